@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "tl_internal.cuh"
+#include "tl_persist.cuh"
 #include "tl_solvers.h"
 
 using namespace tl;
@@ -110,7 +111,9 @@ extern "C" int tl_create(tl_ctx **out, const tl_config *cfg) {
   for (int k = 0; k < TL_NFIELDS; ++k) ctx->field_ptr[k] = f[k];
 
   const size_t tab = (size_t)cfg->maxiters + 2;
-  CK(cudaMalloc(&ctx->small, sizeof(double) * (4 * tab + (size_t)MAX_RED * max_blocks) + sizeof(DevScalars) + 256));
+  const size_t small = sizeof(double) * (4 * tab + (size_t)MAX_RED * max_blocks) + sizeof(DevScalars) + 256;
+  ctx->small_bytes = (small + 255) / 256 * 256 + sizeof(GridSums);
+  CK(cudaMalloc(&ctx->small, ctx->small_bytes));
   char *s = reinterpret_cast<char *>(ctx->small);
   F.cgalpha = reinterpret_cast<double *>(s);
   F.cgbeta = F.cgalpha + tab;
@@ -119,7 +122,7 @@ extern "C" int tl_create(tl_ctx **out, const tl_config *cfg) {
   F.partials = F.chebybeta + tab;
   F.sc = reinterpret_cast<DevScalars *>(F.partials + (size_t)MAX_RED * max_blocks);
   F.counter = reinterpret_cast<unsigned *>(reinterpret_cast<char *>(F.sc) + sizeof(DevScalars));
-  ctx->small_bytes = sizeof(double) * (4 * tab + (size_t)MAX_RED * max_blocks) + sizeof(DevScalars) + 256;
+  ctx->grid_sums = s + (small + 255) / 256 * 256;
   CK(cudaMemsetAsync(ctx->small, 0, ctx->small_bytes, ctx->stream));
   CK(cudaMallocHost(&ctx->host_sc, sizeof(DevScalars)));
 

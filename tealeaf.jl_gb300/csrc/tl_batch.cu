@@ -633,7 +633,7 @@ int batch_solve_ir(tl_batch *b, const double *rx, const double *ry, const tl_par
       snprintf(b->msg, sizeof b->msg, "deck %d: not initialised, or maxiters beyond its tables", k);
       return TL_ERR_STATE;
     }
-    const int rc = tl_ensure_ir(ctx, 0);  // the batch walks its own tiles: no single-deck tuning
+    const int rc = tl_ensure_ir(ctx);
     if (rc) {
       snprintf(b->msg, sizeof b->msg, "deck %d: %s", k, ctx->msg);
       return rc;

@@ -41,6 +41,13 @@ struct Walk {
   int warps, rows, blocks, ntx, tiles;
 };
 
+// The barrier of a persistent (cooperative) kernel, zeroed on the stream
+// before each launch.
+struct GridBar {
+  unsigned count;
+  unsigned fail;  // a wait gave up: the launch's results are void
+};
+
 // Scalars of a solve, resident in device memory so that the iteration loop
 // runs inside a CUDA graph with no host round trip.
 struct DevScalars {
@@ -65,6 +72,7 @@ struct DevScalars {
   int refinements;      // FP64 refinement steps taken
   int prestep_switch;   // FP32 CG presteps of Chebyshev: the switch test held (Cheby.jl:25-29)
   double rxh, ryh;      // FP32 stencil from inverse weights: Kx = rxh (iw_l + iw_c), Ky = ryh (iw_d + iw_c)
+  GridBar bar;          // persistent kernels (tl_persist.cuh); read back with the scalars
 };
 
 // Device pointers of one context, passed to kernels by value.

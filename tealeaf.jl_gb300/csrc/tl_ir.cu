@@ -135,10 +135,8 @@ void tune_kind(tl_ctx *ctx, bool tuning) {
 
 constexpr int NBUF = 7;  // FP32 arrays: p, pb, r, x, sd, sdb, iw
 
-// The FP32 buffers of a context, allocated on first use; `tune` autotunes
-// the single-deck kernels' layouts (the batched solve has its own walk and
-// skips it).
-int ensure_ir(tl_ctx *ctx, bool tune = true) {
+// The FP32 buffers of a context, allocated on first use.
+int ensure_ir(tl_ctx *ctx) {
   if (ctx->ir) return TL_OK;
   tl_ir_state *ir = new (std::nothrow) tl_ir_state();
   if (!ir) return TL_ERR_NOMEM;
@@ -152,13 +150,24 @@ int ensure_ir(tl_ctx *ctx, bool tune = true) {
   float *f[NBUF];
   for (int k = 0; k < NBUF; ++k) f[k] = ir->buf + ir->stride * k + ir->lead;
   ir->p = f[0]; ir->pb = f[1]; ir->r = f[2]; ir->x = f[3]; ir->sd = f[4]; ir->sdb = f[5]; ir->iw = f[6];
-  // tune on the zeroed buffers, then zero them again: the trial launches
-  // leave NaN behind (alpha = 0/0)
-  // OpIrDir and each sweep kind: both forms tuned, the faster kept (without
-  // tuning, TEALEAF_GB300_TUNE=0: the fixed layout, the direction step with
-  // rows two ahead and the sweeps with rows as reached)
+  return TL_OK;
+}
+
+// The layouts of OpIrDir and each sweep kind, on first use (Chebyshev, PPCG and
+// the kernel benchmarks; CG runs in its own kernel): both forms tuned on
+// zeroed buffers, the faster kept, and the buffers zeroed again, because the
+// trial launches leave NaN behind (alpha = 0/0).  Without tuning
+// (TEALEAF_GB300_TUNE=0): the fixed layout, the direction step with rows two
+// ahead and the sweeps with rows as reached.  Call it before a solve's state
+// is in the FP32 buffers.
+int ensure_tuned(tl_ctx *ctx) {
+  int rc = ensure_ir(ctx);
+  if (rc) return rc;
+  tl_ir_state *ir = ctx->ir;
+  if (ir->tuned) return TL_OK;
   const char *env = getenv("TEALEAF_GB300_TUNE");
-  const bool tuning = tune && !(env && !strcmp(env, "0"));
+  const bool tuning = !(env && !strcmp(env, "0"));
+  CK(cudaMemsetAsync(ir->buf, 0, sizeof(float) * ir->stride * NBUF, ctx->stream));
   const Walk d2 = tl_autotune(ctx, 128, occupancy_of<OpIrDir<2>>(128), occupancy_of<OpIrDir<2>>(256),
                               tuning ? tune_dir2 : nullptr);
   const Walk d1 = tl_autotune(ctx, 128, occupancy_of<OpIrDir<1>>(128), occupancy_of<OpIrDir<1>>(256),
@@ -173,72 +182,16 @@ int ensure_ir(tl_ctx *ctx, bool tune = true) {
   tune_kind<SWEEP_PPCG_INNER>(ctx, tuning);
   cudaGetLastError();
   CK(cudaMemsetAsync(ir->buf, 0, sizeof(float) * ir->stride * NBUF, ctx->stream));
-  return TL_OK;
-}
-
-int ir_graph(tl_ctx *ctx, int which, cudaGraphExec_t *out) {
-  tl_ir_state *ir = ctx->ir;
-  if (ir->graph[which]) {
-    *out = ir->graph[which];
-    return TL_OK;
-  }
-  cudaGraph_t graph = nullptr;
-  CK(cudaGraphCreate(&graph, 0));
-  cudaGraphConditionalHandle h;
-  cudaError_t e = cudaGraphConditionalHandleCreate(&h, graph, 1, cudaGraphCondAssignDefault);
-  if (e != cudaSuccess) {
-    cudaGraphDestroy(graph);
-    return tl_cuda_fail(ctx, e, "cudaGraphConditionalHandleCreate", __LINE__);
-  }
-  cudaGraphNodeParams np = {};
-  np.type = cudaGraphNodeTypeConditional;
-  np.conditional.handle = h;
-  np.conditional.type = cudaGraphCondTypeWhile;
-  np.conditional.size = 1;
-  cudaGraphNode_t node;
-  e = cudaGraphAddNode(&node, graph, nullptr, nullptr, 0, &np);
-  if (e != cudaSuccess) {
-    cudaGraphDestroy(graph);
-    return tl_cuda_fail(ctx, e, "cudaGraphAddNode(while)", __LINE__);
-  }
-  cudaGraph_t body = np.conditional.phGraph_out[0];
-  e = cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-  if (e != cudaSuccess) {
-    cudaGraphDestroy(graph);
-    return tl_cuda_fail(ctx, e, "cudaStreamBeginCaptureToGraph", __LINE__);
-  }
-  float *a = which ? ir->pb : ir->p, *b = which ? ir->p : ir->pb;
-  launch_ir_dir(ctx, a, b, 0);
-  launch_ir_update(ctx, b, 0, h, 0);
-  launch_ir_dir(ctx, b, a, 1);
-  launch_ir_update(ctx, a, 1, h, 1);
-  cudaError_t le = cudaGetLastError();
-  cudaGraph_t captured = nullptr;
-  e = cudaStreamEndCapture(ctx->stream, &captured);
-  if (e != cudaSuccess || le != cudaSuccess) {
-    cudaGraphDestroy(graph);
-    return tl_cuda_fail(ctx, e != cudaSuccess ? e : le, "capture of the FP32 loop", __LINE__);
-  }
-  cudaGraphExec_t exec = nullptr;
-  e = cudaGraphInstantiate(&exec, graph, 0);
-  cudaGraphDestroy(graph);
-  if (e != cudaSuccess) return tl_cuda_fail(ctx, e, "cudaGraphInstantiate", __LINE__);
-  ir->graph[which] = exec;
-  *out = exec;
+  ir->tuned = true;
   return TL_OK;
 }
 
 }  // namespace
 
-int tl_ensure_ir(tl_ctx *ctx, int tune) { return ensure_ir(ctx, tune != 0); }
+int tl_ensure_ir(tl_ctx *ctx) { return ensure_ir(ctx); }
 
 void tl_release_ir_graphs(tl_ctx *ctx) {
   if (!ctx->ir) return;
-  for (auto &gx : ctx->ir->graph)
-    if (gx) {
-      cudaGraphExecDestroy(gx);
-      gx = nullptr;
-    }
   for (auto &gx : ctx->ir->ppcg_graph)
     if (gx) {
       cudaGraphExecDestroy(gx);
@@ -286,70 +239,21 @@ static int refine(tl_ctx *ctx, double *rr, float *e = nullptr) {
 // is exported into p.  Returns the last true r.r and its relative value.
 static int ir_loop(tl_ctx *ctx, const tl_params &p, double rx, double ry, double *rr_out, double *rel_out,
                    int *refinements) {
-  const G32 g32 = g32_of(ctx);
   tl_ir_state *ir = ctx->ir;
-  k_ir_convert<<<grid_for((long long)ctx->g.X * ctx->g.Y), 256, 0, ctx->stream>>>(ctx->F, ctx->g, g32, ir->r, ir->p,
-                                                                                  ir->x);
-  k_ir_convert_iw<<<grid_for((long long)ctx->g.X * ctx->g.Y), 256, 0, ctx->stream>>>(ctx->F, ctx->g, g32, ir->iw,
-                                                                                     p.coefficient, rx, ry);
+  k_ir_fields<<<grid_for((long long)ctx->g.X * ctx->g.Y), 256, 0, ctx->stream>>>(ctx->F, ctx->g, g32_of(ctx), ir->r,
+                                                                                 ir->iw, p.coefficient, rx, ry);
   CKL();
-  ctx->launches += 9;
-  int rc = tl_read_scalars(ctx);
-  if (rc) return rc;
-  const double bb = ctx->host_sc->bb;
-  double rr = ctx->host_sc->rro;
-  double rel = bb > 0 ? sqrt(rr / bb) : sqrt(rr);
-  int which = 0, nref = 0, switched = 0;
+  ctx->launches += 8;
   ctx->last_solve_ms = 0.0;
-  while (rel >= p.eps && ctx->host_sc->iter < p.maxiters && !switched) {
-    k_ir_start<<<1, 1, 0, ctx->stream>>>(ctx->F.sc, rr, IR_DELTA * IR_DELTA);
-    CKL();
-    cudaGraphExec_t exec = nullptr;
-    if (!ctx->host_loop && (rc = ir_graph(ctx, which, &exec))) return rc;
-    const int before = ctx->host_sc->iter;
-    CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    if (ctx->host_loop) {
-      // the same kernels launched from the host (see run_host_loop_cg)
-      float *a = which ? ir->pb : ir->p, *b = which ? ir->p : ir->pb;
-      for (;;) {
-        for (int k = 0; k < 8; ++k) {
-          launch_ir_dir(ctx, a, b, 1);
-          launch_ir_update(ctx, b, 1, 0, 0);
-          launch_ir_dir(ctx, b, a, 1);
-          launch_ir_update(ctx, a, 1, 0, 0);
-        }
-        CKL();
-        if ((rc = tl_read_scalars(ctx))) return rc;
-        if (ctx->host_sc->done) break;
-      }
-    } else {
-      CK(cudaGraphLaunch(exec, ctx->stream));
-    }
-    CK(cudaEventRecord(ctx->ev1, ctx->stream));
-    CK(cudaEventSynchronize(ctx->ev1));
-    float t = 0.f;
-    CK(cudaEventElapsedTime(&t, ctx->ev0, ctx->ev1));
-    ctx->last_solve_ms += t;
-    if ((rc = tl_read_scalars(ctx))) return rc;
-    const int trips = ctx->host_sc->iter - before;
-    switched = ctx->host_sc->prestep_switch;
-    ctx->launches += 1 + 4LL * ((trips + 1) / 2);
-    if (trips & 1) which ^= 1;  // the last step wrote p into the other buffer
-    if ((rc = refine(ctx, &rr))) return rc;
-    ++nref;
-    rel = bb > 0 ? sqrt(rr / bb) : sqrt(rr);
-  }
-  float *pcur = which ? ir->pb : ir->p;
-  ir->pwhich = which;
-  k_ir_export_p<<<grid_for((long long)ctx->g.nx * ctx->g.ny), 256, 0, ctx->stream>>>(ctx->F, ctx->g, g32, pcur);
-  CKL();
+  int rc = tl_ir_cg_run(ctx);
+  if (rc) return rc;
+  ir->pwhich = 0;
   const int up[2] = {TL_EX_U, TL_EX_P};
   if ((rc = tl_halo_update(ctx, 1, up, 2, 1))) return rc;
-  ctx->launches += 2;
-  if ((rc = tl_read_scalars(ctx))) return rc;
-  *rr_out = rr;
-  *rel_out = rel;
-  *refinements = nref;
+  ctx->launches += 1;
+  *rr_out = ctx->host_sc->red[0];
+  *rel_out = ctx->host_sc->red[1];
+  *refinements = ctx->host_sc->refinements;
   return TL_OK;
 }
 
@@ -393,7 +297,7 @@ int tl_ir_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_resu
 // same presteps serve PPCG (PPCG.jl:27-31 is the same test).
 int tl_ir_presteps(tl_ctx *ctx, double rx, double ry, const tl_params *prm, int *refinements, double *rr_out,
                    double *rel_out, int *switched) {
-  int rc = ensure_ir(ctx);
+  int rc = ensure_tuned(ctx);  // before the presteps' state is in the FP32 buffers
   if (rc) return rc;
   tl_params p = *prm;
   p.criterion = TL_CRIT_RELATIVE;
@@ -410,7 +314,7 @@ int tl_ir_presteps(tl_ctx *ctx, double rx, double ry, const tl_params *prm, int 
 }
 
 tl::Walk *tl_ir_walk(tl_ctx *ctx, int kernel) {
-  if (ensure_ir(ctx)) return nullptr;
+  if (ensure_tuned(ctx)) return nullptr;
   switch (kernel) {
     case 8: return &ctx->ir->walk_dir;
     case 9: return &ctx->ir->walk_sweep[SWEEP_CG];
@@ -673,7 +577,7 @@ int tl_ppcg32_run(tl_ctx *ctx, const tl_params *prm, double rr, int *refinements
 // in tl_bench_kernel): 6 the Chebyshev step, 7 a PPCG inner sweep, 8 OpIrDir,
 // 9 the CG update step.
 int tl_ir_bench_kernel(tl_ctx *ctx, int kernel, int reps, double *ms_per_launch) {
-  int rc = ensure_ir(ctx);
+  int rc = ensure_tuned(ctx);
   if (rc) return rc;
   if (kernel < 6 || kernel > 9) return TL_ERR_ARG;
   tl_ir_state *ir = ctx->ir;

@@ -23,10 +23,10 @@ struct tl_ir_state {
   tl::Walk walk_sweep[4]{};         // autotuned layouts of OpIrSweep, by kind (the last inner sweep shares slot 3)
   int dir_ahead = 2;                // the faster OpIrDir form after tuning (its AHEAD)
   int sweep_ahead[4] = {1, 1, 1, 1};
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};  // p in the first / second buffer
+  bool tuned = false;               // the layouts of the Chebyshev and PPCG kernels
   cudaGraphExec_t ppcg_graph[2] = {nullptr, nullptr};
   int ppcg_inner = -1;  // inner sweeps recorded in ppcg_graph
-  int pwhich = 0;       // after a CG loop: 1 when the search direction is in pb
+  int pwhich = 0;       // after a PPCG loop: 1 when the search direction is in pb
 };
 
 namespace tl {
@@ -519,6 +519,24 @@ struct OpIrResid : NoSkip {
   }
   __device__ void fin(const double *tot) const { F.sc->red[0] = tot[0]; }
 };
+
+// The start of a single-deck FP32 CG loop: r32 = (float) r on the interior (0
+// in the halo) and the inverse weights (see k_ir_convert_iw).
+__global__ void k_ir_fields(Fields F, Geom g, G32 g32, float *r, float *iw, int coefficient, double rx, double ry) {
+  const long long n = (long long)g.X * g.Y;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    F.sc->rxh = 0.5 * rx;
+    F.sc->ryh = 0.5 * ry;
+  }
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+    const int I = (int)(k % g.X), J = (int)(k / g.X);
+    const size_t c = (size_t)I + (size_t)J * g.pitch, c32 = (size_t)I + (size_t)J * g32.pitch;
+    const bool interior = I >= g.hd && I < g.X - g.hd && J >= g.hd && J < g.Y - g.hd;
+    const double rho = F.density[c];
+    r[c32] = interior ? (float)F.r[c] : 0.f;
+    iw[c32] = (float)(coefficient == TL_CONDUCTIVITY ? 1.0 / rho : rho);
+  }
+}
 
 // The start of an FP32 CG loop: p32 = r32 = (float) r on the interior (0 in
 // the halo) and x = 0.

@@ -51,6 +51,12 @@ int tl_read_scalars(tl_ctx *ctx) {
   return TL_OK;
 }
 
+int tl_persist_check(tl_ctx *ctx) {
+  if (!ctx->host_sc->bar.fail) return TL_OK;
+  tl_set_error(ctx, "a wait of the persistent iteration kernel gave up: the blocks of its grid did not all arrive");
+  return TL_ERR_CUDA;
+}
+
 const Walk &tl_walk_for(tl_ctx *ctx, int exact) {
   return (ctx->cfg.mode == TL_MODE_REFERENCE || exact) ? ctx->walk_exact : ctx->walk_ur64;
 }

@@ -39,6 +39,7 @@ struct tl_ctx {
   tl::Fields F{};
   double *field_ptr[TL_NFIELDS] = {};
   tl::DevScalars *host_sc = nullptr;
+  void *grid_sums = nullptr;  // GridSums of the persistent kernels (tl_persist.cuh)
   int toexchange[TL_NEX] = {};
   int initialised = 0;
   double last_solve_ms = 0.0;
@@ -83,7 +84,11 @@ int tl_cheby_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_r
 int tl_ppcg_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_result *res);
 int tl_jacobi_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_result *res);
 int tl_ir_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_result *res);
-int tl_ensure_ir(tl_ctx *ctx, int tune = 1);  // allocates and tunes the FP32 refinement buffers
+int tl_ensure_ir(tl_ctx *ctx);  // allocates the FP32 refinement buffers
+// The FP32-refined CG loop as one persistent kernel (tl_ir_cg.cu).
+int tl_ir_cg_run(tl_ctx *ctx);
+// TL_OK, or the error of a persistent kernel whose grid barrier gave up (after tl_read_scalars)
+int tl_persist_check(tl_ctx *ctx);
 // Chebyshev after its first step, in FP32 inside FP64 refinement (tl_ir.cu)
 int tl_cheby32_run(tl_ctx *ctx, const tl_params *prm, int *refinements, double *rel_out);
 int tl_ir_presteps(tl_ctx *ctx, double rx, double ry, const tl_params *prm, int *refinements, double *rr_out,
