@@ -70,7 +70,7 @@ __device__ __forceinline__ void ir_pass(const IrCg &A, const PassArgs &q, unsign
   const unsigned slot0 = ring + 16 * lane;
   sum = 0;
   tile = Pair{0.f, 0.f};
-  const bool fixed_tiles = TileWalk::fixed_tiles(A.t);
+  const bool fixed_tiles = A.t.tiles <= A.t.warps;  // one each
   TileWalk walk(A.t, ny, q.mirrored, &A.sums->next_tile, handed);
   handed += walk.requests();
   while (walk.valid()) {
@@ -217,21 +217,12 @@ struct Shared {
   int done, sw;
 };
 
-// What a step's end decides, on warp 0 from the three sums of the new r.
-struct StepEnd {
-  double bb, eps, above, refine_below, epslim;
-  bool above_ok, prestep_rule, lead;
-  int presteps, errorswitch, maxiters;
-};
-
-// Non-negative doubles in integer order: a compare on the FP64 pipe takes 64 cycles.
-__device__ __forceinline__ bool below(double a, double b) { return __double_as_longlong(a) < __double_as_longlong(b); }
-
 // alpha of the next step and 1/gamma, from delta and rho of the current r: both
 // quotients in one division, on lanes 0 and 1.
 __device__ __forceinline__ void next_scalars(Shared &S, double gamma, double beta, double delta, double rho) {
   const int lane = threadIdx.x & 31;
   const double sigma = fma(beta, fma(beta, S.sigma, rho + rho), delta);
+  __syncwarp();  // every lane has read the last step's scalars
   const double quot = (lane == 0 ? gamma : 1.0) / (lane == 0 ? sigma : gamma);
   const float f = (float)(lane == 0 ? quot : beta);
   if (lane == 0) {
@@ -275,18 +266,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ir_cg(const IrCg A) {
   const double eps = sc->eps, bb = sc->bb, epslim = sc->epslim;
   const int maxiters = sc->maxiters, presteps = sc->presteps, errorswitch = sc->errorswitch;
   const bool prestep_rule = sc->switch_rule == 1;
-  StepEnd E;
-  E.bb = bb;
-  E.eps = eps;
-  E.epslim = epslim;
-  E.presteps = presteps;
-  E.errorswitch = errorswitch;
-  E.maxiters = maxiters;
-  E.prestep_rule = prestep_rule;
-  // r.r above this is not converged whatever the rounding of the exact test,
-  // sqrt(r.r / bb) < eps; a limit that is not a normal number decides nothing
-  E.above = eps * eps * bb * (1.0 + 1e-9);
-  E.above_ok = E.above > 1e-290 && E.above < 1e290;
+  const RootTest test(eps, bb);
   double rr = sc->rro;
   double rel = bb > 0 ? sqrt(rr / bb) : sqrt(rr);
   int iter = sc->iter, nref = 0, sw = 0;
@@ -294,13 +274,13 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ir_cg(const IrCg A) {
   bool sv = false, pv = false, xv = false, pend = false, mirrored = false;
   float alpha0 = 0.f, beta0 = 0.f;
   unsigned target = 0, set = 0, handed = 0;
-  const bool fixed_tiles = TileWalk::fixed_tiles(A.t);
+  const bool fixed_tiles = A.t.tiles <= A.t.warps;
   double beta = 0.0, err = 0.0;
   if (threadIdx.x == 0) S.sigma = 0.0;
   __syncthreads();
 
   while (rel >= eps && iter < maxiters && !sw) {
-    E.refine_below = A.delta2 * rr;
+    const double refine_below = A.delta2 * rr;
     double ref = rr;  // the sums' scale follows the last r.r
     {  // the sums of the residual that the refinement (or the start) left
       PassArgs q{};
@@ -313,8 +293,8 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ir_cg(const IrCg A) {
       Pair w;
       ir_pass<PASS_START>(A, q, ring, rxh, ryh, scale, handed, v, w);
       auto fin = [&](double, double f, double r) { next_scalars(S, rr, beta, rr + f, r); };
-      if (!(fixed_tiles ? grid_sums<false>(S.sum, bar, A.sums, v, scale, w, target, set, fin)
-                        : grid_sums<true>(S.sum, bar, A.sums, v, scale, w, target, set, fin)))
+      if (!(fixed_tiles ? grid_sum3<false>(S.sum, bar, A.sums, v, scale, w, target, set, fin)
+                        : grid_sum3<true>(S.sum, bar, A.sums, v, scale, w, target, set, fin)))
         return;
       mirrored = !mirrored;
     }
@@ -340,14 +320,14 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ir_cg(const IrCg A) {
       else ir_pass<PASS_STEP>(A, q, ring, rxh, ryh, scale, handed, v, w);
       auto fin = [&](double g, double f, double r) {
         const double b = g * S.inv_gamma;
-        const bool claim = !(E.above_ok && below(E.above, g)) && sqrt(g / E.bb) < E.eps;
+        const bool claim = test.met(g);
         bool switched = false;
-        if (E.prestep_rule) {
+        if (prestep_rule) {
           const int tt = iter + 2;  // the solver loop's next trip (Cheby.jl:25-29, PPCG.jl:27-31)
-          switched = E.errorswitch ? (g < E.epslim && tt > CGEIGENITERS) : (tt > E.presteps && g < ERROR_SWITCH_MAX);
-          if (lead && iter < E.maxiters) A.F.cgbeta[iter + 1] = b;
+          switched = errorswitch ? (g < epslim && tt > CGEIGENITERS) : (tt > presteps && g < ERROR_SWITCH_MAX);
+          if (lead && iter < maxiters) A.F.cgbeta[iter + 1] = b;
         }
-        const bool done = claim || below(g, E.refine_below) || switched || iter + 1 >= E.maxiters;
+        const bool done = claim || below(g, refine_below) || switched || iter + 1 >= maxiters;
         if (!done) {
           next_scalars(S, g, b, g + f, r);
         } else if (lane == 0) {
@@ -357,8 +337,8 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ir_cg(const IrCg A) {
         }
         if (lane == 0) S.done = done;
       };
-      if (!(fixed_tiles ? grid_sums<false>(S.sum, bar, A.sums, v, scale, w, target, set, fin)
-                        : grid_sums<true>(S.sum, bar, A.sums, v, scale, w, target, set, fin)))
+      if (!(fixed_tiles ? grid_sum3<false>(S.sum, bar, A.sums, v, scale, w, target, set, fin)
+                        : grid_sum3<true>(S.sum, bar, A.sums, v, scale, w, target, set, fin)))
         return;
       mirrored = !mirrored;
       float *t = rc;
@@ -453,10 +433,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ir_cg(const IrCg A) {
       share += to_fixed(acc, scale);
       walk.take(asked);
     }
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1) share += shfl_xor(share, off);
-    if (lane) share = 0;
-    if (!grid_sums<true>(S.sum, bar, A.sums, share, scale, Pair{}, target, set, [&](double a, double, double) {
+    if (!grid_sum1(S.sum, bar, A.sums, warp_fixed(share), scale, target, set, [&](double a) {
           if (lane == 0) S.tot = a;
         }))
       return;
@@ -522,9 +499,9 @@ int tl_ir_cg_run(tl_ctx *ctx) {
   A.iw = ir->iw;
   A.delta2 = IR_DELTA * IR_DELTA;
   // cycles and issue slots of a row and a tile, from the kernel's own counters
-  const TileCost pass{2.0, 300.0, 1500.0, 200.0, 400.0, 32}, resid{1.0, 1200.0, 1500.0, 1100.0, 200.0, 0};
-  A.t = make_tiling(ctx->g.nx, ctx->g.ny, STRIP, pass, persist_blocks(ctx->sm_count));
-  A.t64 = make_tiling(ctx->g.nx, ctx->g.ny, 64, resid, A.t.blocks);
+  const TileCost pass{2.0, 300.0, 1500.0, 200.0, 400.0, 32, 24, 8}, resid{1.0, 1200.0, 1500.0, 1100.0, 200.0, 0, 48, 4};
+  A.t = make_tiling(ctx->g.nx, ctx->g.ny, STRIP, pass, persist_blocks(ctx->sm_count), PERSIST_WARPS);
+  A.t64 = make_tiling_on(A.t, ctx->g.nx, ctx->g.ny, 64, resid, PERSIST_WARPS);
   A.sums = static_cast<GridSums *>(ctx->grid_sums);
   CK(cudaFuncSetAttribute(k_ir_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES * PERSIST_WARPS));
   CK(cudaMemsetAsync(&ctx->F.sc->bar, 0, sizeof(GridBar), ctx->stream));

@@ -13,7 +13,7 @@
 
 namespace tl {
 
-constexpr int PERSIST_WARPS = 16;                 // warps of a persistent block
+constexpr int PERSIST_WARPS = 16;                 // warps of a persistent block at most
 constexpr int PERSIST_THREADS = 32 * PERSIST_WARPS;
 constexpr unsigned BAR_POLLS = 1u << 23;          // a wait gives up after some seconds
 
@@ -68,29 +68,37 @@ __device__ __forceinline__ Pair warp_pairs(const Pair (&v)[3]) {
 // instructions, where one FP64 addition takes 66.
 typedef __int128 Fixed;
 
-// The scale at which a number of the size of `ref` becomes about 2^60: 66 bits
-// above it for sums that grow, 60 bits below it before anything is cut off.
+// The scale at which a number of the size of `ref` becomes about 2^62: 44 bits
+// above it for sums that grow (p.A p against r.r: the operator's eigenvalues),
+// 62 below it before anything is rounded off (a million addends, each rounded
+// to nearest, are off by some 2^-52 of the sum).
 __device__ __forceinline__ int fixed_scale(double ref) {
-  return 60 + 1023 - (int)((__double_as_longlong(ref) >> 52) & 0x7ff);
+  return 62 + 1023 - (int)((__double_as_longlong(ref) >> 52) & 0x7ff);
 }
-// v 2^scale, cut off below 1.  What would reach 2^100 (infinities and NaN among
-// it) becomes 2^100: far beyond anything plausible beside 2^60, and 2^26 of them
-// still add up.  `m` has `bits` bits at most.
+// v 2^scale, rounded.  What would reach FIXED_MOST (infinities and NaN
+// among it) becomes FIXED_MOST: far beyond anything plausible beside 2^62.  A
+// warp's sum is cut to it once more (fixed_cut), so that no number of such
+// addends wraps round to a plausible sum.  `m` has `bits` bits at most.
+constexpr int FIXED_BITS = 106;
 __device__ __forceinline__ Fixed fixed_shift(unsigned long long m, int bits, int shift, bool neg) {
   Fixed q;
-  if (shift >= 0) q = shift <= 100 - bits ? (Fixed)m << shift : (Fixed)(m != 0) << 100;
-  else q = shift > -64 ? (Fixed)(m >> -shift) : (Fixed)0;
+  if (shift >= 0) q = shift <= FIXED_BITS - bits ? (Fixed)m << shift : (Fixed)(m != 0) << FIXED_BITS;
+  else q = shift > -64 ? (Fixed)((m >> -shift) + ((m >> (-shift - 1)) & 1)) : (Fixed)0;
   return neg ? -q : q;
+}
+__device__ __forceinline__ Fixed fixed_cut(Fixed q) {
+  const Fixed most = (Fixed)1 << FIXED_BITS;
+  return q > most ? most : q < -most ? -most : q;
 }
 __device__ __forceinline__ Fixed to_fixed(float v, int scale) {
   const unsigned u = __float_as_uint(v), e = (u >> 23) & 255u;
   const unsigned m = (u & 0x7fffffu) | (e ? 0x800000u : 0u);
-  return fixed_shift(e == 255u ? 1u : m, 24, e == 255u ? 100 : (int)(e ? e : 1u) - 150 + scale, u >> 31);
+  return fixed_shift(e == 255u ? 1u : m, 24, e == 255u ? FIXED_BITS : (int)(e ? e : 1u) - 150 + scale, u >> 31);
 }
 __device__ __forceinline__ Fixed to_fixed(double v, int scale) {
   const unsigned long long u = (unsigned long long)__double_as_longlong(v), e = (u >> 52) & 2047u;
   const unsigned long long m = (u & 0xfffffffffffffull) | (e ? 0x10000000000000ull : 0ull);
-  return fixed_shift(e == 2047u ? 1ull : m, 53, e == 2047u ? 100 : (int)(e ? e : 1u) - 1075 + scale, u >> 63);
+  return fixed_shift(e == 2047u ? 1ull : m, 53, e == 2047u ? FIXED_BITS : (int)(e ? e : 1u) - 1075 + scale, u >> 63);
 }
 // The number a whole number of 2^-scale stands for, cut to 53 bits.
 __device__ __forceinline__ double from_fixed(Fixed q, int scale) {
@@ -141,37 +149,58 @@ __device__ __forceinline__ void stcg_fixed(Fixed *p, Fixed v) {
   __stcg(reinterpret_cast<ulonglong2 *>(p), make_ulonglong2((unsigned long long)u, (unsigned long long)(u >> 64)));
 }
 
-// One thread's arrival at a barrier over the blocks of a cooperative launch and
-// its wait; `target` is the arrivals expected so far (start at 0).  False when
-// the wait gave up: the kernel returns at once, every block by its own limit.
-// What the block wrote before its last block barrier is visible to every block
-// after its wait (release, then acquire, both by this thread).
-__device__ __forceinline__ bool grid_arrive_wait(GridBar *g, unsigned &target) {
-  target += gridDim.x;
-  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&g->count) : "memory");
-  unsigned v, n = 0;
-  for (;;) {
+// A block's arrival at a barrier over the blocks of a cooperative launch and its
+// wait for `target` arrivals in all, by one whole warp.  False when the wait
+// gave up: the kernel returns at once, every block by its own limit.  What the
+// block wrote before its last block barrier, and this warp before the call, is
+// visible to every block after its wait.  All lanes wait, on one load: where
+// lane 0 alone waited, the compiler ran all that follows once for it and once
+// for the others (3 us a sum) and moved the others' loads ahead of the wait.
+__device__ __forceinline__ bool grid_arrive_wait(GridBar *g, unsigned target) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&g->count) : "memory");
+  unsigned n = 0;
+  bool there;
+  do {
+    unsigned v;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&g->count) : "memory");
-    if ((int)(v - target) >= 0 || ++n >= BAR_POLLS) break;
-  }
+    there = __all_sync(FULL, (int)(v - target) >= 0);
+  } while (!there && ++n < BAR_POLLS);
   asm volatile("fence.acq_rel.gpu;" ::: "memory");
-  const bool ok = (int)(v - target) >= 0;
-  if (!ok) atomicExch(&g->fail, 1u);
-  return ok;
+  if (!there && (threadIdx.x & 31) == 0) atomicExch(&g->fail, 1u);
+  return there;
 }
 
-// The barrier for whole blocks.
+// The barrier for whole blocks; `target` counts the arrivals expected so far on
+// every thread (start at 0).
 __device__ __forceinline__ bool grid_barrier(GridBar *g, unsigned &target) {
   __shared__ int ok;
   __syncthreads();
   if (gridDim.x == 1) return true;
-  if (threadIdx.x == 0) ok = grid_arrive_wait(g, target);
-  else target += gridDim.x;
+  target += gridDim.x;
+  if (threadIdx.x < 32) ok = grid_arrive_wait(g, target);
   __syncthreads();
   return ok != 0;
 }
 
-inline int persist_blocks(int sm_count) { return sm_count < PERSIST_MAX_BLOCKS ? sm_count : PERSIST_MAX_BLOCKS; }
+// Non-negative doubles in integer order: a compare on the FP64 pipe takes 64 cycles.
+__device__ __forceinline__ bool below(double a, double b) { return __double_as_longlong(a) < __double_as_longlong(b); }
+
+// A convergence test sqrt(e) < eps with e = error / bb (bb 1 for the absolute
+// test): what lies above `limit` fails it whatever its rounding, so that most
+// trips need no root and no division.  A limit that is not a normal number
+// decides nothing.
+struct RootTest {
+  double eps, bb, limit;
+  bool usable;
+  __device__ __forceinline__ RootTest(double eps, double bb) : eps(eps), bb(bb), limit(eps * eps * bb * (1.0 + 1e-9)) {
+    usable = limit > 1e-290 && limit < 1e290;
+  }
+  __device__ __forceinline__ bool met(double error) const {
+    if (usable && below(limit, error)) return false;
+    return sqrt(bb == 1.0 ? error : error / bb) < eps;
+  }
+};
 
 struct SumShared {
   Fixed warp[PERSIST_WARPS][3];
@@ -179,41 +208,67 @@ struct SumShared {
   int ok;
 };
 
-// Up to three sums over the grid and what follows from them: each warp's share
-// in lanes 0, 8 and 16, `fin(a, b, c)` on warp 0 with the totals, and the block
-// meets.  One block barrier before the grid's, one after `fin`.  `set` counts
-// the calls of a launch; target as in grid_arrive_wait.  Two forms: `v`, whole
-// numbers of 2^-scale, for tiles taken in any order; `w`, pairs, which are
-// cheaper to form and to add (1.3 us of an iteration of 7.9 at 256^2), where
-// every warp has its one fixed tile.
+// Sums over the grid and what follows from them: `fin(totals...)` on warp 0, and
+// the block meets.  One block barrier before the grid's, one after `fin`.
+// `set` counts the calls of a launch; target as in grid_barrier.
+// Between reading and writing shared scalars `fin` needs a warp barrier.
+//
+// One sum: each warp's share in lane 0, in whole numbers of 2^-scale.
+template <class Fin>
+__device__ __forceinline__ bool grid_sum1(SumShared &S, GridBar *bar, GridSums *G, Fixed v, int scale, unsigned &target,
+                                          unsigned &set, Fin &&fin) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = gridDim.x, nw = blockDim.x >> 5;
+  target += nb;
+  if (lane == 0) S.warp[warp][0] = fixed_cut(v);
+  __syncthreads();
+  if (warp == 0) {
+    Fixed t = lane < nw ? S.warp[lane][0] : (Fixed)0;
+    for (int off = nw >> 1; off >= 1; off >>= 1) t += shfl_xor(t, off);
+    if (nb > 1) {
+      Fixed *part = &G->part[set & 1][0][0];
+      if (lane == 0) stcg_fixed(part + blockIdx.x, t);
+      S.ok = grid_arrive_wait(bar, target);
+      Fixed q[5];
+#pragma unroll
+      for (int m = 0; m < 5; ++m) q[m] = lane + 32 * m < nb ? ldcg_fixed(part + lane + 32 * m) : (Fixed)0;
+      t = q[0] + q[1] + q[2] + q[3] + q[4];
+#pragma unroll
+      for (int off = 16; off >= 1; off >>= 1) t += shfl_xor(t, off);
+    }
+    fin(from_fixed(shfl(t, 0), scale));
+  }
+  ++set;
+  __syncthreads();
+  return nb == 1 || S.ok != 0;
+}
+
+// Three sums, each warp's share in lanes 0, 8 and 16.  Two forms: `v`, whole
+// numbers, for tiles taken in any order; `w`, pairs, which are cheaper to form
+// and to add (1.3 us of an iteration of 7.9 at 256^2), where every warp has its
+// one fixed tile.
 template <bool FIXED, class Fin>
-__device__ __forceinline__ bool grid_sums(SumShared &S, GridBar *bar, GridSums *G, Fixed v, int scale, Pair w,
+__device__ __forceinline__ bool grid_sum3(SumShared &S, GridBar *bar, GridSums *G, Fixed v, int scale, Pair w,
                                           unsigned &target, unsigned &set, Fin &&fin) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = gridDim.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = gridDim.x, nw = blockDim.x >> 5;
+  target += nb;
   if ((lane & 7) == 0 && lane < 24) {
-    if (FIXED) S.warp[warp][lane >> 3] = v;
+    if (FIXED) S.warp[warp][lane >> 3] = fixed_cut(v);
     else S.pair[warp][lane >> 3] = w;
   }
   __syncthreads();
   if (warp == 0) {
     const int d = lane < 24 ? lane >> 3 : 2, c = lane & 7;
-    bool ok = true;
-    auto meet = [&]() {
-      __syncwarp();
-      if (lane == 0) ok = grid_arrive_wait(bar, target);
-      else target += nb;
-      ok = __shfl_sync(FULL, (int)ok, 0) != 0;
-    };
     double tot;
     if (FIXED) {
-      Fixed t = S.warp[c][d] + S.warp[c + 8][d];
+      Fixed t = c < nw ? S.warp[c][d] : (Fixed)0;
+      if (nw > 8) t += S.warp[c + 8][d];
       t += shfl_xor(t, 4);
       t += shfl_xor(t, 2);
       t += shfl_xor(t, 1);
       if (nb > 1) {
         Fixed(*part)[4] = G->part[set & 1];
         if (lane < 24 && c == 0) stcg_fixed(&part[blockIdx.x][d], t);
-        meet();
+        S.ok = grid_arrive_wait(bar, target);
         t = 0;
         for (int k0 = c; k0 < nb; k0 += 80) {  // ten loads in flight
           Fixed q[10];
@@ -229,7 +284,7 @@ __device__ __forceinline__ bool grid_sums(SumShared &S, GridBar *bar, GridSums *
       tot = from_fixed(t, scale);
     } else {
       Pair q[3] = {};
-      if (lane < PERSIST_WARPS) {
+      if (lane < nw) {
 #pragma unroll
         for (int m = 0; m < 3; ++m) q[m] = S.pair[lane][m];
       }
@@ -237,37 +292,39 @@ __device__ __forceinline__ bool grid_sums(SumShared &S, GridBar *bar, GridSums *
       if (nb > 1) {
         Pair(*part)[8] = reinterpret_cast<Pair(*)[8]>(G->part[set & 1]);
         if (lane < 24 && c == 0) __stcg(reinterpret_cast<float2 *>(&part[blockIdx.x][d]), make_float2(t.hi, t.lo));
-        meet();
+        S.ok = grid_arrive_wait(bar, target);
+        float4 ab[5];
+        float2 e[5];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) {
+          const int k = lane + 32 * m;
+          ab[m] = k < nb ? __ldcg(reinterpret_cast<const float4 *>(&part[k][0])) : make_float4(0.f, 0.f, 0.f, 0.f);
+          e[m] = k < nb ? __ldcg(reinterpret_cast<const float2 *>(&part[k][2])) : make_float2(0.f, 0.f);
+        }
 #pragma unroll
         for (int m = 0; m < 3; ++m) q[m] = Pair{0.f, 0.f};
-        for (int k0 = lane; k0 < nb; k0 += 160) {  // five loads in flight: 152 blocks in one trip
-          float4 ab[5];
-          float2 e[5];
 #pragma unroll
-          for (int m = 0; m < 5; ++m) {
-            const int k = k0 + 32 * m;
-            ab[m] = k < nb ? __ldcg(reinterpret_cast<const float4 *>(&part[k][0])) : make_float4(0.f, 0.f, 0.f, 0.f);
-            e[m] = k < nb ? __ldcg(reinterpret_cast<const float2 *>(&part[k][2])) : make_float2(0.f, 0.f);
-          }
-#pragma unroll
-          for (int m = 0; m < 5; ++m) {
-            q[0].add(Pair{ab[m].x, ab[m].y});
-            q[1].add(Pair{ab[m].z, ab[m].w});
-            q[2].add(Pair{e[m].x, e[m].y});
-          }
+        for (int m = 0; m < 5; ++m) {
+          q[0].add(Pair{ab[m].x, ab[m].y});
+          q[1].add(Pair{ab[m].z, ab[m].w});
+          q[2].add(Pair{e[m].x, e[m].y});
         }
         t = warp_pairs(q);
       }
       tot = (double)t.hi + (double)t.lo;
     }
     fin(__shfl_sync(FULL, tot, 0), __shfl_sync(FULL, tot, 8), __shfl_sync(FULL, tot, 16));
-    if (lane == 0) S.ok = ok;
-  } else if (nb > 1) {
-    target += nb;
   }
   ++set;
   __syncthreads();
-  return S.ok != 0;
+  return nb == 1 || S.ok != 0;
+}
+
+// Adds a warp's lanes, in every lane.
+__device__ __forceinline__ Fixed warp_fixed(Fixed v) {
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) v += shfl_xor(v, off);
+  return v;
 }
 
 // Copies into a ring of shared memory where every thread reads back only what
@@ -296,14 +353,17 @@ __device__ __forceinline__ double2 lds2d(unsigned a) {
 
 // How a persistent kernel shares an nx x ny grid: warp tiles of `cols` columns,
 // numbered along a row band first, bands of `rows` rows up to row `split` and of
-// `rows2` from there.  The short bands come last, so that the warps finish
-// together.  A deck with fewer tiles than warps spreads them over the blocks, one
+// `rows2` from there.  Fewer tiles than warps are spread over the blocks, one
 // warp of each after another; otherwise a block's warps start on neighbouring
-// strips of the same rows and every warp takes the next free tile after its own
-// first.
+// strips of the same rows.  After its first tile a warp takes every (number of
+// warps)th one, or, with `handed`, the next that is free: the SMs of one GPU do
+// not get the same memory bandwidth (with equal shares the fast ones waited 110
+// of 400 us for the slow ones at 8192^2, FP32 CG).  The short bands come last, so
+// that the warps finish together.
 struct Tiling {
   int ntx, rows, split, rows2;
-  int tiles1, tiles, blocks;
+  int tiles1, tiles, blocks, warps;
+  bool handed;
 };
 
 struct TileWalk {
@@ -315,8 +375,8 @@ struct TileWalk {
   unsigned base;
   __device__ __forceinline__ TileWalk(const Tiling &T, int ny, bool mirrored, unsigned *next, unsigned base)
       : T(T), ny(ny), mirrored(mirrored), next(next), base(base) {
-    const int warp = threadIdx.x >> 5, warps = gridDim.x * PERSIST_WARPS;
-    t = T.tiles < warps ? warp * gridDim.x + blockIdx.x : blockIdx.x * PERSIST_WARPS + warp;
+    const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    t = T.tiles < T.warps ? warp * gridDim.x + blockIdx.x : blockIdx.x * nw + warp;
   }
   __device__ __forceinline__ bool valid() const { return t < T.tiles; }
   // strip, and rows [j0, j1)
@@ -335,37 +395,38 @@ struct TileWalk {
   // asked for while the current tile is still ahead, so that its latency is hidden
   __device__ __forceinline__ unsigned ask() const {
     unsigned v = 0;
-    if (!fixed_tiles(T) && (threadIdx.x & 31) == 0) v = atomicAdd(next, 1u);
+    if (T.handed && (threadIdx.x & 31) == 0) v = atomicAdd(next, 1u);
     return v;
   }
   __device__ __forceinline__ void take(unsigned asked) {
-    t = fixed_tiles(T) ? T.tiles : (int)(gridDim.x * PERSIST_WARPS + __shfl_sync(FULL, asked, 0) - base);
+    t = T.handed ? T.warps + (int)(__shfl_sync(FULL, asked, 0) - base) : t + T.warps;
   }
-  __device__ __forceinline__ static bool fixed_tiles(const Tiling &T) { return T.tiles <= (int)gridDim.x * PERSIST_WARPS; }
   // requests a whole pass makes: each warp asks once for each of its tiles
-  __device__ __forceinline__ unsigned requests() const {
-    return fixed_tiles(T) ? 0u : (unsigned)T.tiles;
-  }
+  __device__ __forceinline__ unsigned requests() const { return T.handed ? (unsigned)T.tiles : 0u; }
 };
 
-// The shape: on decks of up to one tile a warp the rows that make the slowest
-// SM's pass shortest (a tile takes `lat` cycles a row and `lat0` besides when
-// its warp runs alone, `issue` and `issue0` of a sub-partition's issue slots,
-// and `extra` rows overlap the next tile); on larger ones tall bands, whose overlap is small,
-// for the first three quarters and short ones for the rest.  A deck of at most
-// `solo` strip rows runs on one block, which needs no grid barrier.
+inline int persist_blocks(int sm_count) { return sm_count < PERSIST_MAX_BLOCKS ? sm_count : PERSIST_MAX_BLOCKS; }
+
+// The shape.  Up to `hand_from` strip rows a warp: the rows that make the slowest
+// SM's pass shortest, in equal shares.  Beyond: tall bands, whose overlap is
+// small, for the first three quarters and bands of `rows2` for the rest, handed
+// out.  A tile takes `lat` cycles a row and `lat0` besides when its warp runs
+// alone, `issue` and `issue0` of a sub-partition's issue (or FP64) slots; `extra`
+// rows overlap the next tile.  A deck of at most `solo` strip rows runs on one
+// block, which needs no grid barrier.
 struct TileCost {
   double extra, lat, lat0, issue, issue0;
-  int solo;
+  int solo, hand_from, rows2;
 };
-inline Tiling make_tiling(int nx, int ny, int cols, const TileCost &c, int max_blocks) {
+inline Tiling make_tiling(int nx, int ny, int cols, const TileCost &c, int max_blocks, int block_warps) {
   Tiling t;
   t.ntx = (nx + cols - 1) / cols;
   const long long strip_rows = (long long)t.ntx * ny;
   const int cap = strip_rows <= c.solo ? 1 : max_blocks;
-  const long long warps = (long long)cap * PERSIST_WARPS;
-  t.rows2 = 8;
-  if (strip_rows > 24 * warps) {
+  const long long warps = (long long)cap * block_warps;
+  t.rows2 = c.rows2;
+  t.handed = strip_rows > c.hand_from * warps;
+  if (t.handed) {
     t.rows = strip_rows > 128 * warps ? 32 : 16;
     t.split = (int)(0.75 * ny) / t.rows * t.rows;
   } else {
@@ -374,7 +435,7 @@ inline Tiling make_tiling(int nx, int ny, int cols, const TileCost &c, int max_b
     for (int rows = 1; rows <= (ny < 64 ? ny : 64); ++rows) {
       const long long tiles = (long long)t.ntx * ((ny + rows - 1) / rows);
       const long long per_block = (tiles + cap - 1) / cap;
-      const long long rounds = (per_block + PERSIST_WARPS - 1) / PERSIST_WARPS;
+      const long long rounds = (per_block + block_warps - 1) / block_warps;
       const double lat = rounds * ((rows + c.extra) * c.lat + c.lat0);
       const double issue = (double)((per_block + 3) / 4) * ((rows + c.extra) * c.issue + c.issue0);
       const double cost = lat > issue ? lat : issue;
@@ -388,6 +449,16 @@ inline Tiling make_tiling(int nx, int ny, int cols, const TileCost &c, int max_b
   t.tiles1 = t.ntx * ((t.split + t.rows - 1) / t.rows);
   t.tiles = t.tiles1 + t.ntx * ((ny - t.split + t.rows2 - 1) / t.rows2);
   t.blocks = t.tiles < cap ? t.tiles : cap;
+  t.warps = t.blocks * block_warps;
+  return t;
+}
+
+// The same grid of blocks for another pass.
+inline Tiling make_tiling_on(const Tiling &first, int nx, int ny, int cols, const TileCost &c, int block_warps) {
+  Tiling t = make_tiling(nx, ny, cols, c, first.blocks, block_warps);
+  t.blocks = first.blocks;
+  t.warps = first.warps;
+  if (t.handed && t.tiles <= t.warps) t.handed = false;
   return t;
 }
 

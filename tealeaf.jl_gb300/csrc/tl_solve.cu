@@ -102,15 +102,12 @@ static int record_body(tl_ctx *ctx, int which, cudaGraphConditionalHandle h) {
       }
       break;
     }
-    case TL_GRAPH_CG_EXACT:
-    case TL_GRAPH_CG_FAST: {
-      const int exact = which == TL_GRAPH_CG_EXACT;
-      const Walk &ww = exact ? ctx->walk_exact : ctx->walk_w64;
-      const Walk &wu = exact ? ctx->walk_exact : ctx->walk_ur64;
-      launch_tl_w(st, F, g, ww, F.p, F.pb, exact, 0);
-      launch_tl_ur(st, F, g, wu, F.pb, exact, 0, h, 0);
-      launch_tl_w(st, F, g, ww, F.pb, F.p, exact, 1);
-      launch_tl_ur(st, F, g, wu, F.p, exact, 1, h, 1);
+    case TL_GRAPH_CG_EXACT: {
+      const Walk &wk = ctx->walk_exact;
+      launch_tl_w(st, F, g, wk, F.p, F.pb, 1, 0);
+      launch_tl_ur(st, F, g, wk, F.pb, 1, 0, h, 0);
+      launch_tl_w(st, F, g, wk, F.pb, F.p, 1, 1);
+      launch_tl_ur(st, F, g, wk, F.p, 1, 1, h, 1);
       break;
     }
     default:
@@ -175,22 +172,21 @@ void tl_release_graphs(tl_ctx *ctx) {
     }
 }
 
-// The same loop launched from the host: batches of eight two-iteration
+// The exact CG loop launched from the host: batches of eight two-iteration
 // bodies whose kernels all skip once the device has set `done`, with the flag
 // read back after each batch.  Profilers cannot see kernels inside graphs
 // that hold conditional nodes; this mode (TEALEAF_GB300_LOOP=host) runs the
 // identical kernels where they can.
-static int run_host_loop_cg(tl_ctx *ctx, int exact) {
+static int run_host_loop_cg(tl_ctx *ctx) {
   const Fields &F = ctx->F;
   const Geom &g = ctx->g;
-  const Walk &ww = exact ? ctx->walk_exact : ctx->walk_w64;
-  const Walk &wu = exact ? ctx->walk_exact : ctx->walk_ur64;
+  const Walk &wk = ctx->walk_exact;
   for (;;) {
     for (int b = 0; b < 8; ++b) {
-      launch_tl_w(ctx->stream, F, g, ww, F.p, F.pb, exact, 1);
-      launch_tl_ur(ctx->stream, F, g, wu, F.pb, exact, 1, 0, 0);
-      launch_tl_w(ctx->stream, F, g, ww, F.pb, F.p, exact, 1);
-      launch_tl_ur(ctx->stream, F, g, wu, F.p, exact, 1, 0, 0);
+      launch_tl_w(ctx->stream, F, g, wk, F.p, F.pb, 1, 1);
+      launch_tl_ur(ctx->stream, F, g, wk, F.pb, 1, 1, 0, 0);
+      launch_tl_w(ctx->stream, F, g, wk, F.pb, F.p, 1, 1);
+      launch_tl_ur(ctx->stream, F, g, wk, F.p, 1, 1, 0, 0);
     }
     CKL();
     int rc = tl_read_scalars(ctx);
@@ -201,7 +197,7 @@ static int run_host_loop_cg(tl_ctx *ctx, int exact) {
 
 // Runs one loop graph, timing it with events on the context stream.
 int tl_run_graph(tl_ctx *ctx, int which, double *ms) {
-  const bool host = ctx->host_loop && (which == TL_GRAPH_CG_EXACT || which == TL_GRAPH_CG_FAST);
+  const bool host = ctx->host_loop && which == TL_GRAPH_CG_EXACT;
   cudaGraphExec_t exec = nullptr;
   if (!host) {
     int rc = tl_get_graph(ctx, which, &exec);
@@ -209,7 +205,7 @@ int tl_run_graph(tl_ctx *ctx, int which, double *ms) {
   }
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   if (host) {
-    int rc = run_host_loop_cg(ctx, which == TL_GRAPH_CG_EXACT);
+    int rc = run_host_loop_cg(ctx);
     if (rc) return rc;
   } else {
     CK(cudaGraphLaunch(exec, ctx->stream));
@@ -365,24 +361,30 @@ int tl_cg_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_resu
       return TL_OK;
     }
   }
-  const int which = ref ? TL_GRAPH_CG_REF : (exact ? TL_GRAPH_CG_EXACT : TL_GRAPH_CG_FAST);
+  const int which = ref ? TL_GRAPH_CG_REF : TL_GRAPH_CG_EXACT;  // the fused arithmetic has its own kernel
   double rel = -1.0;
   int ran = 0;
   for (int restart = 0; restart < 8 && prm->maxiters >= 1; ++restart) {
-    const int before = ctx->host_sc->iter;
-    if ((rc = tl_run_graph(ctx, which, &ctx->last_solve_ms))) return rc;
-    if ((rc = tl_read_scalars(ctx))) return rc;
-    const int trips = ctx->host_sc->iter - (restart ? before : 0);
-    ctx->launches += ref ? 4LL * trips : 4LL * ((trips + 1) / 2);
-    ran = 1;
-    if (!ref) {
-      // the last iteration's p! and haloupdate! of u, p
-      const double *pcur = (ctx->host_sc->iter & 1) ? ctx->F.pb : ctx->F.p;
-      launch_tl_p(ctx->stream, ctx->F, ctx->g, tl_walk_for(ctx, exact), pcur, ctx->F.p, exact);
-      CKL();
+    if (!exact) {
+      if ((rc = tl_cg64_run(ctx, &ctx->last_solve_ms))) return rc;
       if ((rc = tl_halo_update(ctx, 1, nullptr, -1, 1))) return rc;
-      ctx->launches += 2;
+      ctx->launches += 1;
+    } else {
+      const int before = ctx->host_sc->iter;
+      if ((rc = tl_run_graph(ctx, which, &ctx->last_solve_ms))) return rc;
+      if ((rc = tl_read_scalars(ctx))) return rc;
+      const int trips = ctx->host_sc->iter - (restart ? before : 0);
+      ctx->launches += ref ? 4LL * trips : 4LL * ((trips + 1) / 2);
+      if (!ref) {
+        // the last iteration's p! and haloupdate! of u, p
+        const double *pcur = (ctx->host_sc->iter & 1) ? ctx->F.pb : ctx->F.p;
+        launch_tl_p(ctx->stream, ctx->F, ctx->g, ctx->walk_exact, pcur, ctx->F.p, 1);
+        CKL();
+        if ((rc = tl_halo_update(ctx, 1, nullptr, -1, 1))) return rc;
+        ctx->launches += 2;
+      }
     }
+    ran = 1;
     if (prm->criterion != TL_CRIT_RELATIVE) break;
     double tr;
     if ((rc = true_residual(ctx, 0, &tr))) return rc;

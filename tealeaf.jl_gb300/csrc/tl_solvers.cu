@@ -188,8 +188,12 @@ int cg_phase(tl_ctx *ctx, double rx, double ry, const tl_params *prm, int exact,
     if ((rc = tl_copy_u(ctx))) return rc;
   }
   ctx->last_solve_ms = 0.0;
+  if (!ref && !exact && prm->maxiters >= 1) {
+    if ((rc = tl_cg64_run(ctx, &ctx->last_solve_ms))) return rc;
+    return tl_halo_update(ctx, 1, nullptr, -1, 1);
+  }
   if (prm->maxiters >= 1) {
-    const int which = ref ? TL_GRAPH_CG_REF_NOHALO : (exact ? TL_GRAPH_CG_EXACT : TL_GRAPH_CG_FAST);
+    const int which = ref ? TL_GRAPH_CG_REF_NOHALO : TL_GRAPH_CG_EXACT;
     if ((rc = tl_run_graph(ctx, which, &ctx->last_solve_ms))) return rc;
   }
   if ((rc = tl_read_scalars(ctx))) return rc;

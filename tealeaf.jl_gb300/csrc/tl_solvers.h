@@ -8,7 +8,6 @@ enum {
   TL_GRAPH_CG_REF = 0,       // reference-mode CG step + halo of u, p
   TL_GRAPH_CG_REF_NOHALO,    // reference-mode CG step without the halo (Cheby/PPCG presteps)
   TL_GRAPH_CG_EXACT,         // tealeaf fused CG, reference operation order
-  TL_GRAPH_CG_FAST,          // tealeaf fused CG, FMA
   TL_GRAPH_CHEBY_EXACT,      // Chebyshev steps, the first of the pair reading ub
   TL_GRAPH_CHEBY_FAST,
   TL_GRAPH_PPCG_EXACT,       // two PPCG outer steps with their inner sweeps
@@ -87,6 +86,8 @@ int tl_ir_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_resu
 int tl_ensure_ir(tl_ctx *ctx);  // allocates the FP32 refinement buffers
 // The FP32-refined CG loop as one persistent kernel (tl_ir_cg.cu).
 int tl_ir_cg_run(tl_ctx *ctx);
+// The fused FP64 CG loop with the last step's p!, as one persistent kernel (tl_cg64.cu).
+int tl_cg64_run(tl_ctx *ctx, double *ms);
 // TL_OK, or the error of a persistent kernel whose grid barrier gave up (after tl_read_scalars)
 int tl_persist_check(tl_ctx *ctx);
 // Chebyshev after its first step, in FP32 inside FP64 refinement (tl_ir.cu)

@@ -43,3 +43,30 @@ def test_fp32_cg_tilings(tl, built_lib, nx, ny):
     # whatever warp took which tile, the sums and the solution are the same bits
     np.testing.assert_array_equal(u, runs["again"][0])
     assert [r.iters for r in res] == [r.iters for r in runs["again"][1]]
+
+
+@pytest.mark.parametrize("nx,ny,hd", [
+    (1, 7, 2), (59, 5, 1), (60, 4, 3), (61, 9, 2), (62, 3, 1), (119, 40, 2), (121, 33, 2), (3, 400, 2),  # strip edges, one block
+    (513, 511, 2), (1023, 401, 1),      # one tile a warp
+    (1801, 1403, 2),                    # tiles handed out
+])
+def test_fp64_cg_tilings(tl, built_lib, nx, ny, hd):
+    """Fused FP64 CG against exact FP64 CG: the same bound on u, iteration
+    counts within one (the arithmetic differs in rounding alone), and p, w of
+    the last step where both took the same steps: p within 1e-6 of its norm
+    (CG's vectors drift apart by rounding, by some 1e-9 here)."""
+    text = random_deck(nx, 82, ny=ny, nrect=4, steps=2, eps=1e-10, halo_depth=hd)
+    runs = {}
+    for name, kw in (("fused", {}), ("again", {}), ("exact", dict(exact=True))):
+        c, res, _, _ = gpu_run(tl, text, TEA, criterion=1, **kw)
+        runs[name] = ({f: _interior(c.field(f), hd) for f in ("u", "u0", "p")}, res)
+        c.close()
+    (f, res), (g, ref) = runs["fused"], runs["exact"]
+    for a, b in zip(res, ref):
+        assert a.converged and 0 <= a.rel_residual < 1e-10 and b.converged
+        assert abs(a.iters - b.iters) <= 1, (a.iters, b.iters)
+    assert np.linalg.norm(f["u"] - g["u"]) <= 4e-10 * np.linalg.norm(g["u0"])
+    if [r.iters for r in res] == [r.iters for r in ref] and min(nx, ny) > 30:
+        assert np.linalg.norm(f["p"] - g["p"]) <= 1e-6 * np.linalg.norm(g["p"])
+    for k in f:
+        np.testing.assert_array_equal(f[k], runs["again"][0][k], err_msg=k)
