@@ -75,8 +75,8 @@ typedef __int128 Fixed;
 __device__ __forceinline__ int fixed_scale(double ref) {
   return 62 + 1023 - (int)((__double_as_longlong(ref) >> 52) & 0x7ff);
 }
-// v 2^scale, rounded.  What would reach FIXED_MOST (infinities and NaN
-// among it) becomes FIXED_MOST: far beyond anything plausible beside 2^62.  A
+// v 2^scale, rounded.  What would reach 2^106 (infinities and NaN
+// among it) becomes 2^106: far beyond anything plausible beside 2^62.  A
 // warp's sum is cut to it once more (fixed_cut), so that no number of such
 // addends wraps round to a plausible sum.  `m` has `bits` bits at most.
 constexpr int FIXED_BITS = 106;
@@ -100,12 +100,14 @@ __device__ __forceinline__ Fixed to_fixed(double v, int scale) {
   const unsigned long long m = (u & 0xfffffffffffffull) | (e ? 0x10000000000000ull : 0ull);
   return fixed_shift(e == 2047u ? 1ull : m, 53, e == 2047u ? FIXED_BITS : (int)(e ? e : 1u) - 1075 + scale, u >> 63);
 }
-// The number a whole number of 2^-scale stands for, cut to 53 bits.
+// The number a whole number of 2^-scale stands for, cut to 53 bits; NaN for a sum
+// that holds something cut to 2^106.
 __device__ __forceinline__ double from_fixed(Fixed q, int scale) {
   const bool neg = q < 0;
   unsigned __int128 a = neg ? (unsigned __int128)(-q) : (unsigned __int128)q;
   const unsigned long long hi = (unsigned long long)(a >> 64), lo = (unsigned long long)a;
   if (!(hi | lo)) return 0.0;
+  if (hi >> (FIXED_BITS - 64)) return __longlong_as_double(0x7ff8000000000000ll);
   const int top = hi ? 127 - __clzll(hi) : 63 - __clzll(lo);  // of the leading bit
   a = top > 52 ? a >> (top - 52) : a << (52 - top);
   const int e = top - scale + 1023;

@@ -217,43 +217,35 @@ int tl_record_solver_body(tl_ctx *ctx, int which, cudaGraphConditionalHandle h) 
   const Geom &g = ctx->g;
   cudaStream_t st = ctx->stream;
   switch (which) {
-    case TL_GRAPH_CHEBY_EXACT:
-    case TL_GRAPH_CHEBY_FAST: {
-      const int exact = which == TL_GRAPH_CHEBY_EXACT;
-      const Walk &wk = exact ? ctx->walk_exact : ctx->walk_w64;
-      launch_cheby_step(st, F, g, wk, F.ub, F.u, exact, 0, 0, h, 0);
-      launch_cheby_step(st, F, g, wk, F.u, F.ub, exact, 1, 0, h, 1);
+    case TL_GRAPH_CHEBY_EXACT: {
+      const Walk &wk = ctx->walk_exact;
+      launch_cheby_step(st, F, g, wk, F.ub, F.u, 1, 0, 0, h, 0);
+      launch_cheby_step(st, F, g, wk, F.u, F.ub, 1, 1, 0, h, 1);
       break;
     }
-    case TL_GRAPH_PPCG_EXACT:
-    case TL_GRAPH_PPCG_FAST: {
-      const int exact = which == TL_GRAPH_PPCG_EXACT;
-      const Walk &ww = exact ? ctx->walk_exact : ctx->walk_w64;
-      const Walk &wu = exact ? ctx->walk_exact : ctx->walk_ur64;
+    case TL_GRAPH_PPCG_EXACT: {
+      const Walk &wk = ctx->walk_exact;
       const int n = ctx->ppcg_graph_inner;
       for (int outer = 0; outer < 2; ++outer) {
         const int guard = outer;
         double *pin = outer ? F.pb : F.p, *pout = outer ? F.p : F.pb;
-        launch_tl_w(st, F, g, ww, pin, pout, exact, guard, 0);
-        launch_ppcg_ur(st, F, g, wu, pout, F.sd, exact, guard);
+        launch_tl_w(st, F, g, wk, pin, pout, 1, guard, 0);
+        launch_ppcg_ur(st, F, g, wk, pout, F.sd, 1, guard);
         for (int pp = 1; pp <= n; ++pp) {
           const double *src = (pp & 1) ? F.sd : F.sdb;
           double *dst = (pp & 1) ? F.sdb : F.sd;
           const int last = pp == n;
-          launch_ppcg_inner(st, F, g, ww, src, dst, pp, last, exact, guard, h, last && outer == 1);
+          launch_ppcg_inner(st, F, g, wk, src, dst, pp, last, 1, guard, h, last && outer == 1);
         }
       }
       break;
     }
-    case TL_GRAPH_JACOBI:
-    case TL_GRAPH_JACOBI_FAST: {
-      const int exact = which == TL_GRAPH_JACOBI;
-      const Walk &wk = exact ? ctx->walk_exact : ctx->walk_w64;
-      const Walk &wc = ctx->walk_exact;
-      launch_jacobi(st, F, g, wk, F.u, F.ub, 0, exact);
-      launch_jacobi_check(st, F, g, wc, F.ub, 0, h, 0);
-      launch_jacobi(st, F, g, wk, F.ub, F.u, 1, exact);
-      launch_jacobi_check(st, F, g, wc, F.u, 1, h, 1);
+    case TL_GRAPH_JACOBI: {
+      const Walk &wk = ctx->walk_exact;
+      launch_jacobi(st, F, g, wk, F.u, F.ub, 0, 1);
+      launch_jacobi_check(st, F, g, wk, F.ub, 0, h, 0);
+      launch_jacobi(st, F, g, wk, F.ub, F.u, 1, 1);
+      launch_jacobi_check(st, F, g, wk, F.u, 1, h, 1);
       break;
     }
     default:
@@ -349,8 +341,12 @@ int tl_cheby_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_r
     return TL_OK;
   }
   if (!ctx->host_sc->done) {
-    if ((rc = tl_run_graph(ctx, exact ? TL_GRAPH_CHEBY_EXACT : TL_GRAPH_CHEBY_FAST, &ctx->last_solve_ms))) return rc;
-    if ((rc = tl_read_scalars(ctx))) return rc;
+    if (exact) {
+      if ((rc = tl_run_graph(ctx, TL_GRAPH_CHEBY_EXACT, &ctx->last_solve_ms))) return rc;
+      if ((rc = tl_read_scalars(ctx))) return rc;
+    } else if ((rc = tl_loop64_run(ctx, TL_GRAPH_CHEBY_EXACT, 0, &ctx->last_solve_ms))) {
+      return rc;
+    }
   }
   // u is in ub after an odd number of Chebyshev steps
   if (ctx->host_sc->cheby_iters & 1) {
@@ -442,17 +438,19 @@ int tl_ppcg_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_re
   if ((rc = set_phase(ctx, theta, 0, 0, 1, 2, 2, 0.0))) return rc;
   const int fp = TL_EX_P;
   if ((rc = tl_halo_update(ctx, 1, &fp, 1, 1))) return rc;
-  const int which = exact ? TL_GRAPH_PPCG_EXACT : TL_GRAPH_PPCG_FAST;
-  if (ctx->ppcg_graph_inner != n) {  // the recorded sweeps depend on the inner step count
-    for (int k = TL_GRAPH_PPCG_EXACT; k <= TL_GRAPH_PPCG_FAST; ++k)
-      if (ctx->graph[k]) {
-        cudaGraphExecDestroy(ctx->graph[k]);
-        ctx->graph[k] = nullptr;
+  if (exact) {
+    if (ctx->ppcg_graph_inner != n) {  // the recorded sweeps depend on the inner step count
+      if (ctx->graph[TL_GRAPH_PPCG_EXACT]) {
+        cudaGraphExecDestroy(ctx->graph[TL_GRAPH_PPCG_EXACT]);
+        ctx->graph[TL_GRAPH_PPCG_EXACT] = nullptr;
       }
-    ctx->ppcg_graph_inner = n;
+      ctx->ppcg_graph_inner = n;
+    }
+    if ((rc = tl_run_graph(ctx, TL_GRAPH_PPCG_EXACT, &ctx->last_solve_ms))) return rc;
+    if ((rc = tl_read_scalars(ctx))) return rc;
+  } else if ((rc = tl_loop64_run(ctx, TL_GRAPH_PPCG_EXACT, n, &ctx->last_solve_ms))) {
+    return rc;
   }
-  if ((rc = tl_run_graph(ctx, which, &ctx->last_solve_ms))) return rc;
-  if ((rc = tl_read_scalars(ctx))) return rc;
   const int outer = ctx->host_sc->cheby_iters;
   // the last outer step's p! and halo of p (PPCG.jl:92-93, 31)
   const double *pcur = (outer & 1) ? ctx->F.pb : ctx->F.p;
@@ -508,7 +506,9 @@ int tl_jacobi_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_
   CKL();
   ctx->last_solve_ms = 0.0;
   if (prm->maxiters >= 1) {
-    if ((rc = tl_run_graph(ctx, exact ? TL_GRAPH_JACOBI : TL_GRAPH_JACOBI_FAST, &ctx->last_solve_ms))) return rc;
+    rc = exact ? tl_run_graph(ctx, TL_GRAPH_JACOBI, &ctx->last_solve_ms)
+               : tl_loop64_run(ctx, TL_GRAPH_JACOBI, 0, &ctx->last_solve_ms);
+    if (rc) return rc;
   }
   if ((rc = tl_read_scalars(ctx))) return rc;
   if (ctx->host_sc->iter & 1) {

@@ -3,17 +3,14 @@
 
 #include "tl_internal.cuh"
 
-// Cached iteration-loop graphs.
+// Cached iteration-loop graphs: the exact arithmetic (the fused loops are persistent kernels).
 enum {
   TL_GRAPH_CG_REF = 0,       // reference-mode CG step + halo of u, p
   TL_GRAPH_CG_REF_NOHALO,    // reference-mode CG step without the halo (Cheby/PPCG presteps)
   TL_GRAPH_CG_EXACT,         // tealeaf fused CG, reference operation order
   TL_GRAPH_CHEBY_EXACT,      // Chebyshev steps, the first of the pair reading ub
-  TL_GRAPH_CHEBY_FAST,
   TL_GRAPH_PPCG_EXACT,       // two PPCG outer steps with their inner sweeps
-  TL_GRAPH_PPCG_FAST,
   TL_GRAPH_JACOBI,           // two Jacobi sweeps with their every-50th residual checks
-  TL_GRAPH_JACOBI_FAST,      // the same with the fused sweep
   TL_NGRAPH
 };
 
@@ -88,6 +85,8 @@ int tl_ensure_ir(tl_ctx *ctx);  // allocates the FP32 refinement buffers
 int tl_ir_cg_run(tl_ctx *ctx);
 // The fused FP64 CG loop with the last step's p!, as one persistent kernel (tl_cg64.cu).
 int tl_cg64_run(tl_ctx *ctx, double *ms);
+// The fused FP64 loops of Chebyshev, PPCG and Jacobi (tl_sweeps64.cu).
+int tl_loop64_run(tl_ctx *ctx, int which, int ninner, double *ms);
 // TL_OK, or the error of a persistent kernel whose grid barrier gave up (after tl_read_scalars)
 int tl_persist_check(tl_ctx *ctx);
 // Chebyshev after its first step, in FP32 inside FP64 refinement (tl_ir.cu)

@@ -1,0 +1,436 @@
+// tl_sweeps64.cu -- the fused FP64 loops of Chebyshev, PPCG and Jacobi (tealeaf
+// semantics) as persistent kernels: src/solvers/Cheby.jl:81-106, PPCG.jl:64-94,
+// Jacobi.jl:59-80.
+//
+// Every pass is a ring64 march, bound by the FP64 pipe on large grids; on small
+// ones a pass cost 4-7 us as a kernel of a graph, and costs a grid barrier
+// (1.3 us) here, with the reduction (1.5 us more) only where a test reads it:
+// each Jacobi sweep, the last sweep of a PPCG step, and the Chebyshev steps
+// that take the norm (Cheby.jl:48), which are also the only ones that can be
+// the last and so the only ones that store w and r.
+#include "tl_march.cuh"
+#include "tl_ring64.cuh"
+#include "tl_solvers.h"
+
+namespace tl {
+namespace {
+
+struct Loop64 {
+  Fields F;
+  Geom g;
+  Tiling t;   // strips of 60 columns
+  Tiling te;  // elementwise pass: strips of 64
+  GridSums *sums;
+  int ninner;  // PPCG inner sweeps
+};
+
+struct SharedLoop {
+  SumShared sum;
+  double a, b;
+  int done, conv;
+};
+
+// The state every loop carries.
+struct LoopState {
+  unsigned ring, target = 0, set = 0, handed = 0;
+  bool mirrored = false;
+};
+
+__device__ __forceinline__ Ring64 ring_of(const Loop64 &A, const double *m, const double *o0, const double *o1) {
+  Ring64 q;
+  q.g = A.g;
+  q.m = m;
+  q.m2 = nullptr;
+  q.kx = A.F.kx;
+  q.ky = A.F.ky;
+  q.dg = A.F.diag;
+  q.own[0] = o0;
+  q.own[1] = o1;
+  q.beta = 0.0;
+  q.m_valid = true;
+  return q;
+}
+
+// loop_control's test on the loop's error (no presteps' switch here).
+struct LoopTest {
+  RootTest root;
+  double eps;
+  bool relative;
+  __device__ __forceinline__ LoopTest(const DevScalars *sc)
+      : root(sc->eps, sc->bb), eps(sc->eps), relative(sc->crit == TL_CRIT_RELATIVE) {}
+  __device__ __forceinline__ bool met(double error) const { return relative ? root.met(error) : below(error, eps); }
+};
+
+// ---- Chebyshev ---------------------------------------------------------------
+
+__global__ void __launch_bounds__(WARPS64 * 32, 1) k_cheby64(const Loop64 A) {
+  extern __shared__ __align__(128) unsigned char ring_mem[];
+  __shared__ SharedLoop S;
+  const Fields &F = A.F;
+  DevScalars *sc = F.sc;
+  LoopState L;
+  L.ring = (unsigned)__cvta_generic_to_shared(ring_mem) + (threadIdx.x >> 5) * RING64_BYTES;
+  const LoopTest test(sc);
+  const int maxiters = sc->maxiters, est = sc->est_iters;
+  int k = sc->cheby_iters, iter = sc->iter, conv = 0;
+  double error = sc->error;
+  double *u = (k & 1) ? F.ub : F.u, *un = (k & 1) ? F.u : F.ub;
+  for (;;) {
+    ++k;
+    const int tt = iter + 1, idx = min(k + 1, maxiters + 1);  // the tables hold maxiters + 2 entries
+    const double ca = F.chebyalpha[idx], cb = F.chebybeta[idx];
+    const bool norm = k >= est && (tt + 1) % 10 == 0;  // Cheby.jl:48
+    const bool store = norm || tt >= maxiters;
+    const int scale = fixed_scale(error);
+    double acc = 0.0;
+    Fixed sum = 0;
+    ring64<false, 2>(ring_of(A, u, F.u0, F.p), A.t, L.ring, L.mirrored, &A.sums->next_tile, L.handed,
+                     [&](int j, int i0, bool has1, bool owns, const Row64 &q) {
+                       const double2 w = apply64(q, has1);
+                       const double2 r = make_double2(q.own[0].x - w.x, q.own[0].y - w.y);
+                       const double2 p = make_double2(fma(ca, q.own[1].x, cb * r.x), fma(ca, q.own[1].y, cb * r.y));
+                       if (owns) {
+                         const size_t c = A.g.at(i0, j);
+                         if (norm) {
+                           acc = fma(r.x, r.x, acc);
+                           if (has1) acc = fma(r.y, r.y, acc);
+                         }
+                         if (store) {
+                           put64(F.w + c, w, has1);
+                           put64(F.r + c, r, has1);
+                         }
+                         put64(F.p + c, p, has1);
+                         put64(un + c, make_double2(q.c.x + p.x, q.c.y + p.y), has1);
+                       }
+                     },
+                     [&]() {
+                       if (norm) sum += to_fixed(acc, scale);
+                       acc = 0.0;
+                     });
+    L.mirrored = !L.mirrored;
+    iter = tt;
+    double *t = u;
+    u = un;
+    un = t;
+    if (norm) {
+      if (!grid_sum1(S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double rr) {
+            const bool cv = test.met(rr);
+            if ((threadIdx.x & 31) == 0) {
+              S.a = rr;
+              S.conv = cv;
+            }
+          }))
+        return;
+      error = S.a;
+      conv = S.conv;
+    } else if (!grid_barrier(&sc->bar, L.target)) {
+      return;
+    }
+    if (conv || iter >= maxiters) break;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sc->cheby_iters = k;
+    sc->iter = iter;
+    sc->error = error;
+    sc->converged = conv;
+    sc->done = 1;
+  }
+}
+
+// ---- PPCG --------------------------------------------------------------------
+
+// u += alpha p, r -= alpha w, sd = r / theta on this warp's tiles.
+__device__ __forceinline__ void ppcg_update(const Loop64 &A, LoopState &L, const double *p, double alpha, double rtheta) {
+  const int nx = A.g.nx, lane = threadIdx.x & 31;
+  TileWalk walk(A.te, A.g.ny, L.mirrored, &A.sums->next_tile, L.handed);
+  L.handed += walk.requests();
+  while (walk.valid()) {
+    int strip, j0, j1;
+    walk.place(strip, j0, j1);
+    const unsigned asked = walk.ask();
+    const int i0 = strip * 64 + 2 * lane;
+    if (i0 < nx) {
+      const bool has1 = i0 + 1 < nx;
+#pragma unroll 4
+      for (int j = j0; j < j1; ++j) {
+        const size_t c = A.g.at(i0, j);
+        auto ld = [&](const double *f) { return __ldcg(reinterpret_cast<const double2 *>(f + c)); };
+        const double2 pv = ld(p), wv = ld(A.F.w), uv = ld(A.F.u), rv = ld(A.F.r);
+        const double2 r = make_double2(fma(-alpha, wv.x, rv.x), fma(-alpha, wv.y, rv.y));
+        put64(A.F.u + c, make_double2(fma(alpha, pv.x, uv.x), fma(alpha, pv.y, uv.y)), has1);
+        put64(A.F.r + c, r, has1);
+        put64(A.F.sd + c, make_double2(r.x * rtheta, r.y * rtheta), has1);
+      }
+    }
+    __syncwarp();
+    walk.take(asked);
+  }
+}
+
+__global__ void __launch_bounds__(WARPS64 * 32, 1) k_ppcg64(const Loop64 A) {
+  extern __shared__ __align__(128) unsigned char ring_mem[];
+  __shared__ SharedLoop S;
+  const Fields &F = A.F;
+  DevScalars *sc = F.sc;
+  LoopState L;
+  L.ring = (unsigned)__cvta_generic_to_shared(ring_mem) + (threadIdx.x >> 5) * RING64_BYTES;
+  const LoopTest test(sc);
+  const int maxiters = sc->maxiters;
+  const double rtheta = 1.0 / sc->theta;
+  int outer = sc->cheby_iters, iter = sc->iter;
+  double rro = sc->rro, alpha = 0.0, beta = sc->beta, pw_ref = rro;
+  bool first = sc->first != 0;  // the first direction is p itself
+  double *p = F.p, *pn = F.pb;
+  for (;;) {
+    double acc = 0.0;
+    Fixed sum = 0;
+    int scale = fixed_scale(pw_ref);
+    auto tile_end = [&]() {
+      sum += to_fixed(acc, scale);
+      acc = 0.0;
+    };
+    auto direction = [&](int j, int i0, bool has1, bool owns, const Row64 &q) {
+      const double2 w = apply64(q, has1);
+      if (owns) {
+        const size_t c = A.g.at(i0, j);
+        acc = fma(w.y, q.c.y, fma(w.x, q.c.x, acc));
+        put64(F.w + c, w, has1);
+        put64(pn + c, q.c, has1);
+      }
+    };
+    Ring64 d = ring_of(A, p, nullptr, nullptr);
+    d.m2 = F.r;
+    d.beta = beta;
+    if (first) ring64<false, 0>(d, A.t, L.ring, L.mirrored, &A.sums->next_tile, L.handed, direction, tile_end);
+    else ring64<true, 0>(d, A.t, L.ring, L.mirrored, &A.sums->next_tile, L.handed, direction, tile_end);
+    if (!grid_sum1(S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double pw) {
+          const double a = ddiv(rro, pw);
+          if ((threadIdx.x & 31) == 0) {
+            S.a = a;
+            S.b = pw;
+          }
+        }))
+      return;
+    alpha = S.a;
+    pw_ref = S.b;
+    {
+      double *t = p;
+      p = pn;
+      pn = t;
+    }
+    first = false;
+    L.mirrored = !L.mirrored;
+    ppcg_update(A, L, p, alpha, rtheta);
+    if (!grid_barrier(&sc->bar, L.target)) return;
+    scale = fixed_scale(rro);
+    sum = 0;
+    for (int pp = 1; pp <= A.ninner; ++pp) {
+      const double ca = F.chebyalpha[pp], cb = F.chebybeta[pp];
+      const double *src = (pp & 1) ? F.sd : F.sdb;
+      double *dst = (pp & 1) ? F.sdb : F.sd;
+      const bool last = pp == A.ninner;
+      L.mirrored = !L.mirrored;
+      ring64<false, 2>(ring_of(A, src, F.r, F.u), A.t, L.ring, L.mirrored, &A.sums->next_tile, L.handed,
+                       [&](int j, int i0, bool has1, bool owns, const Row64 &q) {
+                         const double2 a = apply64(q, has1);
+                         const double2 r = make_double2(q.own[0].x - a.x, q.own[0].y - a.y);
+                         if (owns) {
+                           const size_t c = A.g.at(i0, j);
+                           if (last) {
+                             acc = fma(r.x, r.x, acc);
+                             if (has1) acc = fma(r.y, r.y, acc);
+                           }
+                           put64(F.r + c, r, has1);
+                           put64(F.u + c, make_double2(q.own[1].x + q.c.x, q.own[1].y + q.c.y), has1);
+                           put64(dst + c, make_double2(fma(ca, q.c.x, cb * r.x), fma(ca, q.c.y, cb * r.y)), has1);
+                         }
+                       },
+                       [&]() {
+                         if (last) sum += to_fixed(acc, scale);
+                         acc = 0.0;
+                       });
+      if (!last && !grid_barrier(&sc->bar, L.target)) return;
+    }
+    if (!grid_sum1(S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double rrn) {
+          const double b = ddiv(rrn, rro);  // PPCG.jl:89-92
+          const bool cv = test.met(rrn);
+          if ((threadIdx.x & 31) == 0) {
+            S.a = b;
+            S.b = rrn;
+            S.conv = cv;
+            S.done = cv || iter + 1 >= maxiters;
+          }
+        }))
+      return;
+    beta = S.a;
+    rro = S.b;
+    L.mirrored = !L.mirrored;
+    ++iter;
+    ++outer;
+    if (S.done) break;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sc->alpha = alpha;
+    sc->pw = pw_ref;
+    sc->beta = beta;
+    sc->rro = rro;
+    sc->error = rro;
+    sc->iter = iter;
+    sc->cheby_iters = outer;
+    sc->first = 0;
+    sc->converged = S.conv;
+    sc->done = 1;
+  }
+}
+
+// ---- Jacobi ------------------------------------------------------------------
+
+__global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64(const Loop64 A) {
+  extern __shared__ __align__(128) unsigned char ring_mem[];
+  __shared__ SharedLoop S;
+  const Fields &F = A.F;
+  DevScalars *sc = F.sc;
+  LoopState L;
+  L.ring = (unsigned)__cvta_generic_to_shared(ring_mem) + (threadIdx.x >> 5) * RING64_BYTES;
+  const LoopTest test(sc);
+  const int maxiters = sc->maxiters, lane = threadIdx.x & 31;
+  int iter = sc->iter;
+  // a sweep changes no sum of |u' - u| beyond sqrt(cells) times |u|
+  double ref = sqrt(sc->bb), error = sc->error;
+  double *u = F.u, *un = F.ub;
+  bool checked = false;
+  for (;;) {
+    int scale = fixed_scale(ref);
+    double acc = 0.0;
+    Fixed sum = 0;
+    ring64<false, 1>(ring_of(A, u, F.u0, nullptr), A.t, L.ring, L.mirrored, &A.sums->next_tile, L.handed,
+                     [&](int j, int i0, bool has1, bool owns, const Row64 &q) {
+                       double a = fma(q.kx.y, has1 ? q.c.y : q.c.x, q.own[0].x), b = fma(q.kxe, q.e, q.own[0].y);
+                       a = fma(q.kx.x, q.w, a);
+                       b = fma(q.kx.y, q.c.x, b);
+                       a = fma(q.kyn.x, q.n.x, a);
+                       b = fma(q.kyn.y, q.n.y, b);
+                       a = fma(q.ky.x, q.s.x, a) * q.dg.x;  // diag holds 1 / (1 + sum k)
+                       b = fma(q.ky.y, q.s.y, b) * q.dg.y;
+                       if (owns) {
+                         acc = dadd(acc, fabs(dsub(a, q.c.x)));
+                         if (has1) acc = dadd(acc, fabs(dsub(b, q.c.y)));
+                         put64(un + A.g.at(i0, j), make_double2(a, b), has1);
+                       }
+                     },
+                     [&]() {
+                       sum += to_fixed(acc, scale);
+                       acc = 0.0;
+                     });
+    ++iter;
+    checked = iter % 50 == 0;
+    if (!grid_sum1(S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double e) {
+          const bool cv = !checked && test.met(e);
+          if (lane == 0) {
+            S.a = e;
+            S.conv = cv;
+            S.done = !checked && (cv || iter >= maxiters);
+          }
+        }))
+      return;
+    error = S.a;
+    L.mirrored = !L.mirrored;
+    double *t = u;
+    u = un;
+    un = t;
+    if (checked) {  // every 50th sweep r = u0 - A u joins the error (Jacobi.jl:16-21)
+      const double scale_ref = sc->bb;
+      scale = fixed_scale(scale_ref);
+      sum = 0;
+      ring64<false, 1>(ring_of(A, u, F.u0, nullptr), A.t, L.ring, L.mirrored, &A.sums->next_tile, L.handed,
+                       [&](int j, int i0, bool has1, bool owns, const Row64 &q) {
+                         const Nbr c0 = {q.c.x, has1 ? q.c.y : q.c.x, q.w, q.n.x, q.s.x, q.kx.x, q.kx.y, q.ky.x, q.kyn.x, 0.0};
+                         const Nbr c1 = {q.c.y, q.e, q.c.x, q.n.y, q.s.y, q.kx.y, q.kxe, q.ky.y, q.kyn.y, 0.0};
+                         const double r0 = dsub(q.own[0].x, apply_a<true>(c0)), r1 = dsub(q.own[0].y, apply_a<true>(c1));
+                         if (owns) {
+                           put64(F.r + A.g.at(i0, j), make_double2(r0, r1), has1);
+                           acc = dadd(acc, dmul(r0, r0));
+                           if (has1) acc = dadd(acc, dmul(r1, r1));
+                         }
+                       },
+                       [&]() {
+                         sum += to_fixed(acc, scale);
+                         acc = 0.0;
+                       });
+      if (!grid_sum1(S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double rr) {
+            const double e = dadd(error, rr);
+            const bool cv = test.met(e);
+            if (lane == 0) {
+              S.a = e;
+              S.conv = cv;
+              S.done = cv || iter >= maxiters;
+            }
+          }))
+        return;
+      L.mirrored = !L.mirrored;
+    }
+    const double e = S.a;
+    if (!checked && e > 0.0) ref = e;
+    error = e;
+    if (S.done) break;
+  }
+  // r .= u copies the last sweep's input, its depth-1 halo (the reflection)
+  // included; after a check the interior holds the residual
+  const int nx = A.g.nx, ny = A.g.ny, chunks = (nx + 31) / 32, warps = gridDim.x * WARPS64;
+  const long long n = (long long)chunks * ny, pitch = A.g.pitch;
+  for (long long k = blockIdx.x * WARPS64 + (threadIdx.x >> 5); k < n; k += warps) {
+    const int j = (int)(k / chunks), i = (int)(k % chunks) * 32 + lane;
+    if (i >= nx) continue;
+    const size_t c = A.g.at(i, j);
+    const double v = __ldcg(un + c);
+    if (!checked) F.r[c] = v;
+    if (i == 0) F.r[c - 1] = v;
+    if (i == nx - 1) F.r[c + 1] = v;
+    if (j == 0) F.r[c - pitch] = v;
+    if (j == ny - 1) F.r[c + pitch] = v;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sc->error = error;
+    sc->iter = iter;
+    sc->converged = S.conv;
+    sc->done = 1;
+  }
+}
+
+}  // namespace
+}  // namespace tl
+
+using namespace tl;
+
+// Runs one of the loops from the state its solver has set up, as
+// TL_GRAPH_CHEBY_EXACT, TL_GRAPH_PPCG_EXACT or TL_GRAPH_JACOBI name them; the
+// scalars are read back.  One launch.
+int tl_loop64_run(tl_ctx *ctx, int which, int ninner, double *ms) {
+  Loop64 A;
+  A.F = ctx->F;
+  A.g = ctx->g;
+  A.sums = static_cast<GridSums *>(ctx->grid_sums);
+  A.ninner = ninner;
+  const void *kernel = which == TL_GRAPH_CHEBY_EXACT  ? (const void *)k_cheby64
+                       : which == TL_GRAPH_PPCG_EXACT ? (const void *)k_ppcg64
+                                                      : (const void *)k_jacobi64;
+  // a row holds the FP64 pipe for 14 to 20 instructions of 64 cycles; see tl_cg64_run for the rule
+  const TileCost sweep{0.1, 1200.0, 1500.0, 1150.0, 200.0, 32, 48, 4}, each{0.0, 500.0, 1000.0, 400.0, 150.0, 0, 24, 8};
+  A.t = make_tiling(ctx->g.nx, ctx->g.ny, STRIP64, sweep, persist_blocks(ctx->sm_count), WARPS64);
+  A.te = make_tiling_on(A.t, ctx->g.nx, ctx->g.ny, 64, each, WARPS64);
+  const size_t smem = (size_t)RING64_BYTES * WARPS64;
+  CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(cudaMemsetAsync(&ctx->F.sc->bar, 0, sizeof(GridBar), ctx->stream));
+  CK(cudaMemsetAsync(&A.sums->next_tile, 0, sizeof(unsigned), ctx->stream));
+  CK(cudaEventRecord(ctx->ev0, ctx->stream));
+  void *args[] = {&A};
+  CK(cudaLaunchCooperativeKernel(kernel, dim3(A.t.blocks), dim3(WARPS64 * 32), args, smem, ctx->stream));
+  CK(cudaEventRecord(ctx->ev1, ctx->stream));
+  ctx->launches += 1;
+  int rc = tl_read_scalars(ctx);
+  if (rc) return rc;
+  float t = 0.f;
+  CK(cudaEventElapsedTime(&t, ctx->ev0, ctx->ev1));
+  if (ms) *ms += t;
+  return tl_persist_check(ctx);
+}

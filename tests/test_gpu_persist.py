@@ -70,3 +70,52 @@ def test_fp64_cg_tilings(tl, built_lib, nx, ny, hd):
         assert np.linalg.norm(f["p"] - g["p"]) <= 1e-6 * np.linalg.norm(g["p"])
     for k in f:
         np.testing.assert_array_equal(f[k], runs["again"][0][k], err_msg=k)
+
+
+@pytest.mark.parametrize("nx,ny,hd", [(1, 9, 2), (59, 7, 1), (61, 33, 3), (120, 40, 2), (243, 131, 2), (3100, 2500, 2)])
+def test_jacobi_tilings(tl, built_lib, nx, ny, hd):
+    """Fused Jacobi against exact Jacobi over 53 sweeps (one residual check
+    among them): each sweep is a weighted mean of neighbours and the
+    right-hand side, so the two drift by a few roundings a sweep: u within
+    1e-13 of its maximum, r (the last sweep's input) alike, and its faces."""
+    text = random_deck(nx, 83, ny=ny, nrect=4, steps=1, eps=0.0, solver="jacobi", halo_depth=hd)
+    text = text.replace("max_iters=5000", "max_iters=53")
+    f = {}
+    for name, exact in (("fused", False), ("exact", True)):
+        st = tl.Settings.from_text(text, mode=TEA, exact=exact)
+        c = tl.initialiseapp(st)
+        tl.haloupdate(c, st, 1, ["energy", "density"])
+        res = tl.Jacobi.solve(c, st, st.dtinit / st.dx ** 2, st.dtinit / st.dy ** 2)  # solvefinished! overwrites r
+        f[name] = (c.field("u"), c.field("r"), res)
+        c.close()
+    (u, r, a), (v, s, b) = f["fused"], f["exact"]
+    assert a.iters == b.iters == 53
+    assert abs(a.error - b.error) <= 1e-9 * abs(b.error) + 1e-13 * np.max(np.abs(v)) * nx * ny
+    scale = np.max(np.abs(v))
+    assert np.max(np.abs(u - v)) <= 1e-13 * scale
+    # the halo layers past the first hold what the solve before it left: faces and interior are compared
+    k = hd - 1
+    cut = lambda x: x[k:x.shape[0] - k, k:x.shape[1] - k]
+    rf, sf = cut(r)[:, 1:-1], cut(s)[:, 1:-1]
+    assert np.max(np.abs(rf - sf)) <= 1e-13 * scale
+    assert np.max(np.abs(cut(r)[1:-1] - cut(s)[1:-1])) <= 1e-13 * scale
+
+
+@pytest.mark.parametrize("solver", ["cheby", "ppcg"])
+@pytest.mark.parametrize("nx,ny,hd", [(61, 120, 1), (119, 64, 3), (181, 240, 2), (513, 300, 2)])
+def test_cheby_ppcg_tilings(tl, built_lib, solver, nx, ny, hd):
+    """Fused Chebyshev and PPCG against their exact form, 40 presteps: the
+    tolerances of test_gpu_solvers.py (iterations within 2, u within 1e-9 of
+    its maximum)."""
+    text = random_deck(nx, 84, ny=ny, nrect=5, steps=2, eps=1e-12, solver=solver, halo_depth=hd, presteps=40,
+                       ppcg_inner_steps=5)
+    f = {}
+    for name, exact in (("fused", False), ("again", False), ("exact", True)):
+        c, res, _, _ = gpu_run(tl, text, TEA, exact=exact)
+        f[name] = (_interior(c.field("u"), hd), res)
+        c.close()
+    (u, res), (v, ref) = f["fused"], f["exact"]
+    for a, b in zip(res, ref):
+        assert abs(a.iters - b.iters) <= 2, (a.iters, b.iters)
+    assert np.max(np.abs(u - v)) <= 1e-9 * np.max(np.abs(v))
+    np.testing.assert_array_equal(u, f["again"][0])
