@@ -45,7 +45,8 @@ struct Walk {
 // before each launch.
 struct GridBar {
   unsigned count;
-  unsigned fail;  // a wait gave up: the launch's results are void
+  unsigned fail;       // a wait gave up: the launch's results are void
+  unsigned next_tile;  // tiles handed out so far
 };
 
 // Scalars of a solve, resident in device memory so that the iteration loop

@@ -58,6 +58,12 @@ __device__ __forceinline__ Pair warp_pairs(const Pair (&v)[3]) {
   return c;
 }
 
+// The blocks that work on one deck: the whole launch, or a batch's group of it.
+struct Grid {
+  int nb, id;
+};
+__device__ __forceinline__ Grid whole_grid() { return Grid{(int)gridDim.x, (int)blockIdx.x}; }
+
 // ---- sums over the grid ----------------------------------------------------
 // Warps take their tiles in whatever order they come free (the SMs of one GPU
 // do not get the same memory bandwidth: at 8192^2 the fast ones waited 110 of
@@ -131,15 +137,13 @@ __device__ __forceinline__ Fixed shfl(Fixed v, int lane) {
   return (Fixed)(((unsigned __int128)hi << 64) | lo);
 }
 
-// What a persistent launch keeps in global memory, `next_tile` zeroed before
-// it: two sets of block partials in turn (a block may already be at its next
-// sum while another still reads this one), and the tiles handed out so far.
+// A persistent launch's block partials in global memory, two sets in turn (a
+// block may already be at its next sum while another still reads this one).
 // Each block adds up all partials itself: adding them into one place with
 // atomics instead made an iteration 2.7 us longer (152 blocks on one line).
 constexpr int PERSIST_MAX_BLOCKS = 160;
 struct GridSums {
   Fixed part[2][PERSIST_MAX_BLOCKS][4];  // [.][.][3] pads a block to 64 bytes
-  unsigned next_tile;
 };
 
 __device__ __forceinline__ Fixed ldcg_fixed(const Fixed *p) {
@@ -175,11 +179,11 @@ __device__ __forceinline__ bool grid_arrive_wait(GridBar *g, unsigned target) {
 
 // The barrier for whole blocks; `target` counts the arrivals expected so far on
 // every thread (start at 0).
-__device__ __forceinline__ bool grid_barrier(GridBar *g, unsigned &target) {
+__device__ __forceinline__ bool grid_barrier(Grid G, GridBar *g, unsigned &target) {
   __shared__ int ok;
   __syncthreads();
-  if (gridDim.x == 1) return true;
-  target += gridDim.x;
+  if (G.nb == 1) return true;
+  target += G.nb;
   if (threadIdx.x < 32) ok = grid_arrive_wait(g, target);
   __syncthreads();
   return ok != 0;
@@ -217,9 +221,9 @@ struct SumShared {
 //
 // One sum: each warp's share in lane 0, in whole numbers of 2^-scale.
 template <class Fin>
-__device__ __forceinline__ bool grid_sum1(SumShared &S, GridBar *bar, GridSums *G, Fixed v, int scale, unsigned &target,
+__device__ __forceinline__ bool grid_sum1(Grid grid, SumShared &S, GridBar *bar, GridSums *G, Fixed v, int scale, unsigned &target,
                                           unsigned &set, Fin &&fin) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = gridDim.x, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = grid.nb, nw = blockDim.x >> 5;
   target += nb;
   if (lane == 0) S.warp[warp][0] = fixed_cut(v);
   __syncthreads();
@@ -228,7 +232,7 @@ __device__ __forceinline__ bool grid_sum1(SumShared &S, GridBar *bar, GridSums *
     for (int off = nw >> 1; off >= 1; off >>= 1) t += shfl_xor(t, off);
     if (nb > 1) {
       Fixed *part = &G->part[set & 1][0][0];
-      if (lane == 0) stcg_fixed(part + blockIdx.x, t);
+      if (lane == 0) stcg_fixed(part + grid.id, t);
       S.ok = grid_arrive_wait(bar, target);
       Fixed q[5];
 #pragma unroll
@@ -249,9 +253,9 @@ __device__ __forceinline__ bool grid_sum1(SumShared &S, GridBar *bar, GridSums *
 // and to add (1.3 us of an iteration of 7.9 at 256^2), where every warp has its
 // one fixed tile.
 template <bool FIXED, class Fin>
-__device__ __forceinline__ bool grid_sum3(SumShared &S, GridBar *bar, GridSums *G, Fixed v, int scale, Pair w,
+__device__ __forceinline__ bool grid_sum3(Grid grid, SumShared &S, GridBar *bar, GridSums *G, Fixed v, int scale, Pair w,
                                           unsigned &target, unsigned &set, Fin &&fin) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = gridDim.x, nw = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = grid.nb, nw = blockDim.x >> 5;
   target += nb;
   if ((lane & 7) == 0 && lane < 24) {
     if (FIXED) S.warp[warp][lane >> 3] = fixed_cut(v);
@@ -269,7 +273,7 @@ __device__ __forceinline__ bool grid_sum3(SumShared &S, GridBar *bar, GridSums *
       t += shfl_xor(t, 1);
       if (nb > 1) {
         Fixed(*part)[4] = G->part[set & 1];
-        if (lane < 24 && c == 0) stcg_fixed(&part[blockIdx.x][d], t);
+        if (lane < 24 && c == 0) stcg_fixed(&part[grid.id][d], t);
         S.ok = grid_arrive_wait(bar, target);
         t = 0;
         for (int k0 = c; k0 < nb; k0 += 80) {  // ten loads in flight
@@ -293,7 +297,7 @@ __device__ __forceinline__ bool grid_sum3(SumShared &S, GridBar *bar, GridSums *
       Pair t = warp_pairs(q);
       if (nb > 1) {
         Pair(*part)[8] = reinterpret_cast<Pair(*)[8]>(G->part[set & 1]);
-        if (lane < 24 && c == 0) __stcg(reinterpret_cast<float2 *>(&part[blockIdx.x][d]), make_float2(t.hi, t.lo));
+        if (lane < 24 && c == 0) __stcg(reinterpret_cast<float2 *>(&part[grid.id][d]), make_float2(t.hi, t.lo));
         S.ok = grid_arrive_wait(bar, target);
         float4 ab[5];
         float2 e[5];
@@ -375,10 +379,10 @@ struct TileWalk {
   int t;
   unsigned *next;
   unsigned base;
-  __device__ __forceinline__ TileWalk(const Tiling &T, int ny, bool mirrored, unsigned *next, unsigned base)
+  __device__ __forceinline__ TileWalk(Grid grid, const Tiling &T, int ny, bool mirrored, unsigned *next, unsigned base)
       : T(T), ny(ny), mirrored(mirrored), next(next), base(base) {
     const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    t = T.tiles < T.warps ? warp * gridDim.x + blockIdx.x : blockIdx.x * nw + warp;
+    t = T.tiles < T.warps ? warp * grid.nb + grid.id : grid.id * nw + warp;
   }
   __device__ __forceinline__ bool valid() const { return t < T.tiles; }
   // strip, and rows [j0, j1)

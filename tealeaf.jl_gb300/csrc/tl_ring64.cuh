@@ -56,7 +56,7 @@ __device__ __forceinline__ double2 apply64(const Row64 &q, bool has1) {
 // `tile_end()` after each tile.  A neighbour across the domain's edge is the cell
 // itself; the second cell of a lane that has only one is zero.
 template <bool TWO, int NOWN, class Body, class TileEnd>
-__device__ __forceinline__ void ring64(const Ring64 &A, const Tiling &T, unsigned ring, bool mirrored, unsigned *next,
+__device__ __forceinline__ void ring64(Grid grid, const Ring64 &A, const Tiling &T, unsigned ring, bool mirrored, unsigned *next,
                                        unsigned &handed, Body &&body, TileEnd &&tile_end) {
   constexpr int NARR = 4 + TWO + NOWN;
   constexpr int DEPTH = RING64_BYTES / (NARR * 512) < 6 ? RING64_BYTES / (NARR * 512) : 6;
@@ -64,7 +64,7 @@ __device__ __forceinline__ void ring64(const Ring64 &A, const Tiling &T, unsigne
   const int nx = A.g.nx, ny = A.g.ny;
   const int lane = threadIdx.x & 31;
   const unsigned slot0 = ring + 16 * lane;
-  TileWalk walk(T, ny, mirrored, next, handed);
+  TileWalk walk(grid, T, ny, mirrored, next, handed);
   handed += walk.requests();
   while (walk.valid()) {
     int strip, j0, j1;

@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_cheby64(const Loop64 A) {
     const int scale = fixed_scale(error);
     double acc = 0.0;
     Fixed sum = 0;
-    ring64<false, 2>(ring_of(A, u, F.u0, F.p), A.t, L.ring, L.mirrored, &A.sums->next_tile, L.handed,
+    ring64<false, 2>(whole_grid(), ring_of(A, u, F.u0, F.p), A.t, L.ring, L.mirrored, &A.F.sc->bar.next_tile, L.handed,
                      [&](int j, int i0, bool has1, bool owns, const Row64 &q) {
                        const double2 w = apply64(q, has1);
                        const double2 r = make_double2(q.own[0].x - w.x, q.own[0].y - w.y);
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_cheby64(const Loop64 A) {
     u = un;
     un = t;
     if (norm) {
-      if (!grid_sum1(S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double rr) {
+      if (!grid_sum1(whole_grid(), S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double rr) {
             const bool cv = test.met(rr);
             if ((threadIdx.x & 31) == 0) {
               S.a = rr;
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_cheby64(const Loop64 A) {
         return;
       error = S.a;
       conv = S.conv;
-    } else if (!grid_barrier(&sc->bar, L.target)) {
+    } else if (!grid_barrier(whole_grid(), &sc->bar, L.target)) {
       return;
     }
     if (conv || iter >= maxiters) break;
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_cheby64(const Loop64 A) {
 // u += alpha p, r -= alpha w, sd = r / theta on this warp's tiles.
 __device__ __forceinline__ void ppcg_update(const Loop64 &A, LoopState &L, const double *p, double alpha, double rtheta) {
   const int nx = A.g.nx, lane = threadIdx.x & 31;
-  TileWalk walk(A.te, A.g.ny, L.mirrored, &A.sums->next_tile, L.handed);
+  TileWalk walk(whole_grid(), A.te, A.g.ny, L.mirrored, &A.F.sc->bar.next_tile, L.handed);
   L.handed += walk.requests();
   while (walk.valid()) {
     int strip, j0, j1;
@@ -201,9 +201,9 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_ppcg64(const Loop64 A) {
     Ring64 d = ring_of(A, p, nullptr, nullptr);
     d.m2 = F.r;
     d.beta = beta;
-    if (first) ring64<false, 0>(d, A.t, L.ring, L.mirrored, &A.sums->next_tile, L.handed, direction, tile_end);
-    else ring64<true, 0>(d, A.t, L.ring, L.mirrored, &A.sums->next_tile, L.handed, direction, tile_end);
-    if (!grid_sum1(S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double pw) {
+    if (first) ring64<false, 0>(whole_grid(), d, A.t, L.ring, L.mirrored, &A.F.sc->bar.next_tile, L.handed, direction, tile_end);
+    else ring64<true, 0>(whole_grid(), d, A.t, L.ring, L.mirrored, &A.F.sc->bar.next_tile, L.handed, direction, tile_end);
+    if (!grid_sum1(whole_grid(), S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double pw) {
           const double a = ddiv(rro, pw);
           if ((threadIdx.x & 31) == 0) {
             S.a = a;
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_ppcg64(const Loop64 A) {
     first = false;
     L.mirrored = !L.mirrored;
     ppcg_update(A, L, p, alpha, rtheta);
-    if (!grid_barrier(&sc->bar, L.target)) return;
+    if (!grid_barrier(whole_grid(), &sc->bar, L.target)) return;
     scale = fixed_scale(rro);
     sum = 0;
     for (int pp = 1; pp <= A.ninner; ++pp) {
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_ppcg64(const Loop64 A) {
       double *dst = (pp & 1) ? F.sdb : F.sd;
       const bool last = pp == A.ninner;
       L.mirrored = !L.mirrored;
-      ring64<false, 2>(ring_of(A, src, F.r, F.u), A.t, L.ring, L.mirrored, &A.sums->next_tile, L.handed,
+      ring64<false, 2>(whole_grid(), ring_of(A, src, F.r, F.u), A.t, L.ring, L.mirrored, &A.F.sc->bar.next_tile, L.handed,
                        [&](int j, int i0, bool has1, bool owns, const Row64 &q) {
                          const double2 a = apply64(q, has1);
                          const double2 r = make_double2(q.own[0].x - a.x, q.own[0].y - a.y);
@@ -249,9 +249,9 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_ppcg64(const Loop64 A) {
                          if (last) sum += to_fixed(acc, scale);
                          acc = 0.0;
                        });
-      if (!last && !grid_barrier(&sc->bar, L.target)) return;
+      if (!last && !grid_barrier(whole_grid(), &sc->bar, L.target)) return;
     }
-    if (!grid_sum1(S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double rrn) {
+    if (!grid_sum1(whole_grid(), S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double rrn) {
           const double b = ddiv(rrn, rro);  // PPCG.jl:89-92
           const bool cv = test.met(rrn);
           if ((threadIdx.x & 31) == 0) {
@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64(const Loop64 A) {
     int scale = fixed_scale(ref);
     double acc = 0.0;
     Fixed sum = 0;
-    ring64<false, 1>(ring_of(A, u, F.u0, nullptr), A.t, L.ring, L.mirrored, &A.sums->next_tile, L.handed,
+    ring64<false, 1>(whole_grid(), ring_of(A, u, F.u0, nullptr), A.t, L.ring, L.mirrored, &A.F.sc->bar.next_tile, L.handed,
                      [&](int j, int i0, bool has1, bool owns, const Row64 &q) {
                        double a = fma(q.kx.y, has1 ? q.c.y : q.c.x, q.own[0].x), b = fma(q.kxe, q.e, q.own[0].y);
                        a = fma(q.kx.x, q.w, a);
@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64(const Loop64 A) {
                      });
     ++iter;
     checked = iter % 50 == 0;
-    if (!grid_sum1(S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double e) {
+    if (!grid_sum1(whole_grid(), S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double e) {
           const bool cv = !checked && test.met(e);
           if (lane == 0) {
             S.a = e;
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64(const Loop64 A) {
       const double scale_ref = sc->bb;
       scale = fixed_scale(scale_ref);
       sum = 0;
-      ring64<false, 1>(ring_of(A, u, F.u0, nullptr), A.t, L.ring, L.mirrored, &A.sums->next_tile, L.handed,
+      ring64<false, 1>(whole_grid(), ring_of(A, u, F.u0, nullptr), A.t, L.ring, L.mirrored, &A.F.sc->bar.next_tile, L.handed,
                        [&](int j, int i0, bool has1, bool owns, const Row64 &q) {
                          const Nbr c0 = {q.c.x, has1 ? q.c.y : q.c.x, q.w, q.n.x, q.s.x, q.kx.x, q.kx.y, q.ky.x, q.kyn.x, 0.0};
                          const Nbr c1 = {q.c.y, q.e, q.c.x, q.n.y, q.s.y, q.kx.y, q.kxe, q.ky.y, q.kyn.y, 0.0};
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64(const Loop64 A) {
                          sum += to_fixed(acc, scale);
                          acc = 0.0;
                        });
-      if (!grid_sum1(S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double rr) {
+      if (!grid_sum1(whole_grid(), S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double rr) {
             const double e = dadd(error, rr);
             const bool cv = test.met(e);
             if (lane == 0) {
@@ -421,7 +421,7 @@ int tl_loop64_run(tl_ctx *ctx, int which, int ninner, double *ms) {
   const size_t smem = (size_t)RING64_BYTES * WARPS64;
   CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   CK(cudaMemsetAsync(&ctx->F.sc->bar, 0, sizeof(GridBar), ctx->stream));
-  CK(cudaMemsetAsync(&A.sums->next_tile, 0, sizeof(unsigned), ctx->stream));
+  CK(cudaMemsetAsync(&A.F.sc->bar.next_tile, 0, sizeof(unsigned), ctx->stream));
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   void *args[] = {&A};
   CK(cudaLaunchCooperativeKernel(kernel, dim3(A.t.blocks), dim3(WARPS64 * 32), args, smem, ctx->stream));

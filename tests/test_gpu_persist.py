@@ -119,3 +119,30 @@ def test_cheby_ppcg_tilings(tl, built_lib, solver, nx, ny, hd):
         assert abs(a.iters - b.iters) <= 2, (a.iters, b.iters)
     assert np.max(np.abs(u - v)) <= 1e-9 * np.max(np.abs(v))
     np.testing.assert_array_equal(u, f["again"][0])
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_batch_groups(tl, built_lib, precision):
+    """More decks than a batch has groups of blocks, from three cells to some
+    hundred thousand (one block of a group against all of it): each deck
+    converged and, as two solutions of a system A >= I that both meet 1e-10,
+    within 2e-10 ||u0|| of its own single-deck solve."""
+    sizes = [(700, 611), (3, 1), (121, 33), (512, 256), (64, 64), (31, 200), (901, 40), (240, 240), (5, 5), (333, 222),
+             (120, 120), (60, 61), (450, 300), (17, 19), (256, 129), (128, 500), (77, 78), (19, 350), (404, 404), (90, 30)]
+    texts = [random_deck(nx, 500 + k, ny=ny, nrect=3, steps=1, eps=1e-10) for k, (nx, ny) in enumerate(sizes)]
+    kw = dict(mode=TEA, criterion=1, precision=precision)
+    sets = [tl.Settings.from_text(t, **kw) for t in texts]
+    chunks = [tl.initialiseapp(s) for s in sets]
+    hist = tl.diffuse_batch(chunks, sets, steps=1)
+    for k, t in enumerate(texts):
+        s = tl.Settings.from_text(t, **kw)
+        c = tl.initialiseapp(s)
+        tl.haloupdate(c, s, 1, ["energy", "density"])
+        one = tl.CG.solve(c, s, s.dtinit / s.dx ** 2, s.dtinit / s.dy ** 2)
+        b = hist[0][k]
+        assert b.converged and 0 <= b.rel_residual < 1e-10, (sizes[k], b)
+        assert abs(b.iters - one.iters) <= max(1, 0.05 * one.iters), (sizes[k], b.iters, one.iters)
+        d = _interior(chunks[k].field("u")) - _interior(c.field("u"))
+        assert np.linalg.norm(d) <= 2e-10 * np.linalg.norm(_interior(c.field("u0"))), sizes[k]
+        c.close()
+        chunks[k].close()
