@@ -270,22 +270,21 @@ def run_e2e(tl, n, precision, steps, warmup, warm=0):
     return statistics.mean(times), 2 * X * Y * 8, X * Y * 8, times, results, phases
 
 
-# FP32 CG iteration: the direction step (read p, r, iw; write p': 16 B) and
-# the update step (read p', iw, x, r; write x, r: 24 B)
-IR_ITER_BYTES = 40
+# FP32 CG iteration: one pass (read r, s, iw; write r, s: 20 B); every second
+# one also reads the older r, p and x and writes p and x (40 B)
+IR_ITER_BYTES = 30
 KERNELS = {"fp64": ((0, "cg_w_step", W_STEP_BYTES + 8), (1, "cg_ur_step", UR_STEP_BYTES)),
-           "fp32_ir": ((8, "ir_dir_step", 16), (9, "ir_update_step", 24))}
+           "fp32_ir": ((8, "ir_pass", 20), (9, "ir_pass_px", 40))}
 # DRAM bytes (read + write) per interior cell of one launch, from ncu
 # captures at 4096^2; traffic grows with the cells, so a full launch moves
 # this times n^2.
-TRAFFIC_BYTES_PER_CELL = {"ir_dir_step": 247.4e6 / 4096 ** 2, "ir_update_step": 362.5e6 / 4096 ** 2,
-                          "cg_w_step": 923.7e6 / 4096 ** 2}
+TRAFFIC_BYTES_PER_CELL = {"cg_w_step": 923.7e6 / 4096 ** 2}
 
 
 def kernel_roofline(tl, chunk, kind, peak):
-    """Average duration of the two iteration kernels of one precision, each
-    launched 20 times back to back on the library's stream and timed with
-    CUDA events; algorithmic bytes = compulsory reads + writes per interior
+    """Average duration of the two iteration kernels (FP32: passes of the one
+    iteration kernel) of one precision, 20 back to back on the library's
+    stream, timed with CUDA events; algorithmic bytes = compulsory reads + writes per interior
     cell (the FP64 stencil step also reads the stored diagonal: 56 B)."""
     lib = chunk.lib
     cells = chunk.settings.xcells * chunk.settings.ycells
@@ -563,7 +562,7 @@ state 5 density=0.1 energy=0.1 geometry=rectangle xmin=5.0 xmax=10.0 ymin=7.0 ym
 """
 # algorithmic bytes per interior cell of each timed kernel
 CONFIG2_KERNELS = ((0, "cg_w_step", 48), (1, "cg_ur_step", 48), (4, "cheby_step", 72), (5, "ppcg_inner_sweep", 64),
-                   (6, "cheby32_step", 24), (7, "ppcg32_inner_sweep", 28))
+                   (6, "cheby32_step", 12), (7, "ppcg32_inner_sweep", 14))
 
 
 def config2_deck(n: int, solver: str) -> str:
@@ -819,10 +818,10 @@ KERNEL_TABLE = (
     (12, "ppcg_outer_update", 56, 3),  # u += a p, r -= a w (2), sd = r / theta (1 division)
     (10, "jacobi_sweep", 48, 10),      # u' = (u0 + sum k u_nbr) / (1 + sum k): 4 DFMA, 4 DADD, 1 DDIV, |u'-u| sum
     (11, "halo_u_p", None, 0),         # four face strips of two fields
-    (6, "cheby32_step", 24, None),
-    (7, "ppcg32_inner_sweep", 28, None),
-    (8, "ir_dir_step", 16, None),
-    (9, "ir_update_step", 24, None),
+    (6, "cheby32_step", 12, None),       # two steps in a pass of 24 B
+    (7, "ppcg32_inner_sweep", 14, None),  # two sweeps in a pass of 28 B
+    (8, "ir_pass", 20, None),
+    (9, "ir_pass_px", 40, None),
 )
 
 
@@ -849,7 +848,7 @@ def run_kernels(args):
     s.precision = 1
     tl.CG.solve(chunk, s, s.dtinit / s.dx ** 2, s.dtinit / s.dy ** 2)
     cells = n * n
-    for k, name in ((0, "cg_w_step"), (1, "cg_ur_step"), (8, "ir_dir_step"), (9, "ir_update_step")):
+    for k, name in ((0, "cg_w_step"), (1, "cg_ur_step"), (8, "ir_pass"), (9, "ir_pass_px")):
         w, r, blk = C.c_int(), C.c_int(), C.c_int()
         chunk.check(chunk.lib.tl_get_layout(chunk.ctx, k, C.byref(w), C.byref(r), C.byref(blk)))
         out.setdefault("layouts", {})[name] = {"warps": w.value, "rows": r.value, "blocks": blk.value}

@@ -181,9 +181,11 @@ int tl_get_cg_coefficients(tl_ctx *ctx, double *alpha, double *beta, int n);
 int tl_reduction_layout(tl_ctx *ctx, int *warps, int *rows, int *blocks);
 
 /* Launch layout (warps per block, rows per tile, persistent blocks) of one
- * fused iteration kernel (ids as in tl_bench_kernel): get the autotuned
- * choice, or override it (both for tuning studies; a set layout holds until
- * the context is destroyed). */
+ * iteration kernel (ids as in tl_bench_kernel; 8 and 9 are one kernel): get the
+ * choice made, or override it (both for tuning studies; a set layout holds
+ * until the context is destroyed).  The FP32 CG passes (8, 9) always run 16
+ * warps a block and at most one block per SM: of a layout set for them, rows
+ * and blocks take effect. */
 int tl_get_layout(tl_ctx *ctx, int kernel, int *warps, int *rows, int *blocks);
 int tl_set_layout(tl_ctx *ctx, int kernel, int warps, int rows, int blocks);
 
@@ -198,16 +200,18 @@ int tl_last_solve_ms(tl_ctx *ctx, double *ms);
 int tl_timer_start(tl_ctx *ctx);
 int tl_timer_stop(tl_ctx *ctx, double *ms);
 
-/* Times `reps` back-to-back launches of one fused iteration kernel (0: the CG
- * p-update + stencil + p.w step, 1: the u/r update + r.r step, 4: the
- * Chebyshev step, 5: a PPCG inner sweep, 6: the FP32 Chebyshev step, 7: an
- * FP32 PPCG inner sweep, 8: the FP32 CG direction step p' = beta p + r with
- * p'.A p', 9: the FP32 CG update step with A p' recomputed; 8 and 9 are the
- * FP32 CG iteration; 10: a Jacobi sweep, 11: the depth-1 halo update of u and
- * p, 12: PPCG's outer u/r update; 2 and 3, an earlier FP32 pair, are retired
- * and return TL_ERR_ARG) on the current fields; for roofline measurements.  The launches overwrite
- * solver work fields (p, w, r, u, sd, their second buffers and the FP32
- * copies): call it after the solves whose fields matter. */
+/* Times `reps` back-to-back launches (6 to 9: passes of one launch) of one
+ * fused iteration kernel (0: the FP64 CG p-update + stencil + p.w step of the
+ * exact arithmetic's two-kernel form, fused, 1: its u/r update + r.r step, 4: the
+ * Chebyshev step, 5: a PPCG inner sweep, 6: the FP32 Chebyshev step, 7: an FP32
+ * PPCG inner sweep (6 and 7 run two in a pass: half a pass's time), 8: a pass
+ * of the FP32 CG iteration that leaves p and x, 9: one that forms two steps' p
+ * and x (the passes alternate); 10: a Jacobi sweep, 11: the depth-1 halo update
+ * of u and p, 12: PPCG's outer u/r update; 2 and 3, an earlier FP32 pair, are
+ * retired and return TL_ERR_ARG) on the current fields; for roofline
+ * measurements.  The launches overwrite solver work fields (p, w, r, u, sd,
+ * their second buffers and the FP32 copies): call it after the solves whose
+ * fields matter. */
 int tl_bench_kernel(tl_ctx *ctx, int kernel, int reps, double *ms_per_launch);
 
 /* Many independent decks (tealeaf-mode contexts of any sizes on the current

@@ -465,35 +465,45 @@ static Walk *layout_of(tl_ctx *ctx, int kernel) {
   switch (kernel) {
     case 0: return &ctx->walk_w64;
     case 1: return &ctx->walk_ur64;
-    case 8:
-    case 9: return tl_ir_walk(ctx, kernel);
     default: return nullptr;
   }
 }
 
+static bool fp32_pass(tl_ctx *ctx, int kernel) {
+  return ctx->cfg.mode == TL_MODE_TEALEAF && (kernel == 8 || kernel == 9);
+}
+
 extern "C" int tl_get_layout(tl_ctx *ctx, int kernel, int *warps, int *rows, int *blocks) {
   if (!ctx) return TL_ERR_ARG;
-  Walk *w = layout_of(ctx, kernel);
-  if (!w) {
+  int w = 0, r = 0, b = 0;
+  if (fp32_pass(ctx, kernel)) {
+    const int rc = tl_ir_get_layout(ctx, &w, &r, &b);
+    if (rc) return rc;
+  } else if (const Walk *wk = layout_of(ctx, kernel)) {
+    w = wk->warps;
+    r = wk->rows;
+    b = wk->blocks;
+  } else {
     tl_set_error(ctx, "no tuned layout for kernel %d in this mode", kernel);
     return TL_ERR_ARG;
   }
-  if (warps) *warps = w->warps;
-  if (rows) *rows = w->rows;
-  if (blocks) *blocks = w->blocks;
+  if (warps) *warps = w;
+  if (rows) *rows = r;
+  if (blocks) *blocks = b;
   return TL_OK;
 }
 
 extern "C" int tl_set_layout(tl_ctx *ctx, int kernel, int warps, int rows, int blocks) {
   if (!ctx) return TL_ERR_ARG;
   Walk *w = layout_of(ctx, kernel);
-  if (!w || (warps != 4 && warps != 8) || rows < 1 || blocks < 1 || blocks > ctx->max_blocks) {
+  const bool fp32 = fp32_pass(ctx, kernel);
+  if ((!w && !fp32) || (warps != 4 && warps != 8) || rows < 1 || blocks < 1 || blocks > ctx->max_blocks) {
     tl_set_error(ctx, "invalid layout for kernel %d: %d warps, %d rows, %d blocks (at most %d)", kernel, warps, rows,
                  blocks, ctx->max_blocks);
     return TL_ERR_ARG;
   }
-  const int cols = kernel >= 2 ? 128 : 64;
-  const int TW = cols * warps;
+  if (fp32) return tl_ir_set_layout(ctx, warps, rows, blocks);
+  const int TW = 64 * warps;
   Walk n;
   n.warps = warps;
   n.rows = rows;
@@ -501,9 +511,6 @@ extern "C" int tl_set_layout(tl_ctx *ctx, int kernel, int warps, int rows, int b
   n.tiles = n.ntx * ((ctx->g.ny + rows - 1) / rows);
   n.blocks = blocks < n.tiles ? blocks : n.tiles;
   *w = n;
-  // graphs hold the old launch configuration
-  tl_release_graphs(ctx);
-  tl_release_ir_graphs(ctx);
   return TL_OK;
 }
 

@@ -211,10 +211,107 @@ __device__ __forceinline__ void ir_pass(Grid grid, const IrCg &A, const PassArgs
 
 // ---- the solve ---------------------------------------------------------------
 
+// u read past L1: the refinement before this launch's last grid barrier wrote it.
+struct SrcU {
+  const double *f;
+  struct Raw {
+    double2 v;
+    double ev;
+  };
+  __device__ __forceinline__ void load(Raw &o, size_t c, long long ec) const {
+    o.v = __ldcg(reinterpret_cast<const double2 *>(f + c));
+    if (ec >= 0) o.ev = __ldcg(f + ec);
+  }
+  __device__ __forceinline__ double2 val(const Raw &o) const { return o.v; }
+  __device__ __forceinline__ double val_edge(const Raw &o) const { return o.ev; }
+};
+
+// The true residual r = u0 - A u in FP64, its FP32 copy in `r32` and r.r in
+// `rr` (on entry the r.r of the residual before, for the sum's scale).  In
+// difference form: the couplings multiply differences of neighbouring cells, so
+// u's own rounding is not scaled by them.
+__device__ __forceinline__ bool ir_residual(Grid grid, const Fields &F, const Geom &g, const G32 &g32, const Tiling &T,
+                                            GridSums *sums, SumShared &S, float *r32, unsigned &target, unsigned &set,
+                                            unsigned &handed, double &rr) {
+  __shared__ double tot;
+  const int lane = threadIdx.x & 31;
+  SrcU src;
+  src.f = F.u;
+  const int scale = fixed_scale(rr);
+  Fixed share = 0;
+  TileWalk walk(grid, T, g.ny, false, &F.sc->bar.next_tile, handed);
+  handed += walk.requests();
+  while (walk.valid()) {
+    int strip, j0, j1;
+    walk.place(strip, j0, j1);
+    const unsigned asked = walk.ask();
+    const int i0 = strip * 64 + 2 * lane;
+    double acc = 0.0;
+    march<false>(g, F.kx, F.ky, nullptr, src, i0, j0, j1,
+                 [&](int j, const Nbr &c0, const Nbr &c1, bool has1, double2) {
+                   const size_t c = g.at(i0, j), c32 = g32.at(i0, j);
+                   auto resid = [](const Nbr &n, double u0) {
+                     double t = u0 - n.c;
+                     t = fma(n.kx1, n.e - n.c, t);
+                     t = fma(n.kx0, n.w - n.c, t);
+                     t = fma(n.ky1, n.n - n.c, t);
+                     return fma(n.ky0, n.s - n.c, t);
+                   };
+                   const double2 b = ld2(F.u0 + c);
+                   const double t0 = resid(c0, b.x);
+                   acc = fma(t0, t0, acc);
+                   if (has1) {
+                     const double t1 = resid(c1, b.y);
+                     acc = fma(t1, t1, acc);
+                     st2(F.r + c, make_double2(t0, t1));
+                     *reinterpret_cast<float2 *>(r32 + c32) = make_float2((float)t0, (float)t1);
+                   } else {
+                     F.r[c] = t0;
+                     r32[c32] = (float)t0;
+                   }
+                 });
+    share += to_fixed(acc, scale);
+    walk.take(asked);
+  }
+  if (!grid_sum1(grid, S, &F.sc->bar, sums, warp_fixed(share), scale, target, set, [&](double a) {
+        if (lane == 0) tot = a;
+      }))
+    return false;
+  rr = tot;
+  return true;
+}
+
+// Up to four FP32 numbers added to, or stored as, the FP64 cells at `c`.
+__device__ __forceinline__ void add_f32(double *c, float4 v, int cells) {
+  if (cells >= 4) {
+    const double2 a = __ldcg(reinterpret_cast<const double2 *>(c)), b = __ldcg(reinterpret_cast<const double2 *>(c + 2));
+    st2(c, make_double2(a.x + (double)v.x, a.y + (double)v.y));
+    st2(c + 2, make_double2(b.x + (double)v.z, b.y + (double)v.w));
+  } else {
+    for (int m = 0; m < cells; ++m) c[m] = __ldcg(c + m) + (double)comp(v, m);
+  }
+}
+// An FP32 field's interior in FP64.
+__device__ __forceinline__ void export_f32(Grid grid, const Geom &g, const G32 &g32, const float *src, double *dst) {
+  const int nx = g.nx, lane = threadIdx.x & 31, chunks = (nx + 127) / 128;
+  const long long n = (long long)chunks * g.ny;
+  for (long long w = grid.id * PERSIST_WARPS + (threadIdx.x >> 5); w < n; w += grid.nb * PERSIST_WARPS) {
+    const int j = (int)(w / chunks), i0 = (int)(w % chunks) * 128 + 4 * lane;
+    if (i0 >= nx) continue;
+    const float4 v = __ldcg(reinterpret_cast<const float4 *>(src + g32.at(i0, j)));
+    double *p = dst + g.at(i0, j);
+    if (i0 + 3 < nx) {
+      st2(p, make_double2((double)v.x, (double)v.y));
+      st2(p + 2, make_double2((double)v.z, (double)v.w));
+    } else {
+      for (int m = 0; m < nx - i0; ++m) p[m] = (double)comp(v, m);
+    }
+  }
+}
+
 // Scalars of one block, the same on every block.
 struct Shared {
   SumShared sum;
-  double tot;
   double alpha, beta, gamma, inv_gamma, sigma;
   float alpha_f, beta_f;  // of the next step
   int done, sw;
@@ -239,21 +336,6 @@ __device__ __forceinline__ void next_scalars(Shared &S, double gamma, double bet
     S.beta_f = f;
   }
 }
-
-// u read past L1: the refinement before this launch's last grid barrier wrote it.
-struct SrcU {
-  const double *f;
-  struct Raw {
-    double2 v;
-    double ev;
-  };
-  __device__ __forceinline__ void load(Raw &o, size_t c, long long ec) const {
-    o.v = __ldcg(reinterpret_cast<const double2 *>(f + c));
-    if (ec >= 0) o.ev = __ldcg(f + ec);
-  }
-  __device__ __forceinline__ double2 val(const Raw &o) const { return o.v; }
-  __device__ __forceinline__ double val_edge(const Raw &o) const { return o.ev; }
-};
 
 // The solve of one deck by the blocks of `grid`; false when a wait gave up.
 __device__ __forceinline__ bool ir_solve(Grid grid, const IrCg &A, Shared &S, unsigned ring) {
@@ -376,90 +458,20 @@ __device__ __forceinline__ bool ir_solve(Grid grid, const IrCg &A, Shared &S, un
         xo = f4(fmaf(alpha0, p1.x, xo.x), fmaf(alpha0, p1.y, xo.y), fmaf(alpha0, p1.z, xo.z), fmaf(alpha0, p1.w, xo.w));
         st4(A.p + c, p1);
       }
-      const float xs[4] = {xo.x, xo.y, xo.z, xo.w};
-      if (i0 + 3 < nx) {
-        double2 a = __ldcg(reinterpret_cast<const double2 *>(A.F.u + cu));
-        double2 b = __ldcg(reinterpret_cast<const double2 *>(A.F.u + cu + 2));
-        st2(A.F.u + cu, make_double2(a.x + (double)xs[0], a.y + (double)xs[1]));
-        st2(A.F.u + cu + 2, make_double2(b.x + (double)xs[2], b.y + (double)xs[3]));
-      } else {
-        for (int m = 0; m < nx - i0; ++m) A.F.u[cu + m] = __ldcg(A.F.u + cu + m) + (double)xs[m];
-      }
+      add_f32(A.F.u + cu, xo, nx - i0);
     }
     pv = pv || pend;
     pend = false;
     xv = false;
     if (!grid_barrier(grid, bar, target)) return false;
-    // the true residual r = u0 - A u in FP64, in difference form: the
-    // couplings multiply differences of neighbouring cells, so u's own
-    // rounding is not scaled by them
-    SrcU src;
-    src.f = A.F.u;
     rc = A.r[0];
     rn = A.r[1];
-    // the refinement's residual is some 100 times smaller than the one it refines
-    const int scale = fixed_scale(rr);
-    Fixed share = 0;
-    TileWalk walk(grid, A.t64, ny, false, &A.F.sc->bar.next_tile, handed);
-    handed += walk.requests();
-    while (walk.valid()) {
-      int strip, j0, j1;
-      walk.place(strip, j0, j1);
-      const unsigned asked = walk.ask();
-      const int i0 = strip * 64 + 2 * lane;
-      double acc = 0.0;
-      march<false>(A.g, A.F.kx, A.F.ky, nullptr, src, i0, j0, j1,
-                   [&](int j, const Nbr &c0, const Nbr &c1, bool has1, double2) {
-                     const size_t c = A.g.at(i0, j), c32 = A.g32.at(i0, j);
-                     auto resid = [](const Nbr &n, double u0) {
-                       double t = u0 - n.c;
-                       t = fma(n.kx1, n.e - n.c, t);
-                       t = fma(n.kx0, n.w - n.c, t);
-                       t = fma(n.ky1, n.n - n.c, t);
-                       return fma(n.ky0, n.s - n.c, t);
-                     };
-                     const double2 b = ld2(A.F.u0 + c);
-                     const double t0 = resid(c0, b.x);
-                     acc = fma(t0, t0, acc);
-                     if (has1) {
-                       const double t1 = resid(c1, b.y);
-                       acc = fma(t1, t1, acc);
-                       st2(A.F.r + c, make_double2(t0, t1));
-                       *reinterpret_cast<float2 *>(rc + c32) = make_float2((float)t0, (float)t1);
-                     } else {
-                       A.F.r[c] = t0;
-                       rc[c32] = (float)t0;
-                     }
-                   });
-      share += to_fixed(acc, scale);
-      walk.take(asked);
-    }
-    if (!grid_sum1(grid, S.sum, bar, A.sums, warp_fixed(share), scale, target, set, [&](double a) {
-          if (lane == 0) S.tot = a;
-        }))
-      return false;
-    rr = S.tot;
+    if (!ir_residual(grid, A.F, A.g, A.g32, A.t64, A.sums, S.sum, rc, target, set, handed, rr)) return false;
     rel = bb > 0 ? sqrt(rr / bb) : sqrt(rr);
     ++nref;
   }
   // the last search direction in FP64
-  if (pv) {
-    const int chunks = (nx + 127) / 128;
-    const long long n = (long long)chunks * ny;
-    for (long long w = me; w < n; w += warps) {
-      const int j = (int)(w / chunks), i0 = (int)(w % chunks) * 128 + 4 * lane;
-      if (i0 >= nx) continue;
-      const float4 v = __ldcg(reinterpret_cast<const float4 *>(A.p + A.g32.at(i0, j)));
-      const float vs[4] = {v.x, v.y, v.z, v.w};
-      double *p = A.F.p + A.g.at(i0, j);
-      if (i0 + 3 < nx) {
-        st2(p, make_double2((double)vs[0], (double)vs[1]));
-        st2(p + 2, make_double2((double)vs[2], (double)vs[3]));
-      } else {
-        for (int m = 0; m < nx - i0; ++m) p[m] = (double)vs[m];
-      }
-    }
-  }
+  if (pv) export_f32(grid, A.g, A.g32, A.p, A.F.p);
   if (lead) {  // none of these is read above once another block may still be at its start
     sc->red[0] = rr;
     sc->red[1] = rel;
@@ -495,6 +507,14 @@ inline void ir_cg_args(IrCg &A, tl_ctx *ctx, int blocks) {
   // cycles and issue slots of a row and a tile, from the kernel's own counters
   const TileCost pass{2.0, 300.0, 1500.0, 200.0, 400.0, 32, 24, 8}, resid{1.0, 1200.0, 1500.0, 1100.0, 200.0, 0, 48, 4};
   A.t = make_tiling(ctx->g.nx, ctx->g.ny, STRIP, pass, blocks, PERSIST_WARPS);
+  if (ir->set_rows) {  // tl_set_layout: equal shares of bands of these rows
+    A.t.rows = ir->set_rows < ctx->g.ny ? ir->set_rows : ctx->g.ny;
+    A.t.split = ctx->g.ny;
+    A.t.tiles = A.t.tiles1 = A.t.ntx * ((ctx->g.ny + A.t.rows - 1) / A.t.rows);
+    A.t.blocks = ir->set_blocks < blocks ? ir->set_blocks : blocks;
+    A.t.warps = A.t.blocks * PERSIST_WARPS;
+    A.t.handed = false;
+  }
   A.t64 = make_tiling_on(A.t, ctx->g.nx, ctx->g.ny, 64, resid, PERSIST_WARPS);
 }
 

@@ -326,7 +326,7 @@ int tl_cheby_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_r
     // the rest of the iteration in FP32 inside FP64 refinement
     int nref = 0;
     double rel = -1.0;
-    if ((rc = tl_cheby32_run(ctx, prm, &nref, &rel))) return rc;
+    if ((rc = tl_cheby32_run(ctx, &nref, &rel))) return rc;
     const int ex = TL_EX_U;
     if ((rc = tl_halo_update(ctx, 1, &ex, 1, 1))) return rc;
     if ((rc = tl_read_scalars(ctx))) return rc;

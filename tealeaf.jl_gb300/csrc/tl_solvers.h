@@ -63,7 +63,6 @@ void tl_launch_w64_for_tuning(tl_ctx *ctx, const tl::Walk &wk);
 void tl_launch_ur64_for_tuning(tl_ctx *ctx, const tl::Walk &wk);
 void tl_release_graphs(tl_ctx *ctx);
 void tl_release_ir(tl_ctx *ctx);
-void tl_release_ir_graphs(tl_ctx *ctx);
 
 // shared solver pieces (tl_solve.cu)
 int tl_set_loop_params(tl_ctx *ctx, const tl_params *prm, int switch_rule, int stale_rro);
@@ -90,12 +89,13 @@ int tl_loop64_run(tl_ctx *ctx, int which, int ninner, double *ms);
 // TL_OK, or the error of a persistent kernel whose grid barrier gave up (after tl_read_scalars)
 int tl_persist_check(tl_ctx *ctx);
 // Chebyshev after its first step, in FP32 inside FP64 refinement (tl_ir.cu)
-int tl_cheby32_run(tl_ctx *ctx, const tl_params *prm, int *refinements, double *rel_out);
+int tl_cheby32_run(tl_ctx *ctx, int *refinements, double *rel_out);
 int tl_ir_presteps(tl_ctx *ctx, double rx, double ry, const tl_params *prm, int *refinements, double *rr_out,
                    double *rel_out, int *switched);
 int tl_ppcg32_run(tl_ctx *ctx, const tl_params *prm, double rr, int *refinements, double *rel_out);
 int tl_ir_bench_kernel(tl_ctx *ctx, int kernel, int reps, double *ms_per_launch);
-tl::Walk *tl_ir_walk(tl_ctx *ctx, int kernel);  // the FP32 kernels' layouts (kernel 2, 3)
+int tl_ir_get_layout(tl_ctx *ctx, int *warps, int *rows, int *blocks);  // the FP32 CG passes'
+int tl_ir_set_layout(tl_ctx *ctx, int warps, int rows, int blocks);
 
 // warm start (tl_warm.cu): after init + copyu!, maybe replace the plain start
 // by the projected prediction; always records u^n for the next step.

@@ -146,3 +146,25 @@ def test_batch_groups(tl, built_lib, precision):
         assert np.linalg.norm(d) <= 2e-10 * np.linalg.norm(_interior(c.field("u0"))), sizes[k]
         c.close()
         chunks[k].close()
+
+
+@pytest.mark.parametrize("solver,inner", [("cheby", 10), ("ppcg", 1), ("ppcg", 4), ("ppcg", 5)])
+@pytest.mark.parametrize("nx,ny,hd", [(61, 120, 1), (119, 64, 3), (121, 200, 2), (513, 300, 2), (1201, 1000, 2)])
+def test_fp32_sweep_tilings(tl, built_lib, solver, inner, nx, ny, hd):
+    """FP32 Chebyshev and PPCG (an odd and an even number of sweeps after the
+    first, or none) at the edges of strips and bands: every step meets 1e-10 on
+    the true residual, so u is within 2e-10 ||u0|| of exact FP64 CG's (4e-10 at
+    the second step, see above), and two runs are the same bits."""
+    text = random_deck(nx, 84, ny=ny, nrect=5, steps=2, eps=1e-10, solver=solver, halo_depth=hd, presteps=40,
+                       ppcg_inner_steps=inner)
+    c, _, _, _ = gpu_run(tl, text.replace(f"use_{solver}", "use_cg"), TEA, exact=True, criterion=1)
+    v, u0 = _interior(c.field("u"), hd), _interior(c.field("u0"), hd)
+    c.close()
+    u = []
+    for _ in range(2):
+        c, res, _, _ = gpu_run(tl, text, TEA, criterion=1, precision=1)
+        assert all(r.converged and 0 <= r.rel_residual < 1e-10 for r in res), res
+        u.append(_interior(c.field("u"), hd))
+        c.close()
+    assert np.linalg.norm(u[0] - v) <= 4e-10 * np.linalg.norm(u0)
+    np.testing.assert_array_equal(u[0], u[1])
