@@ -968,98 +968,185 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB) k_conv3x3_ws(ConvArgs
 
 // Weight and bias gradients: dW[co][tap][ci] = sum_p dz[p][co] x[p + off(tap)][ci]
 // as a GEMM with M = COUT, N = 9*CIN, K = pixels; db[co] = sum_p dz[p][co].
-// Block b walks row segments b, b + G, ...; A (dz, stored [p][co]) and B (the
-// shifted input, stored [p][ci]) fragments come from ldmatrix.trans.  Each
-// block writes its partial sums; k_sum_partials adds them in block order.
+// A (dz, stored [p][co]) and B (the shifted input, stored [p][ci]) fragments
+// come from ldmatrix.trans.  Each block writes its partial sums;
+// k_sum_partials adds them in block order.
+//
+// A block takes an equal share of the rows of 64-pixel columns of the images and
+// marches down them two rows a step: of x only two new rows arrive (the four
+// that a step needs stay in a ring of eight), copied asynchronously two steps
+// ahead, one barrier a step.  Warp (dy, ks) of the twelve does the three taps of
+// input row y + dy - 1 over the ks-th 16 pixels, so the four ks are summed once
+// at the end.  The earlier form reloaded three rows for each row behind two
+// barriers, with nothing in flight, and summed the bias in a chain of 64 loads.
+//
+// What bounds it: the warp-level tensor path (24 m16n8k16 a warp and row, some 14
+// clocks each on a quarter of an SM) and the latency of its operands.  With the
+// sum below, 32 -> 32 channels: 109 to 41 us on 32 images of 128 x 128, 519 to
+// 125 at 256 x 256, 30 to 14 on 4 of 64 x 64 (one row a step: 49, 139 and 18.5).
+constexpr int DW_WARPS = 12, DW_ROWS = 2, DW_RING = 8;
+
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(128) k_conv_dw(const bf16 *__restrict__ x, const bf16 *__restrict__ dz,
-                                                 float *__restrict__ part, int N, int H, int W) {
+constexpr int dw_smem_bytes() {
+  constexpr int ring = 2 * DW_RING * ((TP + 2) * (CIN + 8) + TP * (COUT + 8));
+  constexpr int sums = 4 * 4 * (COUT * 9 * CIN + COUT);
+  return ring > sums ? ring : sums;
+}
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(32 * DW_WARPS, 1) k_conv_dw(const bf16 *__restrict__ x, const bf16 *__restrict__ dz,
+                                                              float *__restrict__ part, int N, int H, int W) {
   constexpr int PS = CIN + 8, ZS = COUT + 8;
-  constexpr int MT = COUT / 16;
-  constexpr int NTT = 9 * CIN / 8;
-  constexpr int NPW = (NTT + 3) / 4;
+  constexpr int MT = COUT / 16, NP = CIN / 16;  // m-tiles; pairs of n-tiles a tap
   constexpr int NW = COUT * 9 * CIN + COUT;
   constexpr int VX = CIN / 8, VZ = COUT / 8;
-  __shared__ __align__(16) bf16 sx[3][TP + 2][PS];
-  __shared__ __align__(16) bf16 sz[TP][ZS];
+  extern __shared__ __align__(16) unsigned char dw_smem[];
+  bf16 *sx = reinterpret_cast<bf16 *>(dw_smem);  // [DW_RING][TP + 2][PS]
+  bf16 *sz = sx + DW_RING * (TP + 2) * PS;       // [DW_RING][TP][ZS]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int dy = warp % 3, ks = warp / 3;
   const int g = lane >> 2, t = lane & 3;
   const size_t plane = (size_t)H * W;
   const int segs = (W + TP - 1) / TP;
-  const long long tiles = (long long)N * H * segs;
-  float acc[MT][NPW][4];
+  const long long rows = (long long)N * segs * H;
+  const long long r0 = rows * blockIdx.x / gridDim.x, r1 = rows * (blockIdx.x + 1) / gridDim.x;
+  float acc[MT][3 * NP][2][4];
+  float bias[MT][2];
 #pragma unroll
-  for (int m = 0; m < MT; ++m)
+  for (int m = 0; m < MT; ++m) {
+    bias[m][0] = bias[m][1] = 0.f;
 #pragma unroll
-    for (int q = 0; q < NPW; ++q) acc[m][q][0] = acc[m][q][1] = acc[m][q][2] = acc[m][q][3] = 0.f;
-  float bacc = 0.f;
-  for (long long tt = blockIdx.x; tt < tiles; tt += gridDim.x) {
-    const int seg = (int)(tt % segs);
-    const long long rr = tt / segs;
-    const int y = (int)(rr % H), img = (int)(rr / H), x0 = seg * TP;
-    __syncthreads();
-    for (int v = tid; v < 3 * (TP + 2) * VX; v += 128) {
-      const int c8 = v % VX, col = (v / VX) % (TP + 2), r = v / (VX * (TP + 2));
-      const int yy = y + r - 1, xx = x0 + col - 1;
-      uint4 val = make_uint4(0, 0, 0, 0);
-      if (yy >= 0 && yy < H && xx >= 0 && xx < W)
-        val = *reinterpret_cast<const uint4 *>(x + ((size_t)img * plane + (size_t)yy * W + xx) * CIN + c8 * 8);
-      *reinterpret_cast<uint4 *>(&sx[r][col][c8 * 8]) = val;
-    }
-    for (int v = tid; v < TP * VZ; v += 128) {
-      const int c8 = v % VZ, p = v / VZ, xx = x0 + p;
-      uint4 val = make_uint4(0, 0, 0, 0);
-      if (xx < W) val = *reinterpret_cast<const uint4 *>(dz + ((size_t)img * plane + (size_t)y * W + xx) * COUT + c8 * 8);
-      *reinterpret_cast<uint4 *>(&sz[p][c8 * 8]) = val;
-    }
-    __syncthreads();
-    if (tid < COUT)
-      for (int p = 0; p < TP; ++p) bacc += __bfloat162float(sz[p][tid]);
+    for (int q = 0; q < 3 * NP; ++q)
 #pragma unroll
-    for (int ks = 0; ks < TP / 16; ++ks) {
-      const int p0 = ks * 16;
-      uint32_t af[MT][4];
-#pragma unroll
-      for (int m = 0; m < MT; ++m) {
-        const int j = lane >> 3, r = lane & 7;
-        ldsm_x4_trans(af[m], &sz[p0 + (j >> 1) * 8 + r][m * 16 + (j & 1) * 8]);
+      for (int h = 0; h < 2; ++h) acc[m][q][h][0] = acc[m][q][h][1] = acc[m][q][h][2] = acc[m][q][h][3] = 0.f;
+  }
+  for (long long rr = r0; rr < r1;) {
+    const int ya = (int)(rr % H);
+    const long long col = rr / H;
+    const int img = (int)(col / segs), x0 = (int)(col % segs) * TP;
+    const int yb = (int)(ya + (r1 - rr) < H ? ya + (r1 - rr) : H);
+    const bf16 *xi = x + (size_t)img * plane * CIN, *zi = dz + (size_t)img * plane * COUT;
+    // the copies of x rows yy .. yy + n - 1 and of dz rows; a row's ring slot is its distance from ya
+    auto copy_x = [&](int yy, int n) {
+      for (int v = tid; v < n * (TP + 2) * VX; v += 32 * DW_WARPS) {
+        const int c8 = v % VX, q = v / VX, row = q / (TP + 2), p = q - row * (TP + 2);
+        const int y = yy + row, xx = x0 + p - 1;
+        const bool in = y >= 0 && y < H && xx >= 0 && xx < W;
+        cp_async16(sx + (((y - ya) & (DW_RING - 1)) * (TP + 2) + p) * PS + c8 * 8,
+                   in ? xi + ((size_t)y * W + xx) * CIN + c8 * 8 : x, in ? 16 : 0);
       }
+    };
+    auto copy_z = [&](int yy, int n) {
+      for (int v = tid; v < n * TP * VZ; v += 32 * DW_WARPS) {
+        const int c8 = v % VZ, q = v / VZ, row = q / TP, p = q - row * TP;
+        const int y = yy + row, xx = x0 + p;
+        const bool in = y < yb && xx < W;
+        cp_async16(sz + (((y - ya) & (DW_RING - 1)) * TP + p) * ZS + c8 * 8,
+                   in ? zi + ((size_t)y * W + xx) * COUT + c8 * 8 : dz, in ? 16 : 0);
+      }
+    };
+    __syncthreads();  // the ring's last readers
+    copy_x(ya - 1, 2);
 #pragma unroll
-      for (int q = 0; q < NPW; ++q) {
-        const int nt = warp + 4 * q;
-        if (nt < NTT) {
-          const int n0 = nt * 8, tap = n0 / CIN, ci0 = n0 % CIN, dy = tap / 3, dx = tap % 3;
-          const int j = (lane >> 3) & 1, r = lane & 7;
-          uint32_t bfr[2];
-          ldsm_x2_trans(bfr, &sx[dy][p0 + j * 8 + r + dx][ci0]);
+    for (int s = 0; s < 2 * DW_ROWS; s += DW_ROWS) {
+      if (ya + s < yb) {
+        copy_x(ya + s + 1, DW_ROWS);
+        copy_z(ya + s, DW_ROWS);
+      }
+      cp_async_commit();
+    }
+    for (int y = ya; y < yb; y += DW_ROWS) {
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+      __syncthreads();
+      if (y + 2 * DW_ROWS < yb) {
+        copy_x(y + 2 * DW_ROWS + 1, DW_ROWS);
+        copy_z(y + 2 * DW_ROWS, DW_ROWS);
+      }
+      cp_async_commit();
 #pragma unroll
-          for (int m = 0; m < MT; ++m) mma_bf16(acc[m][q], af[m], bfr);
+      for (int r = 0; r < DW_ROWS; ++r) {
+        if (y + r >= yb) break;
+        const bf16 *zr = sz + (((y + r - ya) & (DW_RING - 1)) * TP + ks * 16) * ZS;
+        const bf16 *xr = sx + (((y + r + dy - 1 - ya) & (DW_RING - 1)) * (TP + 2) + ks * 16) * PS;
+        uint32_t af[MT][4];
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+          ldsm_x4_trans(af[m], zr + ((lane >> 4) * 8 + (lane & 7)) * ZS + m * 16 + ((lane >> 3) & 1) * 8);
+        if (dy == 1) {
+#pragma unroll
+          for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {  // fragments 0, 2: channel g; 1, 3: channel g + 8
+              const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&af[m][h]));
+              bias[m][h & 1] += f.x + f.y;
+            }
         }
+#pragma unroll
+        for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+          for (int c = 0; c < NP; ++c) {
+            uint32_t bfr[4];
+            ldsm_x4_trans(bfr, xr + (((lane >> 3) & 1) * 8 + (lane & 7) + dx) * PS + c * 16 + (lane >> 4) * 8);
+            const uint32_t b0[2] = {bfr[0], bfr[1]}, b1[2] = {bfr[2], bfr[3]};
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+              mma_bf16(acc[m][dx * NP + c][0], af[m], b0);
+              mma_bf16(acc[m][dx * NP + c][1], af[m], b1);
+            }
+          }
+      }
+    }
+    rr += yb - ya;
+  }
+  // each ks into its own quarter of the shared memory, then their sums are the block's partial
+  cp_async_wait_all();
+  __syncthreads();
+  float *sums = reinterpret_cast<float *>(dw_smem), *sum = sums + ks * NW;
+#pragma unroll
+  for (int m = 0; m < MT; ++m) {
+#pragma unroll
+    for (int q = 0; q < 3 * NP; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int nn = (dy * 3 + q / NP) * CIN + (q % NP) * 16 + h * 8 + 2 * t;
+        const float *v = acc[m][q][h];
+        float *lo = sum + (m * 16 + g) * 9 * CIN + nn;
+        *reinterpret_cast<float2 *>(lo) = make_float2(v[0], v[1]);
+        *reinterpret_cast<float2 *>(lo + 8 * 9 * CIN) = make_float2(v[2], v[3]);
+      }
+    if (dy == 1) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float v = bias[m][h];
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        if (t == 0) sum[COUT * 9 * CIN + m * 16 + h * 8 + g] = v;
       }
     }
   }
+  __syncthreads();
   float *out = part + (size_t)blockIdx.x * NW;
-#pragma unroll
-  for (int m = 0; m < MT; ++m)
-#pragma unroll
-    for (int q = 0; q < NPW; ++q) {
-      const int nt = warp + 4 * q;
-      if (nt < NTT) {
-        const int nn = nt * 8 + 2 * t, ca = m * 16 + g, cb = ca + 8;
-        out[(size_t)ca * 9 * CIN + nn] = acc[m][q][0];
-        out[(size_t)ca * 9 * CIN + nn + 1] = acc[m][q][1];
-        out[(size_t)cb * 9 * CIN + nn] = acc[m][q][2];
-        out[(size_t)cb * 9 * CIN + nn + 1] = acc[m][q][3];
-      }
-    }
-  if (tid < COUT) out[COUT * 9 * CIN + tid] = bacc;
+#pragma unroll 4
+  for (int k = tid; k < NW; k += 32 * DW_WARPS)
+    out[k] = ((sums[k] + sums[NW + k]) + sums[2 * NW + k]) + sums[3 * NW + k];
 }
 
-__global__ void k_sum_partials(const float *part, int nparts, int n, float *out) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int b = 0; b < nparts; ++b) s += part[(size_t)b * n + k];
-    out[k] = s;
+// out[k] = the sum of part[.][k]: eight threads a value take an eighth of the
+// blocks each, in order, and their sums are added in order.
+__global__ void __launch_bounds__(256) k_sum_partials(const float *part, int nparts, int n, float *out) {
+  __shared__ float s[8][32];
+  const int c = threadIdx.x & 31, e = threadIdx.x >> 5, k = blockIdx.x * 32 + c;
+  const int b0 = nparts * e / 8, b1 = nparts * (e + 1) / 8;
+  float v = 0.f;
+  if (k < n) {
+#pragma unroll 8
+    for (int b = b0; b < b1; ++b) v += part[(size_t)b * n + k];
+  }
+  s[e][c] = v;
+  __syncthreads();
+  if (e == 0 && k < n) {
+    for (int m = 1; m < 8; ++m) v += s[m][c];
+    out[k] = v;
   }
 }
 
@@ -1395,6 +1482,13 @@ void launch_conv(const ConvArgs &a, int mode, cudaStream_t st) {
   else launch_conv_mode<CIN, COUT, 2>(a, st);
 }
 
+template <int CIN, int COUT>
+void launch_dw(const bf16 *x, const bf16 *dz, float *part, int blocks, int N, int H, int W, cudaStream_t st) {
+  constexpr int smem = dw_smem_bytes<CIN, COUT>();
+  cudaFuncSetAttribute(k_conv_dw<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  k_conv_dw<CIN, COUT><<<blocks, 32 * DW_WARPS, smem, st>>>(x, dz, part, N, H, W);
+}
+
 }  // namespace
 
 int tl_conv_forward(const void *x, const void *w, const float *bias, const void *gz, void *z, void *out, float *out32,
@@ -1452,11 +1546,19 @@ extern "C" int tl_conv3x3_weight_grad(const void *x, const void *dz, float *part
   auto X = static_cast<const bf16 *>(x);
   auto Z = static_cast<const bf16 *>(dz);
   const int nw = cout * 9 * cin + cout;
-  if (cin == 16 && cout == 32) k_conv_dw<16, 32><<<nparts, 128, 0, st>>>(X, Z, partials, N, H, W);
-  else if (cin == 32 && cout == 32) k_conv_dw<32, 32><<<nparts, 128, 0, st>>>(X, Z, partials, N, H, W);
-  else if (cin == 32 && cout == 16) k_conv_dw<32, 16><<<nparts, 128, 0, st>>>(X, Z, partials, N, H, W);
-  else return TL_ERR_ARG;
-  k_sum_partials<<<grid_for(nw), 256, 0, st>>>(partials, nparts, nw, dw);
+  auto launch = cin == 16 && cout == 32   ? launch_dw<16, 32>
+                : cin == 32 && cout == 32 ? launch_dw<32, 32>
+                : cin == 32 && cout == 16 ? launch_dw<32, 16>
+                                          : nullptr;
+  if (!launch) return TL_ERR_ARG;
+  // one block per SM runs at a time; more partials than that would only be more to add up
+  int device = 0, sms = 0;
+  if (cudaGetDevice(&device) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+    return TL_ERR_CUDA;
+  const int blocks = nparts < sms ? nparts : sms;
+  launch(X, Z, partials, blocks, N, H, W, st);
+  k_sum_partials<<<(nw + 31) / 32, 256, 0, st>>>(partials, blocks, nw, dw);
   return cudaGetLastError() == cudaSuccess ? TL_OK : TL_ERR_CUDA;
 }
 
