@@ -89,6 +89,11 @@ extern "C" int tl_create(tl_ctx **out, const tl_config *cfg) {
   CK(cudaEventCreate(&ctx->tev1));
 
   ctx->walk_exact = make_walk(g.nx, g.ny, EXACT_WARPS, EXACT_ROWS, 2 * ctx->sm_count);
+  {  // up to two warps on each quarter of an SM, then longer tiles
+    const long long rows = (long long)((g.nx + 63) / 64) * g.ny / (8LL * ctx->sm_count);
+    ctx->walk_short = make_walk(g.nx, g.ny, EXACT_WARPS, (int)(rows < 1 ? 1 : rows > EXACT_ROWS ? EXACT_ROWS : rows),
+                                4 * ctx->sm_count);
+  }
   ctx->max_blocks = 8 * ctx->sm_count;  // the autotuner tries at most 8 resident blocks per SM
   const int max_blocks = ctx->max_blocks;
   const char *loop = getenv("TEALEAF_GB300_LOOP");
@@ -354,10 +359,14 @@ extern "C" int tl_finalise(tl_ctx *ctx) {
 extern "C" int tl_solve_finished(tl_ctx *ctx, int checkresult) {  // kernels.jl:166-170
   if (!ctx) return TL_ERR_ARG;
   int rc;
-  if (checkresult && (rc = tl_residual(ctx))) return rc;
-  if ((rc = tl_finalise(ctx))) return rc;
-  const int ex = TL_EX_ENERGY;
-  if ((rc = tl_halo_update(ctx, 1, &ex, 1, 0))) return rc;
+  if (ctx->cfg.mode == TL_MODE_TEALEAF) {
+    if ((rc = tl_solve_end(ctx, checkresult))) return rc;
+  } else {
+    if (checkresult && (rc = tl_residual(ctx))) return rc;
+    if ((rc = tl_finalise(ctx))) return rc;
+    const int ex = TL_EX_ENERGY;
+    if ((rc = tl_halo_update(ctx, 1, &ex, 1, 0))) return rc;
+  }
   CK(cudaStreamSynchronize(ctx->stream));
   return TL_OK;
 }

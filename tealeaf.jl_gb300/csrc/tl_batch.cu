@@ -232,24 +232,6 @@ extern "C" const char *tl_batch_last_error(const tl_batch *b) { return b ? b->ms
 
 namespace {
 
-int grid_cells_of(const Geom &g) {
-  long long blocks = ((long long)g.X * g.Y + 255) / 256;
-  if (blocks > 152LL * 32) blocks = 152LL * 32;
-  return (int)(blocks < 1 ? 1 : blocks);
-}
-
-// A deck's tea_leaf_init, halo of u, p and copyu!, on its current stream.
-int start_deck(tl_ctx *ctx, double rx, double ry, const tl_params *p, int exact) {
-  ctx->launches = 0;
-  int rc = tl_cg_init(ctx, rx, ry, p->coefficient, exact);
-  if (!rc) rc = tl_set_loop_params(ctx, p, 0, 0);
-  const int up[2] = {TL_EX_U, TL_EX_P};
-  if (!rc) rc = tl_halo_update(ctx, 1, up, 2, 1);
-  if (!rc) rc = tl_copy_u(ctx);
-  if (!rc) CK(cudaMemsetAsync(&ctx->F.sc->bar, 0, sizeof(GridBar), ctx->stream));
-  return rc;
-}
-
 int fetch_scalars(tl_ctx *ctx) {
   CK(cudaMemcpyAsync(ctx->host_sc, ctx->F.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, ctx->stream));
   return TL_OK;
@@ -266,13 +248,9 @@ int batch_solve(tl_batch *b, const double *rx, const double *ry, const tl_params
     tl_ctx *ctx = b->ctx[k];
     memset(&results[k], 0, sizeof(tl_result));
     if (ir) results[k].r0_plain = results[k].r0_pred = -1.0;
-    rc = start_deck(ctx, rx[k], ry[k], &p, ir ? 1 : 0);
-    if (!rc && ir) {
-      // the FP32 copies, and the end state of a deck that needs no iteration
-      k_ir_fields<<<grid_cells_of(ctx->g), 256, 0, b->stream>>>(ctx->F, ctx->g, g32_of(ctx), ctx->ir->r, ctx->ir->iw,
-                                                                p.coefficient, rx[k], ry[k]);
-      if (cudaGetLastError() != cudaSuccess) rc = TL_ERR_CUDA;
-    }
+    ctx->launches = 0;
+    rc = tl_solve_start(ctx, rx[k], ry[k], &p, 0, ir ? TL_START_FP32 : TL_START_FP64);
+    ctx->bar_clean = 0;  // the batch's kernel uses it
     if (rc) snprintf(b->msg, sizeof b->msg, "deck %d: %.480s", k, ctx->msg);
   }
   if (rc) return rc;
@@ -284,13 +262,13 @@ int batch_solve(tl_batch *b, const double *rx, const double *ry, const tl_params
                    (size_t)RING64_BYTES * WARPS64);
   }
   if (rc) return rc;
-  // per deck the halo of u, p and, FP64 under the relative criterion, the true
-  // residual as in the single-deck solve; one wait for all
+  // per deck, FP32, the halo of u, p and, FP64 under the relative criterion, the
+  // true residual as in the single-deck solve; one wait for all
   for (int k = 0; k < n && !rc; ++k) {
     tl_ctx *ctx = b->ctx[k];
-    if (ir || p.maxiters >= 1) rc = tl_halo_update(ctx, 1, nullptr, -1, 1);
-    if (!rc && !ir && p.criterion == TL_CRIT_RELATIVE)
-      launch_true_resid(ctx->stream, ctx->F, ctx->g, ctx->walk_exact, TL_MODE_TEALEAF, 0);
+    if (ir) rc = tl_halo_update(ctx, 1, nullptr, -1, 1);
+    if (!ir && p.criterion == TL_CRIT_RELATIVE)
+      launch_true_resid(ctx->stream, ctx->F, ctx->g, ctx->walk_short, TL_MODE_TEALEAF, 0);
     if (!rc) rc = fetch_scalars(ctx);
     if (rc) snprintf(b->msg, sizeof b->msg, "deck %d: %.480s", k, ctx->msg);
   }
@@ -363,6 +341,7 @@ extern "C" int tl_batch_solve(tl_batch *b, const double *rx, const double *ry, c
                   A.F = ctx->F;
                   A.g = ctx->g;
                   A.sums = static_cast<GridSums *>(ctx->grid_sums);
+                  A.check = 0;
                   cg64_tilings(A, size);
                 });
   if (rc) return rc;

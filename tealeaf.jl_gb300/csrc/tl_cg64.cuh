@@ -24,6 +24,7 @@ struct Cg64 {
   Geom g;
   Tiling tw, tr;  // W (strips of 60 columns), R (64)
   GridSums *sums;
+  int check;  // the relative test before the first iteration
 };
 
 struct Shared64 {
@@ -90,6 +91,7 @@ __device__ __forceinline__ bool cg64_solve(Grid grid, const Cg64 &A, Shared64 &S
   const double bb = sc->bb, eps = sc->eps, epslim = sc->epslim;
   const int maxiters = sc->maxiters, presteps = sc->presteps, errorswitch = sc->errorswitch, rule = sc->switch_rule;
   const bool relative = sc->crit == TL_CRIT_RELATIVE, rooted = relative || rule == 0;
+  if (A.check && sqrt(bb > 0 ? ddiv(sc->rro, bb) : sc->rro) < eps) return true;
   const RootTest test(eps, relative ? bb : 1.0);
   double *p = A.F.p, *pn = A.F.pb;
   double rro = sc->rro, alpha = 0.0, beta = 0.0, pw_ref = rro, rr = rro;
@@ -181,7 +183,7 @@ __device__ __forceinline__ bool cg64_solve(Grid grid, const Cg64 &A, Shared64 &S
     ++iter;
     if (S.done) break;
   }
-  // the last step's u, and p! of the next one (CG.jl:22)
+  // the last step's u, and p! of the next one (CG.jl:22), with their halo
   const int nx = A.g.nx, ny = A.g.ny, chunks = (nx + 63) / 64;
   const int warps = grid.nb * WARPS64;
   const long long n = (long long)chunks * ny;
@@ -191,8 +193,18 @@ __device__ __forceinline__ bool cg64_solve(Grid grid, const Cg64 &A, Shared64 &S
     const size_t c = A.g.at(i0, j);
     auto ld = [&](const double *f) { return __ldcg(reinterpret_cast<const double2 *>(f + c)); };
     const double2 pv = ld(p), rv = ld(A.F.r), uv = ld(A.F.u);
-    put64(A.F.u + c, make_double2(fma(alpha, pv.x, uv.x), fma(alpha, pv.y, uv.y)), i0 + 1 < nx);
-    put64(A.F.p + c, make_double2(fma(beta, pv.x, rv.x), fma(beta, pv.y, rv.y)), i0 + 1 < nx);
+    const double2 un = make_double2(fma(alpha, pv.x, uv.x), fma(alpha, pv.y, uv.y));
+    const double2 pw = make_double2(fma(beta, pv.x, rv.x), fma(beta, pv.y, rv.y));
+    put64(A.F.u + c, un, i0 + 1 < nx);
+    put64(A.F.p + c, pw, i0 + 1 < nx);
+    if (j == 0 || j == ny - 1 || i0 == 0 || i0 + 2 >= nx) {
+      put_faces(A.F.u, A.g, c, i0, j, un.x);
+      put_faces(A.F.p, A.g, c, i0, j, pw.x);
+      if (i0 + 1 < nx) {
+        put_faces(A.F.u, A.g, c + 1, i0 + 1, j, un.y);
+        put_faces(A.F.p, A.g, c + 1, i0 + 1, j, pw.y);
+      }
+    }
   }
   if (lead) {
     sc->alpha = alpha;

@@ -76,6 +76,12 @@ struct DevScalars {
   GridBar bar;          // persistent kernels (tl_persist.cuh); read back with the scalars
 };
 
+// The parameters of a loop that its epilogues read from DevScalars.
+struct LoopParams {
+  double eps, epslim;
+  int maxiters, presteps, errorswitch, stale_rro, crit, switch_rule;
+};
+
 // Device pointers of one context, passed to kernels by value.
 struct Fields {
   double *density0, *density, *energy0, *energy, *u, *u0, *p, *r, *mi, *w, *kx, *ky, *sd, *volume;

@@ -23,6 +23,15 @@
 
 using namespace tl;
 
+// r32 = (float) r on the interior.
+static __global__ void k_ir_residual(const double *r, Geom g, G32 g32, float *r32) {
+  const long long n = (long long)g.nx * g.ny;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(k % g.nx), j = (int)(k / g.nx);
+    r32[g32.at(i, j)] = (float)r[g.at(i, j)];
+  }
+}
+
 static int grid_for(long long n) {
   long long b = (n + 255) / 256;
   if (b > 152LL * 32) b = 152LL * 32;
@@ -55,18 +64,12 @@ void tl_release_ir(tl_ctx *ctx) {
   ctx->ir = nullptr;
 }
 
-// The inner loop with its refinements, from the state tl_cg_init and copyu
-// left (u, r = p = u0 - A u, r.r in rro).  Runs until the relative true
+// The inner loop with its refinements, from the state tl_solve_start left (u,
+// r = p = u0 - A u, r.r in rro, the FP32 copies).  Runs until the relative true
 // residual is below eps, the iteration budget is spent or, as CG presteps of
 // Chebyshev (switch rule 1), the switch test held; the FP32 search direction
 // is exported into p.  Returns the last true r.r and its relative value.
-static int ir_loop(tl_ctx *ctx, const tl_params &p, double rx, double ry, double *rr_out, double *rel_out,
-                   int *refinements) {
-  tl_ir_state *ir = ctx->ir;
-  k_ir_fields<<<grid_for((long long)ctx->g.X * ctx->g.Y), 256, 0, ctx->stream>>>(ctx->F, ctx->g, g32_of(ctx), ir->r,
-                                                                                 ir->iw, p.coefficient, rx, ry);
-  CKL();
-  ctx->launches += 8;
+static int ir_loop(tl_ctx *ctx, double *rr_out, double *rel_out, int *refinements) {
   ctx->last_solve_ms = 0.0;
   int rc = tl_ir_cg_run(ctx);
   if (rc) return rc;
@@ -88,15 +91,18 @@ int tl_ir_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_resu
   if (rc) return rc;
   tl_params p = *prm;
   p.criterion = TL_CRIT_RELATIVE;
-  if ((rc = tl_cg_init(ctx, rx, ry, p.coefficient, 1))) return rc;
-  if ((rc = tl_set_loop_params(ctx, &p, 0, 0))) return rc;
-  const int up[2] = {TL_EX_U, TL_EX_P};
-  if ((rc = tl_halo_update(ctx, 1, up, 2, 1))) return rc;
-  if ((rc = tl_copy_u(ctx))) return rc;
-  if (prm->warmstart && (rc = tl_warm_try(ctx, rx, ry, prm->warmstart, res))) return rc;
+  if ((rc = tl_solve_start(ctx, rx, ry, &p, 0, TL_START_FP32))) return rc;
+  if (prm->warmstart) {
+    if ((rc = tl_warm_try(ctx, rx, ry, prm->warmstart, res))) return rc;
+    // the residual of the start it chose
+    const Geom &g = ctx->g;
+    k_ir_residual<<<grid_for((long long)g.nx * g.ny), 256, 0, ctx->stream>>>(ctx->F.r, g, g32_of(ctx), ctx->ir->r);
+    CKL();
+    ctx->launches += 1;
+  }
   double rr = 0.0, rel = 0.0;
   int refinements = 0;
-  if ((rc = ir_loop(ctx, p, rx, ry, &rr, &rel, &refinements))) return rc;
+  if ((rc = ir_loop(ctx, &rr, &rel, &refinements))) return rc;
   res->iters = ctx->host_sc->iter;
   res->cg_iters = ctx->host_sc->iter;
   res->error = rr;
@@ -123,14 +129,9 @@ int tl_ir_presteps(tl_ctx *ctx, double rx, double ry, const tl_params *prm, int 
   if (rc) return rc;
   tl_params p = *prm;
   p.criterion = TL_CRIT_RELATIVE;
-  // exact 0: the stored diagonal, which the FP64 Chebyshev steps after the
-  // switch read
-  if ((rc = tl_cg_init(ctx, rx, ry, p.coefficient, 0))) return rc;
-  if ((rc = tl_set_loop_params(ctx, &p, 1, 0))) return rc;
-  const int up[2] = {TL_EX_U, TL_EX_P};
-  if ((rc = tl_halo_update(ctx, 1, up, 2, 1))) return rc;
-  if ((rc = tl_copy_u(ctx))) return rc;
-  if ((rc = ir_loop(ctx, p, rx, ry, rr_out, rel_out, refinements))) return rc;
+  // with the stored diagonal, which the FP64 Chebyshev step after the switch reads
+  if ((rc = tl_solve_start(ctx, rx, ry, &p, 1, TL_START_FP32_DIAG))) return rc;
+  if ((rc = ir_loop(ctx, rr_out, rel_out, refinements))) return rc;
   *switched = ctx->host_sc->prestep_switch && *rel_out >= p.eps;
   return TL_OK;
 }

@@ -22,15 +22,15 @@ int tl_ir_cg_run(tl_ctx *ctx) {
   IrCg A;
   ir_cg_args(A, ctx, persist_blocks(ctx->sm_count));
   CK(cudaFuncSetAttribute(k_ir_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES * PERSIST_WARPS));
-  CK(cudaMemsetAsync(&ctx->F.sc->bar, 0, sizeof(GridBar), ctx->stream));
+  int rc = tl_bar_ready(ctx);
+  if (rc) return rc;
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   void *args[] = {&A};
   CK(cudaLaunchCooperativeKernel((const void *)k_ir_cg, dim3(A.t.blocks), dim3(PERSIST_THREADS), args,
                                  RING_BYTES * PERSIST_WARPS, ctx->stream));
   CK(cudaEventRecord(ctx->ev1, ctx->stream));
   ctx->launches += 1;
-  int rc = tl_read_scalars(ctx);
-  if (rc) return rc;
+  if ((rc = tl_read_scalars(ctx))) return rc;
   float ms = 0.f;
   CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
   ctx->last_solve_ms += ms;

@@ -1,5 +1,8 @@
-// tl_ir_ops.cuh -- the FP32 buffers of the refinement path and the FP32 copies
-// a solve starts from, shared by the single-deck solves and the batch.
+// tl_ir_ops.cuh -- the FP32 buffers of the refinement path, shared by the
+// single-deck solves and the batch.  A solve starts (tl_start.cu) from the FP32
+// residual and the inverse weights iw = 1/w over the whole array (w = rho for
+// conductivity, 1/rho for its reciprocal: CG.jl:57-60), with rx/2, ry/2, so that
+// Kx = rx (w_l + w_c) / (2 w_l w_c) = rx/2 (iw_l + iw_c) (CG.jl:62-67).
 //
 // FP32 arrays are pitched like the FP64 fields, 32 floats per pitch unit, first
 // interior cell of each row 128-byte aligned; a lane owns 4 consecutive cells
@@ -36,27 +39,6 @@ struct G32 {
 
 __device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
 __device__ __forceinline__ float comp(const float4 &v, int k) { return k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w; }
-
-// The start of an FP32 solve: r32 = (float) r on the interior (0 in the halo),
-// the inverse weights iw = 1/w over the whole array (w = rho for conductivity,
-// 1/rho for its reciprocal: CG.jl:57-60 over the whole array, the tealeaf-mode
-// range) and the face factors rx/2, ry/2, so that
-// Kx = rx (w_l + w_c) / (2 w_l w_c) = rx/2 (iw_l + iw_c) (CG.jl:62-67).
-__global__ void k_ir_fields(Fields F, Geom g, G32 g32, float *r, float *iw, int coefficient, double rx, double ry) {
-  const long long n = (long long)g.X * g.Y;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    F.sc->rxh = 0.5 * rx;
-    F.sc->ryh = 0.5 * ry;
-  }
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-    const int I = (int)(k % g.X), J = (int)(k / g.X);
-    const size_t c = (size_t)I + (size_t)J * g.pitch, c32 = (size_t)I + (size_t)J * g32.pitch;
-    const bool interior = I >= g.hd && I < g.X - g.hd && J >= g.hd && J < g.Y - g.hd;
-    const double rho = F.density[c];
-    r[c32] = interior ? (float)F.r[c] : 0.f;
-    iw[c32] = (float)(coefficient == TL_CONDUCTIVITY ? 1.0 / rho : rho);
-  }
-}
 
 G32 g32_of(tl_ctx *ctx) {
   G32 g;

@@ -627,14 +627,14 @@ int run_sweeps(tl_ctx *ctx, const void *kernel, int ninner, double rr) {
   IrSweeps A = sweep_args(ctx, ninner, rr);
   const size_t smem = (size_t)RING_BYTES * PERSIST_WARPS;
   CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  CK(cudaMemsetAsync(&ctx->F.sc->bar, 0, sizeof(GridBar), ctx->stream));
+  int rc = tl_bar_ready(ctx);
+  if (rc) return rc;
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   void *args[] = {&A};
   CK(cudaLaunchCooperativeKernel(kernel, dim3(A.t.blocks), dim3(PERSIST_THREADS), args, smem, ctx->stream));
   CK(cudaEventRecord(ctx->ev1, ctx->stream));
   ctx->launches += 1;
-  int rc = tl_read_scalars(ctx);
-  if (rc) return rc;
+  if ((rc = tl_read_scalars(ctx))) return rc;
   float ms = 0.f;
   CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
   ctx->last_solve_ms = ms;
@@ -708,7 +708,7 @@ int tl_ir_bench_kernel(tl_ctx *ctx, int kernel, int reps, double *ms_per_launch)
   ir_cg_args(C, ctx, persist_blocks(ctx->sm_count));
   const size_t smem = (size_t)RING_BYTES * PERSIST_WARPS;
   CK(cudaFuncSetAttribute(k_bench32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  CK(cudaMemsetAsync(&ctx->F.sc->bar, 0, sizeof(GridBar), ctx->stream));
+  if ((rc = tl_bar_ready(ctx))) return rc;
   CK(cudaEventRecord(ctx->tev0, ctx->stream));
   void *args[] = {&A, &C, &kernel, &reps};
   CK(cudaLaunchCooperativeKernel((const void *)k_bench32, dim3(kernel >= 8 ? C.t.blocks : A.t.blocks),

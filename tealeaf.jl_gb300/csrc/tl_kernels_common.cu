@@ -354,6 +354,7 @@ struct OpSummary : NoSkip {
     acc[3] = dadd(acc[3], dmul(m, F.u[c]));
   }
   __device__ void tile(int i0, int j0, int j1, double (&acc)[4]) const {
+#pragma unroll 4  // the loads of four rows in flight
     for (int j = j0; j < j1; ++j) {
       if (i0 < g.nx) cell(i0, j, acc);
       if (i0 + 1 < g.nx) cell(i0 + 1, j, acc);

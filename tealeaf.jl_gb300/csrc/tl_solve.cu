@@ -12,25 +12,11 @@ using namespace tl;
 
 namespace {
 
-struct LoopParams {
-  double eps, epslim;
-  int maxiters, presteps, errorswitch, stale_rro, crit, switch_rule;
-};
-
-__global__ void k_set_params(DevScalars *sc, LoopParams p) {
-  sc->eps = p.eps;
-  sc->epslim = p.epslim;
-  sc->maxiters = p.maxiters;
-  sc->presteps = p.presteps;
-  sc->errorswitch = p.errorswitch;
-  sc->stale_rro = p.stale_rro;
-  sc->crit = p.crit;
-  sc->switch_rule = p.switch_rule;
-}
+__global__ void k_set_params(DevScalars *sc, LoopParams p) { set_params(sc, p); }
 
 }  // namespace
 
-int tl_set_loop_params(tl_ctx *ctx, const tl_params *prm, int switch_rule, int stale_rro) {
+LoopParams loop_params(const tl_params *prm, int switch_rule, int stale_rro) {
   LoopParams p;
   p.eps = prm->eps;
   p.epslim = prm->epslim;
@@ -40,7 +26,11 @@ int tl_set_loop_params(tl_ctx *ctx, const tl_params *prm, int switch_rule, int s
   p.stale_rro = stale_rro;
   p.crit = prm->criterion;
   p.switch_rule = switch_rule;
-  k_set_params<<<1, 1, 0, ctx->stream>>>(ctx->F.sc, p);
+  return p;
+}
+
+int tl_set_loop_params(tl_ctx *ctx, const tl_params *prm, int switch_rule, int stale_rro) {
+  k_set_params<<<1, 1, 0, ctx->stream>>>(ctx->F.sc, loop_params(prm, switch_rule, stale_rro));
   CKL();
   return TL_OK;
 }
@@ -61,20 +51,22 @@ const Walk &tl_walk_for(tl_ctx *ctx, int exact) {
   return (ctx->cfg.mode == TL_MODE_REFERENCE || exact) ? ctx->walk_exact : ctx->walk_ur64;
 }
 
-// CG.init! (CG.jl:47-79).  Also stores the fused kernels' diagonal.
-int tl_cg_init(tl_ctx *ctx, double rx, double ry, int coefficient, int exact) {
+int tl_check_coefficient(tl_ctx *ctx, int coefficient) {
   if (coefficient != TL_CONDUCTIVITY && coefficient != TL_RECIP_CONDUCTIVITY) {
     tl_set_error(ctx, "Coefficient %d is not valid (src/solvers/CG.jl:49)", coefficient);
     return TL_ERR_COEF;
   }
+  return TL_OK;
+}
+
+// CG.init! (CG.jl:47-79), in the exact path's order of summation.
+int tl_cg_init(tl_ctx *ctx, double rx, double ry, int coefficient) {
+  int rc = tl_check_coefficient(ctx, coefficient);
+  if (rc) return rc;
   launch_init_pre(ctx->stream, ctx->F, ctx->g, coefficient, ctx->cfg.mode);
   CKL();
   launch_init_coef(ctx->stream, ctx->F, ctx->g, rx, ry, 0, coefficient);
   CKL();
-  if (ctx->cfg.mode == TL_MODE_TEALEAF && !exact) {
-    launch_init_diag(ctx->stream, ctx->F, ctx->g);
-    CKL();
-  }
   launch_init_resid(ctx->stream, ctx->F, ctx->g, ctx->walk_exact, ctx->cfg.mode);
   CKL();
   return TL_OK;
@@ -323,8 +315,8 @@ void tl_launch_ur64_for_tuning(tl_ctx *ctx, const Walk &wk) {
 // recursive residual; the true residual u0 - A u is then measured and, if it
 // has drifted above eps, CG restarts from it (r = p = u0 - A u) within the
 // remaining iteration budget.
-static int true_residual(tl_ctx *ctx, int write, double *rr) {
-  launch_true_resid(ctx->stream, ctx->F, ctx->g, ctx->walk_exact, ctx->cfg.mode, write);
+static int true_residual(tl_ctx *ctx, int exact, int write, double *rr) {
+  launch_true_resid(ctx->stream, ctx->F, ctx->g, exact ? ctx->walk_exact : ctx->walk_short, ctx->cfg.mode, write);
   ctx->launches += 1;
   CKL();
   int rc = tl_read_scalars(ctx);
@@ -336,39 +328,37 @@ static int true_residual(tl_ctx *ctx, int write, double *rr) {
 int tl_cg_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_result *res) {
   const int ref = ctx->cfg.mode == TL_MODE_REFERENCE;
   const int exact = ref || prm->exact;
-  int rc = tl_cg_init(ctx, rx, ry, prm->coefficient, exact);
+  int rc = tl_solve_start(ctx, rx, ry, prm, 0, exact ? TL_START_EXACT : TL_START_FP64);
   if (rc) return rc;
-  ctx->launches += exact ? 3 : 4;
-  if ((rc = tl_set_loop_params(ctx, prm, 0, 0))) return rc;
-  const int up[2] = {TL_EX_U, TL_EX_P};
-  if ((rc = tl_halo_update(ctx, 1, up, 2, 1))) return rc;   // CG.jl:11
-  if ((rc = tl_copy_u(ctx))) return rc;                     // CG.jl:12
-  ctx->launches += 3;
   if (prm->warmstart && (rc = tl_warm_try(ctx, rx, ry, prm->warmstart, res))) return rc;
   ctx->last_solve_ms = 0.0;
-  if (prm->criterion == TL_CRIT_RELATIVE) {
-    // the relative test also holds before the first iteration (an exact
-    // start, where CG's alpha would be 0/0)
-    if ((rc = tl_read_scalars(ctx))) return rc;
+  // The relative test also holds before the first iteration (an exact start,
+  // where CG's alpha would be 0/0).
+  auto met_at_start = [&]() {
     const DevScalars &s0 = *ctx->host_sc;
     const double rel0 = s0.bb > 0 ? sqrt(s0.rro / s0.bb) : sqrt(s0.rro);
-    if (rel0 < prm->eps) {
-      res->iters = res->cg_iters = 0;
-      res->error = s0.rro;
-      res->converged = 1;
-      res->rel_residual = rel0;
-      res->launches = (int)ctx->launches;
-      return TL_OK;
-    }
+    if (!(rel0 < prm->eps)) return false;
+    res->iters = res->cg_iters = 0;
+    res->error = s0.rro;
+    res->converged = 1;
+    res->rel_residual = rel0;
+    res->launches = (int)ctx->launches;
+    return true;
+  };
+  // The persistent kernel makes the test itself, one wait of the host less.
+  const bool in_kernel = !exact && prm->maxiters >= 1;
+  if (prm->criterion == TL_CRIT_RELATIVE && !in_kernel) {
+    if ((rc = tl_read_scalars(ctx))) return rc;
+    if (met_at_start()) return TL_OK;
   }
   const int which = ref ? TL_GRAPH_CG_REF : TL_GRAPH_CG_EXACT;  // the fused arithmetic has its own kernel
   double rel = -1.0;
   int ran = 0;
   for (int restart = 0; restart < 8 && prm->maxiters >= 1; ++restart) {
     if (!exact) {
-      if ((rc = tl_cg64_run(ctx, &ctx->last_solve_ms))) return rc;
-      if ((rc = tl_halo_update(ctx, 1, nullptr, -1, 1))) return rc;
-      ctx->launches += 1;
+      const int check = prm->criterion == TL_CRIT_RELATIVE && restart == 0;
+      if ((rc = tl_cg64_run(ctx, check, &ctx->last_solve_ms))) return rc;
+      if (check && !ctx->host_sc->done && met_at_start()) return TL_OK;
     } else {
       const int before = ctx->host_sc->iter;
       if ((rc = tl_run_graph(ctx, which, &ctx->last_solve_ms))) return rc;
@@ -387,13 +377,14 @@ int tl_cg_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_resu
     ran = 1;
     if (prm->criterion != TL_CRIT_RELATIVE) break;
     double tr;
-    if ((rc = true_residual(ctx, 0, &tr))) return rc;
+    if ((rc = true_residual(ctx, exact, 0, &tr))) return rc;
     const double bb = ctx->host_sc->bb;
     rel = bb > 0 ? sqrt(tr / bb) : sqrt(tr);
     if (rel < prm->eps || ref || ctx->host_sc->iter >= prm->maxiters) break;
-    if ((rc = true_residual(ctx, 1, &tr))) return rc;  // restart from the true residual
+    if ((rc = true_residual(ctx, exact, 1, &tr))) return rc;  // restart from the true residual
   }
-  if ((rc = tl_read_scalars(ctx))) return rc;
+  // each way through the loop has read the scalars after its last change of them
+  if (!ran && (rc = tl_read_scalars(ctx))) return rc;
   const DevScalars &sc = *ctx->host_sc;
   res->iters = sc.iter;
   res->cg_iters = sc.iter;

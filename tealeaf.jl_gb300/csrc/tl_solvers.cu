@@ -179,18 +179,16 @@ int set_phase(tl_ctx *ctx, double theta, int cheby_iters, int est, int first, in
 // scalars hold the loop's end state.
 int cg_phase(tl_ctx *ctx, double rx, double ry, const tl_params *prm, int exact, int stale_rro) {
   const int ref = ctx->cfg.mode == TL_MODE_REFERENCE;
-  int rc = tl_cg_init(ctx, rx, ry, prm->coefficient, exact);
-  if (rc) return rc;
-  if ((rc = tl_set_loop_params(ctx, prm, 1, stale_rro))) return rc;
-  if (!ref) {
-    const int up[2] = {TL_EX_U, TL_EX_P};
-    if ((rc = tl_halo_update(ctx, 1, up, 2, 1))) return rc;
-    if ((rc = tl_copy_u(ctx))) return rc;
+  int rc;
+  if (ref) {
+    if ((rc = tl_cg_init(ctx, rx, ry, prm->coefficient))) return rc;
+    if ((rc = tl_set_loop_params(ctx, prm, 1, stale_rro))) return rc;
+  } else if ((rc = tl_solve_start(ctx, rx, ry, prm, 1, exact ? TL_START_EXACT : TL_START_FP64))) {
+    return rc;
   }
   ctx->last_solve_ms = 0.0;
   if (!ref && !exact && prm->maxiters >= 1) {
-    if ((rc = tl_cg64_run(ctx, &ctx->last_solve_ms))) return rc;
-    return tl_halo_update(ctx, 1, nullptr, -1, 1);
+    return tl_cg64_run(ctx, 0, &ctx->last_solve_ms);
   }
   if (prm->maxiters >= 1) {
     const int which = ref ? TL_GRAPH_CG_REF_NOHALO : TL_GRAPH_CG_EXACT;

@@ -26,6 +26,7 @@ struct tl_ctx {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   tl::Walk walk_exact{};            // fixed layout of the bit-reproducible kernels
+  tl::Walk walk_short{};            // the same kernels on the fused path: shorter tiles on small decks
   tl::Walk walk_w64{}, walk_ur64{};  // autotuned layouts of the fused FP64 CG kernels
   int max_blocks = 0;                // capacity of the reduction partials
   int host_loop = 0;                 // iteration loops launched from the host (TEALEAF_GB300_LOOP=host)
@@ -36,6 +37,7 @@ struct tl_ctx {
   double *field_ptr[TL_NFIELDS] = {};
   tl::DevScalars *host_sc = nullptr;
   void *grid_sums = nullptr;  // GridSums of the persistent kernels (tl_persist.cuh)
+  int bar_clean = 0;          // the grid barrier is at zero
   int toexchange[TL_NEX] = {};
   int initialised = 0;
   double last_solve_ms = 0.0;
@@ -65,10 +67,23 @@ void tl_release_graphs(tl_ctx *ctx);
 void tl_release_ir(tl_ctx *ctx);
 
 // shared solver pieces (tl_solve.cu)
+tl::LoopParams loop_params(const tl_params *prm, int switch_rule, int stale_rro);
 int tl_set_loop_params(tl_ctx *ctx, const tl_params *prm, int switch_rule, int stale_rro);
 int tl_read_scalars(tl_ctx *ctx);
 const tl::Walk &tl_walk_for(tl_ctx *ctx, int exact);
-int tl_cg_init(tl_ctx *ctx, double rx, double ry, int coefficient, int exact);
+int tl_check_coefficient(tl_ctx *ctx, int coefficient);
+int tl_cg_init(tl_ctx *ctx, double rx, double ry, int coefficient);
+// The start of a solve in tealeaf mode (tl_start.cu): CG.init!, the loop's
+// parameters, the halo of u and p, copyu!.  The fused starts are one launch.
+enum {
+  TL_START_EXACT,      // bit-identical to the oracle
+  TL_START_FP64,       // with the fused kernels' diagonal
+  TL_START_FP32,       // with the FP32 loop's residual and inverse weights
+  TL_START_FP32_DIAG,  // both
+};
+int tl_solve_start(tl_ctx *ctx, double rx, double ry, const tl_params *prm, int switch_rule, int kind);
+int tl_solve_end(tl_ctx *ctx, int checkresult);
+int tl_bar_ready(tl_ctx *ctx);
 int tl_get_graph(tl_ctx *ctx, int which, cudaGraphExec_t *out);
 int tl_run_graph(tl_ctx *ctx, int which, double *ms);
 int tl_cg_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_result *res);
@@ -83,7 +98,8 @@ int tl_ensure_ir(tl_ctx *ctx);  // allocates the FP32 refinement buffers
 // The FP32-refined CG loop as one persistent kernel (tl_ir_cg.cu).
 int tl_ir_cg_run(tl_ctx *ctx);
 // The fused FP64 CG loop with the last step's p!, as one persistent kernel (tl_cg64.cu).
-int tl_cg64_run(tl_ctx *ctx, double *ms);
+// With `check` it ends at once, the state untouched, if the start meets the relative test.
+int tl_cg64_run(tl_ctx *ctx, int check, double *ms);
 // The fused FP64 loops of Chebyshev, PPCG and Jacobi (tl_sweeps64.cu).
 int tl_loop64_run(tl_ctx *ctx, int which, int ninner, double *ms);
 // TL_OK, or the error of a persistent kernel whose grid barrier gave up (after tl_read_scalars)

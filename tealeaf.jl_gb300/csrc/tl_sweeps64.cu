@@ -420,15 +420,14 @@ int tl_loop64_run(tl_ctx *ctx, int which, int ninner, double *ms) {
   A.te = make_tiling_on(A.t, ctx->g.nx, ctx->g.ny, 64, each, WARPS64);
   const size_t smem = (size_t)RING64_BYTES * WARPS64;
   CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  CK(cudaMemsetAsync(&ctx->F.sc->bar, 0, sizeof(GridBar), ctx->stream));
-  CK(cudaMemsetAsync(&A.F.sc->bar.next_tile, 0, sizeof(unsigned), ctx->stream));
+  int rc = tl_bar_ready(ctx);
+  if (rc) return rc;
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   void *args[] = {&A};
   CK(cudaLaunchCooperativeKernel(kernel, dim3(A.t.blocks), dim3(WARPS64 * 32), args, smem, ctx->stream));
   CK(cudaEventRecord(ctx->ev1, ctx->stream));
   ctx->launches += 1;
-  int rc = tl_read_scalars(ctx);
-  if (rc) return rc;
+  if ((rc = tl_read_scalars(ctx))) return rc;
   float t = 0.f;
   CK(cudaEventElapsedTime(&t, ctx->ev0, ctx->ev1));
   if (ms) *ms += t;

@@ -39,6 +39,27 @@ __device__ __forceinline__ double acc_mul(double acc, double x, double y) {
 __device__ __forceinline__ double2 ld2(const double *p) { return __ldg(reinterpret_cast<const double2 *>(p)); }
 __device__ __forceinline__ void st2(double *p, double2 v) { *reinterpret_cast<double2 *>(p) = v; }
 
+__device__ __forceinline__ void set_params(DevScalars *sc, const LoopParams &p) {
+  sc->eps = p.eps;
+  sc->epslim = p.epslim;
+  sc->maxiters = p.maxiters;
+  sc->presteps = p.presteps;
+  sc->errorswitch = p.errorswitch;
+  sc->stale_rro = p.stale_rro;
+  sc->crit = p.crit;
+  sc->switch_rule = p.switch_rule;
+}
+
+// The halo (depth 1, tealeaf semantics: kernels.jl:191-210) of a field whose
+// cell (i, j), at c, got the value v: a cell at the domain's edge also owns the
+// cells across it.
+__device__ __forceinline__ void put_faces(double *f, const Geom &g, size_t c, int i, int j, double v) {
+  if (i == 0) f[c - 1] = v;
+  if (i == g.nx - 1) f[c + 1] = v;
+  if (j == 0) f[c - g.pitch] = v;
+  if (j == g.ny - 1) f[c + g.pitch] = v;
+}
+
 __device__ __forceinline__ double warp_butterfly(double v) {
 #pragma unroll
   for (int off = 16; off >= 1; off >>= 1) v = dadd(v, __shfl_xor_sync(FULL, v, off));

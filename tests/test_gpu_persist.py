@@ -168,3 +168,35 @@ def test_fp32_sweep_tilings(tl, built_lib, solver, inner, nx, ny, hd):
         c.close()
     assert np.linalg.norm(u[0] - v) <= 4e-10 * np.linalg.norm(u0)
     np.testing.assert_array_equal(u[0], u[1])
+
+
+@pytest.mark.parametrize("hd", [1, 2, 3])
+@pytest.mark.parametrize("coefficient", [1, 2])
+@pytest.mark.parametrize("nx,ny", [(1, 1), (2, 3), (26, 5), (28, 1), (29, 31), (61, 64), (90, 7), (700, 611)])
+def test_start_and_end_of_a_solve(tl, built_lib, nx, ny, hd, coefficient):
+    """The one-kernel start and end of a step against the separate kernels of the
+    exact path, halo included: the same operations per cell, so equal bit for
+    bit.  A bound on the residual that the start already meets ends the solve
+    there."""
+    text = random_deck(nx, 7, ny=ny, nrect=3, eps=1e10).replace("halo_depth=2", f"halo_depth={hd}")
+    text = text.replace("coefficient=1", f"coefficient={coefficient}")
+    chunks, results = [], []
+    for exact in (False, True):
+        s = tl.Settings.from_text(text, mode=TEA, exact=exact, criterion=1)
+        c = tl.initialiseapp(s)
+        tl.haloupdate(c, s, 1, ["energy", "density"])
+        results.append(tl.CG.solve(c, s, s.dtinit / s.dx ** 2, s.dtinit / s.dy ** 2))
+        chunks.append((c, s))
+    (a, sa), (b, sb) = chunks
+    assert results[0].iters == results[1].iters == 0 and results[0].converged
+    assert abs(results[0].error - results[1].error) <= 1e-12 * results[1].error
+    for f in ("u", "u0", "p", "r", "w", "kx", "ky"):
+        np.testing.assert_array_equal(a.field(f), b.field(f), err_msg=f)
+    tl.solvefinished(a, sa)
+    tl.residual(b)
+    tl.finalise(b)
+    tl.haloupdate(b, sb, 1, ["energy"])
+    for f in ("r", "energy"):
+        np.testing.assert_array_equal(a.field(f), b.field(f), err_msg=f)
+    a.close()
+    b.close()
