@@ -503,11 +503,13 @@ int tl_jacobi_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_
   k_jacobi_start<<<1, 1, 0, ctx->stream>>>(ctx->F.sc);
   CKL();
   ctx->last_solve_ms = 0.0;
-  if (prm->maxiters >= 1) {
-    rc = exact ? tl_run_graph(ctx, TL_GRAPH_JACOBI, &ctx->last_solve_ms)
-               : tl_loop64_run(ctx, TL_GRAPH_JACOBI, 0, &ctx->last_solve_ms);
-    if (rc) return rc;
+  if (prm->maxiters >= 1 && !exact) {  // u, r with their halos; the scalars read
+    if ((rc = tl_loop64_run(ctx, TL_GRAPH_JACOBI, 0, &ctx->last_solve_ms))) return rc;
+    fill_result(ctx, res, 0);
+    res->inner_iters = 0;
+    return TL_OK;
   }
+  if (prm->maxiters >= 1 && (rc = tl_run_graph(ctx, TL_GRAPH_JACOBI, &ctx->last_solve_ms))) return rc;
   if ((rc = tl_read_scalars(ctx))) return rc;
   if (ctx->host_sc->iter & 1) {
     launch_copy_interior(ctx->stream, ctx->F.u, ctx->F.ub, g);

@@ -200,3 +200,42 @@ def test_start_and_end_of_a_solve(tl, built_lib, nx, ny, hd, coefficient):
         np.testing.assert_array_equal(a.field(f), b.field(f), err_msg=f)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(1, 1), (2, 2), (61, 33), (62, 1), (243, 131), (600, 449),  # the blocks hold the deck
+                                   (600, 481), (901, 700)])
+@pytest.mark.parametrize("iters,eps", [(1, 0.0), (2, 0.0), (3, 0.0), (50, 0.0), (51, 0.0), (52, 0.0),
+                                       (400, 3.0), (400, 2.0), (400, 1.4)])
+def test_jacobi_pairs(tl, built_lib, nx, ny, iters, eps):
+    """Fused Jacobi, two sweeps a pass, against the exact sweeps where it can end:
+    after the first or the second of a pair, at a check, by its bound or its
+    budget.  The bounds are in units of the 7th sweep's change.  Tolerances as
+    in test_jacobi_tilings."""
+    text = random_deck(nx, 84, ny=ny, nrect=4, steps=1, eps=0.0, solver="jacobi")
+    if eps:
+        changes = []
+        for k in (1, 7):
+            s = tl.Settings.from_text(text.replace("max_iters=5000", f"max_iters={k}"), mode=TEA, exact=True)
+            c = tl.initialiseapp(s)
+            tl.haloupdate(c, s, 1, ["energy", "density"])
+            changes.append(tl.Jacobi.solve(c, s, s.dtinit / s.dx ** 2, s.dtinit / s.dy ** 2).error)
+            c.close()
+        eps *= max(changes[1], 1e-8 * changes[0])  # not a bound within rounding, on decks that are done by then
+    text = text.replace("max_iters=5000", f"max_iters={iters}").replace("eps=0.0", f"eps={eps!r}")
+    f = []
+    for exact in (False, True):
+        s = tl.Settings.from_text(text, mode=TEA, exact=exact)
+        c = tl.initialiseapp(s)
+        tl.haloupdate(c, s, 1, ["energy", "density"])
+        res = tl.Jacobi.solve(c, s, s.dtinit / s.dx ** 2, s.dtinit / s.dy ** 2)
+        f.append((_interior(c.field("u"), 1), _interior(c.field("r"), 1), res))
+        k = 1 + 2 * (np.max(np.abs(_interior(c.field("kx")))) + np.max(np.abs(_interior(c.field("ky")))))
+        c.close()
+    (u, r, a), (v, s, b) = f
+    assert (a.iters, a.converged) == (b.iters, b.converged)
+    scale = np.max(np.abs(v))
+    assert np.max(np.abs(u - v)) <= 1e-13 * scale
+    # after a check r is u0 - A u, which multiplies what u is off by up to 1 + sum k
+    at_check = b.iters % 50 == 0
+    assert np.max(np.abs(r - s)) <= 1e-13 * scale * (k if at_check else 1)
+    assert abs(a.error - b.error) <= 1e-9 * abs(b.error) + 1e-13 * scale * nx * ny
