@@ -61,6 +61,7 @@ struct ConvArgs {
   bf16 *z, *out;
   float *out32;
   int N, H, W;
+  int wide;  // gz, z and out start on 32-byte boundaries
 };
 
 __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void *p) {
@@ -680,6 +681,37 @@ struct WsWalk {
   }
 };
 
+// A pixel's channels (8 a vector) to or from memory: 32 bytes an instruction, a
+// whole sector a lane, where the buffers' alignment lets it (the forward pass
+// of 32 images of 128 x 128 in 29 us; with 16 bytes, half a sector, 35).
+template <int N>
+__device__ __forceinline__ void store_channels(bf16 *p, const uint4 (&v)[N], int wide) {
+  if (N > 1 && wide) {
+#pragma unroll
+    for (int q = 0; q + 1 < N; q += 2)
+      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p + 8 * q), "r"(v[q].x), "r"(v[q].y),
+                   "r"(v[q].z), "r"(v[q].w), "r"(v[q + 1].x), "r"(v[q + 1].y), "r"(v[q + 1].z), "r"(v[q + 1].w)
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int q = 0; q < N; ++q) reinterpret_cast<uint4 *>(p)[q] = v[q];
+  }
+}
+template <int N>
+__device__ __forceinline__ void load_channels(uint4 (&v)[N], const bf16 *p, int wide) {
+  if (N > 1 && wide) {
+#pragma unroll
+    for (int q = 0; q + 1 < N; q += 2)
+      asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                   : "=r"(v[q].x), "=r"(v[q].y), "=r"(v[q].z), "=r"(v[q].w), "=r"(v[q + 1].x), "=r"(v[q + 1].y),
+                     "=r"(v[q + 1].z), "=r"(v[q + 1].w)
+                   : "l"(p + 8 * q));
+  } else {
+#pragma unroll
+    for (int q = 0; q < N; ++q) v[q] = reinterpret_cast<const uint4 *>(p)[q];
+  }
+}
+
 template <int CIN, int COUT, int MODE, class CFG>
 __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB) k_conv3x3_ws(ConvArgs a, int tiles_x, int th,
                                                              const __grid_constant__ ConvMaps maps) {
@@ -886,10 +918,7 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB) k_conv3x3_ws(ConvArgs
         const int y = T.y0 + i;
         uint4 gzv[MODE == 2 ? CW / 8 : 1];
         if (MODE == 2 && xx < a.W) {
-          const uint4 *gp = reinterpret_cast<const uint4 *>(
-              a.gz + ((size_t)T.img * plane + (size_t)y * a.W + xx) * COUT + half * CW);
-#pragma unroll
-          for (int q = 0; q < (MODE == 2 ? CW / 8 : 1); ++q) gzv[q] = gp[q];
+          load_channels(gzv, a.gz + ((size_t)T.img * plane + (size_t)y * a.W + xx) * COUT + half * CW, a.wide);
         }
         const int acc_i = O % NACC;
         if (!ws_wait(tfull + acc_i, (O / NACC) & 1u, abort_flag)) {
@@ -943,16 +972,8 @@ __global__ void __launch_bounds__(CFG::THREADS, CFG::MINB) k_conv3x3_ws(ConvArgs
               op[h] = __floats2bfloat162_rn(o0, o1);
             }
           }
-          if (MODE == 1 && a.z) {
-            uint4 *zd = reinterpret_cast<uint4 *>(a.z + pix * COUT + half * CW);
-#pragma unroll
-            for (int q = 0; q < CW / 8; ++q) zd[q] = zo[q];
-          }
-          if (a.out) {
-            uint4 *od = reinterpret_cast<uint4 *>(a.out + pix * COUT + half * CW);
-#pragma unroll
-            for (int q = 0; q < CW / 8; ++q) od[q] = oo[q];
-          }
+          if (MODE == 1 && a.z) store_channels(a.z + pix * COUT + half * CW, zo, a.wide);
+          if (a.out) store_channels(a.out + pix * COUT + half * CW, oo, a.wide);
         }
       }
     }
@@ -1339,10 +1360,8 @@ int conv_sm_count() {
 }
 
 // The warp-specialised kernel's producer and epilogue (TEALEAF_GB300_CONV_WS):
-//   0 (default) a tensor copy per row into a 4-slot ring; the GELU forward
-//     (mode 1) with the row-parallel epilogue at three blocks per SM, the
-//     plain output (0) and the input gradient (2) with every epilogue warp
-//     on every row at four blocks per SM (each measured best for its mode);
+//   0 (default) a tensor copy per row into a 4-slot ring, row-parallel
+//     epilogue, two blocks per SM;
 //   1 a tensor copy per row, every epilogue warp on every row (half the
 //     channels), three blocks per SM, every mode;
 //   2 cp.async channel chunks into a 6-slot ring with 3 rows ahead, every
@@ -1457,11 +1476,13 @@ void launch_conv_mode(const ConvArgs &a, cudaStream_t st) {
     tc::k_conv3x3_tc<CIN, COUT, MODE><<<grid, 256, smem, st>>>(a);
     return;
   }
-  // GELU forward: the row-parallel epilogue at three blocks per SM; plain
-  // output and input gradient: every epilogue warp on every row at four
-  // blocks per SM (registers capped at 48; measured faster for those two)
-  using TmaCfg = tc::WsCfg<4, 1, 4, true, MODE == 1, MODE == 1 ? 3 : 4>;
-  constexpr int TMA_MAXB = MODE == 1 ? 3 : 4;
+  // The row-parallel epilogue, which moves 64 bytes of a pixel at a time, at two
+  // blocks per SM, forward and input gradient: 84 us each on 32 images of
+  // 256 x 256 (32 -> 32 channels), 29 at 128 x 128, 14.4 on one of 300 x 300.  At
+  // three blocks 89 and 109 (256 x 256); 88 and 100 with every epilogue warp
+  // on every row, a half of the channels each; a ring of six or eight rows, or
+  // eight accumulators, no faster; one block per SM 121 and 135.
+  using TmaCfg = tc::WsCfg<4, 1, 4, true, true, 2>;
   using TmaCfgAll = tc::WsCfg<4, 1, 4, true, false>;
   using CpCfg = tc::WsCfg<6, 3, 4, false>;
   tc::ConvMaps maps;
@@ -1469,7 +1490,7 @@ void launch_conv_mode(const ConvArgs &a, cudaStream_t st) {
   const int cfg = conv_ws_cfg();
   if (cfg != 2 && input_map<CIN>(a, &maps.in)) {
     if (cfg == 1) launch_ws<CIN, COUT, MODE, TmaCfgAll, 3>(a, maps, st);
-    else launch_ws<CIN, COUT, MODE, TmaCfg, TMA_MAXB>(a, maps, st);
+    else launch_ws<CIN, COUT, MODE, TmaCfg, 2>(a, maps, st);
   } else {
     launch_ws<CIN, COUT, MODE, CpCfg, 3>(a, maps, st);
   }
@@ -1513,6 +1534,7 @@ int tl_conv_forward(const void *x, const void *w, const float *bias, const void 
   a.N = N;
   a.H = H;
   a.W = W;
+  a.wide = !misaligned(gz, 31) && !misaligned(z, 31) && !misaligned(out, 31);
   if (cin == 16 && cout == 32) launch_conv<16, 32>(a, mode, st);
   else if (cin == 32 && cout == 32) launch_conv<32, 32>(a, mode, st);
   else if (cin == 32 && cout == 16) launch_conv<32, 16>(a, mode, st);
