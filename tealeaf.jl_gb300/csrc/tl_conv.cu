@@ -1360,8 +1360,8 @@ int conv_sm_count() {
 }
 
 // The warp-specialised kernel's producer and epilogue (TEALEAF_GB300_CONV_WS):
-//   0 (default) a tensor copy per row into a 4-slot ring, row-parallel
-//     epilogue, two blocks per SM;
+//   0 (default) a tensor copy per row into a 4-slot ring, the epilogue and the
+//     blocks per SM by what a launch writes (launch_conv_mode);
 //   1 a tensor copy per row, every epilogue warp on every row (half the
 //     channels), three blocks per SM, every mode;
 //   2 cp.async channel chunks into a 6-slot ring with 3 rows ahead, every
@@ -1476,13 +1476,24 @@ void launch_conv_mode(const ConvArgs &a, cudaStream_t st) {
     tc::k_conv3x3_tc<CIN, COUT, MODE><<<grid, 256, smem, st>>>(a);
     return;
   }
-  // The row-parallel epilogue, which moves 64 bytes of a pixel at a time, at two
-  // blocks per SM, forward and input gradient: 84 us each on 32 images of
-  // 256 x 256 (32 -> 32 channels), 29 at 128 x 128, 14.4 on one of 300 x 300.  At
-  // three blocks 89 and 109 (256 x 256); 88 and 100 with every epilogue warp
-  // on every row, a half of the channels each; a ring of six or eight rows, or
-  // eight accumulators, no faster; one block per SM 121 and 135.
+  // Two streams of 64 bytes a pixel beside the input (the forward pass that keeps
+  // z, the input gradient of 32 channels): memory bounds them, and the row-parallel
+  // epilogue, which moves a pixel whole, at two blocks per SM is the fastest at every
+  // size: 29 and 29 us on 32 images of 128 x 128, 145 and 154 at 2048^2; at three
+  // blocks 29 and 37, 160 and 187; every epilogue warp on every row (half the channels
+  // each) at four 33 and 37, 165 and 170.  Rings of six or eight rows or eight
+  // accumulators are no faster, one block per SM takes 39 and 43 at 128 x 128.
+  // With less to write the epilogue's arithmetic bounds a large image, and more
+  // warps hide its latency: at 2048^2 GELU without z at three blocks 115 against
+  // 142, the plain output at four 86 against 115, the input gradient of 16
+  // channels at four 104 against 138.  A small one gains nothing and waits for the
+  // blocks to start: 300^2 12.4, 16.5, 12.4 against 10.3, 14.4, 12.3.  The lines:
+  // GELU 49 both ways at 1024^2 (512 tiles), the others level at 512^2 (128).
   using TmaCfg = tc::WsCfg<4, 1, 4, true, true, 2>;
+  using TmaCfgOut = tc::WsCfg<4, 1, 4, true, MODE == 1, MODE == 1 ? 3 : 4>;
+  const long long tiles = (long long)a.N * ((a.W + FTP - 1) / FTP) * ((a.H + 15) / 16);
+  const bool two_streams = COUT == 32 && (MODE == 2 || (MODE == 1 && a.z));
+  const bool large = tiles >= (MODE == 1 ? 6 : 2) * (long long)conv_sm_count();
   using TmaCfgAll = tc::WsCfg<4, 1, 4, true, false>;
   using CpCfg = tc::WsCfg<6, 3, 4, false>;
   tc::ConvMaps maps;
@@ -1490,7 +1501,8 @@ void launch_conv_mode(const ConvArgs &a, cudaStream_t st) {
   const int cfg = conv_ws_cfg();
   if (cfg != 2 && input_map<CIN>(a, &maps.in)) {
     if (cfg == 1) launch_ws<CIN, COUT, MODE, TmaCfgAll, 3>(a, maps, st);
-    else launch_ws<CIN, COUT, MODE, TmaCfg, 2>(a, maps, st);
+    else if (two_streams || !large) launch_ws<CIN, COUT, MODE, TmaCfg, 2>(a, maps, st);
+    else launch_ws<CIN, COUT, MODE, TmaCfgOut, TmaCfgOut::MINB>(a, maps, st);
   } else {
     launch_ws<CIN, COUT, MODE, CpCfg, 3>(a, maps, st);
   }
