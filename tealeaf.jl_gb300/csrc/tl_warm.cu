@@ -10,7 +10,7 @@
 // u^n + (1 + g)(u^n - u^{n-1})).  With V the basis, the start
 // x = V c minimises ||x - A^{-1} u0||_A over the span, from the Gram system
 // (V^T A V) c = V^T u0: one pass over the fields forms every A v_j on the fly
-// and the m(m+1)/2 + m sums, the host solves the m x m system (m <= 5), and a
+// and the m(m+1)/2 + m sums, the host solves the m x m system (m <= 8), and a
 // second pass forms x.  The span holds the plain start u^n and the linear
 // extrapolation 2u^n - u^{n-1}, so x is never farther from the solution in
 // the A-norm than either; the network's term enters with the weight that
@@ -79,14 +79,14 @@ __global__ void __launch_bounds__(256) k_warm_stats(Fields F, Geom g, const doub
   }
 }
 
-__global__ void k_warm_stats_fold(double *part, int nblk) {
-  double su = 0.0, sd = 0.0;
-  for (int k = 0; k < nblk; ++k) {
-    su += part[2 * k];
-    sd += part[2 * k + 1];
-  }
-  part[2 * nblk] = su;
-  part[2 * nblk + 1] = sd;
+// The sums of n numbers a block over nblk blocks, behind them in `part`: a warp a
+// number, each lane every 32nd block in order, then the lanes.  One thread a
+// number waited for a load a block, 27 to 29 us.
+__global__ void __launch_bounds__(32) k_warm_fold(double *part, int nblk, int n) {
+  double v = 0.0;
+  for (int b = threadIdx.x; b < nblk; b += 32) v += part[(size_t)b * n + blockIdx.x];
+  v = warp_butterfly(v);
+  if (threadIdx.x == 0) part[(size_t)nblk * n + blockIdx.x] = v;
 }
 
 // The projection basis.  Slot 0 holds u^n; slots 1..WARM_HIST the
@@ -108,21 +108,12 @@ struct ProjBasis {
   int nh;                           // increments in the basis (1..WARM_HIST)
 };
 
-// The right-hand sides u^n, u^{n-1}, ... at one cell (zero past nh).
-__device__ __forceinline__ void hist_at(const ProjBasis &B, size_t c, double (&hv)[WARM_HIST + 1]) {
+// The right-hand sides u^n, u^{n-1}, ... at one cell.
+template <int NH>
+__device__ __forceinline__ void hist_at(const ProjBasis &B, size_t c, double (&hv)[NH + 1]) {
   hv[0] = B.u0[c];
 #pragma unroll
-  for (int i = 1; i <= WARM_HIST; ++i) hv[i] = i <= B.nh ? B.h[i - 1][c] : 0.0;
-}
-
-// The basis slots at one cell.
-__device__ __forceinline__ void basis_at(const ProjBasis &B, size_t c, long long k, double (&v)[PROJ_MAX]) {
-  double hv[WARM_HIST + 1];
-  hist_at(B, c, hv);
-  v[0] = hv[0];
-#pragma unroll
-  for (int j = 1; j <= WARM_HIST; ++j) v[j] = j <= B.nh ? hv[j - 1] - hv[j] : 0.0;
-  v[PROJ_NET] = B.gv ? (double)B.gv[k] * (hv[0] - hv[1]) : 0.0;
+  for (int i = 1; i <= NH; ++i) hv[i] = B.h[i - 1][c];
 }
 
 // The 5-point operator in difference form, v + sum k (v - v_nbr), with the
@@ -132,14 +123,21 @@ __device__ __forceinline__ double stencil(double vc, double ve, double vw, doubl
   return vc + kxE * (vc - ve) + kxW * (vc - vw) + kyN * (vc - vn) + kyS * (vc - vs);
 }
 
-// One pass: A v_j at every interior cell for every basis slot, from A of each
-// earlier right-hand side (an increment's A v is the difference of two), and
-// the sums v_a . A v_b (a <= b) and v_a . u0.  Fixed grid and block order:
-// the sums are deterministic.
+// One pass: A v_j at every interior cell for every basis slot in use (NH
+// increments, NET: the network's term), from A of each earlier right-hand side
+// (an increment's A v is the difference of two), and the sums v_a . A v_b
+// (a <= b) and v_a . u0.  Fixed grid and block order: the sums are deterministic.
+//
+// Bound by the FP64 pipe, some 10 instructions a right-hand side and one for
+// each sum.  At 2048^2: 0.35 ms with one increment and the network, 0.28 with
+// two and no network, 0.58, 0.70 and 0.84 with three to five and the network; one
+// kernel for all eight slots took 1.0 ms each time.
+template <int NH, bool NET>
 __global__ void __launch_bounds__(256) k_warm_gram(Fields F, Geom g, ProjBasis B, double *part) {
-  double acc[PROJ_NACC];
+  constexpr int M = 1 + NH + NET, NACC = M * (M + 1) / 2 + M;
+  double acc[NACC];
 #pragma unroll
-  for (int a = 0; a < PROJ_NACC; ++a) acc[a] = 0.0;
+  for (int a = 0; a < NACC; ++a) acc[a] = 0.0;
   const long long n = (long long)g.nx * g.ny;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(k % g.nx), j = (int)(k / g.nx);
@@ -147,79 +145,81 @@ __global__ void __launch_bounds__(256) k_warm_gram(Fields F, Geom g, ProjBasis B
     const size_t cE = i + 1 < g.nx ? c + 1 : c, cW = i > 0 ? c - 1 : c;
     const size_t cN = j + 1 < g.ny ? c + g.pitch : c, cS = j > 0 ? c - g.pitch : c;
     const double kxE = F.kx[c + 1], kxW = F.kx[c], kyN = F.ky[c + g.pitch], kyS = F.ky[c];
-    double hc[WARM_HIST + 1], ah[WARM_HIST + 1];
-    hist_at(B, c, hc);
+    double hc[NH + 1], ah[NH + 1];
+    hist_at<NH>(B, c, hc);
     ah[0] = stencil(hc[0], B.u0[cE], B.u0[cW], B.u0[cN], B.u0[cS], kxE, kxW, kyN, kyS);
 #pragma unroll
-    for (int q = 1; q <= WARM_HIST; ++q) {
-      ah[q] = 0.0;
-      if (q <= B.nh) {
-        const double *h = B.h[q - 1];
-        ah[q] = stencil(hc[q], h[cE], h[cW], h[cN], h[cS], kxE, kxW, kyN, kyS);
-      }
+    for (int q = 1; q <= NH; ++q) {
+      const double *h = B.h[q - 1];
+      ah[q] = stencil(hc[q], h[cE], h[cW], h[cN], h[cS], kxE, kxW, kyN, kyS);
     }
-    double v[PROJ_MAX], av[PROJ_MAX];
+    double v[M], av[M];
     v[0] = hc[0];
     av[0] = ah[0];
 #pragma unroll
-    for (int q = 1; q <= WARM_HIST; ++q) {
-      v[q] = q <= B.nh ? hc[q - 1] - hc[q] : 0.0;
-      av[q] = q <= B.nh ? ah[q - 1] - ah[q] : 0.0;
+    for (int q = 1; q <= NH; ++q) {
+      v[q] = hc[q - 1] - hc[q];
+      av[q] = ah[q - 1] - ah[q];
     }
-    v[PROJ_NET] = av[PROJ_NET] = 0.0;
-    if (B.gv) {
+    if (NET) {
       const long long kE = i + 1 < g.nx ? k + 1 : k, kW = i > 0 ? k - 1 : k;
       const long long kN = j + 1 < g.ny ? k + g.nx : k, kS = j > 0 ? k - g.nx : k;
       const double *h0 = B.h[0];
       auto t = [&](size_t cc, long long kk) { return (double)B.gv[kk] * (B.u0[cc] - h0[cc]); };
-      v[PROJ_NET] = (double)B.gv[k] * (hc[0] - hc[1]);
-      av[PROJ_NET] = stencil(v[PROJ_NET], t(cE, kE), t(cW, kW), t(cN, kN), t(cS, kS), kxE, kxW, kyN, kyS);
+      v[M - 1] = (double)B.gv[k] * (hc[0] - hc[1]);
+      av[M - 1] = stencil(v[M - 1], t(cE, kE), t(cW, kW), t(cN, kN), t(cS, kS), kxE, kxW, kyN, kyS);
     }
     int tt = 0;
 #pragma unroll
-    for (int a = 0; a < PROJ_MAX; ++a)
+    for (int a = 0; a < M; ++a)
 #pragma unroll
-      for (int b = a; b < PROJ_MAX; ++b, ++tt) acc[tt] = fma(v[a], av[b], acc[tt]);
+      for (int b = a; b < M; ++b, ++tt) acc[tt] = fma(v[a], av[b], acc[tt]);
 #pragma unroll
-    for (int a = 0; a < PROJ_MAX; ++a) acc[PROJ_NG + a] = fma(v[a], v[0], acc[PROJ_NG + a]);
+    for (int a = 0; a < M; ++a) acc[tt + a] = fma(v[a], v[0], acc[tt + a]);
   }
-  __shared__ double ws[8][PROJ_NACC];
+  __shared__ double ws[8][NACC];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int a = 0; a < PROJ_NACC; ++a) {
+  for (int a = 0; a < NACC; ++a) {
     const double val = warp_butterfly(acc[a]);
     if (lane == 0) ws[warp][a] = val;
   }
   __syncthreads();
-  if (threadIdx.x < PROJ_NACC) {
+  if (threadIdx.x < NACC) {
     double val = ws[0][threadIdx.x];
     for (int w = 1; w < (int)(blockDim.x >> 5); ++w) val += ws[w][threadIdx.x];
-    part[(size_t)blockIdx.x * PROJ_NACC + threadIdx.x] = val;
+    part[(size_t)blockIdx.x * NACC + threadIdx.x] = val;
   }
-}
-
-__global__ void k_warm_gram_fold(double *part, int nblk) {
-  if (threadIdx.x >= PROJ_NACC) return;
-  double v = 0.0;
-  for (int b = 0; b < nblk; ++b) v += part[(size_t)b * PROJ_NACC + threadIdx.x];
-  part[(size_t)nblk * PROJ_NACC + threadIdx.x] = v;
 }
 
 struct ProjCoef {
   double c[PROJ_MAX];  // zero on the slots not in use
 };
 
-// x = V c on the interior, into ub.
-__global__ void k_warm_combine(Fields F, Geom g, ProjBasis B, ProjCoef C) {
+// x = V c on the interior with its halo: by the history alone (C) into xh and,
+// NET, with the network's term (D) into xn.
+template <int NH, bool NET>
+__global__ void k_warm_combine(Fields F, Geom g, ProjBasis B, ProjCoef C, ProjCoef D, double *xh, double *xn) {
   const long long n = (long long)g.nx * g.ny;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-    const size_t c = g.at((int)(k % g.nx), (int)(k / g.nx));
-    double v[PROJ_MAX];
-    basis_at(B, c, k, v);
-    double x = 0.0;
+    const int i = (int)(k % g.nx), j = (int)(k / g.nx);
+    const size_t c = g.at(i, j);
+    double hv[NH + 1];
+    hist_at<NH>(B, c, hv);
+    double x = fma(C.c[0], hv[0], 0.0), y = NET ? fma(D.c[0], hv[0], 0.0) : 0.0;
 #pragma unroll
-    for (int a = 0; a < PROJ_MAX; ++a) x = fma(C.c[a], v[a], x);
-    F.ub[c] = x;
+    for (int a = 1; a <= NH; ++a) {
+      const double v = hv[a - 1] - hv[a];
+      x = fma(C.c[a], v, x);
+      if (NET) y = fma(D.c[a], v, y);
+    }
+    xh[c] = x;
+    put_faces(xh, g, c, i, j, x);
+    if (NET) {
+      y = fma(D.c[PROJ_NET], (double)B.gv[k] * (hv[0] - hv[1]), y);
+      xn[c] = y;
+      put_faces(xn, g, c, i, j, y);
+    }
   }
 }
 
@@ -241,36 +241,49 @@ __global__ void k_copy_u0(Fields F, Geom g, double *dst) {
   }
 }
 
-// Residual of the candidate: w = u0 - A ub (true residual, 5-point operator), sum w.w;
-// with write 0 only the sum.
+// The candidates' true residuals w = u0 - A x (5-point operator) and their w.w
+// in red[]: N of them, the second in its own buffers.
+template <int N>
 struct OpWarmResid : NoSkip {
   Fields F;
   Geom g;
-  int write;  // 0: the norm only
-  __device__ void cell(int i, int j, double (&acc)[1]) const {
+  const double *x[N];
+  double *w[N];
+  __device__ void cell(int i, int j, double (&acc)[N]) const {
     const size_t c = g.at(i, j);
-    const double t = dsub(F.u0[c], smvp_exact(F, g, F.ub, c, TL_MODE_TEALEAF));
-    if (write) F.w[c] = t;
-    acc[0] = dadd(acc[0], dmul(t, t));
+#pragma unroll
+    for (int m = 0; m < N; ++m) {
+      const double t = dsub(F.u0[c], smvp_exact(F, g, x[m], c, TL_MODE_TEALEAF));
+      w[m][c] = t;
+      acc[m] = dadd(acc[m], dmul(t, t));
+    }
   }
-  __device__ void tile(int i0, int j0, int j1, double (&acc)[1]) const {
+  __device__ void tile(int i0, int j0, int j1, double (&acc)[N]) const {
     for (int j = j0; j < j1; ++j) {
       if (i0 < g.nx) cell(i0, j, acc);
       if (i0 + 1 < g.nx) cell(i0 + 1, j, acc);
     }
   }
-  __device__ void fin(const double *tot) const { F.sc->red[0] = tot[0]; }
+  __device__ void fin(const double *tot) const {
+    for (int m = 0; m < N; ++m) F.sc->red[m] = tot[m];
+  }
 };
 
-// The prediction won: r = p = w and rr = its r.r.
-__global__ void k_warm_accept(Fields F, Geom g) {
-  const long long n = (long long)g.nx * g.ny;
+// A prediction won: u = x, r = p = w, with their halo, and rr = its r.r (red[m]).
+__global__ void k_warm_accept(Fields F, Geom g, const double *x, const double *w, int m) {
+  const long long n = (long long)g.X * g.Y;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-    const size_t c = g.at((int)(k % g.nx), (int)(k / g.nx));
-    F.r[c] = F.w[c];
-    F.p[c] = F.w[c];
+    const int i = (int)(k % g.X) - g.hd, j = (int)(k / g.X) - g.hd;
+    const size_t c = g.full(i + g.hd, j + g.hd);
+    F.u[c] = x[c];
+    if (i >= 0 && i < g.nx && j >= 0 && j < g.ny) {
+      const double v = w[c];
+      F.r[c] = v;
+      F.p[c] = v;
+      put_faces(F.p, g, c, i, j, v);
+    }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) F.sc->rro = F.sc->red[0];
+  if (blockIdx.x == 0 && threadIdx.x == 0) F.sc->rro = F.sc->red[m];
 }
 
 __global__ void k_to_bf16(const float *src, __nv_bfloat16 *dst, int n) {
@@ -393,7 +406,7 @@ static int run_network(tl_ctx *ctx, double rx, double ry) {
   const Fields &F = ctx->F;
   cudaStream_t st = ctx->stream;
   k_warm_stats<<<STAT_BLOCKS, 256, 0, st>>>(F, g, ws->hist[0], ws->stats);
-  k_warm_stats_fold<<<1, 1, 0, st>>>(ws->stats, STAT_BLOCKS);
+  k_warm_fold<<<2, 32, 0, st>>>(ws->stats, STAT_BLOCKS, 2);
   CKL();
   double tot[2];
   CK(cudaMemcpyAsync(tot, ws->stats + 2 * STAT_BLOCKS, sizeof tot, cudaMemcpyDeviceToHost, st));
@@ -515,43 +528,64 @@ static int solve_dense(int m, const double *G, const double *h, double *c) {
   return 1;
 }
 
-// x = V c into ub, its halo, and ||u0 - A x||^2 (with `write`, the residual
-// itself into w for accept_candidate).
-static int candidate_residual(tl_ctx *ctx, const ProjBasis &B, const ProjCoef &C, int write, double *rr) {
-  const Geom &g = ctx->g;
-  const Fields &F = ctx->F;
-  cudaStream_t st = ctx->stream;
-  k_warm_combine<<<grid_cells(g), 256, 0, st>>>(F, g, B, C);
+// The kernels for the basis in use.
+struct BasisKernels {
+  void (*gram)(Fields, Geom, ProjBasis, double *);
+  void (*combine)(Fields, Geom, ProjBasis, ProjCoef, ProjCoef, double *, double *);
+};
+template <bool NET>
+static BasisKernels basis_kernels(int nh) {
+  static const BasisKernels all[WARM_HIST] = {
+      {k_warm_gram<1, NET>, k_warm_combine<1, NET>}, {k_warm_gram<2, NET>, k_warm_combine<2, NET>},
+      {k_warm_gram<3, NET>, k_warm_combine<3, NET>}, {k_warm_gram<4, NET>, k_warm_combine<4, NET>},
+      {k_warm_gram<5, NET>, k_warm_combine<5, NET>}, {k_warm_gram<6, NET>, k_warm_combine<6, NET>}};
+  return all[nh - 1];
+}
+
+// Where the candidates and their residuals go: by the history alone, and with
+// the network.
+static double *candidate_x(const Fields &F, int m) { return m ? F.sdb : F.ub; }
+static double *candidate_w(const Fields &F, int m) { return m ? F.pb : F.w; }
+
+template <int N>
+static int launch_resid(tl_ctx *ctx) {
+  OpWarmResid<N> op;
+  op.F = ctx->F;
+  op.g = ctx->g;
+  for (int m = 0; m < N; ++m) {
+    op.x[m] = candidate_x(ctx->F, m);
+    op.w[m] = candidate_w(ctx->F, m);
+  }
+  launch_walk<N>(ctx->stream, op, ctx->walk_exact, ctx->g.ny);
   CKL();
-  double *ub = F.ub;
-  launch_halo(st, &ub, 1, g, 1, TL_MODE_TEALEAF);
+  ctx->launches += 1;
+  return tl_read_scalars(ctx);
+}
+
+// x = V c with its halo, its residual and ||u0 - A x||^2: of the candidate by
+// the history alone and, with `net`, of the one with the network's term (both in
+// one pass; a third pass over the winner, and the halos, had their own kernels).
+static int candidate_residuals(tl_ctx *ctx, const ProjBasis &B, const ProjCoef &Ch, const ProjCoef &Cn, int net,
+                               double (&rr)[2]) {
+  const BasisKernels K = net ? basis_kernels<true>(B.nh) : basis_kernels<false>(B.nh);
+  K.combine<<<grid_cells(ctx->g), 256, 0, ctx->stream>>>(ctx->F, ctx->g, B, Ch, Cn, candidate_x(ctx->F, 0),
+                                                         candidate_x(ctx->F, 1));
   CKL();
-  OpWarmResid op;
-  op.F = F;
-  op.g = g;
-  op.write = write;
-  launch_walk<1>(st, op, ctx->walk_exact, g.ny);
-  CKL();
-  ctx->launches += 3;
-  int rc = tl_read_scalars(ctx);
+  ctx->launches += 1;
+  int rc = net ? launch_resid<2>(ctx) : launch_resid<1>(ctx);
   if (rc) return rc;
-  *rr = ctx->host_sc->red[0];
+  rr[0] = ctx->host_sc->red[0];
+  rr[1] = ctx->host_sc->red[1];
   return TL_OK;
 }
 
-// The candidate in ub (its residual in w) becomes the start: u = ub,
-// r = p = w, rr = its r.r, and the halo of u, p.
-static int accept_candidate(tl_ctx *ctx) {
-  const Geom &g = ctx->g;
-  const Fields &F = ctx->F;
-  cudaStream_t st = ctx->stream;
-  launch_copy_full(st, F.u, F.ub, g);
-  k_warm_accept<<<grid_cells(g), 256, 0, st>>>(F, g);
+// Candidate m becomes the start: u, r = p = its residual, rr, the halo of u, p.
+static int accept_candidate(tl_ctx *ctx, int m) {
+  k_warm_accept<<<grid_cells(ctx->g), 256, 0, ctx->stream>>>(ctx->F, ctx->g, candidate_x(ctx->F, m),
+                                                             candidate_w(ctx->F, m), m);
   CKL();
-  const int up[2] = {TL_EX_U, TL_EX_P};
-  int rc = tl_halo_update(ctx, 1, up, 2, 1);
-  if (rc) return rc;
-  ctx->launches += 3;
+  for (int k = 0; k < TL_NEX; ++k) ctx->toexchange[k] = k == TL_EX_U || k == TL_EX_P;
+  ctx->launches += 1;
   return TL_OK;
 }
 
@@ -605,17 +639,21 @@ int tl_warm_try(tl_ctx *ctx, double rx, double ry, int warmstart, tl_result *res
       if (nrc < 0) return -nrc;
       if (nrc == 0) B.gv = ws->g;
     }
-    k_warm_gram<<<GRAM_BLOCKS, 256, 0, st>>>(F, g, B, ws->gram);
-    k_warm_gram_fold<<<1, 64, 0, st>>>(ws->gram, GRAM_BLOCKS);
+    const BasisKernels K = B.gv ? basis_kernels<true>(B.nh) : basis_kernels<false>(B.nh);
+    const int m = 1 + B.nh + (B.gv ? 1 : 0), nacc = m * (m + 1) / 2 + m;
+    K.gram<<<GRAM_BLOCKS, 256, 0, st>>>(F, g, B, ws->gram);
+    k_warm_fold<<<nacc, 32, 0, st>>>(ws->gram, GRAM_BLOCKS, nacc);
     CKL();
     ctx->launches += 2;
     double tot[PROJ_NACC];
-    CK(cudaMemcpyAsync(tot, ws->gram + (size_t)GRAM_BLOCKS * PROJ_NACC, sizeof tot, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(tot, ws->gram + (size_t)GRAM_BLOCKS * nacc, sizeof(double) * nacc, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     double G[PROJ_MAX * PROJ_MAX] = {}, h[PROJ_MAX] = {};
-    for (int a = 0, t = 0; a < PROJ_MAX; ++a)
-      for (int b = a; b < PROJ_MAX; ++b, ++t) G[a * PROJ_MAX + b] = G[b * PROJ_MAX + a] = tot[t];
-    for (int a = 0; a < PROJ_MAX; ++a) h[a] = tot[PROJ_NG + a];
+    auto place = [&](int q) { return q <= B.nh ? q : PROJ_NET; };
+    int t = 0;
+    for (int a = 0; a < m; ++a)
+      for (int b = a; b < m; ++b, ++t) G[place(a) * PROJ_MAX + place(b)] = G[place(b) * PROJ_MAX + place(a)] = tot[t];
+    for (int a = 0; a < m; ++a) h[place(a)] = tot[t + a];
     // the history-only projection (slots 0..nh), and with the network the
     // full one; the network's term is kept only when its candidate's
     // residual is below the history-only candidate's
@@ -627,11 +665,10 @@ int tl_warm_try(tl_ctx *ctx, double rx, double ry, int warmstart, tl_result *res
     const int okh = solve_gram(mh, slot, G, h, Ch.c);
     const int okn = B.gv ? solve_gram(mh + 1, slot, G, h, Cn.c) : 0;
     const ProjCoef *chosen = nullptr;
+    double rr[2] = {0.0, 0.0};
+    if (okh && (rc = candidate_residuals(ctx, B, Ch, Cn, okn, rr))) return rc;
     if (okh && okn) {
-      double rr_h = 0.0, rr_n = 0.0;
-      if ((rc = candidate_residual(ctx, B, Ch, 0, &rr_h))) return rc;
-      if ((rc = candidate_residual(ctx, B, Cn, 0, &rr_n))) return rc;
-      if (rr_n < rr_h) {
+      if (rr[1] < rr[0]) {
         chosen = &Cn;
         res->warm = 1;
         ws->net_backoff = 1;
@@ -647,8 +684,8 @@ int tl_warm_try(tl_ctx *ctx, double rx, double ry, int warmstart, tl_result *res
       res->warm = network ? 3 : 1;
     }
     if (chosen) {
-      double rr_pred = 0.0;
-      if ((rc = candidate_residual(ctx, B, *chosen, 1, &rr_pred))) return rc;
+      const int which = chosen == &Cn;
+      const double rr_pred = rr[which];
       // weights on u^n, u^{n-1}, ...: x = c0 u^n + sum_j c_j (u^{n-j+1} - u^{n-j}) + c_net t
       const double *cc = chosen->c;
       res->warm_coef[0] = cc[0] + cc[1];
@@ -656,7 +693,7 @@ int tl_warm_try(tl_ctx *ctx, double rx, double ry, int warmstart, tl_result *res
       res->warm_coef[TL_WARM_HIST + 1] = cc[PROJ_NET];
       res->r0_pred = bb > 0 ? sqrt(rr_pred / bb) : sqrt(rr_pred);
       if (rr_pred < rr_plain) {
-        if ((rc = accept_candidate(ctx))) return rc;
+        if ((rc = accept_candidate(ctx, which))) return rc;
       } else {
         res->warm = 2;
       }
@@ -666,18 +703,12 @@ int tl_warm_try(tl_ctx *ctx, double rx, double ry, int warmstart, tl_result *res
     double *ub = F.ub;
     launch_halo(st, &ub, 1, g, 1, TL_MODE_TEALEAF);
     CKL();
-    OpWarmResid op;
-    op.F = F;
-    op.g = g;
-    op.write = 1;
-    launch_walk<1>(st, op, ctx->walk_exact, g.ny);
-    CKL();
-    ctx->launches += 2;
-    if ((rc = tl_read_scalars(ctx))) return rc;
+    ctx->launches += 1;
+    if ((rc = launch_resid<1>(ctx))) return rc;
     const double rr_pred = ctx->host_sc->red[0];
     res->r0_pred = bb > 0 ? sqrt(rr_pred / bb) : sqrt(rr_pred);
     if (rr_pred < rr_plain) {
-      if ((rc = accept_candidate(ctx))) return rc;
+      if ((rc = accept_candidate(ctx, 0))) return rc;
       res->warm = 1;
     } else {
       res->warm = 2;
