@@ -76,9 +76,9 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_batch_64(const Cg64 *decks,
   extern __shared__ __align__(128) unsigned char ring_mem[];
   __shared__ Shared64 S;
   __shared__ Cg64 A;
-  const unsigned ring = (unsigned)__cvta_generic_to_shared(ring_mem) + (threadIdx.x >> 5) * RING64_BYTES;
+  const Mem64 mem(ring_mem);
   take_decks(decks, A, Q, n, size, [](const Cg64 &a) { return a.tw.blocks; },
-             [&](Grid g) { return cg64_solve(g, A, S, ring); });
+             [&](Grid g) { return cg64_solve(g, A, S, mem); });
 }
 
 // When the last deck ends with `groups` groups of sms/groups blocks, in
@@ -258,8 +258,7 @@ int batch_solve(tl_batch *b, const double *rx, const double *ry, const tl_params
     rc = run_decks(b, (const void *)k_batch_ir, b->d32, b->groups32, b->size32, PERSIST_THREADS,
                    (size_t)RING_BYTES * PERSIST_WARPS);
   } else if (p.maxiters >= 1) {
-    rc = run_decks(b, (const void *)k_batch_64, b->d64, b->groups64, b->size64, WARPS64 * 32,
-                   (size_t)RING64_BYTES * WARPS64);
+    rc = run_decks(b, (const void *)k_batch_64, b->d64, b->groups64, b->size64, WARPS64 * 32, CG64_SMEM);
   }
   if (rc) return rc;
   // per deck, FP32, the halo of u, p and, FP64 under the relative criterion, the

@@ -7,7 +7,7 @@ namespace {
 __global__ void __launch_bounds__(WARPS64 * 32, 1) k_cg64(const Cg64 A) {
   extern __shared__ __align__(128) unsigned char ring_mem[];
   __shared__ Shared64 S;
-  cg64_solve(whole_grid(), A, S, (unsigned)__cvta_generic_to_shared(ring_mem) + (threadIdx.x >> 5) * RING64_BYTES);
+  cg64_solve(whole_grid(), A, S, Mem64(ring_mem));
 }
 
 }  // namespace
@@ -25,7 +25,7 @@ int tl_cg64_run(tl_ctx *ctx, int check, double *ms) {
   A.sums = static_cast<GridSums *>(ctx->grid_sums);
   A.check = check;
   cg64_tilings(A, persist_blocks(ctx->sm_count));
-  const size_t smem = (size_t)RING64_BYTES * WARPS64;
+  const size_t smem = CG64_SMEM;
   CK(cudaFuncSetAttribute(k_cg64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int rc = tl_bar_ready(ctx);
   if (rc) return rc;

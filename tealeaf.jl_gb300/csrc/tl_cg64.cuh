@@ -25,11 +25,28 @@ struct Cg64 {
   Tiling tw, tr;  // W (strips of 60 columns), R (64)
   GridSums *sums;
   int check;  // the relative test before the first iteration
+  int keep;   // every warp has one tile of KEEP_ROWS rows at most: R works on what W left in shared memory
+};
+
+// Small decks: with one row a warp, r is still in W's ring and w goes beside it, so
+// that R waits for no load and w for no store: 7.1 us an iteration at 64^2 against
+// 7.7, 8.2 against 8.7 at 256^2 (beta's division, formed with alpha's, among it).
+// With two rows a warp it gains nothing (12.9 both ways at 512^2).
+constexpr int KEEP_ROWS = 1, KEEP_BYTES = KEEP_ROWS * 512;
+constexpr int CG64_SMEM = WARPS64 * (RING64_BYTES + KEEP_BYTES);
+// This warp's ring, and where it keeps w.
+struct Mem64 {
+  unsigned ring, w;
+  __device__ __forceinline__ explicit Mem64(const void *smem) {
+    const unsigned base = (unsigned)__cvta_generic_to_shared(smem), warp = threadIdx.x >> 5;
+    ring = base + warp * RING64_BYTES;
+    w = base + WARPS64 * RING64_BYTES + warp * KEEP_BYTES;
+  }
 };
 
 struct Shared64 {
   SumShared sum;
-  double alpha, beta, err;
+  double alpha, beta, err, inv_rro;
   int done, conv, sw;
 };
 
@@ -82,8 +99,30 @@ __device__ __forceinline__ Fixed r_pass(Grid grid, const Cg64 &A, unsigned ring,
   return sum;
 }
 
-// The loop on one deck by the blocks of `grid`; false when a wait gave up.
-__device__ __forceinline__ bool cg64_solve(Grid grid, const Cg64 &A, Shared64 &S, unsigned ring) {
+// The same on the one tile (j0 < 0: none) that this warp's W left in shared memory,
+// in a ring of `arrays` operands a row.
+__device__ __forceinline__ Fixed r_kept(const Cg64 &A, const Mem64 &mem, int strip, int j0, int j1, int arrays,
+                                        double alpha, int scale) {
+  const int lane = threadIdx.x & 31;
+  if (j0 < 0) return 0;
+  const int i0 = strip * STRIP64 - 2 + 2 * lane;
+  if (lane < 1 || lane > 30 || i0 >= A.g.nx) return 0;
+  const bool has1 = i0 + 1 < A.g.nx;
+  double acc = 0.0;
+  for (int j = j0; j < j1; ++j) {
+    double2 r = lds2d(mem.ring + 16 * lane + ((j - j0 + 1) * arrays + 1) * 512);
+    const double2 w = lds2d(mem.w + 16 * lane + (j - j0) * 512);
+    r = make_double2(fma(-alpha, w.x, r.x), fma(-alpha, w.y, r.y));
+    if (!has1) r.y = 0.0;
+    acc = fma(r.y, r.y, fma(r.x, r.x, acc));
+    put64(A.F.r + A.g.at(i0, j), r, has1);
+  }
+  return to_fixed(acc, scale);
+}
+
+template <bool KEEP>
+__device__ __forceinline__ bool cg64_loop(Grid grid, const Cg64 &A, Shared64 &S, const Mem64 &mem) {
+  const unsigned ring = mem.ring;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool lead = grid.id == 0 && threadIdx.x == 0;
   DevScalars *sc = A.F.sc;
@@ -98,6 +137,11 @@ __device__ __forceinline__ bool cg64_solve(Grid grid, const Cg64 &A, Shared64 &S
   int iter = sc->iter;
   bool first = true, mirrored = false;
   unsigned target = 0, set = 0, handed = 0;
+  int tile0 = -1, tile1 = -1, tile_strip = 0;  // with `keep`, this warp's tile
+  if (KEEP) {
+    const TileWalk walk(grid, A.tw, A.g.ny, false, nullptr, 0);
+    if (walk.valid()) walk.place(tile_strip, tile0, tile1);
+  }
   for (;;) {
     // W
     Ring64 q;
@@ -117,12 +161,14 @@ __device__ __forceinline__ bool cg64_solve(Grid grid, const Cg64 &A, Shared64 &S
       sum += to_fixed(acc, scale);
       acc = 0.0;
     };
+    const int arrays = first ? 5 : 6;
     auto direction = [&](int j, int i0, bool has1, bool owns, const Row64 &o) {
       const double2 w = apply64(o, has1);
       if (owns) {
         const size_t c = A.g.at(i0, j);
         acc = fma(w.y, o.c.y, fma(w.x, o.c.x, acc));
-        put64(A.F.w + c, w, has1);
+        if (KEEP) sts2d(mem.w + 16 * lane + (j - tile0) * 512, w);
+        else put64(A.F.w + c, w, has1);
         put64(pn + c, o.c, has1);
       }
     };
@@ -139,17 +185,19 @@ __device__ __forceinline__ bool cg64_solve(Grid grid, const Cg64 &A, Shared64 &S
                       tile_end);
     }
     if (!grid_sum1(grid, S.sum, bar, A.sums, warp_fixed(sum), scale, target, set, [&](double pw) {
-          const double a = ddiv(rro, pw);
+          const double a = ddiv(lane == 0 ? rro : 1.0, lane == 0 ? pw : rro);  // and 1/rro for beta, in one division
           if (lane == 0) {
             S.alpha = a;
             S.err = pw;
+          } else if (lane == 1) {
+            S.inv_rro = a;
           }
           if (lead && iter < maxiters) A.F.cgalpha[iter + 1] = a;  // table holds maxiters + 2 entries
         }))
       return false;
     alpha = S.alpha;
     pw_ref = S.err;
-    mirrored = !mirrored;
+    mirrored = !mirrored && !KEEP;
     {
       double *t = p;
       p = pn;
@@ -157,9 +205,13 @@ __device__ __forceinline__ bool cg64_solve(Grid grid, const Cg64 &A, Shared64 &S
     }
     // R
     scale = fixed_scale(rr);
-    sum = r_pass(grid, A, ring, mirrored, alpha, scale, handed);
+    sum = KEEP ? r_kept(A, mem, tile_strip, tile0, tile1, arrays, alpha, scale)
+                 : r_pass(grid, A, ring, mirrored, alpha, scale, handed);
     if (!grid_sum1(grid, S.sum, bar, A.sums, warp_fixed(sum), scale, target, set, [&](double rrn) {
-          const double b = ddiv(rrn, rro);
+          // rrn / rro from the reciprocal formed before, with one correction (Markstein's), away from its ends
+          double b = rrn * S.inv_rro;
+          if (rro > 1e-290 && rro < 1e290) b = fma(fma(-b, rro, rrn), S.inv_rro, b);
+          else b = ddiv(rrn, rro);
           const bool conv = rooted ? test.met(rrn) : below(rrn, eps);
           bool sw = false;
           if (!conv && rule == 1) {  // Cheby.jl:25-29, PPCG.jl:27-31
@@ -178,10 +230,17 @@ __device__ __forceinline__ bool cg64_solve(Grid grid, const Cg64 &A, Shared64 &S
       return false;
     beta = S.beta;
     rro = rr = S.err;
-    mirrored = !mirrored;
+    mirrored = !mirrored && !KEEP;
     first = false;
     ++iter;
     if (S.done) break;
+  }
+  if (KEEP && tile0 >= 0) {  // the last step's w
+    for (int j = tile0; j < tile1; ++j) {
+      const int i0 = tile_strip * STRIP64 - 2 + 2 * lane;
+      if (lane >= 1 && lane <= 30 && i0 < A.g.nx)
+        put64(A.F.w + A.g.at(i0, j), lds2d(mem.w + 16 * lane + (j - tile0) * 512), i0 + 1 < A.g.nx);
+    }
   }
   // the last step's u, and p! of the next one (CG.jl:22), with their halo
   const int nx = A.g.nx, ny = A.g.ny, chunks = (nx + 63) / 64;
@@ -222,15 +281,21 @@ __device__ __forceinline__ bool cg64_solve(Grid grid, const Cg64 &A, Shared64 &S
   return true;
 }
 
+// The loop on one deck by the blocks of `grid`; false when a wait gave up.
+__device__ __forceinline__ bool cg64_solve(Grid grid, const Cg64 &A, Shared64 &S, const Mem64 &mem) {
+  return A.keep ? cg64_loop<true>(grid, A, S, mem) : cg64_loop<false>(grid, A, S, mem);
+}
+
 // Tilings for `blocks` blocks at most.
 inline void cg64_tilings(Cg64 &A, int blocks) {
   // A row of W holds the FP64 pipe for 17 x 64 cycles, of R for 4 x 64.  W's
   // shares are even up to 48 rows a warp: there its tiles are the coarser, the
   // better (93 us an iteration at 2048^2 against 105-113 with any tiles handed
   // out); beyond, what the SMs get of HBM differs (326 against 401 at 4096^2).
-  const TileCost w{0.25, 1100.0, 1500.0, 1100.0, 200.0, 32, 48, 4}, r{0.0, 300.0, 1000.0, 260.0, 150.0, 0, 24, 8};
+  const TileCost w{0.25, 1100.0, 1500.0, 1100.0, 200.0, 16, 48, 4}, r{0.0, 300.0, 1000.0, 260.0, 150.0, 0, 24, 8};
   A.tw = make_tiling(A.g.nx, A.g.ny, STRIP64, w, blocks, WARPS64);
   A.tr = make_tiling_on(A.tw, A.g.nx, A.g.ny, 64, r, WARPS64);
+  A.keep = !A.tw.handed && A.tw.tiles <= A.tw.warps && A.tw.rows <= KEEP_ROWS;
 }
 
 }  // namespace

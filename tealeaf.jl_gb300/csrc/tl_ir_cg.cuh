@@ -505,7 +505,7 @@ inline void ir_cg_args(IrCg &A, tl_ctx *ctx, int blocks) {
   A.delta2 = IR_DELTA * IR_DELTA;
   A.sums = static_cast<GridSums *>(ctx->grid_sums);
   // cycles and issue slots of a row and a tile, from the kernel's own counters
-  const TileCost pass{2.0, 300.0, 1500.0, 200.0, 400.0, 32, 24, 8}, resid{1.0, 1200.0, 1500.0, 1100.0, 200.0, 0, 48, 4};
+  const TileCost pass{2.0, 300.0, 1500.0, 200.0, 400.0, 16, 24, 8}, resid{1.0, 1200.0, 1500.0, 1100.0, 200.0, 0, 48, 4};
   A.t = make_tiling(ctx->g.nx, ctx->g.ny, STRIP, pass, blocks, PERSIST_WARPS);
   if (ir->set_rows) {  // tl_set_layout: equal shares of bands of these rows
     A.t.rows = ir->set_rows < ctx->g.ny ? ir->set_rows : ctx->g.ny;

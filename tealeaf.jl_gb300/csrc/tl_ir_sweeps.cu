@@ -617,7 +617,7 @@ IrSweeps sweep_args(tl_ctx *ctx, int ninner, double rr) {
   A.rr = rr;
   A.sums = static_cast<GridSums *>(ctx->grid_sums);
   // a row takes both steps' arithmetic; see tl_ir_cg.cuh for the rule
-  const TileCost pass{3.0, 450.0, 1500.0, 300.0, 400.0, 32, 24, 8}, resid{1.0, 1200.0, 1500.0, 1100.0, 200.0, 0, 48, 4};
+  const TileCost pass{3.0, 450.0, 1500.0, 300.0, 400.0, 16, 24, 8}, resid{1.0, 1200.0, 1500.0, 1100.0, 200.0, 0, 48, 4};
   A.t = make_tiling(ctx->g.nx, ctx->g.ny, STRIP, pass, persist_blocks(ctx->sm_count), PERSIST_WARPS);
   A.t64 = make_tiling_on(A.t, ctx->g.nx, ctx->g.ny, 64, resid, PERSIST_WARPS);
   return A;

@@ -363,6 +363,9 @@ __device__ __forceinline__ float4 lds4(unsigned a) {
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
   return v;
 }
+__device__ __forceinline__ void sts2d(unsigned a, double2 v) {
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
+}
 __device__ __forceinline__ double2 lds2d(unsigned a) {
   double2 v;
   asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
@@ -431,7 +434,8 @@ inline int persist_blocks(int sm_count) { return sm_count < PERSIST_MAX_BLOCKS ?
 // out.  A tile takes `lat` cycles a row and `lat0` besides when its warp runs
 // alone, `issue` and `issue0` of a sub-partition's issue (or FP64) slots; `extra`
 // rows overlap the next tile.  A deck of at most `solo` strip rows runs on one
-// block, which needs no grid barrier.
+// block, which needs no grid barrier: a row a warp (28^2 by FP64 CG: 8.1 us an
+// iteration spread over blocks, 10.6 with two rows a warp on one).
 struct TileCost {
   double extra, lat, lat0, issue, issue0;
   int solo, hand_from, rows2;

@@ -664,7 +664,7 @@ int tl_loop64_run(tl_ctx *ctx, int which, int ninner, double *ms) {
                        : which == TL_GRAPH_PPCG_EXACT ? (const void *)k_ppcg64
                                                       : (const void *)k_jacobi64;
   // a row holds the FP64 pipe for 14 to 20 instructions of 64 cycles; see tl_cg64_run for the rule
-  const TileCost sweep{0.1, 1200.0, 1500.0, 1150.0, 200.0, 32, 48, 4}, each{0.0, 500.0, 1000.0, 400.0, 150.0, 0, 24, 8};
+  const TileCost sweep{0.1, 1200.0, 1500.0, 1150.0, 200.0, 16, 48, 4}, each{0.0, 500.0, 1000.0, 400.0, 150.0, 0, 24, 8};
   A.t = make_tiling(ctx->g.nx, ctx->g.ny, STRIP64, sweep, blocks, WARPS64);
   A.te = make_tiling_on(A.t, ctx->g.nx, ctx->g.ny, 64, each, WARPS64);
   return run_loop(ctx, kernel, A.t.blocks, &A, (size_t)RING64_BYTES * WARPS64, ms);

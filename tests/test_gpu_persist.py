@@ -239,3 +239,30 @@ def test_jacobi_pairs(tl, built_lib, nx, ny, iters, eps):
     at_check = b.iters % 50 == 0
     assert np.max(np.abs(r - s)) <= 1e-13 * scale * (k if at_check else 1)
     assert abs(a.error - b.error) <= 1e-9 * abs(b.error) + 1e-13 * scale * nx * ny
+
+
+@pytest.mark.parametrize("nx,ny", [(1, 1), (60, 16), (60, 17), (61, 8), (61, 9), (300, 480), (300, 487), (540, 271)])
+@pytest.mark.parametrize("iters", [1, 2, 7])
+def test_fp64_cg_one_row_a_warp(tl, built_lib, nx, ny, iters):
+    """FP64 CG where a warp has one row (r and w stay with it between the passes)
+    and on either side of that line, stopped early: u, p, r and w of the last
+    step against the exact loop's.  Their roundings, some 1e-16 of a vector a step
+    before the residual's own fall (by less than 1e3 in seven steps of these
+    decks) scales them up, stay below 1e-9 of its norm."""
+    text = random_deck(nx, 85, ny=ny, nrect=4, steps=1, eps=1e-300).replace("max_iters=5000", f"max_iters={iters}")
+    f = []
+    for exact in (False, True):
+        s = tl.Settings.from_text(text, mode=TEA, exact=exact)
+        c = tl.initialiseapp(s)
+        tl.haloupdate(c, s, 1, ["energy", "density"])
+        res = tl.CG.solve(c, s, s.dtinit / s.dx ** 2, s.dtinit / s.dy ** 2)
+        f.append(({k: c.field(k) for k in ("u", "p", "r", "w")}, res))
+        c.close()
+    (a, ra), (b, rb) = f
+    if min(nx, ny) > 1:
+        assert ra.iters == rb.iters == iters
+        for k in "uprw":
+            x, y = _interior(a[k], 1 if k in "up" else 2), _interior(b[k], 1 if k in "up" else 2)
+            assert np.linalg.norm(x - y) <= 1e-9 * np.linalg.norm(y), k
+    else:
+        assert np.max(np.abs(_interior(a["u"]) - _interior(b["u"]))) <= 1e-14 * np.max(np.abs(b["u"]))
