@@ -63,7 +63,7 @@ __device__ __forceinline__ float4 f4(float a, float b, float c, float d) { retur
 
 // One pass over the grid: this warp's share of gamma, the face sums and rho in
 // lanes 0, 8 and 16, as whole numbers where tiles are handed out, else as pairs.
-template <int PASS>
+template <int PASS, bool FIXED>
 __device__ __forceinline__ void ir_pass(Grid grid, const IrCg &A, const PassArgs &q, unsigned ring, float rxh, float ryh,
                                         int scale, unsigned &handed, Fixed &sum, Pair &tile) {
   constexpr int NARR = PASS == PASS_STEP2 ? 6 : 3;
@@ -73,7 +73,6 @@ __device__ __forceinline__ void ir_pass(Grid grid, const IrCg &A, const PassArgs
   const unsigned slot0 = ring + 16 * lane;
   sum = 0;
   tile = Pair{0.f, 0.f};
-  const bool fixed_tiles = A.t.tiles <= A.t.warps;  // one each
   TileWalk walk(grid, A.t, ny, q.mirrored, &A.F.sc->bar.next_tile, handed);
   handed += walk.requests();
   while (walk.valid()) {
@@ -204,7 +203,7 @@ __device__ __forceinline__ void ir_pass(Grid grid, const IrCg &A, const PassArgs
       if (lane == 0 || lane == 31) acc[d] = Pair{0.f, 0.f};
     }
     tile = warp_pairs(acc);
-    if (!fixed_tiles) sum += to_fixed(tile.hi, scale) + to_fixed(tile.lo, scale);
+    if (FIXED) sum += to_fixed(tile.hi, scale) + to_fixed(tile.lo, scale);
     walk.take(asked);
   }
 }
@@ -337,8 +336,9 @@ __device__ __forceinline__ void next_scalars(Shared &S, double gamma, double bet
   }
 }
 
-// The solve of one deck by the blocks of `grid`; false when a wait gave up.
-__device__ __forceinline__ bool ir_solve(Grid grid, const IrCg &A, Shared &S, unsigned ring) {
+// FIXED: tiles are handed out or several a warp, and the sums are whole numbers.
+template <bool FIXED>
+__device__ __forceinline__ bool ir_loop(Grid grid, const IrCg &A, Shared &S, unsigned ring) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int warps = grid.nb * PERSIST_WARPS, me = grid.id * PERSIST_WARPS + warp;
   GridBar *bar = &A.F.sc->bar;
@@ -357,7 +357,6 @@ __device__ __forceinline__ bool ir_solve(Grid grid, const IrCg &A, Shared &S, un
   bool sv = false, pv = false, xv = false, pend = false, mirrored = false;
   float alpha0 = 0.f, beta0 = 0.f;
   unsigned target = 0, set = 0, handed = 0;
-  const bool fixed_tiles = A.t.tiles <= A.t.warps;
   double beta = 0.0, err = 0.0;
   if (threadIdx.x == 0) S.sigma = 0.0;
   __syncthreads();
@@ -374,11 +373,9 @@ __device__ __forceinline__ bool ir_solve(Grid grid, const IrCg &A, Shared &S, un
       const int scale = fixed_scale(ref);
       Fixed v;
       Pair w;
-      ir_pass<PASS_START>(grid, A, q, ring, rxh, ryh, scale, handed, v, w);
+      ir_pass<PASS_START, FIXED>(grid, A, q, ring, rxh, ryh, scale, handed, v, w);
       auto fin = [&](double, double f, double r) { next_scalars(S, rr, beta, rr + f, r); };
-      if (!(fixed_tiles ? grid_sum3<false>(grid, S.sum, bar, A.sums, v, scale, w, target, set, fin)
-                        : grid_sum3<true>(grid, S.sum, bar, A.sums, v, scale, w, target, set, fin)))
-        return false;
+      if (!grid_sum3<FIXED>(grid, S.sum, bar, A.sums, v, scale, w, target, set, fin)) return false;
       mirrored = !mirrored;
     }
     for (;;) {
@@ -399,8 +396,8 @@ __device__ __forceinline__ bool ir_solve(Grid grid, const IrCg &A, Shared &S, un
       const int scale = fixed_scale(ref);
       Fixed v;
       Pair w;
-      if (pend) ir_pass<PASS_STEP2>(grid, A, q, ring, rxh, ryh, scale, handed, v, w);
-      else ir_pass<PASS_STEP>(grid, A, q, ring, rxh, ryh, scale, handed, v, w);
+      if (pend) ir_pass<PASS_STEP2, FIXED>(grid, A, q, ring, rxh, ryh, scale, handed, v, w);
+      else ir_pass<PASS_STEP, FIXED>(grid, A, q, ring, rxh, ryh, scale, handed, v, w);
       auto fin = [&](double g, double f, double r) {
         const double b = g * S.inv_gamma;
         const bool claim = test.met(g);
@@ -420,9 +417,7 @@ __device__ __forceinline__ bool ir_solve(Grid grid, const IrCg &A, Shared &S, un
         }
         if (lane == 0) S.done = done;
       };
-      if (!(fixed_tiles ? grid_sum3<false>(grid, S.sum, bar, A.sums, v, scale, w, target, set, fin)
-                        : grid_sum3<true>(grid, S.sum, bar, A.sums, v, scale, w, target, set, fin)))
-        return false;
+      if (!grid_sum3<FIXED>(grid, S.sum, bar, A.sums, v, scale, w, target, set, fin)) return false;
       mirrored = !mirrored;
       float *t = rc;
       rc = rn;
@@ -488,6 +483,11 @@ __device__ __forceinline__ bool ir_solve(Grid grid, const IrCg &A, Shared &S, un
     }
   }
   return true;
+}
+
+// The solve of one deck by the blocks of `grid`; false when a wait gave up.
+__device__ __forceinline__ bool ir_solve(Grid grid, const IrCg &A, Shared &S, unsigned ring) {
+  return A.t.tiles <= A.t.warps ? ir_loop<false>(grid, A, S, ring) : ir_loop<true>(grid, A, S, ring);
 }
 
 inline void ir_cg_args(IrCg &A, tl_ctx *ctx, int blocks) {

@@ -91,24 +91,24 @@ struct PassSums {
 };
 
 // One tile's three sums into the pass's.
-__device__ __forceinline__ void tile_sums(PassSums &S, Pair (&acc)[3], bool fixed_tiles, int scale) {
+template <bool FIXED>
+__device__ __forceinline__ void tile_sums(PassSums &S, Pair (&acc)[3], int scale) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int d = 0; d < 3; ++d)
     if (lane == 0 || lane == 31) acc[d] = Pair{0.f, 0.f};
   S.w = warp_pairs(acc);
-  if (!fixed_tiles) S.v += to_fixed(S.w.hi, scale) + to_fixed(S.w.lo, scale);
+  if (FIXED) S.v += to_fixed(S.w.hi, scale) + to_fixed(S.w.lo, scale);
 }
 
 // One pass of one or two steps; sums r1.r1 and r2.r2 when `sums`.
-template <int KIND, int STEPS>
+template <int KIND, int STEPS, bool FIXED>
 __device__ __forceinline__ void step_pass(Grid grid, const IrSweeps &A, const StepArgs &q, unsigned ring, float rxh,
                                           float ryh, bool sums, int scale, unsigned &handed, PassSums &S) {
   constexpr int DEPTH = RING_BYTES / 2048;
   const int nx = A.g32.nx, ny = A.g32.ny;
   const int lane = threadIdx.x & 31;
   const unsigned slot0 = ring + 16 * lane;
-  const bool fixed_tiles = A.t.tiles <= A.t.warps;
   TileWalk walk(grid, A.t, ny, q.mirrored, &A.F.sc->bar.next_tile, handed);
   handed += walk.requests();
   while (walk.valid()) {
@@ -235,12 +235,13 @@ __device__ __forceinline__ void step_pass(Grid grid, const IrSweeps &A, const St
     cp_wait<0>();
     acc[0].add(ps[0]);
     acc[1].add(ps[1]);
-    if (sums) tile_sums(S, acc, fixed_tiles, scale);
+    if (sums) tile_sums<FIXED>(S, acc, scale);
     walk.take(asked);
   }
 }
 
 // p' = beta p + r into `pn`; p'.p' and its face sums (p'.A p' is both together).
+template <bool FIXED>
 __device__ __forceinline__ void direction_pass(Grid grid, const IrSweeps &A, const float *p, const float *r, float *pn,
                                                float beta, unsigned ring, float rxh, float ryh, bool mirrored, int scale,
                                                unsigned &handed, PassSums &S) {
@@ -248,7 +249,6 @@ __device__ __forceinline__ void direction_pass(Grid grid, const IrSweeps &A, con
   const int nx = A.g32.nx, ny = A.g32.ny;
   const int lane = threadIdx.x & 31;
   const unsigned slot0 = ring + 16 * lane;
-  const bool fixed_tiles = A.t.tiles <= A.t.warps;
   TileWalk walk(grid, A.t, ny, mirrored, &A.F.sc->bar.next_tile, handed);
   handed += walk.requests();
   while (walk.valid()) {
@@ -314,7 +314,7 @@ __device__ __forceinline__ void direction_pass(Grid grid, const IrSweeps &A, con
     cp_wait<0>();
     acc[0].add(s[0]);
     acc[1].add(s[1]);
-    tile_sums(S, acc, fixed_tiles, scale);
+    tile_sums<FIXED>(S, acc, scale);
     walk.take(asked);
   }
 }
@@ -337,6 +337,7 @@ __device__ __forceinline__ void fold_correction(Grid grid, const IrSweeps &A, co
   }
 }
 
+template <bool FIXED>
 __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A) {
   extern __shared__ __align__(128) unsigned char ring_mem[];
   __shared__ SweepShared S;
@@ -348,7 +349,6 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A
   const double eps = sc->eps, bb = sc->bb;
   const int maxiters = sc->maxiters;
   const RootTest test(eps, bb);
-  const bool fixed_tiles = A.t.tiles <= A.t.warps;
   int iter = sc->iter, ci = sc->cheby_iters, nref = 0;
   unsigned target = 0, set = 0, handed = 0;
   bool mirrored = false;
@@ -380,8 +380,8 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A
       q.mirrored = mirrored;
       const int scale = fixed_scale(ref);
       PassSums sums;
-      if (two) step_pass<STEP_CHEBY, 2>(grid, A, q, ring, rxh, ryh, true, scale, handed, sums);
-      else step_pass<STEP_CHEBY, 1>(grid, A, q, ring, rxh, ryh, true, scale, handed, sums);
+      if (two) step_pass<STEP_CHEBY, 2, FIXED>(grid, A, q, ring, rxh, ryh, true, scale, handed, sums);
+      else step_pass<STEP_CHEBY, 1, FIXED>(grid, A, q, ring, rxh, ryh, true, scale, handed, sums);
       const int steps = two ? 2 : 1;
       auto fin = [&](double g1, double g2, double) {
         const double g = two ? g2 : g1;
@@ -391,9 +391,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A
           S.done = hit || iter + steps >= maxiters;
         }
       };
-      if (!(fixed_tiles ? grid_sum3<false>(grid, S.sum, &sc->bar, A.sums, sums.v, scale, sums.w, target, set, fin)
-                        : grid_sum3<true>(grid, S.sum, &sc->bar, A.sums, sums.v, scale, sums.w, target, set, fin)))
-        return;
+      if (!grid_sum3<FIXED>(grid, S.sum, &sc->bar, A.sums, sums.v, scale, sums.w, target, set, fin)) return;
       float *t = e;
       e = en;
       en = t;
@@ -425,6 +423,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A
   }
 }
 
+template <bool FIXED>
 __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ppcg32(const IrSweeps A) {
   extern __shared__ __align__(128) unsigned char ring_mem[];
   __shared__ SweepShared S;
@@ -438,7 +437,6 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ppcg32(const IrSweeps A)
   const int maxiters = sc->maxiters, n = A.ninner;
   const float rtheta = (float)(1.0 / sc->theta);
   const RootTest test(eps, bb);
-  const bool fixed_tiles = A.t.tiles <= A.t.warps;
   int iter = sc->iter, outer = sc->cheby_iters, nref = 0;
   unsigned target = 0, set = 0, handed = 0;
   bool mirrored = false;
@@ -453,7 +451,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ppcg32(const IrSweeps A)
     for (;;) {
       int scale = fixed_scale(ref);
       PassSums sums;
-      direction_pass(grid, A, p, r, spare, (float)beta, ring, rxh, ryh, mirrored, scale, handed, sums);
+      direction_pass<FIXED>(grid, A, p, r, spare, (float)beta, ring, rxh, ryh, mirrored, scale, handed, sums);
       auto step = [&](double pp, double faces, double) {
         const double pw = pp + faces, a = gamma / pw;
         if (lane == 0) {
@@ -462,9 +460,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ppcg32(const IrSweeps A)
           S.af = (float)a;
         }
       };
-      if (!(fixed_tiles ? grid_sum3<false>(grid, S.sum, bar, A.sums, sums.v, scale, sums.w, target, set, step)
-                        : grid_sum3<true>(grid, S.sum, bar, A.sums, sums.v, scale, sums.w, target, set, step)))
-        return;
+      if (!grid_sum3<FIXED>(grid, S.sum, bar, A.sums, sums.v, scale, sums.w, target, set, step)) return;
       mirrored = !mirrored;
       alpha = S.a;
       ref = S.b;
@@ -493,9 +489,9 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ppcg32(const IrSweeps A)
         q.store_m = end < n;  // the last sweep's sd starts nothing
         q.mirrored = mirrored;
         const bool last = end == n;
-        if (update) step_pass<STEP_UPDATE, 2>(grid, A, q, ring, rxh, ryh, last, scale, handed, sums);
-        else if (two) step_pass<STEP_SWEEP, 2>(grid, A, q, ring, rxh, ryh, last, scale, handed, sums);
-        else step_pass<STEP_SWEEP, 1>(grid, A, q, ring, rxh, ryh, last, scale, handed, sums);
+        if (update) step_pass<STEP_UPDATE, 2, FIXED>(grid, A, q, ring, rxh, ryh, last, scale, handed, sums);
+        else if (two) step_pass<STEP_SWEEP, 2, FIXED>(grid, A, q, ring, rxh, ryh, last, scale, handed, sums);
+        else step_pass<STEP_SWEEP, 1, FIXED>(grid, A, q, ring, rxh, ryh, last, scale, handed, sums);
         mirrored = !mirrored;
         xv = true;
         t = r;
@@ -518,9 +514,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ppcg32(const IrSweeps A)
               S.done = hit || iter + 1 >= maxiters;
             }
           };
-          if (!(fixed_tiles ? grid_sum3<false>(grid, S.sum, bar, A.sums, sums.v, scale, sums.w, target, set, fin)
-                            : grid_sum3<true>(grid, S.sum, bar, A.sums, sums.v, scale, sums.w, target, set, fin)))
-            return;
+          if (!grid_sum3<FIXED>(grid, S.sum, bar, A.sums, sums.v, scale, sums.w, target, set, fin)) return;
         }
         pp = end + 1;
       }
@@ -576,8 +570,8 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_bench32(const IrSweeps A
       q.sn = C.s[odd ^ 1];
       q.s_valid = q.p_valid = q.x_valid = true;
       q.mirrored = odd;
-      if (kind == 8) ir_pass<PASS_STEP>(grid, C, q, ring, rxh, ryh, scale, handed, sums.v, sums.w);
-      else ir_pass<PASS_STEP2>(grid, C, q, ring, rxh, ryh, scale, handed, sums.v, sums.w);
+      if (kind == 8) ir_pass<PASS_STEP, true>(grid, C, q, ring, rxh, ryh, scale, handed, sums.v, sums.w);
+      else ir_pass<PASS_STEP2, true>(grid, C, q, ring, rxh, ryh, scale, handed, sums.v, sums.w);
     } else {
       StepArgs q{};
       q.m = kind == 6 ? (odd ? A.pb : A.x) : odd ? A.sdb : A.sd;
@@ -588,8 +582,8 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_bench32(const IrSweeps A
       q.zo = kind == 6 ? (odd ? A.p : A.sd) : A.x;
       q.m_valid = q.z_valid = q.store_m = true;
       q.mirrored = odd;
-      if (kind == 6) step_pass<STEP_CHEBY, 2>(grid, A, q, ring, rxh, ryh, true, scale, handed, sums);
-      else step_pass<STEP_SWEEP, 2>(grid, A, q, ring, rxh, ryh, false, scale, handed, sums);
+      if (kind == 6) step_pass<STEP_CHEBY, 2, true>(grid, A, q, ring, rxh, ryh, true, scale, handed, sums);
+      else step_pass<STEP_SWEEP, 2, true>(grid, A, q, ring, rxh, ryh, false, scale, handed, sums);
     }
     if (kind == 7) {
       if (!grid_barrier(grid, bar, target)) return;
@@ -623,8 +617,10 @@ IrSweeps sweep_args(tl_ctx *ctx, int ninner, double rr) {
   return A;
 }
 
-int run_sweeps(tl_ctx *ctx, const void *kernel, int ninner, double rr) {
+// `one`: the kernel for one tile a warp; `more`: for several, or tiles handed out.
+int run_sweeps(tl_ctx *ctx, const void *one, const void *more, int ninner, double rr) {
   IrSweeps A = sweep_args(ctx, ninner, rr);
+  const void *kernel = A.t.tiles <= A.t.warps ? one : more;
   const size_t smem = (size_t)RING_BYTES * PERSIST_WARPS;
   CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int rc = tl_bar_ready(ctx);
@@ -675,7 +671,7 @@ int tl_cheby32_run(tl_ctx *ctx, int *refinements, double *rel_out) {
   if (blocks > 152LL * 32) blocks = 152LL * 32;
   k_ir_import_p<<<(int)blocks, 256, 0, ctx->stream>>>(ctx->F, ctx->g, g32_of(ctx), ctx->ir->p);
   CKL();
-  if ((rc = run_sweeps(ctx, (const void *)k_cheby32, 0, 0.0))) return rc;
+  if ((rc = run_sweeps(ctx, (const void *)k_cheby32<false>, (const void *)k_cheby32<true>, 0, 0.0))) return rc;
   *refinements = ctx->host_sc->refinements;
   *rel_out = ctx->host_sc->red[1];
   return TL_OK;
@@ -690,7 +686,7 @@ int tl_cheby32_run(tl_ctx *ctx, int *refinements, double *rel_out) {
 // residual in FP64 and replaces the FP32 residual with it.  Stops on the
 // relative true residual ||u0 - A u|| / ||u0|| < eps or the iteration budget.
 int tl_ppcg32_run(tl_ctx *ctx, const tl_params *prm, double rr, int *refinements, double *rel_out) {
-  int rc = run_sweeps(ctx, (const void *)k_ppcg32, prm->ppcginnersteps, rr);
+  int rc = run_sweeps(ctx, (const void *)k_ppcg32<false>, (const void *)k_ppcg32<true>, prm->ppcginnersteps, rr);
   if (rc) return rc;
   *refinements = ctx->host_sc->refinements;
   *rel_out = ctx->host_sc->red[1];
