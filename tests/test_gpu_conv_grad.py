@@ -3,10 +3,10 @@ edges of its 64-pixel columns, images of one row, fewer rows than blocks, a
 block that ends inside one column and starts in the next, one block for all.
 
 The reference is torch's FP64 gradient of the same BF16 inputs.  Their products
-are exact in FP32.  A block adds one product of 16 pixels per row it marches to
-each of four accumulators, and a tensor-core addition may cut off up to 2^-23
-of the running sum: steps * 2^-23 for the rows of one block.  The additions
-after that (four accumulators, at most 152 blocks in eight chains) round to
+are exact in FP32.  A block adds two products of 16 pixels per row it marches to
+each of its accumulators, and a tensor-core addition may cut off up to 2^-23 of the
+running sum, half of that on average: steps * 2^-23 for the rows of one block.  The
+additions after that (two accumulators, the blocks in eight chains) round to
 nearest: 2 + 3 + 19 + 8 of them at 2^-24 each are 2e-6.
 """
 import ctypes
