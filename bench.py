@@ -169,8 +169,8 @@ def gpu_setup(tl, n, precision, maxiters=40000, warm=0):
 def restart_deck(tl, chunk, s):
     """Puts the context back to the deck's initial state (initialiseapp!: the
     states, the halo of density, energy0, energy, energy = energy0) and clears
-    the warm start's history, keeping the tuned layouts and the instantiated
-    graphs: the next timestep is timestep 1 of the deck."""
+    the warm start's history, keeping the context and its tuned layouts: the
+    next timestep is timestep 1 of the deck."""
     arr = tl._state_array(s, chunk.mode)
     chunk.check(chunk.lib.tl_initialise(chunk.ctx, arr, len(s.states)))
     s.resettoexchange()
@@ -538,7 +538,7 @@ def gpu_arm(args):
 
 def config4_leg(tl):
     """The batched workload beside the headline: 128 decks of uneven sizes,
-    10 timesteps each, one batched graph launch per timestep against the same
+    10 timesteps each, one batched launch per timestep against the same
     decks solved one after another, FP64 and FP32-refined CG to 1e-10."""
     sizes, texts = config4_decks(128)
     out = {"workload": "128 random-rectangle decks, nx, ny in 256..2048 step 128, 10 steps, CG to 1e-10 relative",
@@ -664,7 +664,7 @@ def config4_decks(count: int = 128, seed: int = DECK_SEED + 4):
 
 def run_config4(args):
     """128 independent decks of uneven sizes, 10 timesteps each, CG to 1e-10
-    relative residual, FP64 and FP32-refined: one batched graph launch per
+    relative residual, FP64 and FP32-refined: one batched launch per
     timestep against the same decks solved one after another by the
     single-deck solver of the same precision."""
     import torch

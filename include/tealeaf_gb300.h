@@ -114,7 +114,7 @@ typedef struct {
   int converged;            /* the loop ended on its convergence test           */
   int refinements;          /* FP64 refinement passes (TL_PREC_FP32_IR)         */
   double rel_residual;      /* ||u0 - A u|| / ||u0|| after the solve (TL_CRIT_RELATIVE), else -1 */
-  int launches;             /* kernels this solve launched (graph-body kernels counted per trip) */
+  int launches;             /* kernels this solve launched (graph-body kernels of the exact loops counted per trip) */
   int warm;                 /* 0: plain start (no warm start asked or no previous step), 1: the
                                prediction was used, 2: the prediction lost to the plain start,
                                3 (TL_WARM_NETWORK): the projection without the network's term had
@@ -215,10 +215,9 @@ int tl_timer_stop(tl_ctx *ctx, double *ms);
 int tl_bench_kernel(tl_ctx *ctx, int kernel, int reps, double *ms_per_launch);
 
 /* Many independent decks (tealeaf-mode contexts of any sizes on the current
- * device) solved by the fused FP64 CG in one graph launch: the persistent
- * blocks are shared over the decks in proportion to their cells, a converged
- * deck drops out (per-deck convergence mask) and its blocks go to the decks
- * still running.  Each deck's solve is CG.solve! (src/solvers/CG.jl:7-29)
+ * device) solved by the fused FP64 CG, or the FP32-refined CG, in one launch:
+ * groups of blocks take decks from a queue, the largest first, and run each
+ * deck's whole loop among themselves.  Each deck's solve is CG.solve! (src/solvers/CG.jl:7-29)
  * with that deck's rx[k], ry[k]; results[k] is the deck's result.  The batch
  * borrows the contexts: destroy it before them. */
 typedef struct tl_batch tl_batch;

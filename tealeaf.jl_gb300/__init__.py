@@ -302,7 +302,7 @@ def diffuse(chunk: Chunk, settings: Settings, problemfile: Optional[str] = None)
 
 class Batch:
     """Many independent decks (tealeaf-mode Chunks of any sizes) whose CG
-    solves run together in one graph launch (tl_batch_*)."""
+    solves run together in one launch (tl_batch_*)."""
 
     def __init__(self, chunks):
         self.lib = _abi.load()

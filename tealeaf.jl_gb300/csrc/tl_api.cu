@@ -1,7 +1,8 @@
 // tl_api.cu -- the C ABI (include/tealeaf_gb300.h): context, copies, and the
-// host orchestration of each reference entry point.  Iteration loops run as
-// CUDA graphs whose while-node is driven by the convergence test on the
-// device; the host only reads the scalars back once a solve has ended.
+// host orchestration of each reference entry point.  Iteration loops run on
+// the device to their convergence test, the fused ones as one persistent kernel,
+// the exact ones as CUDA graphs with a while-node; the host reads the scalars
+// back once a solve has ended.
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>

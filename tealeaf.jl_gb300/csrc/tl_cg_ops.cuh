@@ -1,6 +1,6 @@
 // tl_cg_ops.cuh -- the fused CG step operations (tealeaf semantics), shared
-// by the single-deck loop (tl_kernels_cg.cu) and the batched loop
-// (tl_batch.cu).
+// by the exact loop's kernels and the fused ones that tl_bench_kernel times
+// (tl_kernels_cg.cu).
 #pragma once
 
 #include "tl_march.cuh"

@@ -50,7 +50,7 @@ struct GridBar {
 };
 
 // Scalars of a solve, resident in device memory so that the iteration loop
-// runs inside a CUDA graph with no host round trip.
+// runs with no host round trip.
 struct DevScalars {
   // loop state
   double rro, pw, alpha, beta, rrn, error, bb, theta;
@@ -65,11 +65,7 @@ struct DevScalars {
   int iter_base;        // 1-based loop index of this loop's first trip minus 1
   int cheby_iters, est_iters, calc_every;  // Chebyshev loop bookkeeping
   int first;            // the next fused CG step starts from p itself (no beta update)
-  double rr_ref;        // FP32 refinement: r.r at the last refinement
-  double delta2;        // FP32 refinement: refine once r.r < delta2 * rr_ref
-  // batched FP32 refinement (tl_batch.cu)
-  int pbuf;             // 1: the current FP32 search direction is in the second buffer
-  int finished;         // the deck's solve is over (converged or out of iterations)
+  // FP32 refinement
   int refinements;      // FP64 refinement steps taken
   int prestep_switch;   // FP32 CG presteps of Chebyshev: the switch test held (Cheby.jl:25-29)
   double rxh, ryh;      // FP32 stencil from inverse weights: Kx = rxh (iw_l + iw_c), Ky = ryh (iw_d + iw_c)

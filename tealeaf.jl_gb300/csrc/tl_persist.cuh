@@ -4,7 +4,7 @@
 // A persistent kernel runs a whole iteration loop in one launch of at most one
 // block per SM: a graph with a while-node spends 9 us on each kernel boundary
 // of a small deck (18-20 us per CG iteration up to 512^2, whatever the
-// deck), a barrier here 1.25 us.  Every block adds the block partials of a
+// deck), a barrier here 1.5 us.  Every block adds the block partials of a
 // reduction itself, in the same order, so all blocks hold the same scalars bit
 // for bit and take the same decisions without another broadcast.
 #pragma once

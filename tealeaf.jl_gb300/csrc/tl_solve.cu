@@ -1,6 +1,6 @@
 // tl_solve.cu -- solve!(chunk, set, rx, ry) for the CG plugin
 // (src/solvers/CG.jl:7-29) and the shared pieces of the other solvers:
-// tea_leaf_init, loop parameters, and the while-node iteration graphs.
+// tea_leaf_init, loop parameters, and the exact path's while-node iteration graphs.
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
