@@ -50,15 +50,18 @@ struct Shared64 {
   int done, conv, sw;
 };
 
-// r -= alpha w over this warp's tiles; this lane's share of r.r.
-__device__ __forceinline__ Fixed r_pass(Grid grid, const Cg64 &A, unsigned ring, bool mirrored, double alpha, int scale,
-                                        unsigned &handed) {
+// r -= alpha w over this warp's tiles; its share of r.r.
+template <bool LATE>
+__device__ __forceinline__ Digits r_pass(Grid grid, const Cg64 &A, unsigned ring, bool mirrored, double alpha,
+                                         unsigned &handed) {
   constexpr int DEPTH = RING64_BYTES / 1024;
   const int nx = A.g.nx, ny = A.g.ny, lane = threadIdx.x & 31;
   const unsigned slot0 = ring + 16 * lane;
-  Fixed sum = 0;
+  Digits sum;
+  double acc = 0.0;
   TileWalk walk(grid, A.tr, ny, mirrored, &A.F.sc->bar.next_tile, handed);
   handed += walk.requests();
+  bool any = false;
   while (walk.valid()) {
     int strip, j0, j1;
     walk.place(strip, j0, j1);
@@ -77,7 +80,9 @@ __device__ __forceinline__ Fixed r_pass(Grid grid, const Cg64 &A, unsigned ring,
     };
 #pragma unroll
     for (int d = 0; d < DEPTH - 1; ++d) issue(j0 + d, d);
-    double acc = 0.0;
+    if (LATE && any) add_lanes(sum, acc);  // of the tile before
+    any = true;
+    acc = 0.0;
     unsigned slot = 0, prev = DEPTH - 1;
     for (int j = j0; j < j1; ++j) {
       cp_wait<DEPTH - 2>();
@@ -85,42 +90,47 @@ __device__ __forceinline__ Fixed r_pass(Grid grid, const Cg64 &A, unsigned ring,
       const double2 w = lds2d(slot0 + slot * 1024 + 512);
       r = make_double2(fma(-alpha, w.x, r.x), fma(-alpha, w.y, r.y));
       if (!has1) r.y = 0.0;
-      acc = fma(r.y, r.y, fma(r.x, r.x, acc));
-      if (in) put64(A.F.r + c, r, has1);
+      if (in) {
+        acc = fma(r.x, r.x, fma(r.y, r.y, acc));
+        put64(A.F.r + c, r, has1);
+      }
       c += step;
       issue(j + DEPTH - 1, prev);
       prev = slot;
       slot = slot + 1 == DEPTH ? 0 : slot + 1;
     }
     cp_wait<0>();
-    if (in) sum += to_fixed(acc, scale);
+    if (!LATE) add_lanes(sum, acc);
     walk.take(asked);
   }
+  if (LATE && any) add_lanes(sum, acc);
   return sum;
 }
 
 // The same on the one tile (j0 < 0: none) that this warp's W left in shared memory,
 // in a ring of `arrays` operands a row.
-__device__ __forceinline__ Fixed r_kept(const Cg64 &A, const Mem64 &mem, int strip, int j0, int j1, int arrays,
-                                        double alpha, int scale) {
+__device__ __forceinline__ Digits r_kept(const Cg64 &A, const Mem64 &mem, int strip, int j0, int j1, int arrays,
+                                         double alpha) {
   const int lane = threadIdx.x & 31;
-  if (j0 < 0) return 0;
+  Digits sum;
+  if (j0 < 0) return sum;
   const int i0 = strip * STRIP64 - 2 + 2 * lane;
-  if (lane < 1 || lane > 30 || i0 >= A.g.nx) return 0;
-  const bool has1 = i0 + 1 < A.g.nx;
+  const bool owns = lane >= 1 && lane <= 30 && i0 < A.g.nx, has1 = i0 + 1 < A.g.nx;
   double acc = 0.0;
-  for (int j = j0; j < j1; ++j) {
+  for (int j = j0; owns && j < j1; ++j) {
     double2 r = lds2d(mem.ring + 16 * lane + ((j - j0 + 1) * arrays + 1) * 512);
     const double2 w = lds2d(mem.w + 16 * lane + (j - j0) * 512);
     r = make_double2(fma(-alpha, w.x, r.x), fma(-alpha, w.y, r.y));
     if (!has1) r.y = 0.0;
-    acc = fma(r.y, r.y, fma(r.x, r.x, acc));
+    acc = fma(r.x, r.x, fma(r.y, r.y, acc));
     put64(A.F.r + A.g.at(i0, j), r, has1);
   }
-  return to_fixed(acc, scale);
+  add_lanes(sum, acc);
+  return sum;
 }
 
-template <bool KEEP>
+// HANDED: W's tiles are handed out (and R's, if they are more than the warps).
+template <bool KEEP, bool HANDED>
 __device__ __forceinline__ bool cg64_loop(Grid grid, const Cg64 &A, Shared64 &S, const Mem64 &mem) {
   const unsigned ring = mem.ring;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -133,7 +143,7 @@ __device__ __forceinline__ bool cg64_loop(Grid grid, const Cg64 &A, Shared64 &S,
   if (A.check && sqrt(bb > 0 ? ddiv(sc->rro, bb) : sc->rro) < eps) return true;
   const RootTest test(eps, relative ? bb : 1.0);
   double *p = A.F.p, *pn = A.F.pb;
-  double rro = sc->rro, alpha = 0.0, beta = 0.0, pw_ref = rro, rr = rro;
+  double rro = sc->rro, alpha = 0.0, beta = 0.0, pw = 0.0;
   int iter = sc->iter;
   bool first = true, mirrored = false;
   unsigned target = 0, set = 0, handed = 0;
@@ -155,10 +165,9 @@ __device__ __forceinline__ bool cg64_loop(Grid grid, const Cg64 &A, Shared64 &S,
     q.beta = beta;
     q.m_valid = !first;  // the first direction is r
     double acc = 0.0;
-    Fixed sum = 0;
-    int scale = fixed_scale(pw_ref);
+    Digits sum;
     auto tile_end = [&]() {
-      sum += to_fixed(acc, scale);
+      add_lanes(sum, acc);
       acc = 0.0;
     };
     const int arrays = first ? 5 : 6;
@@ -173,9 +182,9 @@ __device__ __forceinline__ bool cg64_loop(Grid grid, const Cg64 &A, Shared64 &S,
       }
     };
     if (first) {
-      ring64<true, 0>(grid, q, A.tw, ring, mirrored, &A.F.sc->bar.next_tile, handed, direction, tile_end);
+      ring64<true, 0, HANDED>(grid, q, A.tw, ring, mirrored, &A.F.sc->bar.next_tile, handed, direction, tile_end);
     } else {
-      ring64<true, 1>(grid, q, A.tw, ring, mirrored, &A.F.sc->bar.next_tile, handed,
+      ring64<true, 1, HANDED>(grid, q, A.tw, ring, mirrored, &A.F.sc->bar.next_tile, handed,
                       [&](int j, int i0, bool has1, bool owns, const Row64 &o) {
                         direction(j, i0, has1, owns, o);
                         if (owns)
@@ -184,7 +193,7 @@ __device__ __forceinline__ bool cg64_loop(Grid grid, const Cg64 &A, Shared64 &S,
                       },
                       tile_end);
     }
-    if (!grid_sum1(grid, S.sum, bar, A.sums, warp_fixed(sum), scale, target, set, [&](double pw) {
+    if (!grid_sum<1>(grid, S.sum, bar, A.sums, sum, target, set, [&](double pw) {
           const double a = ddiv(lane == 0 ? rro : 1.0, lane == 0 ? pw : rro);  // and 1/rro for beta, in one division
           if (lane == 0) {
             S.alpha = a;
@@ -196,7 +205,7 @@ __device__ __forceinline__ bool cg64_loop(Grid grid, const Cg64 &A, Shared64 &S,
         }))
       return false;
     alpha = S.alpha;
-    pw_ref = S.err;
+    pw = S.err;
     mirrored = !mirrored && !KEEP;
     {
       double *t = p;
@@ -204,10 +213,8 @@ __device__ __forceinline__ bool cg64_loop(Grid grid, const Cg64 &A, Shared64 &S,
       pn = t;
     }
     // R
-    scale = fixed_scale(rr);
-    sum = KEEP ? r_kept(A, mem, tile_strip, tile0, tile1, arrays, alpha, scale)
-                 : r_pass(grid, A, ring, mirrored, alpha, scale, handed);
-    if (!grid_sum1(grid, S.sum, bar, A.sums, warp_fixed(sum), scale, target, set, [&](double rrn) {
+    sum = KEEP ? r_kept(A, mem, tile_strip, tile0, tile1, arrays, alpha) : r_pass<HANDED>(grid, A, ring, mirrored, alpha, handed);
+    if (!grid_sum<1>(grid, S.sum, bar, A.sums, sum, target, set, [&](double rrn) {
           // rrn / rro from the reciprocal formed before, with one correction (Markstein's), away from its ends
           double b = rrn * S.inv_rro;
           if (rro > 1e-290 && rro < 1e290) b = fma(fma(-b, rro, rrn), S.inv_rro, b);
@@ -229,7 +236,7 @@ __device__ __forceinline__ bool cg64_loop(Grid grid, const Cg64 &A, Shared64 &S,
         }))
       return false;
     beta = S.beta;
-    rro = rr = S.err;
+    rro = S.err;
     mirrored = !mirrored && !KEEP;
     first = false;
     ++iter;
@@ -268,10 +275,10 @@ __device__ __forceinline__ bool cg64_loop(Grid grid, const Cg64 &A, Shared64 &S,
   if (lead) {
     sc->alpha = alpha;
     sc->beta = beta;
-    sc->pw = pw_ref;
-    sc->rrn = rr;
-    sc->rro = rr;
-    sc->error = rr;
+    sc->pw = pw;
+    sc->rrn = rro;
+    sc->rro = rro;
+    sc->error = rro;
     sc->iter = iter;
     sc->first = 0;
     sc->converged = S.conv;
@@ -283,7 +290,8 @@ __device__ __forceinline__ bool cg64_loop(Grid grid, const Cg64 &A, Shared64 &S,
 
 // The loop on one deck by the blocks of `grid`; false when a wait gave up.
 __device__ __forceinline__ bool cg64_solve(Grid grid, const Cg64 &A, Shared64 &S, const Mem64 &mem) {
-  return A.keep ? cg64_loop<true>(grid, A, S, mem) : cg64_loop<false>(grid, A, S, mem);
+  if (A.keep) return cg64_loop<true, false>(grid, A, S, mem);
+  return A.tw.handed ? cg64_loop<false, true>(grid, A, S, mem) : cg64_loop<false, false>(grid, A, S, mem);
 }
 
 // Tilings for `blocks` blocks at most.

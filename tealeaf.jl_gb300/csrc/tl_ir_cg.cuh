@@ -62,17 +62,15 @@ struct PassArgs {
 __device__ __forceinline__ float4 f4(float a, float b, float c, float d) { return make_float4(a, b, c, d); }
 
 // One pass over the grid: this warp's share of gamma, the face sums and rho in
-// lanes 0, 8 and 16, as whole numbers where tiles are handed out, else as pairs.
-template <int PASS, bool FIXED>
+// lanes 0, 8 and 16, as digits where tiles are handed out, else as pairs.
+template <int PASS, bool HANDED>
 __device__ __forceinline__ void ir_pass(Grid grid, const IrCg &A, const PassArgs &q, unsigned ring, float rxh, float ryh,
-                                        int scale, unsigned &handed, Fixed &sum, Pair &tile) {
+                                        unsigned &handed, PassSums &sums) {
   constexpr int NARR = PASS == PASS_STEP2 ? 6 : 3;
   constexpr int DEPTH = RING_BYTES / (NARR * 512);
   const int nx = A.g32.nx, ny = A.g32.ny;
   const int lane = threadIdx.x & 31;
   const unsigned slot0 = ring + 16 * lane;
-  sum = 0;
-  tile = Pair{0.f, 0.f};
   TileWalk walk(grid, A.t, ny, q.mirrored, &A.F.sc->bar.next_tile, handed);
   handed += walk.requests();
   while (walk.valid()) {
@@ -202,8 +200,7 @@ __device__ __forceinline__ void ir_pass(Grid grid, const IrCg &A, const PassArgs
       acc[d].add(ps[d]);
       if (lane == 0 || lane == 31) acc[d] = Pair{0.f, 0.f};
     }
-    tile = warp_pairs(acc);
-    if (FIXED) sum += to_fixed(tile.hi, scale) + to_fixed(tile.lo, scale);
+    add_tile<HANDED>(sums, warp_pairs(acc));
     walk.take(asked);
   }
 }
@@ -226,9 +223,8 @@ struct SrcU {
 };
 
 // The true residual r = u0 - A u in FP64, its FP32 copy in `r32` and r.r in
-// `rr` (on entry the r.r of the residual before, for the sum's scale).  In
-// difference form: the couplings multiply differences of neighbouring cells, so
-// u's own rounding is not scaled by them.
+// `rr`.  In difference form: the couplings multiply differences of neighbouring
+// cells, so u's own rounding is not scaled by them.
 __device__ __forceinline__ bool ir_residual(Grid grid, const Fields &F, const Geom &g, const G32 &g32, const Tiling &T,
                                             GridSums *sums, SumShared &S, float *r32, unsigned &target, unsigned &set,
                                             unsigned &handed, double &rr) {
@@ -236,8 +232,7 @@ __device__ __forceinline__ bool ir_residual(Grid grid, const Fields &F, const Ge
   const int lane = threadIdx.x & 31;
   SrcU src;
   src.f = F.u;
-  const int scale = fixed_scale(rr);
-  Fixed share = 0;
+  Digits share;
   TileWalk walk(grid, T, g.ny, false, &F.sc->bar.next_tile, handed);
   handed += walk.requests();
   while (walk.valid()) {
@@ -269,10 +264,10 @@ __device__ __forceinline__ bool ir_residual(Grid grid, const Fields &F, const Ge
                      r32[c32] = (float)t0;
                    }
                  });
-    share += to_fixed(acc, scale);
+    add_lanes(share, acc);
     walk.take(asked);
   }
-  if (!grid_sum1(grid, S, &F.sc->bar, sums, warp_fixed(share), scale, target, set, [&](double a) {
+  if (!grid_sum<1>(grid, S, &F.sc->bar, sums, share, target, set, [&](double a) {
         if (lane == 0) tot = a;
       }))
     return false;
@@ -336,8 +331,8 @@ __device__ __forceinline__ void next_scalars(Shared &S, double gamma, double bet
   }
 }
 
-// FIXED: tiles are handed out or several a warp, and the sums are whole numbers.
-template <bool FIXED>
+// HANDED: tiles are handed out.
+template <bool HANDED>
 __device__ __forceinline__ bool ir_loop(Grid grid, const IrCg &A, Shared &S, unsigned ring) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int warps = grid.nb * PERSIST_WARPS, me = grid.id * PERSIST_WARPS + warp;
@@ -363,19 +358,16 @@ __device__ __forceinline__ bool ir_loop(Grid grid, const IrCg &A, Shared &S, uns
 
   while (rel >= eps && iter < maxiters && !sw) {
     const double refine_below = A.delta2 * rr;
-    double ref = rr;  // the sums' scale follows the last r.r
     {  // the sums of the residual that the refinement (or the start) left
       PassArgs q{};
       q.rc = rc;
       q.sc = sc_;
       q.s_valid = sv;
       q.mirrored = mirrored;
-      const int scale = fixed_scale(ref);
-      Fixed v;
-      Pair w;
-      ir_pass<PASS_START, FIXED>(grid, A, q, ring, rxh, ryh, scale, handed, v, w);
+      PassSums sums;
+      ir_pass<PASS_START, HANDED>(grid, A, q, ring, rxh, ryh, handed, sums);
       auto fin = [&](double, double f, double r) { next_scalars(S, rr, beta, rr + f, r); };
-      if (!grid_sum3<FIXED>(grid, S.sum, bar, A.sums, v, scale, w, target, set, fin)) return false;
+      if (!grid_sums<HANDED>(grid, S.sum, bar, A.sums, sums, target, set, fin)) return false;
       mirrored = !mirrored;
     }
     for (;;) {
@@ -393,11 +385,9 @@ __device__ __forceinline__ bool ir_loop(Grid grid, const IrCg &A, Shared &S, uns
       q.p_valid = pv;
       q.x_valid = xv;
       q.mirrored = mirrored;
-      const int scale = fixed_scale(ref);
-      Fixed v;
-      Pair w;
-      if (pend) ir_pass<PASS_STEP2, FIXED>(grid, A, q, ring, rxh, ryh, scale, handed, v, w);
-      else ir_pass<PASS_STEP, FIXED>(grid, A, q, ring, rxh, ryh, scale, handed, v, w);
+      PassSums sums;
+      if (pend) ir_pass<PASS_STEP2, HANDED>(grid, A, q, ring, rxh, ryh, handed, sums);
+      else ir_pass<PASS_STEP, HANDED>(grid, A, q, ring, rxh, ryh, handed, sums);
       auto fin = [&](double g, double f, double r) {
         const double b = g * S.inv_gamma;
         const bool claim = test.met(g);
@@ -417,7 +407,7 @@ __device__ __forceinline__ bool ir_loop(Grid grid, const IrCg &A, Shared &S, uns
         }
         if (lane == 0) S.done = done;
       };
-      if (!grid_sum3<FIXED>(grid, S.sum, bar, A.sums, v, scale, w, target, set, fin)) return false;
+      if (!grid_sums<HANDED>(grid, S.sum, bar, A.sums, sums, target, set, fin)) return false;
       mirrored = !mirrored;
       float *t = rc;
       rc = rn;
@@ -431,7 +421,6 @@ __device__ __forceinline__ bool ir_loop(Grid grid, const IrCg &A, Shared &S, uns
       alpha0 = q.alpha;
       beta0 = q.beta;
       ++iter;
-      ref = S.gamma;
       if (S.done) break;
     }
     beta = S.beta;
@@ -487,7 +476,7 @@ __device__ __forceinline__ bool ir_loop(Grid grid, const IrCg &A, Shared &S, uns
 
 // The solve of one deck by the blocks of `grid`; false when a wait gave up.
 __device__ __forceinline__ bool ir_solve(Grid grid, const IrCg &A, Shared &S, unsigned ring) {
-  return A.t.tiles <= A.t.warps ? ir_loop<false>(grid, A, S, ring) : ir_loop<true>(grid, A, S, ring);
+  return A.t.handed ? ir_loop<true>(grid, A, S, ring) : ir_loop<false>(grid, A, S, ring);
 }
 
 inline void ir_cg_args(IrCg &A, tl_ctx *ctx, int blocks) {

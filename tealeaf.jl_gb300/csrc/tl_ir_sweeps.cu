@@ -84,27 +84,20 @@ __device__ __forceinline__ float4 face_row(float ryh, float4 a, float4 b) {
   return f4(ryh * (a.x + b.x), ryh * (a.y + b.y), ryh * (a.z + b.z), ryh * (a.w + b.w));
 }
 
-// The sums of a pass: whole numbers where tiles are handed out, else pairs.
-struct PassSums {
-  Fixed v = 0;
-  Pair w{0.f, 0.f};
-};
-
 // One tile's three sums into the pass's.
-template <bool FIXED>
-__device__ __forceinline__ void tile_sums(PassSums &S, Pair (&acc)[3], int scale) {
+template <bool HANDED>
+__device__ __forceinline__ void tile_sums(PassSums &S, Pair (&acc)[3]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int d = 0; d < 3; ++d)
     if (lane == 0 || lane == 31) acc[d] = Pair{0.f, 0.f};
-  S.w = warp_pairs(acc);
-  if (FIXED) S.v += to_fixed(S.w.hi, scale) + to_fixed(S.w.lo, scale);
+  add_tile<HANDED>(S, warp_pairs(acc));
 }
 
 // One pass of one or two steps; sums r1.r1 and r2.r2 when `sums`.
-template <int KIND, int STEPS, bool FIXED>
+template <int KIND, int STEPS, bool HANDED>
 __device__ __forceinline__ void step_pass(Grid grid, const IrSweeps &A, const StepArgs &q, unsigned ring, float rxh,
-                                          float ryh, bool sums, int scale, unsigned &handed, PassSums &S) {
+                                          float ryh, bool sums, unsigned &handed, PassSums &S) {
   constexpr int DEPTH = RING_BYTES / 2048;
   const int nx = A.g32.nx, ny = A.g32.ny;
   const int lane = threadIdx.x & 31;
@@ -235,15 +228,15 @@ __device__ __forceinline__ void step_pass(Grid grid, const IrSweeps &A, const St
     cp_wait<0>();
     acc[0].add(ps[0]);
     acc[1].add(ps[1]);
-    if (sums) tile_sums<FIXED>(S, acc, scale);
+    if (sums) tile_sums<HANDED>(S, acc);
     walk.take(asked);
   }
 }
 
 // p' = beta p + r into `pn`; p'.p' and its face sums (p'.A p' is both together).
-template <bool FIXED>
+template <bool HANDED>
 __device__ __forceinline__ void direction_pass(Grid grid, const IrSweeps &A, const float *p, const float *r, float *pn,
-                                               float beta, unsigned ring, float rxh, float ryh, bool mirrored, int scale,
+                                               float beta, unsigned ring, float rxh, float ryh, bool mirrored,
                                                unsigned &handed, PassSums &S) {
   constexpr int DEPTH = RING_BYTES / 1536;
   const int nx = A.g32.nx, ny = A.g32.ny;
@@ -314,7 +307,7 @@ __device__ __forceinline__ void direction_pass(Grid grid, const IrSweeps &A, con
     cp_wait<0>();
     acc[0].add(s[0]);
     acc[1].add(s[1]);
-    tile_sums<FIXED>(S, acc, scale);
+    tile_sums<HANDED>(S, acc);
     walk.take(asked);
   }
 }
@@ -337,7 +330,7 @@ __device__ __forceinline__ void fold_correction(Grid grid, const IrSweeps &A, co
   }
 }
 
-template <bool FIXED>
+template <bool HANDED>
 __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A) {
   extern __shared__ __align__(128) unsigned char ring_mem[];
   __shared__ SweepShared S;
@@ -353,12 +346,11 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A
   unsigned target = 0, set = 0, handed = 0;
   bool mirrored = false;
   float *e = A.x, *en = A.pb, *p = A.p, *pn = A.sd;
-  double err = sc->error, rr = err;
+  double err = sc->error, rr = 0.0;
   if (!ir_residual(grid, A.F, A.g, A.g32, A.t64, A.sums, S.sum, A.r, target, set, handed, rr)) return;
   double rel = bb > 0 ? sqrt(rr / bb) : sqrt(rr);
   while (rel >= eps && iter < maxiters) {
     const double refine_below = A.delta2 * rr;
-    double ref = rr;
     bool ev = false;
     for (;;) {
       const bool two = iter + 2 <= maxiters;
@@ -378,10 +370,9 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A
       q.z_valid = true;
       q.store_m = true;
       q.mirrored = mirrored;
-      const int scale = fixed_scale(ref);
       PassSums sums;
-      if (two) step_pass<STEP_CHEBY, 2, FIXED>(grid, A, q, ring, rxh, ryh, true, scale, handed, sums);
-      else step_pass<STEP_CHEBY, 1, FIXED>(grid, A, q, ring, rxh, ryh, true, scale, handed, sums);
+      if (two) step_pass<STEP_CHEBY, 2, HANDED>(grid, A, q, ring, rxh, ryh, true, handed, sums);
+      else step_pass<STEP_CHEBY, 1, HANDED>(grid, A, q, ring, rxh, ryh, true, handed, sums);
       const int steps = two ? 2 : 1;
       auto fin = [&](double g1, double g2, double) {
         const double g = two ? g2 : g1;
@@ -391,7 +382,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A
           S.done = hit || iter + steps >= maxiters;
         }
       };
-      if (!grid_sum3<FIXED>(grid, S.sum, &sc->bar, A.sums, sums.v, scale, sums.w, target, set, fin)) return;
+      if (!grid_sums<HANDED>(grid, S.sum, &sc->bar, A.sums, sums, target, set, fin)) return;
       float *t = e;
       e = en;
       en = t;
@@ -402,7 +393,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A
       mirrored = !mirrored;
       iter += steps;
       ci += steps;
-      ref = err = S.a;
+      err = S.a;
       if (S.done) break;
     }
     fold_correction(grid, A, e);
@@ -423,7 +414,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A
   }
 }
 
-template <bool FIXED>
+template <bool HANDED>
 __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ppcg32(const IrSweeps A) {
   extern __shared__ __align__(128) unsigned char ring_mem[];
   __shared__ SweepShared S;
@@ -446,29 +437,25 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ppcg32(const IrSweeps A)
   double rel = bb > 0 ? sqrt(rr / bb) : sqrt(rr);
   while (rel >= eps && iter < maxiters) {
     const double refine_below = A.delta2 * rr;
-    double gamma = rr, ref = rr;
+    double gamma = rr;
     bool xv = false;
     for (;;) {
-      int scale = fixed_scale(ref);
       PassSums sums;
-      direction_pass<FIXED>(grid, A, p, r, spare, (float)beta, ring, rxh, ryh, mirrored, scale, handed, sums);
+      direction_pass<HANDED>(grid, A, p, r, spare, (float)beta, ring, rxh, ryh, mirrored, handed, sums);
       auto step = [&](double pp, double faces, double) {
         const double pw = pp + faces, a = gamma / pw;
         if (lane == 0) {
           S.a = a;
-          S.b = pw;
           S.af = (float)a;
         }
       };
-      if (!grid_sum3<FIXED>(grid, S.sum, bar, A.sums, sums.v, scale, sums.w, target, set, step)) return;
+      if (!grid_sums<HANDED>(grid, S.sum, bar, A.sums, sums, target, set, step)) return;
       mirrored = !mirrored;
       alpha = S.a;
-      ref = S.b;
       float *t = p;
       p = spare;
       spare = t;
       // the update with the first sweep, then the others two by two
-      scale = fixed_scale(gamma);
       sums = PassSums{};
       for (int pp = 1; pp <= n;) {
         const bool update = pp == 1, two = update || pp + 1 <= n;
@@ -489,9 +476,9 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ppcg32(const IrSweeps A)
         q.store_m = end < n;  // the last sweep's sd starts nothing
         q.mirrored = mirrored;
         const bool last = end == n;
-        if (update) step_pass<STEP_UPDATE, 2, FIXED>(grid, A, q, ring, rxh, ryh, last, scale, handed, sums);
-        else if (two) step_pass<STEP_SWEEP, 2, FIXED>(grid, A, q, ring, rxh, ryh, last, scale, handed, sums);
-        else step_pass<STEP_SWEEP, 1, FIXED>(grid, A, q, ring, rxh, ryh, last, scale, handed, sums);
+        if (update) step_pass<STEP_UPDATE, 2, HANDED>(grid, A, q, ring, rxh, ryh, last, handed, sums);
+        else if (two) step_pass<STEP_SWEEP, 2, HANDED>(grid, A, q, ring, rxh, ryh, last, handed, sums);
+        else step_pass<STEP_SWEEP, 1, HANDED>(grid, A, q, ring, rxh, ryh, last, handed, sums);
         mirrored = !mirrored;
         xv = true;
         t = r;
@@ -514,7 +501,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ppcg32(const IrSweeps A)
               S.done = hit || iter + 1 >= maxiters;
             }
           };
-          if (!grid_sum3<FIXED>(grid, S.sum, bar, A.sums, sums.v, scale, sums.w, target, set, fin)) return;
+          if (!grid_sums<HANDED>(grid, S.sum, bar, A.sums, sums, target, set, fin)) return;
         }
         pp = end + 1;
       }
@@ -560,7 +547,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_bench32(const IrSweeps A
   const float rxh = (float)A.F.sc->rxh, ryh = (float)A.F.sc->ryh;
   unsigned target = 0, set = 0, handed = 0;
   for (int k = 0; k < reps; ++k) {
-    const int odd = k & 1, scale = fixed_scale(1.0);
+    const int odd = k & 1;
     PassSums sums;
     if (kind >= 8) {
       PassArgs q{};
@@ -570,8 +557,8 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_bench32(const IrSweeps A
       q.sn = C.s[odd ^ 1];
       q.s_valid = q.p_valid = q.x_valid = true;
       q.mirrored = odd;
-      if (kind == 8) ir_pass<PASS_STEP, true>(grid, C, q, ring, rxh, ryh, scale, handed, sums.v, sums.w);
-      else ir_pass<PASS_STEP2, true>(grid, C, q, ring, rxh, ryh, scale, handed, sums.v, sums.w);
+      if (kind == 8) ir_pass<PASS_STEP, true>(grid, C, q, ring, rxh, ryh, handed, sums);
+      else ir_pass<PASS_STEP2, true>(grid, C, q, ring, rxh, ryh, handed, sums);
     } else {
       StepArgs q{};
       q.m = kind == 6 ? (odd ? A.pb : A.x) : odd ? A.sdb : A.sd;
@@ -582,12 +569,12 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_bench32(const IrSweeps A
       q.zo = kind == 6 ? (odd ? A.p : A.sd) : A.x;
       q.m_valid = q.z_valid = q.store_m = true;
       q.mirrored = odd;
-      if (kind == 6) step_pass<STEP_CHEBY, 2, true>(grid, A, q, ring, rxh, ryh, true, scale, handed, sums);
-      else step_pass<STEP_SWEEP, 2, true>(grid, A, q, ring, rxh, ryh, false, scale, handed, sums);
+      if (kind == 6) step_pass<STEP_CHEBY, 2, true>(grid, A, q, ring, rxh, ryh, true, handed, sums);
+      else step_pass<STEP_SWEEP, 2, true>(grid, A, q, ring, rxh, ryh, false, handed, sums);
     }
     if (kind == 7) {
       if (!grid_barrier(grid, bar, target)) return;
-    } else if (!grid_sum3<true>(grid, S, bar, A.sums, sums.v, scale, sums.w, target, set, [](double, double, double) {})) {
+    } else if (!grid_sums<true>(grid, S, bar, A.sums, sums, target, set, [](double, double, double) {})) {
       return;
     }
   }
@@ -617,10 +604,10 @@ IrSweeps sweep_args(tl_ctx *ctx, int ninner, double rr) {
   return A;
 }
 
-// `one`: the kernel for one tile a warp; `more`: for several, or tiles handed out.
-int run_sweeps(tl_ctx *ctx, const void *one, const void *more, int ninner, double rr) {
+// `fixed`: the kernel where every warp has its tiles; `handed`: where they are handed out.
+int run_sweeps(tl_ctx *ctx, const void *fixed, const void *handed, int ninner, double rr) {
   IrSweeps A = sweep_args(ctx, ninner, rr);
-  const void *kernel = A.t.tiles <= A.t.warps ? one : more;
+  const void *kernel = A.t.handed ? handed : fixed;
   const size_t smem = (size_t)RING_BYTES * PERSIST_WARPS;
   CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int rc = tl_bar_ready(ctx);

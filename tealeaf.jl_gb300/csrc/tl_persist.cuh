@@ -13,7 +13,7 @@
 
 namespace tl {
 
-constexpr int PERSIST_WARPS = 16;                 // warps of a persistent block at most
+constexpr int PERSIST_WARPS = 16;                 // warps of a persistent block
 constexpr int PERSIST_THREADS = 32 * PERSIST_WARPS;
 constexpr unsigned BAR_POLLS = 1u << 23;          // a wait gives up after some seconds
 
@@ -68,73 +68,140 @@ __device__ __forceinline__ Grid whole_grid() { return Grid{(int)gridDim.x, (int)
 // Warps take their tiles in whatever order they come free (the SMs of one GPU
 // do not get the same memory bandwidth: at 8192^2 the fast ones waited 110 of
 // 400 us for the slow ones with equal shares).  The sums stay the same bit for
-// bit all the same: each tile's sum, whose inner order is fixed, is turned
-// into a 128-bit whole number of 2^-scale, and whole numbers add up exactly in
-// any order, over warps, blocks and the grid.  They also add in 4-cycle
-// instructions, where one FP64 addition takes 66.
-typedef __int128 Fixed;
+// bit all the same.  A number is cut into digits of 25 bits whose places are the
+// same for all doubles (digit b counts 2^(25 b - 1074)); a sum keeps the digits of
+// the four highest places that any addend has reached, each as a whole number of
+// its own, with no carries between them.  What an addend puts into a place does
+// not depend on the others, nor does the highest place, so neither does the sum
+// on the order, over warps, blocks and the grid.  Whole numbers also add
+// in 4-cycle instructions, where one FP64 addition takes 66.
+//
+// The places come from the addends themselves, not from an earlier sum: whatever
+// a step did to the sum, the highest addend is held to its last bit and every
+// other one to 2^-75 of it at least (2^22 addends, all cut the same way, are off by
+// 2^-53).  There is room for 2^27 addends; a deck of 2^31 cells has fewer than 10^8.
+constexpr int DIGIT = 25, DIGITS = 4;
+constexpr int TOP_MIN = 2;  // of zero and the smallest doubles
+// Infinities and NaN: a place above all others, in which digit 0 counts what
+// holds +Inf, digit 2 what holds -Inf, NaN being both, so that none cancels another.
+constexpr int TOP_SPECIAL = 100;
 
-// The scale at which a number of the size of `ref` becomes about 2^62: 44 bits
-// above it for sums that grow (p.A p against r.r: the operator's eigenvalues),
-// 62 below it before anything is rounded off (a million addends, each rounded
-// to nearest, are off by some 2^-52 of the sum).
-__device__ __forceinline__ int fixed_scale(double ref) {
-  return 62 + 1023 - (int)((__double_as_longlong(ref) >> 52) & 0x7ff);
+typedef __int128 Whole;
+
+// +-m 2^(at - 1074)
+struct Addend {
+  unsigned long long m;
+  int at, top;  // top: the place of its highest digit
+  bool neg;
+};
+__device__ __forceinline__ Addend addend(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v);
+  const int e = (int)(hi >> 20) & 2047;
+  Addend a;
+  a.m = ((unsigned long long)((hi & 0xfffffu) | (e ? 0x100000u : 0u)) << 32) | (unsigned)__double2loint(v);
+  a.at = max(e, 1) - 1;
+  a.top = e == 2047 ? TOP_SPECIAL : (a.at + 52) / DIGIT;
+  a.neg = hi >> 31;
+  return a;
 }
-// v 2^scale, rounded.  What would reach 2^106 (infinities and NaN
-// among it) becomes 2^106: far beyond anything plausible beside 2^62.  A
-// warp's sum is cut to it once more (fixed_cut), so that no number of such
-// addends wraps round to a plausible sum.  `m` has `bits` bits at most.
-constexpr int FIXED_BITS = 106;
-__device__ __forceinline__ Fixed fixed_shift(unsigned long long m, int bits, int shift, bool neg) {
-  Fixed q;
-  if (shift >= 0) q = shift <= FIXED_BITS - bits ? (Fixed)m << shift : (Fixed)(m != 0) << FIXED_BITS;
-  else q = shift > -64 ? (Fixed)((m >> -shift) + ((m >> (-shift - 1)) & 1)) : (Fixed)0;
-  return neg ? -q : q;
+__device__ __forceinline__ Addend addend(float v) {
+  const unsigned u = __float_as_uint(v);
+  const int e = (int)(u >> 23) & 255;
+  Addend a;
+  a.m = (unsigned long long)((u & 0x7fffffu) | (e ? 0x800000u : 0u)) << 29;  // the leading bit as a double's
+  a.at = max(e, 1) + 895;
+  a.top = e == 255 ? TOP_SPECIAL : a.m ? (a.at + 52) / DIGIT : TOP_MIN;
+  a.neg = u >> 31;
+  return a;
 }
-__device__ __forceinline__ Fixed fixed_cut(Fixed q) {
-  const Fixed most = (Fixed)1 << FIXED_BITS;
-  return q > most ? most : q < -most ? -most : q;
+// Its four digits up to place `top`, at or above its own.
+__device__ __forceinline__ void digits(const Addend &a, int top, int (&d)[DIGITS]) {
+  constexpr unsigned ONES = (1u << DIGIT) - 1;
+  const int s = a.at - (top - (DIGITS - 1)) * DIGIT, left = max(s, 0);  // at most 47
+  const unsigned long long m = a.m >> min(max(-s, 0), 63), lo = m << left, hi = (m >> 1) >> (63 - left);
+  d[0] = (int)((unsigned)lo & ONES);
+  d[1] = (int)((unsigned)(lo >> DIGIT) & ONES);
+  d[2] = (int)(((unsigned)(lo >> 2 * DIGIT) | ((unsigned)hi << (64 - 2 * DIGIT))) & ONES);
+  d[3] = (int)((unsigned)(hi >> (3 * DIGIT - 64)) & ONES);
+#pragma unroll
+  for (int k = 0; k < DIGITS; ++k) d[k] = a.neg ? -d[k] : d[k];
 }
-__device__ __forceinline__ Fixed to_fixed(float v, int scale) {
-  const unsigned u = __float_as_uint(v), e = (u >> 23) & 255u;
-  const unsigned m = (u & 0x7fffffu) | (e ? 0x800000u : 0u);
-  return fixed_shift(e == 255u ? 1u : m, 24, e == 255u ? FIXED_BITS : (int)(e ? e : 1u) - 150 + scale, u >> 31);
+// Whether it counts in digit k of the special place.
+__device__ __forceinline__ bool counts(const Addend &a, int k) {
+  const bool nan = a.m & 0xfffffffffffffull;
+  return a.top == TOP_SPECIAL && (k == 0 ? nan || !a.neg : k == 2 && (nan || a.neg));
 }
-__device__ __forceinline__ Fixed to_fixed(double v, int scale) {
-  const unsigned long long u = (unsigned long long)__double_as_longlong(v), e = (u >> 52) & 2047u;
-  const unsigned long long m = (u & 0xfffffffffffffull) | (e ? 0x10000000000000ull : 0ull);
-  return fixed_shift(e == 2047u ? 1ull : m, 53, e == 2047u ? FIXED_BITS : (int)(e ? e : 1u) - 1075 + scale, u >> 63);
+__device__ __forceinline__ int pick(const int (&d)[DIGITS], int k) {
+  return k & 2 ? (k & 1 ? d[3] : d[2]) : (k & 1 ? d[1] : d[0]);
 }
-// The number a whole number of 2^-scale stands for, cut to 53 bits; NaN for a sum
-// that holds something cut to 2^106.
-__device__ __forceinline__ double from_fixed(Fixed q, int scale) {
+
+// A warp's share of a sum: each lane holds digit (lane & 3).
+struct Digits {
+  int top = TOP_MIN;
+  long long d = 0;
+};
+// The digits counted from a higher top: those below the four are dropped.
+__device__ __forceinline__ void raise_top(Digits &s, int top) {
+  const int k = (threadIdx.x & 3) + top - s.top;
+  const long long v = __shfl_sync(FULL, s.d, (threadIdx.x & 28) | (k & 3));
+  s.d = k < DIGITS ? v : 0;
+  s.top = top;
+}
+// Adds one number of each lane.
+__device__ __forceinline__ void add_lanes(Digits &s, double v) {
+  const Addend a = addend(v);
+  const int top = max(s.top, __reduce_max_sync(FULL, a.top)), k = threadIdx.x & 3;
+  if (top != s.top) raise_top(s, top);
+  if (top == TOP_SPECIAL) {
+    const bool plus = __any_sync(FULL, counts(a, 0)), minus = __any_sync(FULL, counts(a, 2));
+    s.d += k == 0 ? plus : k == 2 && minus;
+    return;
+  }
+  int d[DIGITS];
+  digits(a, top, d);
+#pragma unroll
+  for (int q = 0; q < DIGITS; ++q) d[q] = __reduce_add_sync(FULL, d[q]);
+  s.d += pick(d, k);
+}
+// Adds a pair to each of the warp's sums: eight lanes a sum, its pair in their first.
+__device__ __forceinline__ void add_pairs(Digits &s, Pair v) {
+  const int k = threadIdx.x & 3, first = threadIdx.x & 24;
+  const Addend hi = addend(__shfl_sync(FULL, v.hi, first)), lo = addend(__shfl_sync(FULL, v.lo, first));
+  raise_top(s, max(s.top, max(hi.top, lo.top)));
+  if (s.top == TOP_SPECIAL) {
+    s.d += counts(hi, k) || counts(lo, k);
+  } else {
+    int d[DIGITS], e[DIGITS];
+    digits(hi, s.top, d);
+    digits(lo, s.top, e);
+    s.d += pick(d, k) + pick(e, k);
+  }
+}
+
+// The four digits as one whole number.
+__device__ __forceinline__ Whole join(long long d0, long long d1, long long d2, long long d3) {
+  return (((((Whole)d3 << DIGIT) + d2) << DIGIT) + d1 << DIGIT) + d0;
+}
+// The double nearest to it.
+__device__ __forceinline__ double to_double(Whole q, int top) {
   const bool neg = q < 0;
-  unsigned __int128 a = neg ? (unsigned __int128)(-q) : (unsigned __int128)q;
-  const unsigned long long hi = (unsigned long long)(a >> 64), lo = (unsigned long long)a;
-  if (!(hi | lo)) return 0.0;
-  if (hi >> (FIXED_BITS - 64)) return __longlong_as_double(0x7ff8000000000000ll);
-  const int top = hi ? 127 - __clzll(hi) : 63 - __clzll(lo);  // of the leading bit
-  a = top > 52 ? a >> (top - 52) : a << (52 - top);
-  const int e = top - scale + 1023;
-  if (e >= 2047) return neg ? -INFINITY : INFINITY;
-  if (e <= 0) return 0.0;  // below the normal numbers: nothing of the sum is left
-  return __longlong_as_double((long long)((unsigned long long)a & 0xfffffffffffffull) | ((long long)e << 52) |
-                              ((long long)neg << 63));
-}
-__device__ __forceinline__ Fixed shfl_xor(Fixed v, int off) {
-  const unsigned __int128 u = (unsigned __int128)v;
-  unsigned long long lo = (unsigned long long)u, hi = (unsigned long long)(u >> 64);
-  lo = __shfl_xor_sync(FULL, lo, off);
-  hi = __shfl_xor_sync(FULL, hi, off);
-  return (Fixed)(((unsigned __int128)hi << 64) | lo);
-}
-__device__ __forceinline__ Fixed shfl(Fixed v, int lane) {
-  const unsigned __int128 u = (unsigned __int128)v;
-  unsigned long long lo = (unsigned long long)u, hi = (unsigned long long)(u >> 64);
-  lo = __shfl_sync(FULL, lo, lane);
-  hi = __shfl_sync(FULL, hi, lane);
-  return (Fixed)(((unsigned __int128)hi << 64) | lo);
+  const unsigned __int128 a = neg ? -(unsigned __int128)q : (unsigned __int128)q;
+  const unsigned long long h = (unsigned long long)(a >> 64), l = (unsigned long long)a, w = h ? h : l;
+  const int c = __clzll(w);
+  const unsigned long long hi = (w << c) | (h ? (l >> 1) >> (63 - c) : 0ull);  // the leading bit at the top
+  const int e = (h ? 127 : 63) - c + (top - (DIGITS - 1)) * DIGIT - 51;        // exponent field
+  unsigned long long m = ((unsigned long long)e << 52) + (hi >> 11) - (1ull << 52) + ((hi >> 10) & 1);
+  if (top == TOP_SPECIAL || !w || e < 1 || e >= 2047) {
+    if (top == TOP_SPECIAL) {
+      const bool plus = l & ((1ull << 2 * DIGIT) - 1), minus = a >> 2 * DIGIT;
+      return plus && minus ? __longlong_as_double(0x7ff8000000000000ll) : plus ? INFINITY : -INFINITY;
+    }
+    if (!w) return 0.0;
+    if (e >= 2047) return neg ? -INFINITY : INFINITY;
+    const int below = min(12 - e, 63);  // below the normal numbers
+    m = (hi >> below) + ((hi >> (below - 1)) & 1);
+  }
+  return __longlong_as_double((long long)(m | ((unsigned long long)neg << 63)));
 }
 
 // A persistent launch's block partials in global memory, two sets in turn (a
@@ -142,22 +209,14 @@ __device__ __forceinline__ Fixed shfl(Fixed v, int lane) {
 // Each block adds up all partials itself: adding them into one place with
 // atomics instead made an iteration 2.7 us longer (152 blocks on one line).
 constexpr int PERSIST_MAX_BLOCKS = 160;
-// The partials of one sum lie side by side: what the blocks' loads cost is the
-// 32-byte sectors that all of them want at once (three sums of 152 blocks, 64
-// bytes a block: 3.2 us a reduction against 3.0).
+// The partials of one sum lie side by side, a block's in one 32-byte sector: what the
+// blocks' loads cost is the sectors that all of them want at once (three sums of 152
+// blocks, 64 bytes a block: 3.2 us a reduction against 3.0).  A word holds a digit above
+// the 7 bits of its top.
 struct GridSums {
-  Fixed part[2][3][PERSIST_MAX_BLOCKS];
+  long long part[2][3][PERSIST_MAX_BLOCKS][DIGITS];
   Pair pair[2][PERSIST_MAX_BLOCKS][4];  // [.][.][3] pads a block to 32 bytes
 };
-
-__device__ __forceinline__ Fixed ldcg_fixed(const Fixed *p) {
-  const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(p));
-  return (Fixed)(((unsigned __int128)v.y << 64) | v.x);
-}
-__device__ __forceinline__ void stcg_fixed(Fixed *p, Fixed v) {
-  const unsigned __int128 u = (unsigned __int128)v;
-  __stcg(reinterpret_cast<ulonglong2 *>(p), make_ulonglong2((unsigned long long)u, (unsigned long long)(u >> 64)));
-}
 
 // A block's arrival at a barrier over the blocks of a cooperative launch and its
 // wait for `target` arrivals in all, by one whole warp.  False when the wait
@@ -214,123 +273,158 @@ struct RootTest {
 };
 
 struct SumShared {
-  Fixed warp[PERSIST_WARPS][3];
+  int top[3][PERSIST_WARPS];
+  long long digit[3][PERSIST_WARPS][DIGITS];
   Pair pair[PERSIST_WARPS][4];  // [.][3] pads a row to 32 bytes
   int ok;
 };
 
+// The digits (lane & 3) of sum `e` of every LANESth warp from the jth on, added up at
+// the highest top of the block's.
+template <int LANES, class Highest>
+__device__ __forceinline__ long long gather_digits(const SumShared &S, int e, int j, int &top, Highest &&highest) {
+  constexpr int N = PERSIST_WARPS / LANES;
+  const int k = threadIdx.x & 3;
+  int t[N];
+  top = TOP_MIN;
+#pragma unroll
+  for (int m = 0; m < N; ++m) top = max(top, t[m] = S.top[e][j + LANES * m]);
+  top = highest(top);
+  long long d = 0;
+#pragma unroll
+  for (int m = 0; m < N; ++m) {
+    const int at = k + top - t[m];
+    const long long x = S.digit[e][j + LANES * m][at & 3];
+    d += at < DIGITS ? x : 0;
+  }
+  return d;
+}
+// The block's digits of the one sum, in every lane; of the three, eight lanes each.
+__device__ __forceinline__ long long block_digits1(const SumShared &S, int &top) {
+  long long d = gather_digits<8>(S, 0, (threadIdx.x & 31) >> 2, top, [](int t) { return __reduce_max_sync(FULL, t); });
+#pragma unroll
+  for (int off = 16; off >= DIGITS; off >>= 1) d += __shfl_xor_sync(FULL, d, off);
+  return d;
+}
+__device__ __forceinline__ long long block_digits3(const SumShared &S, int &top) {
+  const int lane = threadIdx.x & 31;
+  const long long d = gather_digits<2>(S, lane < 24 ? lane >> 3 : 2, (lane & 7) >> 2, top,
+                                       [](int t) { return max(t, __shfl_xor_sync(FULL, t, DIGITS)); });
+  return d + __shfl_xor_sync(FULL, d, DIGITS);
+}
+__device__ __forceinline__ Whole join_lanes(long long d, int first) {
+  const long long d0 = __shfl_sync(FULL, d, first), d1 = __shfl_sync(FULL, d, first + 1), d2 = __shfl_sync(FULL, d, first + 2),
+                  d3 = __shfl_sync(FULL, d, first + 3);
+  return join(d0, d1, d2, d3);
+}
+
+// The blocks' partials of N sums, each warp's eight (and eight of the blocks past 128)
+// added up where its own digits were.  The whole block does it: one warp took
+// 800 cycles a sum, with the digits joined into 16 bytes, 1100 with them in 32.
+template <int N>
+__device__ __forceinline__ void spread_partials(SumShared &S, const long long (*part)[PERSIST_MAX_BLOCKS][DIGITS], int nb) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, b = 8 * warp + (lane >> 2);
+  long long w[N][2];
+#pragma unroll
+  for (int e = 0; e < N; ++e)
+#pragma unroll
+    for (int m = 0; m < 2; ++m) w[e][m] = b + 128 * m < nb ? __ldcg(&part[e][b + 128 * m][lane & 3]) : (long long)TOP_MIN;
+#pragma unroll
+  for (int e = 0; e < N; ++e) {
+    Digits s{(int)w[e][0] & 127, w[e][0] >> 7}, t{(int)w[e][1] & 127, w[e][1] >> 7};
+    const int top = __reduce_max_sync(FULL, max(s.top, t.top));
+    raise_top(s, top);
+    raise_top(t, top);
+    long long d = s.d + t.d;
+#pragma unroll
+    for (int off = 16; off >= DIGITS; off >>= 1) d += __shfl_xor_sync(FULL, d, off);
+    if (lane < DIGITS) S.digit[e][warp][lane] = d;
+    if (lane == 0) S.top[e][warp] = top;
+  }
+}
+
 // Sums over the grid and what follows from them: `fin(totals...)` on warp 0, and
-// the block meets.  One block barrier before the grid's, one after `fin`.
-// `set` counts the calls of a launch; target as in grid_barrier.
+// the block meets.  One block barrier before the grid's, two between it and `fin`,
+// one after.  `set` counts the calls of a launch; target as in grid_barrier.
 // Between reading and writing shared scalars `fin` needs a warp barrier.
 //
-// One sum: each warp's share in lane 0, in whole numbers of 2^-scale.
-template <class Fin>
-__device__ __forceinline__ bool grid_sum1(Grid grid, SumShared &S, GridBar *bar, GridSums *G, Fixed v, int scale, unsigned &target,
-                                          unsigned &set, Fin &&fin) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = grid.nb, nw = blockDim.x >> 5;
+// N = 1: each warp's digits of one sum.  N = 3: of three, the first in its lanes 0..7,
+// the second and third in the next eights.
+template <int N, class Fin>
+__device__ __forceinline__ bool grid_sum(Grid grid, SumShared &S, GridBar *bar, GridSums *G, const Digits &v, unsigned &target,
+                                         unsigned &set, Fin &&fin) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = grid.nb, e = lane >> 3, k = lane & 7;
+  const bool holds = e < N && k < DIGITS;
   target += nb;
-  if (lane == 0) S.warp[warp][0] = fixed_cut(v);
+  if (holds) {
+    S.digit[e][warp][k] = v.d;
+    if (k == 0) S.top[e][warp] = v.top;
+  }
   __syncthreads();
-  if (warp == 0) {
-    Fixed t = lane < nw ? S.warp[lane][0] : (Fixed)0;
-    for (int off = nw >> 1; off >= 1; off >>= 1) t += shfl_xor(t, off);
-    if (nb > 1) {
-      Fixed *part = G->part[set & 1][0];
-      if (lane == 0) stcg_fixed(part + grid.id, t);
+  int top;
+  auto block_digits = [&]() { return N == 1 ? block_digits1(S, top) : block_digits3(S, top); };
+  if (nb > 1) {
+    long long(*part)[PERSIST_MAX_BLOCKS][DIGITS] = G->part[set & 1];
+    if (warp == 0) {
+      const long long d = block_digits();
+      if (holds) __stcg(&part[e][grid.id][k], (d << 7) | top);
       S.ok = grid_arrive_wait(bar, target);
-      Fixed q[5];
-#pragma unroll
-      for (int m = 0; m < 5; ++m) q[m] = lane + 32 * m < nb ? ldcg_fixed(part + lane + 32 * m) : (Fixed)0;
-      t = q[0] + q[1] + q[2] + q[3] + q[4];
-#pragma unroll
-      for (int off = 16; off >= 1; off >>= 1) t += shfl_xor(t, off);
     }
-    fin(from_fixed(shfl(t, 0), scale));
+    __syncthreads();
+    spread_partials<N>(S, part, nb);
+    __syncthreads();
+  }
+  if (warp == 0) {
+    const Whole q = join_lanes(block_digits(), N == 1 ? 0 : lane & 24);
+    const double tot = to_double(q, top);
+    if constexpr (N == 1) fin(tot);
+    else fin(__shfl_sync(FULL, tot, 0), __shfl_sync(FULL, tot, 8), __shfl_sync(FULL, tot, 16));
   }
   ++set;
   __syncthreads();
   return nb == 1 || S.ok != 0;
 }
 
-// Three sums, each warp's share in lanes 0, 8 and 16.  Two forms: `v`, whole
-// numbers, for tiles taken in any order; `w`, pairs, which are cheaper to form
-// and to add (1.3 us of an iteration of 7.9 at 256^2), where every warp has its
-// one fixed tile.
-template <bool FIXED, class Fin>
-__device__ __forceinline__ bool grid_sum3(Grid grid, SumShared &S, GridBar *bar, GridSums *G, Fixed v, int scale, Pair w,
-                                          unsigned &target, unsigned &set, Fin &&fin) {
+// Three sums of pairs, each warp's share in lanes 0, 8 and 16: cheaper to form and
+// to add (1.3 us of an iteration of 7.9 at 256^2), where the warps' tiles are fixed.
+template <class Fin>
+__device__ __forceinline__ bool grid_sum_pairs(Grid grid, SumShared &S, GridBar *bar, GridSums *G, Pair w, unsigned &target,
+                                               unsigned &set, Fin &&fin) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nb = grid.nb, nw = blockDim.x >> 5;
   target += nb;
-  if ((lane & 7) == 0 && lane < 24) {
-    if (FIXED) S.warp[warp][lane >> 3] = fixed_cut(v);
-    else S.pair[warp][lane >> 3] = w;
-  }
+  if ((lane & 7) == 0 && lane < 24) S.pair[warp][lane >> 3] = w;
   __syncthreads();
   if (warp == 0) {
-    const int d = lane < 24 ? lane >> 3 : 2, c = lane & 7;
-    double tot;
-    if (FIXED) {
-      Fixed t = c < nw ? S.warp[c][d] : (Fixed)0;
-      if (nw > 8) t += S.warp[c + 8][d];
-      t += shfl_xor(t, 4);
-      t += shfl_xor(t, 2);
-      t += shfl_xor(t, 1);
-      if (nb > 1) {
-        Fixed(*part)[PERSIST_MAX_BLOCKS] = G->part[set & 1];
-        if (lane < 24 && c == 0) stcg_fixed(&part[d][grid.id], t);
-        S.ok = grid_arrive_wait(bar, target);
-        Fixed q[3][5], x[3];
+    Pair q[3] = {};
+    if (lane < nw) {
 #pragma unroll
-        for (int e = 0; e < 3; ++e)
-#pragma unroll
-          for (int m = 0; m < 5; ++m) q[e][m] = lane + 32 * m < nb ? ldcg_fixed(&part[e][lane + 32 * m]) : (Fixed)0;
-#pragma unroll
-        for (int e = 0; e < 3; ++e) x[e] = q[e][0] + q[e][1] + q[e][2] + q[e][3] + q[e][4];
-        // over the warp: lanes 0..7 end with the first sum, 8..15 the second, the rest the third
-        const bool up = lane & 16;
-        const Fixed a = shfl_xor(up ? x[0] : x[2], 16), b = shfl_xor(x[1], 16);
-        x[0] = up ? x[2] + a : x[0] + a;
-        x[1] = up ? (Fixed)0 : x[1] + b;
-        const bool second = !up && (lane & 8);
-        const Fixed f = shfl_xor(second || up ? x[0] : x[1], 8);
-        t = (second ? x[1] : x[0]) + f;
-        t += shfl_xor(t, 4);
-        t += shfl_xor(t, 2);
-        t += shfl_xor(t, 1);
-      }
-      tot = from_fixed(t, scale);
-    } else {
-      Pair q[3] = {};
-      if (lane < nw) {
-#pragma unroll
-        for (int m = 0; m < 3; ++m) q[m] = S.pair[lane][m];
-      }
-      Pair t = warp_pairs(q);
-      if (nb > 1) {
-        Pair(*part)[4] = G->pair[set & 1];
-        if (lane < 24 && c == 0) __stcg(reinterpret_cast<float2 *>(&part[grid.id][d]), make_float2(t.hi, t.lo));
-        S.ok = grid_arrive_wait(bar, target);
-        float4 ab[5];
-        float2 e[5];
-#pragma unroll
-        for (int m = 0; m < 5; ++m) {
-          const int k = lane + 32 * m;
-          ab[m] = k < nb ? __ldcg(reinterpret_cast<const float4 *>(&part[k][0])) : make_float4(0.f, 0.f, 0.f, 0.f);
-          e[m] = k < nb ? __ldcg(reinterpret_cast<const float2 *>(&part[k][2])) : make_float2(0.f, 0.f);
-        }
-#pragma unroll
-        for (int m = 0; m < 3; ++m) q[m] = Pair{0.f, 0.f};
-#pragma unroll
-        for (int m = 0; m < 5; ++m) {
-          q[0].add(Pair{ab[m].x, ab[m].y});
-          q[1].add(Pair{ab[m].z, ab[m].w});
-          q[2].add(Pair{e[m].x, e[m].y});
-        }
-        t = warp_pairs(q);
-      }
-      tot = (double)t.hi + (double)t.lo;
+      for (int m = 0; m < 3; ++m) q[m] = S.pair[lane][m];
     }
+    Pair t = warp_pairs(q);
+    if (nb > 1) {
+      Pair(*part)[4] = G->pair[set & 1];
+      if (lane < 24 && (lane & 7) == 0)
+        __stcg(reinterpret_cast<float2 *>(&part[grid.id][lane >> 3]), make_float2(t.hi, t.lo));
+      S.ok = grid_arrive_wait(bar, target);
+      float4 ab[5];
+      float2 e[5];
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        const int k = lane + 32 * m;
+        ab[m] = k < nb ? __ldcg(reinterpret_cast<const float4 *>(&part[k][0])) : make_float4(0.f, 0.f, 0.f, 0.f);
+        e[m] = k < nb ? __ldcg(reinterpret_cast<const float2 *>(&part[k][2])) : make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int m = 0; m < 3; ++m) q[m] = Pair{0.f, 0.f};
+#pragma unroll
+      for (int m = 0; m < 5; ++m) {
+        q[0].add(Pair{ab[m].x, ab[m].y});
+        q[1].add(Pair{ab[m].z, ab[m].w});
+        q[2].add(Pair{e[m].x, e[m].y});
+      }
+      t = warp_pairs(q);
+    }
+    const double tot = (double)t.hi + (double)t.lo;
     fin(__shfl_sync(FULL, tot, 0), __shfl_sync(FULL, tot, 8), __shfl_sync(FULL, tot, 16));
   }
   ++set;
@@ -338,11 +432,21 @@ __device__ __forceinline__ bool grid_sum3(Grid grid, SumShared &S, GridBar *bar,
   return nb == 1 || S.ok != 0;
 }
 
-// Adds a warp's lanes, in every lane.
-__device__ __forceinline__ Fixed warp_fixed(Fixed v) {
-#pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) v += shfl_xor(v, off);
-  return v;
+// A warp's share of three sums over its tiles, in either form.
+struct PassSums {
+  Digits d;
+  Pair w{0.f, 0.f};
+};
+template <bool HANDED>
+__device__ __forceinline__ void add_tile(PassSums &s, Pair tile) {
+  if (HANDED) add_pairs(s.d, tile);
+  else s.w.add(tile);
+}
+template <bool HANDED, class Fin>
+__device__ __forceinline__ bool grid_sums(Grid grid, SumShared &S, GridBar *bar, GridSums *G, const PassSums &v,
+                                          unsigned &target, unsigned &set, Fin &&fin) {
+  if constexpr (HANDED) return grid_sum<3>(grid, S, bar, G, v.d, target, set, fin);
+  else return grid_sum_pairs(grid, S, bar, G, v.w, target, set, fin);
 }
 
 // Copies into a ring of shared memory where every thread reads back only what

@@ -53,9 +53,11 @@ __device__ __forceinline__ double2 apply64(const Row64 &q, bool has1) {
 
 // Runs `body(j, i0, has1, row)` for every row of every tile this warp takes, on
 // all lanes (body stores and sums on owner lanes only: `owns`), and
-// `tile_end()` after each tile.  A neighbour across the domain's edge is the cell
-// itself; the second cell of a lane that has only one is zero.
-template <bool TWO, int NOWN, class Body, class TileEnd>
+// `tile_end()` after each tile; LATE: once the next tile's first rows are on their way
+// (CG where tiles are handed out: 326 us an iteration at 4096^2 against 331; on decks
+// of a tile a warp it costs more than it hides).  A neighbour across the domain's
+// edge is the cell itself; the second cell of a lane that has only one is zero.
+template <bool TWO, int NOWN, bool LATE = false, class Body, class TileEnd>
 __device__ __forceinline__ void ring64(Grid grid, const Ring64 &A, const Tiling &T, unsigned ring, bool mirrored, unsigned *next,
                                        unsigned &handed, Body &&body, TileEnd &&tile_end) {
   constexpr int NARR = 4 + TWO + NOWN;
@@ -66,6 +68,7 @@ __device__ __forceinline__ void ring64(Grid grid, const Ring64 &A, const Tiling 
   const unsigned slot0 = ring + 16 * lane;
   TileWalk walk(grid, T, ny, mirrored, next, handed);
   handed += walk.requests();
+  bool any = false;
   while (walk.valid()) {
     int strip, j0, j1;
     walk.place(strip, j0, j1);
@@ -99,6 +102,8 @@ __device__ __forceinline__ void ring64(Grid grid, const Ring64 &A, const Tiling 
     };
 #pragma unroll
     for (int d = 0; d < DEPTH - 1; ++d) issue(j0 - 1 + d, d);
+    if (LATE && any) tile_end();
+    any = true;
     Row64 q;
     q.s = q.c = make_double2(0.0, 0.0);
     q.ky = q.c;
@@ -142,9 +147,10 @@ __device__ __forceinline__ void ring64(Grid grid, const Ring64 &A, const Tiling 
       slot = slot + 1 == DEPTH ? 0 : slot + 1;
     }
     cp_wait<0>();
-    tile_end();
+    if (!LATE) tile_end();
     walk.take(asked);
   }
+  if (LATE && any) tile_end();
 }
 
 // Two cells of a row to memory.

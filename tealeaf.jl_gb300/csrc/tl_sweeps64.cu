@@ -81,9 +81,8 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_cheby64(const Loop64 A) {
     const double ca = F.chebyalpha[idx], cb = F.chebybeta[idx];
     const bool norm = k >= est && (tt + 1) % 10 == 0;  // Cheby.jl:48
     const bool store = norm || tt >= maxiters;
-    const int scale = fixed_scale(error);
     double acc = 0.0;
-    Fixed sum = 0;
+    Digits sum;
     ring64<false, 2>(whole_grid(), ring_of(A, u, F.u0, F.p), A.t, L.ring, L.mirrored, &A.F.sc->bar.next_tile, L.handed,
                      [&](int j, int i0, bool has1, bool owns, const Row64 &q) {
                        const double2 w = apply64(q, has1);
@@ -104,7 +103,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_cheby64(const Loop64 A) {
                        }
                      },
                      [&]() {
-                       if (norm) sum += to_fixed(acc, scale);
+                       if (norm) add_lanes(sum, acc);
                        acc = 0.0;
                      });
     L.mirrored = !L.mirrored;
@@ -113,7 +112,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_cheby64(const Loop64 A) {
     u = un;
     un = t;
     if (norm) {
-      if (!grid_sum1(whole_grid(), S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double rr) {
+      if (!grid_sum<1>(whole_grid(), S.sum, &sc->bar, A.sums, sum, L.target, L.set, [&](double rr) {
             const bool cv = test.met(rr);
             if ((threadIdx.x & 31) == 0) {
               S.a = rr;
@@ -178,15 +177,14 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_ppcg64(const Loop64 A) {
   const int maxiters = sc->maxiters;
   const double rtheta = 1.0 / sc->theta;
   int outer = sc->cheby_iters, iter = sc->iter;
-  double rro = sc->rro, alpha = 0.0, beta = sc->beta, pw_ref = rro;
+  double rro = sc->rro, alpha = 0.0, beta = sc->beta, pw = 0.0;
   bool first = sc->first != 0;  // the first direction is p itself
   double *p = F.p, *pn = F.pb;
   for (;;) {
     double acc = 0.0;
-    Fixed sum = 0;
-    int scale = fixed_scale(pw_ref);
+    Digits sum;
     auto tile_end = [&]() {
-      sum += to_fixed(acc, scale);
+      add_lanes(sum, acc);
       acc = 0.0;
     };
     auto direction = [&](int j, int i0, bool has1, bool owns, const Row64 &q) {
@@ -203,7 +201,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_ppcg64(const Loop64 A) {
     d.beta = beta;
     if (first) ring64<false, 0>(whole_grid(), d, A.t, L.ring, L.mirrored, &A.F.sc->bar.next_tile, L.handed, direction, tile_end);
     else ring64<true, 0>(whole_grid(), d, A.t, L.ring, L.mirrored, &A.F.sc->bar.next_tile, L.handed, direction, tile_end);
-    if (!grid_sum1(whole_grid(), S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double pw) {
+    if (!grid_sum<1>(whole_grid(), S.sum, &sc->bar, A.sums, sum, L.target, L.set, [&](double pw) {
           const double a = ddiv(rro, pw);
           if ((threadIdx.x & 31) == 0) {
             S.a = a;
@@ -212,7 +210,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_ppcg64(const Loop64 A) {
         }))
       return;
     alpha = S.a;
-    pw_ref = S.b;
+    pw = S.b;
     {
       double *t = p;
       p = pn;
@@ -222,8 +220,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_ppcg64(const Loop64 A) {
     L.mirrored = !L.mirrored;
     ppcg_update(A, L, p, alpha, rtheta);
     if (!grid_barrier(whole_grid(), &sc->bar, L.target)) return;
-    scale = fixed_scale(rro);
-    sum = 0;
+    sum = Digits{};
     for (int pp = 1; pp <= A.ninner; ++pp) {
       const double ca = F.chebyalpha[pp], cb = F.chebybeta[pp];
       const double *src = (pp & 1) ? F.sd : F.sdb;
@@ -246,12 +243,12 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_ppcg64(const Loop64 A) {
                          }
                        },
                        [&]() {
-                         if (last) sum += to_fixed(acc, scale);
+                         if (last) add_lanes(sum, acc);
                          acc = 0.0;
                        });
       if (!last && !grid_barrier(whole_grid(), &sc->bar, L.target)) return;
     }
-    if (!grid_sum1(whole_grid(), S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double rrn) {
+    if (!grid_sum<1>(whole_grid(), S.sum, &sc->bar, A.sums, sum, L.target, L.set, [&](double rrn) {
           const double b = ddiv(rrn, rro);  // PPCG.jl:89-92
           const bool cv = test.met(rrn);
           if ((threadIdx.x & 31) == 0) {
@@ -271,7 +268,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_ppcg64(const Loop64 A) {
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     sc->alpha = alpha;
-    sc->pw = pw_ref;
+    sc->pw = pw;
     sc->beta = beta;
     sc->rro = rro;
     sc->error = rro;
@@ -317,14 +314,12 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64(const Loop64 A) {
   const LoopTest test(sc);
   const int maxiters = sc->maxiters, lane = threadIdx.x & 31;
   int iter = sc->iter;
-  // a sweep changes no sum of |u' - u| beyond sqrt(cells) times |u|
-  double ref = sqrt(sc->bb), error = sc->error;
+  double error = sc->error;
   double *u = F.u, *un = F.ub;
   bool checked = false;
   for (;;) {
-    int scale = fixed_scale(ref);
     double acc = 0.0;
-    Fixed sum = 0;
+    Digits sum;
     ring64<false, 1>(whole_grid(), ring_of(A, u, F.u0, nullptr), A.t, L.ring, L.mirrored, &A.F.sc->bar.next_tile, L.handed,
                      [&](int j, int i0, bool has1, bool owns, const Row64 &q) {
                        const double2 v = jacobi_row(q, has1);
@@ -334,12 +329,12 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64(const Loop64 A) {
                        }
                      },
                      [&]() {
-                       sum += to_fixed(acc, scale);
+                       add_lanes(sum, acc);
                        acc = 0.0;
                      });
     ++iter;
     checked = iter % 50 == 0;
-    if (!grid_sum1(whole_grid(), S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double e) {
+    if (!grid_sum<1>(whole_grid(), S.sum, &sc->bar, A.sums, sum, L.target, L.set, [&](double e) {
           const bool cv = !checked && test.met(e);
           if (lane == 0) {
             S.a = e;
@@ -354,9 +349,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64(const Loop64 A) {
     u = un;
     un = t;
     if (checked) {  // every 50th sweep r = u0 - A u joins the error (Jacobi.jl:16-21)
-      const double scale_ref = sc->bb;
-      scale = fixed_scale(scale_ref);
-      sum = 0;
+      sum = Digits{};
       ring64<false, 1>(whole_grid(), ring_of(A, u, F.u0, nullptr), A.t, L.ring, L.mirrored, &A.F.sc->bar.next_tile, L.handed,
                        [&](int j, int i0, bool has1, bool owns, const Row64 &q) {
                          const double2 r = residual_row(q, has1);
@@ -367,10 +360,10 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64(const Loop64 A) {
                          }
                        },
                        [&]() {
-                         sum += to_fixed(acc, scale);
+                         add_lanes(sum, acc);
                          acc = 0.0;
                        });
-      if (!grid_sum1(whole_grid(), S.sum, &sc->bar, A.sums, warp_fixed(sum), scale, L.target, L.set, [&](double rr) {
+      if (!grid_sum<1>(whole_grid(), S.sum, &sc->bar, A.sums, sum, L.target, L.set, [&](double rr) {
             const double e = dadd(error, rr);
             const bool cv = test.met(e);
             if (lane == 0) {
@@ -382,9 +375,7 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64(const Loop64 A) {
         return;
       L.mirrored = !L.mirrored;
     }
-    const double e = S.a;
-    if (!checked && e > 0.0) ref = e;
-    error = e;
+    error = S.a;
     if (S.done) break;
   }
   // r .= u copies the last sweep's input, its depth-1 halo (the reflection)
@@ -487,14 +478,12 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64_resident(const Jac
     if (i0 == 0) o.w = o.c.x;
   };
   int iter = sc->iter;
-  // a sweep changes no sum of |u' - u| beyond sqrt(cells) times |u|
-  double ref = sqrt(sc->bb), error = sc->error;
+  double error = sc->error;
   double *u = F.u, *un = F.ub;
   unsigned target = 0, set = 0;
   bool checked = false;
   fetch(u, true);
   for (;;) {
-    const int scale = fixed_scale(ref);
     double acc1 = 0.0, acc2 = 0.0;
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
@@ -522,18 +511,20 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64_resident(const Jac
     }
     // Pairs start at even counts, so that the sweeps checked (every 50th) are their second.
     checked = (iter + 2) % 50 == 0;
-    const Fixed s1 = warp_fixed(to_fixed(acc1, scale)), s2 = warp_fixed(to_fixed(acc2, scale));
-    if (!grid_sum3<true>(whole_grid(), S.sum, &sc->bar, A.sums, lane == 0 ? s1 : lane == 8 ? s2 : (Fixed)0, scale, Pair{},
-                         target, set, [&](double e1, double e2, double) {
-                           const bool met1 = test.met(e1), first = met1 || iter + 1 >= maxiters;
-                           const bool cv = first ? met1 : !checked && test.met(e2);
-                           if (lane == 0) {
-                             S.a = first ? e1 : e2;
-                             S.first = first;
-                             S.conv = cv;
-                             S.done = first || (!checked && (cv || iter + 2 >= maxiters));
-                           }
-                         }))
+    Digits s1, s2;
+    add_lanes(s1, acc1);
+    add_lanes(s2, acc2);
+    const Digits both = lane < 8 ? s1 : lane < 16 ? s2 : Digits{};
+    if (!grid_sum<3>(whole_grid(), S.sum, &sc->bar, A.sums, both, target, set, [&](double e1, double e2, double) {
+          const bool met1 = test.met(e1), first = met1 || iter + 1 >= maxiters;
+          const bool cv = first ? met1 : !checked && test.met(e2);
+          if (lane == 0) {
+            S.a = first ? e1 : e2;
+            S.first = first;
+            S.conv = cv;
+            S.done = first || (!checked && (cv || iter + 2 >= maxiters));
+          }
+        }))
       return;
     error = S.a;
     if (S.first) {  // the first sweep ends it
@@ -547,7 +538,6 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64_resident(const Jac
     un = t;
     if (!S.done) fetch(u, false);
     if (checked) {  // every 50th sweep r = u0 - A u joins the error (Jacobi.jl:16-21)
-      const int rscale = fixed_scale(sc->bb);
       double acc = 0.0;
 #pragma unroll
       for (int m = 0; m < 2; ++m) {
@@ -561,20 +551,19 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64_resident(const Jac
           if (has1) acc = dadd(acc, dmul(r.y, r.y));
         }
       }
-      if (!grid_sum1(whole_grid(), S.sum, &sc->bar, A.sums, warp_fixed(to_fixed(acc, rscale)), rscale, target, set,
-                     [&](double rr) {
-                       const double e = dadd(error, rr);
-                       const bool cv = test.met(e);
-                       if (lane == 0) {
-                         S.a = e;
-                         S.conv = cv;
-                         S.done = cv || iter >= maxiters;
-                       }
-                     }))
+      Digits sum;
+      add_lanes(sum, acc);
+      if (!grid_sum<1>(whole_grid(), S.sum, &sc->bar, A.sums, sum, target, set, [&](double rr) {
+            const double e = dadd(error, rr);
+            const bool cv = test.met(e);
+            if (lane == 0) {
+              S.a = e;
+              S.conv = cv;
+              S.done = cv || iter >= maxiters;
+            }
+          }))
         return;
       error = S.a;
-    } else if (error > 0.0) {
-      ref = error;
     }
     if (S.done) break;
   }
