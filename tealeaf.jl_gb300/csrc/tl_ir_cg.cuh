@@ -55,6 +55,7 @@ struct PassArgs {
   float *rn, *sn;           // the next ones (r_old, for PASS_STEP2, is read from rn first)
   float alpha, beta;        // this step
   float alpha0, beta0;      // PASS_STEP2: the step before, whose p and x are formed here
+  float down;               // the sums' scale
   bool s_valid, p_valid, x_valid;  // false: zero, whatever the buffer holds
   bool mirrored;            // from the last rows to the first
 };
@@ -179,9 +180,9 @@ __device__ __forceinline__ void ir_pass(Grid grid, const IrCg &A, const PassArgs
           rp = r1;
         }
         if (++nrow == 4) {  // 16 products in FP32, then the pair
-          acc[0].add(ps[0]);
-          acc[1].add(ps[1]);
-          acc[2].add(ps[2]);
+          acc[0].add(q.down * ps[0]);
+          acc[1].add(q.down * ps[1]);
+          acc[2].add(q.down * ps[2]);
           ps[0] = ps[1] = ps[2] = 0.f;
           nrow = 0;
         }
@@ -197,7 +198,7 @@ __device__ __forceinline__ void ir_pass(Grid grid, const IrCg &A, const PassArgs
     cp_wait<0>();
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      acc[d].add(ps[d]);
+      acc[d].add(q.down * ps[d]);
       if (lane == 0 || lane == 31) acc[d] = Pair{0.f, 0.f};
     }
     add_tile<HANDED>(sums, warp_pairs(acc));
@@ -308,6 +309,7 @@ struct Shared {
   SumShared sum;
   double alpha, beta, gamma, inv_gamma, sigma;
   float alpha_f, beta_f;  // of the next step
+  Scale scale;
   int done, sw;
 };
 
@@ -358,16 +360,18 @@ __device__ __forceinline__ bool ir_loop(Grid grid, const IrCg &A, Shared &S, uns
 
   while (rel >= eps && iter < maxiters && !sw) {
     const double refine_below = A.delta2 * rr;
+    Scale scale = scale_of(rr, Scale{});
     {  // the sums of the residual that the refinement (or the start) left
       PassArgs q{};
       q.rc = rc;
       q.sc = sc_;
       q.s_valid = sv;
       q.mirrored = mirrored;
+      q.down = scale.down;
       PassSums sums;
       ir_pass<PASS_START, HANDED>(grid, A, q, ring, rxh, ryh, handed, sums);
       auto fin = [&](double, double f, double r) { next_scalars(S, rr, beta, rr + f, r); };
-      if (!grid_sums<HANDED>(grid, S.sum, bar, A.sums, sums, target, set, fin)) return false;
+      if (!grid_sums<HANDED>(grid, S.sum, bar, A.sums, sums, scale.up, target, set, fin)) return false;
       mirrored = !mirrored;
     }
     for (;;) {
@@ -385,6 +389,7 @@ __device__ __forceinline__ bool ir_loop(Grid grid, const IrCg &A, Shared &S, uns
       q.p_valid = pv;
       q.x_valid = xv;
       q.mirrored = mirrored;
+      q.down = scale.down;
       PassSums sums;
       if (pend) ir_pass<PASS_STEP2, HANDED>(grid, A, q, ring, rxh, ryh, handed, sums);
       else ir_pass<PASS_STEP, HANDED>(grid, A, q, ring, rxh, ryh, handed, sums);
@@ -405,9 +410,12 @@ __device__ __forceinline__ bool ir_loop(Grid grid, const IrCg &A, Shared &S, uns
           S.gamma = g;
           S.sw = switched;
         }
-        if (lane == 0) S.done = done;
+        if (lane == 0) {
+          S.done = done;
+          S.scale = scale_of(g, scale);
+        }
       };
-      if (!grid_sums<HANDED>(grid, S.sum, bar, A.sums, sums, target, set, fin)) return false;
+      if (!grid_sums<HANDED>(grid, S.sum, bar, A.sums, sums, scale.up, target, set, fin)) return false;
       mirrored = !mirrored;
       float *t = rc;
       rc = rn;
@@ -421,6 +429,7 @@ __device__ __forceinline__ bool ir_loop(Grid grid, const IrCg &A, Shared &S, uns
       alpha0 = q.alpha;
       beta0 = q.beta;
       ++iter;
+      scale = S.scale;
       if (S.done) break;
     }
     beta = S.beta;

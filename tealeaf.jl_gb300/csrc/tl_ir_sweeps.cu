@@ -46,6 +46,7 @@ struct StepArgs {
   float a1, b1, a2, b2;
   bool m_valid, z_valid;  // false: zero
   bool store_m, mirrored;
+  float down;  // the sums' scale
 };
 
 __device__ __forceinline__ float4 axpy4(float a, float4 x, float4 y) {
@@ -206,8 +207,8 @@ __device__ __forceinline__ void step_pass(Grid grid, const IrSweeps &A, const St
         }
       }
       if (++nrow == 4) {  // 16 products in FP32, then the pair
-        acc[0].add(ps[0]);
-        acc[1].add(ps[1]);
+        acc[0].add(q.down * ps[0]);
+        acc[1].add(q.down * ps[1]);
         ps[0] = ps[1] = 0.f;
         nrow = 0;
       }
@@ -226,8 +227,8 @@ __device__ __forceinline__ void step_pass(Grid grid, const IrSweeps &A, const St
       slot = slot + 1 == DEPTH ? 0 : slot + 1;
     }
     cp_wait<0>();
-    acc[0].add(ps[0]);
-    acc[1].add(ps[1]);
+    acc[0].add(q.down * ps[0]);
+    acc[1].add(q.down * ps[1]);
     if (sums) tile_sums<HANDED>(S, acc);
     walk.take(asked);
   }
@@ -236,7 +237,7 @@ __device__ __forceinline__ void step_pass(Grid grid, const IrSweeps &A, const St
 // p' = beta p + r into `pn`; p'.p' and its face sums (p'.A p' is both together).
 template <bool HANDED>
 __device__ __forceinline__ void direction_pass(Grid grid, const IrSweeps &A, const float *p, const float *r, float *pn,
-                                               float beta, unsigned ring, float rxh, float ryh, bool mirrored,
+                                               float beta, float down, unsigned ring, float rxh, float ryh, bool mirrored,
                                                unsigned &handed, PassSums &S) {
   constexpr int DEPTH = RING_BYTES / 1536;
   const int nx = A.g32.nx, ny = A.g32.ny;
@@ -293,8 +294,8 @@ __device__ __forceinline__ void direction_pass(Grid grid, const IrSweeps &A, con
         if (owns) st4(pn + col + (size_t)row * A.g32.pitch, pv);
       }
       if (++nrow == 4) {
-        acc[0].add(s[0]);
-        acc[1].add(s[1]);
+        acc[0].add(down * s[0]);
+        acc[1].add(down * s[1]);
         s[0] = s[1] = 0.f;
         nrow = 0;
       }
@@ -305,8 +306,8 @@ __device__ __forceinline__ void direction_pass(Grid grid, const IrSweeps &A, con
       slot = slot + 1 == DEPTH ? 0 : slot + 1;
     }
     cp_wait<0>();
-    acc[0].add(s[0]);
-    acc[1].add(s[1]);
+    acc[0].add(down * s[0]);
+    acc[1].add(down * s[1]);
     tile_sums<HANDED>(S, acc);
     walk.take(asked);
   }
@@ -316,6 +317,7 @@ struct SweepShared {
   SumShared sum;
   double a, b;
   float af;
+  Scale scale;
   int done;
 };
 
@@ -352,6 +354,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A
   while (rel >= eps && iter < maxiters) {
     const double refine_below = A.delta2 * rr;
     bool ev = false;
+    Scale scale = scale_of(rr, Scale{});
     for (;;) {
       const bool two = iter + 2 <= maxiters;
       const int i1 = min(ci + 2, maxiters + 1), i2 = min(ci + 3, maxiters + 1);
@@ -370,6 +373,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A
       q.z_valid = true;
       q.store_m = true;
       q.mirrored = mirrored;
+      q.down = scale.down;
       PassSums sums;
       if (two) step_pass<STEP_CHEBY, 2, HANDED>(grid, A, q, ring, rxh, ryh, true, handed, sums);
       else step_pass<STEP_CHEBY, 1, HANDED>(grid, A, q, ring, rxh, ryh, true, handed, sums);
@@ -379,10 +383,11 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A
         const bool hit = test.met(g) || below(g, refine_below) || test.met(g1) || below(g1, refine_below);
         if (lane == 0) {
           S.a = g;
+          S.scale = scale_of(g, scale);
           S.done = hit || iter + steps >= maxiters;
         }
       };
-      if (!grid_sums<HANDED>(grid, S.sum, &sc->bar, A.sums, sums, target, set, fin)) return;
+      if (!grid_sums<HANDED>(grid, S.sum, &sc->bar, A.sums, sums, scale.up, target, set, fin)) return;
       float *t = e;
       e = en;
       en = t;
@@ -394,6 +399,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_cheby32(const IrSweeps A
       iter += steps;
       ci += steps;
       err = S.a;
+      scale = S.scale;
       if (S.done) break;
     }
     fold_correction(grid, A, e);
@@ -438,10 +444,11 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ppcg32(const IrSweeps A)
   while (rel >= eps && iter < maxiters) {
     const double refine_below = A.delta2 * rr;
     double gamma = rr;
+    Scale scale = scale_of(rr, Scale{});
     bool xv = false;
     for (;;) {
       PassSums sums;
-      direction_pass<HANDED>(grid, A, p, r, spare, (float)beta, ring, rxh, ryh, mirrored, handed, sums);
+      direction_pass<HANDED>(grid, A, p, r, spare, (float)beta, scale.down, ring, rxh, ryh, mirrored, handed, sums);
       auto step = [&](double pp, double faces, double) {
         const double pw = pp + faces, a = gamma / pw;
         if (lane == 0) {
@@ -449,7 +456,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ppcg32(const IrSweeps A)
           S.af = (float)a;
         }
       };
-      if (!grid_sums<HANDED>(grid, S.sum, bar, A.sums, sums, target, set, step)) return;
+      if (!grid_sums<HANDED>(grid, S.sum, bar, A.sums, sums, scale.up, target, set, step)) return;
       mirrored = !mirrored;
       alpha = S.a;
       float *t = p;
@@ -475,6 +482,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ppcg32(const IrSweeps A)
         q.z_valid = xv;
         q.store_m = end < n;  // the last sweep's sd starts nothing
         q.mirrored = mirrored;
+        q.down = scale.down;
         const bool last = end == n;
         if (update) step_pass<STEP_UPDATE, 2, HANDED>(grid, A, q, ring, rxh, ryh, last, handed, sums);
         else if (two) step_pass<STEP_SWEEP, 2, HANDED>(grid, A, q, ring, rxh, ryh, last, handed, sums);
@@ -498,15 +506,17 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ppcg32(const IrSweeps A)
             if (lane == 0) {
               S.a = b;
               S.b = g;
+              S.scale = scale_of(g, scale);
               S.done = hit || iter + 1 >= maxiters;
             }
           };
-          if (!grid_sums<HANDED>(grid, S.sum, bar, A.sums, sums, target, set, fin)) return;
+          if (!grid_sums<HANDED>(grid, S.sum, bar, A.sums, sums, scale.up, target, set, fin)) return;
         }
         pp = end + 1;
       }
       beta = S.a;
       gamma = err = S.b;
+      scale = S.scale;
       ++iter;
       ++outer;
       if (S.done) break;
@@ -557,6 +567,7 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_bench32(const IrSweeps A
       q.sn = C.s[odd ^ 1];
       q.s_valid = q.p_valid = q.x_valid = true;
       q.mirrored = odd;
+      q.down = 1.f;
       if (kind == 8) ir_pass<PASS_STEP, true>(grid, C, q, ring, rxh, ryh, handed, sums);
       else ir_pass<PASS_STEP2, true>(grid, C, q, ring, rxh, ryh, handed, sums);
     } else {
@@ -569,12 +580,13 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_bench32(const IrSweeps A
       q.zo = kind == 6 ? (odd ? A.p : A.sd) : A.x;
       q.m_valid = q.z_valid = q.store_m = true;
       q.mirrored = odd;
+      q.down = 1.f;
       if (kind == 6) step_pass<STEP_CHEBY, 2, true>(grid, A, q, ring, rxh, ryh, true, handed, sums);
       else step_pass<STEP_SWEEP, 2, true>(grid, A, q, ring, rxh, ryh, false, handed, sums);
     }
     if (kind == 7) {
       if (!grid_barrier(grid, bar, target)) return;
-    } else if (!grid_sums<true>(grid, S, bar, A.sums, sums, target, set, [](double, double, double) {})) {
+    } else if (!grid_sums<true>(grid, S, bar, A.sums, sums, 0, target, set, [](double, double, double) {})) {
       return;
     }
   }

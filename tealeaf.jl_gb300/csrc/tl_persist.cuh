@@ -432,6 +432,28 @@ __device__ __forceinline__ bool grid_sum_pairs(Grid grid, SumShared &S, GridBar 
   return nb == 1 || S.ok != 0;
 }
 
+// The FP32 passes add up 16 products in FP32, as far as those go (3.4e38), and the pairs
+// of a tile, a warp or the whole grid beyond that: `down` is a power of two that
+// brings them to about 1 where the last r.r was `ref`, and the total gets 2^up back, both
+// exactly.  r.r may grow by 2^127 in a step, or fall by 2^100 and keep its bits.
+struct Scale {
+  float down = 1.f;
+  int up = 0;
+};
+__device__ __forceinline__ Scale scale_of(double ref, Scale last) {
+  const int e = (__double2hiint(ref) >> 20) & 2047, c = min(max(e, 1023 - 120), 1023 + 120);
+  if (e == 0 || e == 2047) return last;  // nothing to go by
+  Scale s;
+  s.down = __int_as_float((127 + 1023 - c) << 23);
+  s.up = c - 1023;
+  return s;
+}
+// v 2^up, for what a sum of FP32 numbers can be.
+__device__ __forceinline__ double scaled_up(double v, int up) {
+  const int hi = __double2hiint(v), e = (hi >> 20) & 2047;
+  return e == 0 || e == 2047 ? v : __hiloint2double(hi + (up << 20), __double2loint(v));
+}
+
 // A warp's share of three sums over its tiles, in either form.
 struct PassSums {
   Digits d;
@@ -443,10 +465,11 @@ __device__ __forceinline__ void add_tile(PassSums &s, Pair tile) {
   else s.w.add(tile);
 }
 template <bool HANDED, class Fin>
-__device__ __forceinline__ bool grid_sums(Grid grid, SumShared &S, GridBar *bar, GridSums *G, const PassSums &v,
+__device__ __forceinline__ bool grid_sums(Grid grid, SumShared &S, GridBar *bar, GridSums *G, const PassSums &v, int up,
                                           unsigned &target, unsigned &set, Fin &&fin) {
-  if constexpr (HANDED) return grid_sum<3>(grid, S, bar, G, v.d, target, set, fin);
-  else return grid_sum_pairs(grid, S, bar, G, v.w, target, set, fin);
+  auto scaled = [&](double a, double b, double c) { fin(scaled_up(a, up), scaled_up(b, up), scaled_up(c, up)); };
+  if constexpr (HANDED) return grid_sum<3>(grid, S, bar, G, v.d, target, set, scaled);
+  else return grid_sum_pairs(grid, S, bar, G, v.w, target, set, scaled);
 }
 
 // Copies into a ring of shared memory where every thread reads back only what

@@ -96,3 +96,16 @@ def test_infinities_and_nan(tl, built_lib, nx, ny, solver):
     (a, _), (b, _) = _solve(tl, text, change), _solve(tl, text, change, exact=True)
     assert (a.iters, a.converged, b.converged) == (b.iters, False, False)
     assert math.isnan(a.error) == math.isnan(b.error)
+
+
+@pytest.mark.parametrize("solver,nx,ny,k", [("cg", 256, 256, 51), ("cheby", 256, 256, 51), ("ppcg", 256, 256, 51),
+                                            ("cg", 1021, 769, 45), ("ppcg", 1021, 769, 45), ("cg", 2700, 2600, 40)])
+def test_fp32_sums_beyond_fp32(tl, built_lib, solver, nx, ny, k):
+    """Energies times 2^k, where r.r of the grid is above 3.4e38 and 16 products still
+    are not: every number of the solve is the unscaled one times a power of two, so the
+    steps are the same and u the same bits times 2^k."""
+    text = random_deck(nx, 6, ny=ny, solver=solver, presteps=40, eps=1e-10, errorswitch=1, epslim=1e250)
+    a, f = _solve(tl, text, precision=1, criterion=1)
+    b, g = _solve(tl, _scaled(text, 2.0 ** k), precision=1, criterion=1)
+    assert a.converged and b.converged and (a.iters, a.refinements) == (b.iters, b.refinements)
+    np.testing.assert_array_equal(g["u"], f["u"] * 2.0 ** k)
