@@ -40,7 +40,8 @@ struct BatchQueue {
 };
 
 // Takes decks for this block's group until none is left.  `solve(grid, args)`
-// runs one deck on the first blocks of the group, as many as its tiling uses.
+// runs one deck on the first blocks of the group, as many as its tiling uses; the
+// others wait at the group's barrier for as long as the deck's own counts on.
 template <class Args, class Solve, class Blocks>
 __device__ __forceinline__ void take_decks(const Args *decks, Args &A, BatchQueue *Q, int n, int size, Blocks &&blocks,
                                            Solve &&solve) {
@@ -49,7 +50,7 @@ __device__ __forceinline__ void take_decks(const Args *decks, Args &A, BatchQueu
   unsigned target = 0;
   for (unsigned turn = 0;; ++turn) {
     if (grid.id == 0 && threadIdx.x == 0) __stcg(&Q->slot[group][turn & 1], atomicAdd(&Q->next, 1u));
-    if (!grid_barrier(grid, &Q->bar[group], target)) return;
+    if (!grid_barrier(grid, &Q->bar[group], target, turn ? &A.F.sc->bar.count : nullptr)) return;
     const int d = (int)__ldcg(&Q->slot[group][turn & 1]);
     if (d >= n) {
       if (grid.id == 0 && threadIdx.x == 0) atomicAdd(&Q->finished, 1u);

@@ -15,7 +15,7 @@ namespace tl {
 
 constexpr int PERSIST_WARPS = 16;                 // warps of a persistent block
 constexpr int PERSIST_THREADS = 32 * PERSIST_WARPS;
-constexpr unsigned BAR_POLLS = 1u << 23;          // a wait gives up after some seconds
+constexpr unsigned BAR_POLLS = 1u << 23;          // a wait gives up after 1.3 s (314 cycles a poll)
 
 // A running sum as an unevaluated pair hi + lo of FP32 numbers (the two-sum of
 // Knuth): about 48 significant bits.  One FP64 instruction holds an SM
@@ -226,16 +226,22 @@ struct GridSums {
 // lane 0 alone waited, the compiler ran all that follows once for it and once
 // for the others (3 us a sum) and moved the others' loads ahead of the wait.
 // Acquiring loads, where plain ones with a fence after them took 0.25 to 0.35 us
-// more.
-__device__ __forceinline__ bool grid_arrive_wait(GridBar *g, unsigned target) {
+// more.  `busy`: a counter that whoever is waited for moves on; the limit counts
+// from its last change.
+__device__ __forceinline__ bool grid_arrive_wait(GridBar *g, unsigned target, const unsigned *busy = nullptr) {
   __syncwarp();
   if ((threadIdx.x & 31) == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&g->count) : "memory");
-  unsigned n = 0;
+  unsigned n = 0, last = 0;
   bool there;
   do {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&g->count) : "memory");
     there = __all_sync(FULL, (int)(v - target) >= 0);
+    if (busy && (n & 1023u) == 1023u) {
+      const unsigned now = __shfl_sync(FULL, *reinterpret_cast<const volatile unsigned *>(busy), 0);
+      if (now != last) n = 0;
+      last = now;
+    }
   } while (!there && ++n < BAR_POLLS);
   if (!there && (threadIdx.x & 31) == 0) atomicExch(&g->fail, 1u);
   return there;
@@ -243,12 +249,12 @@ __device__ __forceinline__ bool grid_arrive_wait(GridBar *g, unsigned target) {
 
 // The barrier for whole blocks; `target` counts the arrivals expected so far on
 // every thread (start at 0).
-__device__ __forceinline__ bool grid_barrier(Grid G, GridBar *g, unsigned &target) {
+__device__ __forceinline__ bool grid_barrier(Grid G, GridBar *g, unsigned &target, const unsigned *busy = nullptr) {
   __shared__ int ok;
   __syncthreads();
   if (G.nb == 1) return true;
   target += G.nb;
-  if (threadIdx.x < 32) ok = grid_arrive_wait(g, target);
+  if (threadIdx.x < 32) ok = grid_arrive_wait(g, target, busy);
   __syncthreads();
   return ok != 0;
 }
@@ -343,6 +349,12 @@ __device__ __forceinline__ void spread_partials(SumShared &S, const long long (*
   }
 }
 
+// A deck on one block has no barrier; its sums move the counter on all the same, for
+// those that wait for the deck (tl_batch.cu).
+__device__ __forceinline__ void count_alone(GridBar *bar) {
+  if (threadIdx.x == 0) asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(&bar->count) : "memory");
+}
+
 // Sums over the grid and what follows from them: `fin(totals...)` on warp 0, and
 // the block meets.  One block barrier before the grid's, two between it and `fin`,
 // one after.  `set` counts the calls of a launch; target as in grid_barrier.
@@ -373,6 +385,8 @@ __device__ __forceinline__ bool grid_sum(Grid grid, SumShared &S, GridBar *bar, 
     __syncthreads();
     spread_partials<N>(S, part, nb);
     __syncthreads();
+  } else {
+    count_alone(bar);
   }
   if (warp == 0) {
     const Whole q = join_lanes(block_digits(), N == 1 ? 0 : lane & 24);
@@ -423,6 +437,8 @@ __device__ __forceinline__ bool grid_sum_pairs(Grid grid, SumShared &S, GridBar 
         q[2].add(Pair{e[m].x, e[m].y});
       }
       t = warp_pairs(q);
+    } else {
+      count_alone(bar);
     }
     const double tot = (double)t.hi + (double)t.lo;
     fin(__shfl_sync(FULL, tot, 0), __shfl_sync(FULL, tot, 8), __shfl_sync(FULL, tot, 16));
