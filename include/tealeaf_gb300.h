@@ -185,7 +185,7 @@ int tl_reduction_layout(tl_ctx *ctx, int *warps, int *rows, int *blocks);
  * choice made, or override it (both for tuning studies; a set layout holds
  * until the context is destroyed).  The FP32 CG passes (8, 9) always run 16
  * warps a block and at most one block per SM: of a layout set for them, rows
- * and blocks take effect. */
+ * and blocks take effect.  A batch lays its decks out by itself. */
 int tl_get_layout(tl_ctx *ctx, int kernel, int *warps, int *rows, int *blocks);
 int tl_set_layout(tl_ctx *ctx, int kernel, int warps, int rows, int blocks);
 

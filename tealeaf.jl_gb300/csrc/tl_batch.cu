@@ -336,7 +336,7 @@ extern "C" int tl_batch_solve(tl_batch *b, const double *rx, const double *ry, c
   }
   // fixed and per-cell microseconds of an iteration: 5.5 and 11.5 at 1024^2 on 152 SMs, FP64 8 and 30
   int rc = ir ? place_decks(b, &b->d32, &b->groups32, &b->size32, 5.5, 0.87e-3,
-                            [](IrCg &A, tl_ctx *ctx, int size) { ir_cg_args(A, ctx, size); })
+                            [](IrCg &A, tl_ctx *ctx, int size) { ir_cg_args(A, ctx, size, false); })
               : place_decks(b, &b->d64, &b->groups64, &b->size64, 8.0, 3.1e-3, [](Cg64 &A, tl_ctx *ctx, int size) {
                   A.F = ctx->F;
                   A.g = ctx->g;

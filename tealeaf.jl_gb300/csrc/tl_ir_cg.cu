@@ -20,7 +20,7 @@ using namespace tl;
 // presteps' switch; the scalars are read back.  One launch.
 int tl_ir_cg_run(tl_ctx *ctx) {
   IrCg A;
-  ir_cg_args(A, ctx, persist_blocks(ctx->sm_count));
+  ir_cg_args(A, ctx, persist_blocks(ctx->sm_count), true);
   CK(cudaFuncSetAttribute(k_ir_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, RING_BYTES * PERSIST_WARPS));
   int rc = tl_bar_ready(ctx);
   if (rc) return rc;

@@ -488,7 +488,8 @@ __device__ __forceinline__ bool ir_solve(Grid grid, const IrCg &A, Shared &S, un
   return A.t.handed ? ir_loop<true>(grid, A, S, ring) : ir_loop<false>(grid, A, S, ring);
 }
 
-inline void ir_cg_args(IrCg &A, tl_ctx *ctx, int blocks) {
+// `set`: in the layout that tl_set_layout has set, if any.
+inline void ir_cg_args(IrCg &A, tl_ctx *ctx, int blocks, bool set) {
   tl_ir_state *ir = ctx->ir;
   A.F = ctx->F;
   A.g = ctx->g;
@@ -505,7 +506,7 @@ inline void ir_cg_args(IrCg &A, tl_ctx *ctx, int blocks) {
   // cycles and issue slots of a row and a tile, from the kernel's own counters
   const TileCost pass{2.0, 300.0, 1500.0, 200.0, 400.0, 16, 24, 8}, resid{1.0, 1200.0, 1500.0, 1100.0, 200.0, 0, 48, 4};
   A.t = make_tiling(ctx->g.nx, ctx->g.ny, STRIP, pass, blocks, PERSIST_WARPS);
-  if (ir->set_rows) {  // tl_set_layout: equal shares of bands of these rows
+  if (set && ir->set_rows) {  // equal shares of bands of these rows
     A.t.rows = ir->set_rows < ctx->g.ny ? ir->set_rows : ctx->g.ny;
     A.t.split = ctx->g.ny;
     A.t.tiles = A.t.tiles1 = A.t.ntx * ((ctx->g.ny + A.t.rows - 1) / A.t.rows);

@@ -700,7 +700,7 @@ int tl_ir_bench_kernel(tl_ctx *ctx, int kernel, int reps, double *ms_per_launch)
   if (rc) return rc;
   IrSweeps A = sweep_args(ctx, 0, 0.0);
   IrCg C;
-  ir_cg_args(C, ctx, persist_blocks(ctx->sm_count));
+  ir_cg_args(C, ctx, persist_blocks(ctx->sm_count), true);
   const size_t smem = (size_t)RING_BYTES * PERSIST_WARPS;
   CK(cudaFuncSetAttribute(k_bench32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if ((rc = tl_bar_ready(ctx))) return rc;
@@ -721,7 +721,7 @@ int tl_ir_get_layout(tl_ctx *ctx, int *warps, int *rows, int *blocks) {
   int rc = tl_ensure_ir(ctx);
   if (rc) return rc;
   IrCg C;
-  ir_cg_args(C, ctx, persist_blocks(ctx->sm_count));
+  ir_cg_args(C, ctx, persist_blocks(ctx->sm_count), true);
   *warps = ctx->ir->set_warps ? ctx->ir->set_warps : PERSIST_WARPS;
   *rows = C.t.rows;
   *blocks = C.t.blocks;
