@@ -269,19 +269,19 @@ struct OpWarmResid : NoSkip {
   }
 };
 
-// A prediction won: u = x, r = p = w, with their halo, and rr = its r.r (red[m]).
+// A prediction won: u = x, r = p = w, with the halo of u and p, and rr = its r.r
+// (red[m]).  Beyond the first layer x holds what its buffer held before.
 __global__ void k_warm_accept(Fields F, Geom g, const double *x, const double *w, int m) {
-  const long long n = (long long)g.X * g.Y;
+  const long long n = (long long)g.nx * g.ny;
   for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(k % g.X) - g.hd, j = (int)(k / g.X) - g.hd;
-    const size_t c = g.full(i + g.hd, j + g.hd);
-    F.u[c] = x[c];
-    if (i >= 0 && i < g.nx && j >= 0 && j < g.ny) {
-      const double v = w[c];
-      F.r[c] = v;
-      F.p[c] = v;
-      put_faces(F.p, g, c, i, j, v);
-    }
+    const int i = (int)(k % g.nx), j = (int)(k / g.nx);
+    const size_t c = g.at(i, j);
+    const double u = x[c], r = w[c];
+    F.u[c] = u;
+    F.r[c] = r;
+    F.p[c] = r;
+    put_faces(F.u, g, c, i, j, u);
+    put_faces(F.p, g, c, i, j, r);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) F.sc->rro = F.sc->red[m];
 }
