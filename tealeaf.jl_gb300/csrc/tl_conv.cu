@@ -1170,9 +1170,11 @@ __global__ void __launch_bounds__(DW_THREADS, 2) k_conv_dw(const bf16 *__restric
         float v[16];
         tc::tld16(tmem + ((uint32_t)(32 * r) << 16) + dx * NCOL + c0, v);
         const int zr = c0 / COUT, dy = r - zr, co = c0 % COUT;
-        if (dy < 0 || dy > 2 || ci >= CIN) continue;
+        if (dy >= 0 && dy <= 2 && ci < CIN) {
 #pragma unroll
-        for (int m = 0; m < 16; ++m) sums[zr * NW + (co + m) * 9 * CIN + (dy * 3 + dx) * CIN + ci] = any ? v[m] : 0.f;
+          for (int m = 0; m < 16; ++m) sums[zr * NW + (co + m) * 9 * CIN + (dy * 3 + dx) * CIN + ci] = any ? v[m] : 0.f;
+        }
+        __syncwarp();  // with 16 input channels half the lanes store nothing; the next load wants them all
       }
   }
   // the bias in both: threads of one pair are COUT / 2 apart
@@ -1192,6 +1194,7 @@ __global__ void __launch_bounds__(DW_THREADS, 2) k_conv_dw(const bf16 *__restric
   float *out = part + (size_t)blockIdx.x * NW;
 #pragma unroll 4
   for (int k = tid; k < NW; k += DW_THREADS) out[k] = sums[k] + sums[NW + k];
+  __syncwarp();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TALLOC));
 }
 
