@@ -259,8 +259,12 @@ __device__ __forceinline__ bool grid_barrier(Grid G, GridBar *g, unsigned &targe
   return ok != 0;
 }
 
-// Non-negative doubles in integer order: a compare on the FP64 pipe takes 64 cycles.
-__device__ __forceinline__ bool below(double a, double b) { return __double_as_longlong(a) < __double_as_longlong(b); }
+// a < b for an `a` that is not negative, in integer order: a compare on the FP64 pipe
+// takes 64 cycles.  Nothing is below NaN or a negative b, nor is NaN below anything.
+__device__ __forceinline__ bool below(double a, double b) {
+  const unsigned long long x = (unsigned long long)__double_as_longlong(a), y = (unsigned long long)__double_as_longlong(b);
+  return x < y && y <= 0x7ff0000000000000ull;
+}
 
 // A convergence test sqrt(e) < eps with e = error / bb (bb 1 for the absolute
 // test): what lies above `limit` fails it whatever its rounding, so that most

@@ -109,3 +109,22 @@ def test_fp32_sums_beyond_fp32(tl, built_lib, solver, nx, ny, k):
     b, g = _solve(tl, _scaled(text, 2.0 ** k), precision=1, criterion=1)
     assert a.converged and b.converged and (a.iters, a.refinements) == (b.iters, b.refinements)
     np.testing.assert_array_equal(g["u"], f["u"] * 2.0 ** k)
+
+
+@pytest.mark.parametrize("eps", [math.nan, -1.0, -0.0])
+@pytest.mark.parametrize("solver,criterion", [("cg", 0), ("cg", 1), ("cheby", 0), ("ppcg", 0), ("jacobi", 0)])
+def test_bounds_that_nothing_meets(tl, built_lib, solver, criterion, eps):
+    """No error is below NaN, a negative number or zero: the fused loops run to their
+    budget as the exact ones do."""
+    text = random_deck(61, 6, ny=47, solver=solver, presteps=10, errorswitch=1, epslim=1e9)
+    text = text.replace("max_iters=5000", "max_iters=40")
+    got = []
+    for exact in (False, True):
+        s = tl.Settings.from_text(text, mode=1, criterion=criterion, exact=exact)
+        s.eps = eps
+        c = tl.initialiseapp(s)
+        tl.haloupdate(c, s, 1, ["energy", "density"])
+        r = tl.SOLVERS[s.solver].solve(c, s, s.dtinit / s.dx ** 2, s.dtinit / s.dy ** 2)
+        got.append((r.converged, r.iters))
+        c.close()
+    assert got[0] == got[1] == (False, 40)
