@@ -47,9 +47,8 @@ DECK_SEED = 2024
 # over the timed timesteps; the GPU arm uses the counts it measures.
 FP64_ITERS_8192 = [4122, 3884, 3643, 3403, 3190, 2993, 2822, 2681, 2531, 2429, 2322, 2220, 2175, 2065, 2016, 1966,
                    1899, 1849, 1783, 1758, 1693, 1642, 1610, 1647, 1615]
-BYTES_PER_CELL_ITER = 104    # 13 FP64 words: stencil 4 + u/r update 6 + p update 3
-W_STEP_BYTES = 48            # fused p-update + stencil + p.w: read p, r, kx, ky; write p, w
-UR_STEP_BYTES = 48           # u/r update + r.r: read u, p, r, w; write u, r
+# 12 FP64 words: the direction pass reads p, r, kx, ky, diag, u and writes p, w, u, the residual's reads r, w and writes r
+BYTES_PER_CELL_ITER = 96
 
 
 def load_package():
@@ -273,23 +272,19 @@ def run_e2e(tl, n, precision, steps, warmup, warm=0):
 # FP32 CG iteration: one pass (read r, s, iw; write r, s: 20 B); every second
 # one also reads the older r, p and x and writes p and x (40 B)
 IR_ITER_BYTES = 30
-KERNELS = {"fp64": ((0, "cg_w_step", W_STEP_BYTES + 8), (1, "cg_ur_step", UR_STEP_BYTES)),
-           "fp32_ir": ((8, "ir_pass", 20), (9, "ir_pass_px", 40))}
-# DRAM bytes (read + write) per interior cell of one launch, from ncu
-# captures at 4096^2; traffic grows with the cells, so a full launch moves
-# this times n^2.
-TRAFFIC_BYTES_PER_CELL = {"cg_w_step": 923.7e6 / 4096 ** 2}
+PASSES = ((8, "ir_pass", 20), (9, "ir_pass_px", 40))
 
 
-def kernel_roofline(tl, chunk, kind, peak):
-    """Average duration of the two iteration kernels (FP32: passes of the one
-    iteration kernel) of one precision, 20 back to back on the library's
-    stream, timed with CUDA events; algorithmic bytes = compulsory reads + writes per interior
-    cell (the FP64 stencil step also reads the stored diagonal: 56 B)."""
+def kernel_roofline(tl, chunk, peak):
+    """Average duration of the two kinds of pass of the FP32 CG iteration, 20 back to
+    back on the library's stream, timed with CUDA events; algorithmic bytes =
+    compulsory reads + writes per interior cell.  (The FP64 loops' passes have no
+    timer of their own: ids 0, 1, 4, 5, 10 and 12 time kernels of the exact loops'
+    form that no fused loop runs.  ms_per_iteration is their rate.)"""
     lib = chunk.lib
     cells = chunk.settings.xcells * chunk.settings.ycells
     out = {}
-    for k, name, b in KERNELS[kind]:
+    for k, name, b in PASSES:
         ms = C.c_double()
         chunk.check(lib.tl_bench_kernel(chunk.ctx, k, 20, C.byref(ms)))
         gbs = b * cells / (ms.value * 1e-3) / 1e9
@@ -474,9 +469,8 @@ def gpu_arm(args):
             elif u64 is not None:
                 variants[name]["final_field_vs_fp64"] = accuracy_against(u, summ, u64, summ64)
             del u
-            if name == "fp64" or name == HEADLINE:
-                roof.update(kernel_roofline(tl, chunk, "fp64" if name == "fp64" else "fp32_ir", peak))
             if name == HEADLINE:
+                roof = kernel_roofline(tl, chunk, peak)
                 headline_res = results
             chunk.close()
     clocks = clk.summary()
@@ -504,16 +498,11 @@ def gpu_arm(args):
             "vs_fp64_gpu": {k: variants["fp64"]["ms_per_step"] / v["ms_per_step"] for k, v in variants.items()
                             if "ms_per_step" in v and "ms_per_step" in variants.get("fp64", {})}}
     if roof:
-        dom = max((v for k, v in roof.items() if k.startswith("ir_")), key=lambda d: d["ms"], default=None)
-        if dom is not None:
-            dname = [k for k, v in roof.items() if v is dom][0]
-            tpc = TRAFFIC_BYTES_PER_CELL.get(dname)
-            line["roofline"] = {"bound": "hbm", "kernel": dname, "achieved": dom["gbs"], "peak": peak,
-                                "unit": "GB/s", "frac": dom["gbs"] / peak,
-                                "traffic": tpc * n * n if tpc else None,
-                                "traffic_source": "ncu capture at 4096^2 scaled by cells" if tpc else None,
-                                "algorithmic_bytes": dom["bytes_per_cell"] * n * n,
-                                "peak_kind": peak_kind, "kernels": roof}
+        dname, dom = max(roof.items(), key=lambda d: d[1]["ms"])
+        line["roofline"] = {"bound": "hbm", "kernel": dname, "achieved": dom["gbs"], "peak": peak, "unit": "GB/s",
+                            "frac": dom["gbs"] / peak, "traffic": None,
+                            "algorithmic_bytes": dom["bytes_per_cell"] * n * n, "peak_kind": peak_kind,
+                            "kernels": roof}
     if rank == 0 and world == 1 and not args.no_config4:
         line["config4"] = config4_leg(tl)
     if rank == 0 and world == 1 and not args.no_cpu:
@@ -531,9 +520,35 @@ def gpu_arm(args):
         if not args.no_single:
             line["cpu_baseline"]["single_thread"] = cpu_single_thread(oracle, n, iters)
     if rank == 0:
-        print(json.dumps(line))
+        if args.detail:
+            Path(args.detail).write_text(json.dumps(line))
+        print(json.dumps(short_line(line)))
     if dist:
         dist.destroy_process_group()
+
+
+def short_line(line):
+    """The line as printed: what it says per step in one number each (a reader may
+    keep no more than the last few kB of the output), numbers to seven digits."""
+    def brief(d):
+        out = {}
+        for k, v in d.items():
+            if isinstance(v, dict):
+                out[k] = brief(v)
+            elif isinstance(v, list):
+                if k in ("iters", "launches", "refinements"):
+                    out[k] = sum(v)
+                elif k == "rel_residual":
+                    out["rel_residual_max"] = max(v)
+                elif k in ("final_summary", "reasons"):
+                    out[k] = v
+            else:
+                out[k] = float(f"{v:.7g}") if isinstance(v, float) else v
+        return out
+    out = brief(line)
+    for k in ("value", "ms_per_step"):
+        out[k] = line[k]
+    return out
 
 
 def config4_leg(tl):
@@ -560,7 +575,8 @@ state 3 density=0.1 energy=0.1 geometry=rectangle xmin=1.0 xmax=6.0 ymin=1.0 yma
 state 4 density=0.1 energy=0.1 geometry=rectangle xmin=5.0 xmax=6.0 ymin=1.0 ymax=8.0
 state 5 density=0.1 energy=0.1 geometry=rectangle xmin=5.0 xmax=10.0 ymin=7.0 ymax=8.0
 """
-# algorithmic bytes per interior cell of each timed kernel
+# algorithmic bytes per interior cell of each timed kernel (the FP64 ones: the exact
+# loops' form with the fused arithmetic, which no fused loop runs)
 CONFIG2_KERNELS = ((0, "cg_w_step", 48), (1, "cg_ur_step", 48), (4, "cheby_step", 72), (5, "ppcg_inner_sweep", 64),
                    (6, "cheby32_step", 12), (7, "ppcg32_inner_sweep", 14))
 
@@ -826,12 +842,12 @@ KERNEL_TABLE = (
 
 
 def run_kernels(args):
-    """Every fused iteration kernel launched from the host (`--reps` back to
-    back launches each, CUDA events on the library's stream) on the fields of
-    the 5-state deck at n^2 (4096 by default) after a short FP64 and a short
-    FP32-refined CG solve: per kernel the time, the algorithmic GB/s and its
-    fraction of the measured HBM peak.  Also the launch source for per-kernel
-    ncu captures (-k regex:<Op name> -c 1)."""
+    """What tl_bench_kernel times (`--reps` back to back, CUDA events on the
+    library's stream) on the fields of the 5-state deck at n^2 (4096 by default)
+    after a short FP64 and a short FP32-refined CG solve: per kernel the time, the
+    algorithmic GB/s and its fraction of the measured HBM peak.  The FP32 ids are
+    the passes of the solves; the FP64 ones are kernels of the exact loops' form,
+    which the fused loops no longer run."""
     import torch
     torch.cuda.set_device(0)
     tl = load_package()
@@ -903,6 +919,7 @@ def main():
     ap.add_argument("--size", type=int, default=8192)
     ap.add_argument("--variant", default="all", choices=["all"] + list(VARIANTS))
     ap.add_argument("--no-cpu", action="store_true")
+    ap.add_argument("--detail", help="timestep: a file for the whole line, with the numbers of each step")
     ap.add_argument("--no-single", action="store_true", help="skip the single-thread CPU sample")
     ap.add_argument("--no-config4", action="store_true", help="skip the batched 128-deck leg of the headline run")
     ap.add_argument("--workload", default="timestep", choices=["timestep", "config2", "config4", "config5", "cpucheck", "kernels"],
