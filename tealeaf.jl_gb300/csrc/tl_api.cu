@@ -126,6 +126,7 @@ extern "C" int tl_create(tl_ctx **out, const tl_config *cfg) {
   F.chebyalpha = F.cgbeta + tab;
   F.chebybeta = F.chebyalpha + tab;
   F.partials = F.chebybeta + tab;
+  ctx->coef_last = cfg->maxiters + 1;
   F.sc = reinterpret_cast<DevScalars *>(F.partials + (size_t)MAX_RED * max_blocks);
   F.counter = reinterpret_cast<unsigned *>(reinterpret_cast<char *>(F.sc) + sizeof(DevScalars));
   ctx->grid_sums = s + (small + 255) / 256 * 256;
@@ -154,6 +155,7 @@ extern "C" int tl_destroy(tl_ctx *ctx) {
   tl_release_graphs(ctx);
   if (ctx->buf) cudaFree(ctx->buf);
   if (ctx->small) cudaFree(ctx->small);
+  if (ctx->coef) cudaFree(ctx->coef);
   if (ctx->host_sc) cudaFreeHost(ctx->host_sc);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);

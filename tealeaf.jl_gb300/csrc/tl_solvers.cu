@@ -127,9 +127,26 @@ int eigenvalues(tl_ctx *ctx, int cgiters, double *emin, double *emax) {
   return TL_OK;
 }
 
+// Room for n coefficients: the context's tables hold one for each iteration, PPCG
+// takes one for each inner step.
+int coef_room(tl_ctx *ctx, int n) {
+  if (n <= ctx->coef_last) return TL_OK;
+  const size_t tab = (size_t)n + 1;
+  double *more = nullptr;
+  CK(cudaMalloc(&more, sizeof(double) * 2 * tab));
+  cudaStreamSynchronize(ctx->stream);
+  tl_release_graphs(ctx);  // they hold the old tables
+  if (ctx->coef) cudaFree(ctx->coef);
+  ctx->coef = more;
+  ctx->F.chebyalpha = more;
+  ctx->F.chebybeta = more + tab;
+  ctx->coef_last = n;
+  return TL_OK;
+}
+
 // coef! (Cheby.jl:121-135) into the device tables (1-based).
 int cheby_coef(tl_ctx *ctx, double emin, double emax, int n, double *theta) {
-  if (n > ctx->cfg.maxiters + 1) n = ctx->cfg.maxiters + 1;
+  if (n > ctx->coef_last) n = ctx->coef_last;
   *theta = (emax + emin) / 2;
   const double delta = (emax - emin) / 2;
   const double sigma = *theta / delta;
@@ -409,6 +426,7 @@ int tl_ppcg_solve(tl_ctx *ctx, double rx, double ry, const tl_params *prm, tl_re
   const int n = prm->ppcginnersteps;
   double emin, emax, theta;
   if ((rc = eigenvalues(ctx, cgiters, &emin, &emax))) return rc;  // PPCG.jl:41-42
+  if ((rc = coef_room(ctx, n))) return rc;
   if ((rc = cheby_coef(ctx, emin, emax, n, &theta))) return rc;
   if (fp32) {
     // the presteps' last refinement measured the true residual, which

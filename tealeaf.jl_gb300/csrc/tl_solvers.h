@@ -36,6 +36,8 @@ struct tl_ctx {
   tl::Fields F{};
   double *field_ptr[TL_NFIELDS] = {};
   tl::DevScalars *host_sc = nullptr;
+  double *coef = nullptr;     // the Chebyshev coefficient tables once PPCG has wanted more inner steps than maxiters + 1
+  int coef_last = 0;          // their last index
   void *grid_sums = nullptr;  // GridSums of the persistent kernels (tl_persist.cuh)
   int bar_clean = 0;          // the grid barrier is at zero
   int toexchange[TL_NEX] = {};
