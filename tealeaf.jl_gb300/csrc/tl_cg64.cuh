@@ -29,9 +29,9 @@ struct Cg64 {
 };
 
 // Small decks: with one row a warp, r is still in W's ring and w goes beside it, so
-// that R waits for no load and w for no store: 7.1 us an iteration at 64^2 against
-// 7.7, 8.2 against 8.7 at 256^2 (beta's division, formed with alpha's, among it).
-// With two rows a warp it gains nothing (12.9 both ways at 512^2).
+// that R waits for no load and w for no store: 7.2 us an iteration at 64^2 against
+// 7.9, 8.4 against 8.9 at 256^2.  With two rows a warp it gained nothing (12.9 both
+// ways at 512^2).
 constexpr int KEEP_ROWS = 1, KEEP_BYTES = KEEP_ROWS * 512;
 constexpr int CG64_SMEM = WARPS64 * (RING64_BYTES + KEEP_BYTES);
 // This warp's ring, and where it keeps w.
@@ -298,7 +298,7 @@ __device__ __forceinline__ bool cg64_solve(Grid grid, const Cg64 &A, Shared64 &S
 inline void cg64_tilings(Cg64 &A, int blocks) {
   // A row of W holds the FP64 pipe for 17 x 64 cycles, of R for 4 x 64.  W's
   // shares are even up to 48 rows a warp: there its tiles are the coarser, the
-  // better (93 us an iteration at 2048^2 against 105-113 with any tiles handed
+  // better (92 us an iteration at 2048^2 against 110 with tiles handed
   // out); beyond, what the SMs get of HBM differs (326 against 401 at 4096^2).
   const TileCost w{0.25, 1100.0, 1500.0, 1100.0, 200.0, 16, 48, 4}, r{0.0, 300.0, 1000.0, 260.0, 150.0, 0, 24, 8};
   A.tw = make_tiling(A.g.nx, A.g.ny, STRIP64, w, blocks, WARPS64);

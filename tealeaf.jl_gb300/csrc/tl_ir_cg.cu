@@ -15,8 +15,8 @@ __global__ void __launch_bounds__(PERSIST_THREADS, 1) k_ir_cg(const IrCg A) {
 
 using namespace tl;
 
-// Runs the FP32-refined CG loop on the state that tl_cg_init, copyu! and the
-// FP32 copies left, to the relative true residual, the iteration budget or the
+// Runs the FP32-refined CG loop on the state that tl_solve_start (or the warm start
+// after it) left, to the relative true residual, the iteration budget or the
 // presteps' switch; the scalars are read back.  One launch.
 int tl_ir_cg_run(tl_ctx *ctx) {
   IrCg A;

@@ -1,12 +1,13 @@
 // tl_persist.cuh -- pieces of the persistent (cooperative) iteration kernels:
-// the grid barrier, thread-private copy rings and the FP32-pair accumulator.
+// the grid barrier, the sums over the grid and thread-private copy rings.
 //
 // A persistent kernel runs a whole iteration loop in one launch of at most one
 // block per SM: a graph with a while-node spends 9 us on each kernel boundary
 // of a small deck (18-20 us per CG iteration up to 512^2, whatever the
-// deck), a barrier here 1.5 us.  Every block adds the block partials of a
-// reduction itself, in the same order, so all blocks hold the same scalars bit
-// for bit and take the same decisions without another broadcast.
+// deck), a barrier here takes 1.2 us over 152 blocks (0.9 over two), with a sum of
+// digits 2.6, with three 3.0, with three sums of pairs 2.1.  Every block adds the
+// block partials of a reduction itself, so all blocks hold the same scalars bit for
+// bit and take the same decisions without another broadcast.
 #pragma once
 
 #include "tl_walk.cuh"
@@ -210,9 +211,8 @@ __device__ __forceinline__ double to_double(Whole q, int top) {
 // atomics instead made an iteration 2.7 us longer (152 blocks on one line).
 constexpr int PERSIST_MAX_BLOCKS = 160;
 // The partials of one sum lie side by side, a block's in one 32-byte sector: what the
-// blocks' loads cost is the sectors that all of them want at once (three sums of 152
-// blocks, 64 bytes a block: 3.2 us a reduction against 3.0).  A word holds a digit above
-// the 7 bits of its top.
+// blocks' loads cost is the sectors that all of them want at once.  A word holds a
+// digit above the 7 bits of its top.
 struct GridSums {
   long long part[2][3][PERSIST_MAX_BLOCKS][DIGITS];
   Pair pair[2][PERSIST_MAX_BLOCKS][4];  // [.][.][3] pads a block to 32 bytes
@@ -404,7 +404,7 @@ __device__ __forceinline__ bool grid_sum(Grid grid, SumShared &S, GridBar *bar, 
 }
 
 // Three sums of pairs, each warp's share in lanes 0, 8 and 16: cheaper to form and
-// to add (1.3 us of an iteration of 7.9 at 256^2), where the warps' tiles are fixed.
+// to add (2.1 us over 152 blocks against 3.0), where the warps' tiles are fixed.
 template <class Fin>
 __device__ __forceinline__ bool grid_sum_pairs(Grid grid, SumShared &S, GridBar *bar, GridSums *G, Pair w, unsigned &target,
                                                unsigned &set, Fin &&fin) {
@@ -581,8 +581,8 @@ inline int persist_blocks(int sm_count) { return sm_count < PERSIST_MAX_BLOCKS ?
 // out.  A tile takes `lat` cycles a row and `lat0` besides when its warp runs
 // alone, `issue` and `issue0` of a sub-partition's issue (or FP64) slots; `extra`
 // rows overlap the next tile.  A deck of at most `solo` strip rows runs on one
-// block, which needs no grid barrier: a row a warp (28^2 by FP64 CG: 8.1 us an
-// iteration spread over blocks, 10.6 with two rows a warp on one).
+// block, which needs no grid barrier: a row a warp (28^2 by FP64 CG: 7.4 us an
+// iteration spread over blocks, 10.2 with two rows a warp on one).
 struct TileCost {
   double extra, lat, lat0, issue, issue0;
   int solo, hand_from, rows2;

@@ -4,7 +4,7 @@
 //
 // Every pass is a ring64 march, bound by the FP64 pipe on large grids; on small
 // ones a pass cost 4-7 us as a kernel of a graph, and costs a grid barrier
-// (1.3 us) here, with the reduction (1.5 us more) only where a test reads it:
+// (1.2 us) here, with the reduction (1.4 us more) only where a test reads it:
 // each Jacobi sweep, the last sweep of a PPCG step, and the Chebyshev steps
 // that take the norm (Cheby.jl:48), which are also the only ones that can be
 // the last and so the only ones that store w and r.
@@ -411,8 +411,9 @@ __global__ void __launch_bounds__(WARPS64 * 32, 1) k_jacobi64(const Loop64 A) {
 // What a sweep of a small deck costs is a grid barrier with its reduction and
 // the latency of its loads, which the pair has once and the operands not at
 // all; 28 FP64 instructions a row and pair, 10 for each of the two more.
-// A sweep: 250^2 3.8 us against 5.1 swept one by one (k_jacobi64), 100^2 3.0,
-// 400^2 5.3; of 7.6 us a pair, 1.2 wait at the barrier and 2.4 add up its sums.
+// A sweep: 250^2 3.5 us against 4.7 swept one by one (k_jacobi64), 100^2 2.6 against
+// 3.9, 400^2 5.0 against 9.1; of 6.9 us a pair at 250^2, 1.2 wait at the barrier and 1.8
+// add up its sums.
 constexpr int RES_ROWS = 30;  // two rows a warp with those on the sides
 
 struct Jacobi64 {
@@ -652,7 +653,7 @@ int tl_loop64_run(tl_ctx *ctx, int which, int ninner, double *ms) {
   const void *kernel = which == TL_GRAPH_CHEBY_EXACT  ? (const void *)k_cheby64
                        : which == TL_GRAPH_PPCG_EXACT ? (const void *)k_ppcg64
                                                       : (const void *)k_jacobi64;
-  // a row holds the FP64 pipe for 14 to 20 instructions of 64 cycles; see tl_cg64_run for the rule
+  // a row holds the FP64 pipe for 14 to 20 instructions of 64 cycles; see cg64_tilings for the rule
   const TileCost sweep{0.1, 1200.0, 1500.0, 1150.0, 200.0, 16, 48, 4}, each{0.0, 500.0, 1000.0, 400.0, 150.0, 0, 24, 8};
   A.t = make_tiling(ctx->g.nx, ctx->g.ny, STRIP64, sweep, blocks, WARPS64);
   A.te = make_tiling_on(A.t, ctx->g.nx, ctx->g.ny, 64, each, WARPS64);
