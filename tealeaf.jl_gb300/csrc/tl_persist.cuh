@@ -118,7 +118,7 @@ __device__ __forceinline__ Addend addend(float v) {
 // Its four digits up to place `top`, at or above its own.
 __device__ __forceinline__ void digits(const Addend &a, int top, int (&d)[DIGITS]) {
   constexpr unsigned ONES = (1u << DIGIT) - 1;
-  const int s = a.at - (top - (DIGITS - 1)) * DIGIT, left = max(s, 0);  // at most 47
+  const int s = a.at - (top - (DIGITS - 1)) * DIGIT, left = min(max(s, 0), 47);  // more for a zero alone
   const unsigned long long m = a.m >> min(max(-s, 0), 63), lo = m << left, hi = (m >> 1) >> (63 - left);
   d[0] = (int)((unsigned)lo & ONES);
   d[1] = (int)((unsigned)(lo >> DIGIT) & ONES);
@@ -471,7 +471,7 @@ __device__ __forceinline__ Scale scale_of(double ref, Scale last) {
 // v 2^up, for what a sum of FP32 numbers can be.
 __device__ __forceinline__ double scaled_up(double v, int up) {
   const int hi = __double2hiint(v), e = (hi >> 20) & 2047;
-  return e == 0 || e == 2047 ? v : __hiloint2double(hi + (up << 20), __double2loint(v));
+  return e == 0 || e == 2047 ? v : __hiloint2double(hi + up * (1 << 20), __double2loint(v));
 }
 
 // A warp's share of three sums over its tiles, in either form.
