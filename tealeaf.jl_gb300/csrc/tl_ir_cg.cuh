@@ -73,11 +73,11 @@ __device__ __forceinline__ void ir_pass(Grid grid, const IrCg &A, const PassArgs
   const int lane = threadIdx.x & 31;
   const unsigned slot0 = ring + 16 * lane;
   TileWalk walk(grid, A.t, ny, q.mirrored, &A.F.sc->bar.next_tile, handed);
-  handed += walk.requests();
+  if (HANDED) handed += walk.requests();
   while (walk.valid()) {
     int strip, j0, j1;
     walk.place(strip, j0, j1);
-    const unsigned asked = walk.ask();
+    const unsigned asked = HANDED ? walk.ask() : 0u;
     const int i0 = strip * STRIP - 4 + 4 * lane;
     const bool in = i0 >= 0 && i0 < nx;
     const bool owns = lane >= 1 && lane <= 30 && i0 < nx;
@@ -202,7 +202,8 @@ __device__ __forceinline__ void ir_pass(Grid grid, const IrCg &A, const PassArgs
       if (lane == 0 || lane == 31) acc[d] = Pair{0.f, 0.f};
     }
     add_tile<HANDED>(sums, warp_pairs(acc));
-    walk.take(asked);
+    if (HANDED) walk.take(asked);
+    else walk.step();
   }
 }
 

@@ -104,11 +104,11 @@ __device__ __forceinline__ void step_pass(Grid grid, const IrSweeps &A, const St
   const int lane = threadIdx.x & 31;
   const unsigned slot0 = ring + 16 * lane;
   TileWalk walk(grid, A.t, ny, q.mirrored, &A.F.sc->bar.next_tile, handed);
-  handed += walk.requests();
+  if (HANDED) handed += walk.requests();
   while (walk.valid()) {
     int strip, j0, j1;
     walk.place(strip, j0, j1);
-    const unsigned asked = walk.ask();
+    const unsigned asked = HANDED ? walk.ask() : 0u;
     const int i0 = strip * STRIP - 4 + 4 * lane;
     const bool in = i0 >= 0 && i0 < nx;
     const bool owns = lane >= 1 && lane <= 30 && i0 < nx;
@@ -230,7 +230,8 @@ __device__ __forceinline__ void step_pass(Grid grid, const IrSweeps &A, const St
     acc[0].add(q.down * ps[0]);
     acc[1].add(q.down * ps[1]);
     if (sums) tile_sums<HANDED>(S, acc);
-    walk.take(asked);
+    if (HANDED) walk.take(asked);
+    else walk.step();
   }
 }
 
@@ -244,11 +245,11 @@ __device__ __forceinline__ void direction_pass(Grid grid, const IrSweeps &A, con
   const int lane = threadIdx.x & 31;
   const unsigned slot0 = ring + 16 * lane;
   TileWalk walk(grid, A.t, ny, mirrored, &A.F.sc->bar.next_tile, handed);
-  handed += walk.requests();
+  if (HANDED) handed += walk.requests();
   while (walk.valid()) {
     int strip, j0, j1;
     walk.place(strip, j0, j1);
-    const unsigned asked = walk.ask();
+    const unsigned asked = HANDED ? walk.ask() : 0u;
     const int i0 = strip * STRIP - 4 + 4 * lane;
     const bool in = i0 >= 0 && i0 < nx;
     const bool owns = lane >= 1 && lane <= 30 && i0 < nx;
@@ -309,7 +310,8 @@ __device__ __forceinline__ void direction_pass(Grid grid, const IrSweeps &A, con
     acc[0].add(down * s[0]);
     acc[1].add(down * s[1]);
     tile_sums<HANDED>(S, acc);
-    walk.take(asked);
+    if (HANDED) walk.take(asked);
+    else walk.step();
   }
 }
 

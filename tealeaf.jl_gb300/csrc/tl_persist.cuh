@@ -569,6 +569,8 @@ struct TileWalk {
   __device__ __forceinline__ void take(unsigned asked) {
     t = T.handed ? T.warps + (int)(__shfl_sync(FULL, asked, 0) - base) : t + T.warps;
   }
+  // the same where it is known that none are handed out
+  __device__ __forceinline__ void step() { t += T.warps; }
   // requests a whole pass makes: each warp asks once for each of its tiles
   __device__ __forceinline__ unsigned requests() const { return T.handed ? (unsigned)T.tiles : 0u; }
 };
