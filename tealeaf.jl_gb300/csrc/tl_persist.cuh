@@ -105,16 +105,6 @@ __device__ __forceinline__ Addend addend(double v) {
   a.neg = hi >> 31;
   return a;
 }
-__device__ __forceinline__ Addend addend(float v) {
-  const unsigned u = __float_as_uint(v);
-  const int e = (int)(u >> 23) & 255;
-  Addend a;
-  a.m = (unsigned long long)((u & 0x7fffffu) | (e ? 0x800000u : 0u)) << 29;  // the leading bit as a double's
-  a.at = max(e, 1) + 895;
-  a.top = e == 255 ? TOP_SPECIAL : a.m ? (a.at + 52) / DIGIT : TOP_MIN;
-  a.neg = u >> 31;
-  return a;
-}
 // Its four digits up to place `top`, at or above its own.
 __device__ __forceinline__ void digits(const Addend &a, int top, int (&d)[DIGITS]) {
   constexpr unsigned ONES = (1u << DIGIT) - 1;
@@ -127,10 +117,9 @@ __device__ __forceinline__ void digits(const Addend &a, int top, int (&d)[DIGITS
 #pragma unroll
   for (int k = 0; k < DIGITS; ++k) d[k] = a.neg ? -d[k] : d[k];
 }
-// Whether it counts in digit k of the special place.
-__device__ __forceinline__ bool counts(const Addend &a, int k) {
-  const bool nan = a.m & 0xfffffffffffffull;
-  return a.top == TOP_SPECIAL && (k == 0 ? nan || !a.neg : k == 2 && (nan || a.neg));
+// Whether a number counts in digit k of the special place.
+__device__ __forceinline__ bool counts(bool special, bool nan, bool neg, int k) {
+  return special && (k == 0 ? nan || !neg : k == 2 && (nan || neg));
 }
 __device__ __forceinline__ int pick(const int (&d)[DIGITS], int k) {
   return k & 2 ? (k & 1 ? d[3] : d[2]) : (k & 1 ? d[1] : d[0]);
@@ -154,7 +143,8 @@ __device__ __forceinline__ void add_lanes(Digits &s, double v) {
   const int top = max(s.top, __reduce_max_sync(FULL, a.top)), k = threadIdx.x & 3;
   if (top != s.top) raise_top(s, top);
   if (top == TOP_SPECIAL) {
-    const bool plus = __any_sync(FULL, counts(a, 0)), minus = __any_sync(FULL, counts(a, 2));
+    const bool special = a.top == TOP_SPECIAL, nan = a.m & 0xfffffffffffffull;
+    const bool plus = __any_sync(FULL, counts(special, nan, a.neg, 0)), minus = __any_sync(FULL, counts(special, nan, a.neg, 2));
     s.d += k == 0 ? plus : k == 2 && minus;
     return;
   }
@@ -165,17 +155,32 @@ __device__ __forceinline__ void add_lanes(Digits &s, double v) {
   s.d += pick(d, k);
 }
 // Adds a pair to each of the warp's sums: eight lanes a sum, its pair in their first.
+// Both numbers go into one integer, cut 52 bits below the larger one's leading bit, of
+// which each lane takes its digit.
 __device__ __forceinline__ void add_pairs(Digits &s, Pair v) {
   const int k = threadIdx.x & 3, first = threadIdx.x & 24;
-  const Addend hi = addend(__shfl_sync(FULL, v.hi, first)), lo = addend(__shfl_sync(FULL, v.lo, first));
-  raise_top(s, max(s.top, max(hi.top, lo.top)));
-  if (s.top == TOP_SPECIAL) {
-    s.d += counts(hi, k) || counts(lo, k);
+  const unsigned u[2] = {__float_as_uint(__shfl_sync(FULL, v.hi, first)), __float_as_uint(__shfl_sync(FULL, v.lo, first))};
+  const int e[2] = {(int)(u[0] >> 23) & 255, (int)(u[1] >> 23) & 255}, most = max(max(e[0], e[1]), 1);
+  long long m = 0;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const unsigned long long x = ((unsigned long long)((u[q] & 0x7fffffu) | (e[q] ? 0x800000u : 0u)) << 29) >>
+                                 min(most - max(e[q], 1), 63);
+    m += u[q] >> 31 ? -(long long)x : (long long)x;
+  }
+  const int at = most + 895;  // below 2^54, it counts 2^(at - 1074)
+  const int top = max(s.top, most == 255 ? TOP_SPECIAL : m ? (at + 53) / DIGIT : TOP_MIN);
+  if (__any_sync(FULL, top != s.top)) raise_top(s, top);
+  if (top == TOP_SPECIAL) {
+    bool count = false;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) count = count || counts(e[q] == 255, u[q] & 0x7fffffu, u[q] >> 31, k);
+    s.d += count;
   } else {
-    int d[DIGITS], e[DIGITS];
-    digits(hi, s.top, d);
-    digits(lo, s.top, e);
-    s.d += pick(d, k) + pick(e, k);
+    const unsigned long long a = m < 0 ? -m : m;
+    const int right = (top - (DIGITS - 1) + k) * DIGIT - at;
+    const int d = (int)((unsigned)(right >= 0 ? a >> min(right, 63) : a << min(-right, 63)) & ((1u << DIGIT) - 1));
+    s.d += m < 0 ? -d : d;
   }
 }
 
